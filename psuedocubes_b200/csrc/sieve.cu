@@ -932,7 +932,23 @@ __global__ void __launch_bounds__(256) k_deep(const DeepArgs a) {
 }
 
 // ------------------------------------------------------------------------------------------
-// plain per-position matcher (pseudocube/gpu.py:147-182): warp per v row, lanes over u
+// plain per-position matcher (pseudocube/gpu.py:147-182)
+//
+// A CTA owns PLAIN_U consecutive u entries and a run of v rows.  Each thread keeps the residues
+// u*B mod q of the first four filters for its u entries in registers; a v row brings its residues
+// v*A mod q and its exact u interval (clipped to the CTA's entries) through shared memory, so a position
+// costs one subtraction and one bitmap lookup per filter (x mod q = (uB - vA) mod q).  The 1 in 81
+// positions that pass are queued per warp and finished 32 at a time in 128-bit arithmetic, filter by
+// filter.  The work is split over u chunks and v runs, so a tile of ten v rows fills the device: with a
+// warp per v row such a tile, and one of 964 rows, took 570 us, bound by the one warp that walked 17,400
+// u entries of a row; now 11 us and 57 us (the latter bound by instruction issue, 0.61 per cycle).
+
+constexpr uint32_t PLAIN_T = 256, PLAIN_PER = 4, PLAIN_U = PLAIN_T * PLAIN_PER;   // threads, u entries per thread, per CTA
+constexpr uint32_t PLAIN_V = 64;                  // v rows staged at a time
+constexpr uint32_t PLAIN_FIRST = 4;               // filters tested from residues (the first group)
+constexpr uint32_t PLAIN_QUEUE = 256;             // queued positions per warp (31 left over and 128 of one row fit)
+constexpr uint32_t PLAIN_WORDS = 256;             // bitmap words per filter (q < 8192)
+constexpr uint64_t PLAIN_RUN_MAX = UINT64_C(1) << 21;   // v rows per CTA (a queue entry holds the row in 22 bits)
 
 struct PlainArgs {
     const uint64_t *us;
@@ -945,49 +961,137 @@ struct PlainArgs {
     uint64_t *counts;
     uint64_t *out;
     uint64_t out_cap;
+    uint64_t run;                                 // v rows per CTA
+    uint32_t aq[PLAIN_FIRST], bq[PLAIN_FIRST];    // A mod q, B mod q of the first filters
 };
 
-__global__ void __launch_bounds__(256) k_plain(const PlainArgs a) {
+__global__ void __launch_bounds__(PLAIN_T) k_plain(const PlainArgs a) {
     __shared__ unsigned long long cnt[PC_MAX_RES / 4 + 4];
-    for (uint32_t k = threadIdx.x; k < a.ng + 3; k += blockDim.x) cnt[k] = 0;
-    __syncthreads();
-    const uint32_t lane = threadIdx.x & 31;
-    const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
-    unsigned long long c0 = 0;
-    for (uint64_t j = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; j < a.nv; j += warps) {
-        const u128 shift = mul_wide(a.vs[j], a.A), upper = add128(shift, a.hi);
-        const uint64_t left = count_le(a.us, a.nu, a.B, add128(shift, a.lo));
-        for (uint64_t i = left + lane; i < a.nu; i += 32) {
-            const u128 pos = mul_wide(a.us[i], a.B);
-            if (less128(upper, pos)) break;
-            if (less128(pos, shift)) {
-                atomicAdd(&cnt[a.ng + 2], 1ull);
-                continue;
+    __shared__ uint32_t bits_s[PLAIN_FIRST][PLAIN_WORDS];
+    __shared__ uint4 row_s[PLAIN_V];              // interval start | end << 16, residues of filters 0-1 and 2-3
+    __shared__ uint32_t queue_s[PLAIN_T / 32][PLAIN_QUEUE];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lanes_below = (1u << lane) - 1u;
+    const uint32_t nf = min(a.nres, PLAIN_FIRST);
+    const uint64_t c0 = blockIdx.x * (uint64_t)PLAIN_U;
+    const uint32_t n_here = (uint32_t)umin64(a.nu - c0, PLAIN_U);
+    const uint64_t j0 = blockIdx.y * a.run, j1 = umin64(a.nv, j0 + a.run);
+    const uint64_t *us = a.us + c0;
+    for (uint32_t k = threadIdx.x; k < a.ng + 3; k += PLAIN_T) cnt[k] = 0;
+    uint32_t q[PLAIN_FIRST], ru[PLAIN_PER][PLAIN_FIRST];
+    // entry (warp, k, lane) of the chunk: a warp owns 128 consecutive entries
+    const uint32_t u0 = warp * 32 * PLAIN_PER + lane;
+#pragma unroll
+    for (uint32_t f = 0; f < PLAIN_FIRST; ++f) {
+        q[f] = 1;                                 // a missing filter (nres < 4) passes residue 0
+#pragma unroll
+        for (uint32_t k = 0; k < PLAIN_PER; ++k) ru[k][f] = 0;
+        if (f < nf) {
+            const FiltConst fc = a.fc[f];
+            q[f] = fc.m.q;
+            for (uint32_t w = threadIdx.x; w < (fc.m.q + 31) / 32; w += PLAIN_T) bits_s[f][w] = a.bits[fc.tab_off + w];
+#pragma unroll
+            for (uint32_t k = 0; k < PLAIN_PER; ++k) {
+                const uint64_t u = u0 + 32 * k < n_here ? __ldg(us + u0 + 32 * k) : 0;
+                ru[k][f] = fastmod32(mod64(u, fc.m) * a.bq[f], fc.m.c, fc.m.q);
             }
-            const u128 x = sub128(pos, shift);
-            ++c0;
-            bool ok = true;
-            for (uint32_t idx = 0; idx < a.nres; ++idx) {
-                const FiltConst fc = a.fc[idx];
-                uint32_t m = mod128(x, fc.m);
-                if (!((__ldg(a.bits + fc.tab_off + (m >> 5)) >> (m & 31)) & 1u)) {
-                    ok = false;
-                    break;
-                }
-                if ((idx & 3) == 3 || idx + 1 == a.nres) atomicAdd(&cnt[idx / 4 + 1], 1ull);
-            }
-            if (!ok) continue;
-            unsigned long long slot = atomicAdd((unsigned long long *)&a.counts[a.ng + 1], 1ull);
-            if (slot < a.out_cap) {
-                a.out[2 * slot] = x.lo;
-                a.out[2 * slot + 1] = x.hi;
-            }
+        } else if (threadIdx.x == 0) {
+            bits_s[f][0] = 1;
         }
     }
-    atomicAdd(&cnt[0], c0);
+    uint32_t passed = 0, qhead = 0, qtail = 0;    // group-1 positions of the lane; warp-uniform queue positions
+
+    // Up to 32 queued positions, one per lane: the remaining filters on x = uB - vA in two limbs.
+    auto drain = [&](uint32_t n) {
+        __syncwarp();
+        const bool mine = lane < n;
+        const uint32_t ent = mine ? queue_s[warp][(qhead + lane) & (PLAIN_QUEUE - 1)] : 0u;
+        __syncwarp();
+        qhead += n;
+        if (!mine) return;
+        const u128 x = sub128(mul_wide(__ldg(us + (ent & (PLAIN_U - 1))), a.B), mul_wide(__ldg(a.vs + j0 + ent / PLAIN_U), a.A));
+        for (uint32_t idx = nf; idx < a.nres; ++idx) {
+            const FiltConst fc = a.fc[idx];
+            const uint32_t m = mod128(x, fc.m);
+            if (!((__ldg(a.bits + fc.tab_off + (m >> 5)) >> (m & 31)) & 1u)) return;
+            if ((idx & 3) == 3 || idx + 1 == a.nres) atomicAdd(&cnt[idx / 4 + 1], 1ull);
+        }
+        const unsigned long long slot = atomicAdd((unsigned long long *)&a.counts[a.ng + 1], 1ull);
+        if (slot < a.out_cap) {
+            a.out[2 * slot] = x.lo;
+            a.out[2 * slot + 1] = x.hi;
+        }
+    };
+
+    for (uint64_t base = j0; base < j1; base += PLAIN_V) {
+        const uint32_t rows = (uint32_t)umin64(PLAIN_V, j1 - base);
+        __syncthreads();                          // every warp has read the previous rows
+        if (threadIdx.x < PLAIN_V) {              // the row's interval inside the chunk
+            uint32_t left = 0, right = 0;
+            if (threadIdx.x < rows) {
+                const u128 shift = mul_wide(a.vs[base + threadIdx.x], a.A), above = add128(shift, a.lo);
+                left = (uint32_t)count_le(us, n_here, a.B, above);
+                right = max(left, (uint32_t)count_le(us, n_here, a.B, add128(shift, a.hi)));
+                if (less128(above, shift)) {      // vA + lo wrapped: positions below vA are flagged, not tested
+                    uint32_t first = left;
+                    while (first < right && less128(mul_wide(__ldg(us + first), a.B), shift)) ++first;
+                    if (first > left) atomicAdd(&cnt[a.ng + 2], (unsigned long long)(first - left));
+                    left = first;
+                }
+                if (right > left) atomicAdd(&cnt[0], (unsigned long long)(right - left));
+            }
+            row_s[threadIdx.x].x = left | right << 16;
+        }
+        {                                         // its residues: one (row, filter) pair per thread
+            const uint32_t r = threadIdx.x / PLAIN_FIRST, f = threadIdx.x % PLAIN_FIRST;
+            uint32_t m = 0;
+            if (r < rows && f < nf) {
+                const FiltConst fc = a.fc[f];
+                m = fastmod32(mod64(a.vs[base + r], fc.m) * a.aq[f], fc.m.c, fc.m.q);
+            }
+            ((uint16_t *)&row_s[r])[2 + f] = (uint16_t)m;
+        }
+        __syncthreads();
+        for (uint32_t r = 0; r < rows; ++r) {
+            const uint4 row = row_s[r];
+            const uint32_t left = row.x & 0xffffu, right = row.x >> 16, w0 = warp * 32 * PLAIN_PER;
+            if (right <= w0 || left >= w0 + 32 * PLAIN_PER || left == right) continue;    // warp-uniform
+            const uint32_t rv[PLAIN_FIRST] = {row.y & 0xffffu, row.y >> 16, row.z & 0xffffu, row.z >> 16};
+#pragma unroll
+            for (uint32_t k = 0; k < PLAIN_PER; ++k) {
+                const uint32_t ul = u0 + 32 * k;
+                uint32_t ok = ul >= left && ul < right;
+#pragma unroll
+                for (uint32_t f = 0; f < PLAIN_FIRST; ++f) {
+                    const uint32_t d = ru[k][f] - rv[f], m = __viaddmin_u32(d, q[f], d);   // (ru - rv) mod q
+                    ok &= bits_s[f][m >> 5] >> (m & 31);
+                }
+                const uint32_t won = __ballot_sync(0xffffffffu, ok);
+                if (won) {
+                    passed += ok;
+                    if (ok)
+                        queue_s[warp][(qtail + __popc(won & lanes_below)) & (PLAIN_QUEUE - 1)] =
+                            ul | (uint32_t)(base - j0 + r) * PLAIN_U;
+                    qtail += __popc(won);
+                }
+            }
+            while (qtail - qhead >= 32) drain(32);
+        }
+    }
+    if (qtail != qhead) drain(qtail - qhead);
+    passed = __reduce_add_sync(0xffffffffu, passed);
+    if (lane == 0 && passed) atomicAdd(&cnt[1], (unsigned long long)passed);
     __syncthreads();
-    for (uint32_t k = threadIdx.x; k < a.ng + 3; k += blockDim.x)
+    for (uint32_t k = threadIdx.x; k < a.ng + 3; k += PLAIN_T)
         if (k != a.ng + 1 && cnt[k]) atomicAdd((unsigned long long *)&a.counts[k], cnt[k]);
+}
+
+// Grid of a plain launch: every u chunk, times as many v runs as one wave of four CTAs per SM (64 registers)
+// holds.  More, shorter runs only repeat the staging of rows and leave fuller last waves.
+dim3 plain_grid(PlainArgs &a, int sm_count) {
+    const uint64_t chunks = (a.nu + PLAIN_U - 1) / PLAIN_U, want = (uint64_t)sm_count * 4;
+    const uint64_t runs = std::max(std::min(a.nv, std::max<uint64_t>(1, want / chunks)), (a.nv + PLAIN_RUN_MAX - 1) / PLAIN_RUN_MAX);
+    a.run = (a.nv + runs - 1) / runs;
+    return dim3((unsigned)chunks, (unsigned)((a.nv + a.run - 1) / a.run));
 }
 
 template <int NB, int K, int NT>
@@ -1682,8 +1786,12 @@ extern "C" int pc_run_plain(pc_ctx *ctx, const pc_filters *f, const pc_buf *us, 
         a.counts = d_counts;
         a.out = d_out;
         a.out_cap = out_cap;
-        uint64_t blocks = std::min<uint64_t>((nv + 7) / 8, (uint64_t)ctx->sm_count * 8);
-        k_plain<<<(unsigned)blocks, 256, 0, st>>>(a);
+        for (uint32_t k = 0; k < std::min(f->nres, PLAIN_FIRST); ++k) {
+            a.aq[k] = (uint32_t)(f->A % f->primes[k]);
+            a.bq[k] = (uint32_t)(f->B % f->primes[k]);
+        }
+        const dim3 grid = plain_grid(a, ctx->sm_count);
+        k_plain<<<grid, PLAIN_T, 0, st>>>(a);
         PC_LAUNCHED(ctx, "plain match");
     }
     PC_CHECK(ctx, cudaEventRecord(ctx->ev[7], st));
@@ -2174,8 +2282,12 @@ static int plain_static_on(int device, const uint64_t *us, uint64_t nu, const ui
         a.counts = (uint64_t *)(base + o_counts);
         a.out = (uint64_t *)(base + o_out);
         a.out_cap = out_cap;
-        uint64_t blocks = std::min<uint64_t>((nv + 7) / 8, (uint64_t)std::max(sm, 1) * 8);
-        k_plain<<<(unsigned)blocks, 256, 0, st>>>(a);
+        for (uint32_t k = 0; k < std::min(nres, PLAIN_FIRST); ++k) {
+            a.aq[k] = (uint32_t)(A % primes[k]);
+            a.bq[k] = (uint32_t)(B % primes[k]);
+        }
+        const dim3 grid = plain_grid(a, std::max(sm, 1));
+        k_plain<<<grid, PLAIN_T, 0, st>>>(a);
         e = cudaGetLastError();
         if (e != cudaSuccess) return static_cuda(err, err_len, e, "plain match launch");
     }
