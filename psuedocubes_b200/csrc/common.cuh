@@ -230,23 +230,25 @@ uint64_t pc_scan_workspace(uint64_t n);
 int pc_exclusive_scan_ws(pc_ctx *ctx, const uint64_t *in, uint64_t *out, uint64_t n, uint64_t *total_dev,
                          uint64_t *ws);
 
-// Many sorted focus windows generated together: one count launch, one scan and one emit launch.
-// Window i is written at base[i] of the shared output; each base is rounded up to a multiple of
-// the window's padding (so a u list can start on a block boundary of the matcher).
+// Many sorted focus windows generated together by one launch.  winbatch_run writes them one after another
+// into a buffer it sizes; winbatch_plan counts them first and gives window i a place that starts on a
+// multiple of pad[i] (so a u list can start on a block boundary of the matcher), for winbatch_emit.
 struct WinBatch {
-    uint32_t n = 0;
+    uint32_t n = 0, rounds = 1;
     uint64_t units = 0;
     void *d_desc = nullptr, *d_foci = nullptr;
-    uint64_t *d_cnt = nullptr, *d_off = nullptr, *d_ws = nullptr, *d_tot = nullptr, *d_base = nullptr;
-    uint32_t *d_bits = nullptr;      // the count pass's unit words for the emit pass (null: recompute)
-    std::vector<uint64_t> total, base;
+    uint64_t *d_scan = nullptr;      // ticket, tile states, window starts and total, stuck flag
+    uint64_t *d_stuck = nullptr;     // set by an emitting pass that gave up (in d_scan, or where the owner reads it)
+    uint64_t *d_delta = nullptr;     // per window: output position minus values before it (null: 0)
+    std::vector<uint64_t> total, base, delta;
+    std::vector<char> has;           // windows with any unit
+    std::vector<unsigned char> staged;   // descriptors as uploaded (kept until the copy has run)
     uint64_t out_len = 0;
 };
 struct pc_focus;
 uint64_t pc_focus_modulus(const pc_focus *f);
 int winbatch_plan(pc_ctx *ctx, Scratch &hold, const pc_focus *const *focus, const uint64_t *low, const uint64_t *high,
-                  const uint64_t *pad, uint32_t n, uint64_t cap, WinBatch &wb, int *launches);
-int winbatch_count(pc_ctx *ctx, const WinBatch &wb);
-int winbatch_emit(pc_ctx *ctx, const WinBatch &wb, uint64_t *out);
-int pc_window_into(pc_ctx *ctx, const pc_focus *f, uint64_t low, uint64_t high, uint64_t cap, uint64_t **out,
-                   uint64_t *out_bytes, uint64_t *total_host, int *launches);
+                  const uint64_t *pad, uint32_t n, uint64_t cap, WinBatch &wb);
+int winbatch_emit(pc_ctx *ctx, const WinBatch &wb, uint64_t *out, uint64_t out_cap);
+int winbatch_run(pc_ctx *ctx, Scratch &hold, const pc_focus *const *focus, const uint64_t *low, const uint64_t *high,
+                 uint32_t n, uint64_t cap, WinBatch &wb, uint64_t **out, uint64_t *out_bytes, int *launches);

@@ -1355,7 +1355,9 @@ struct Engine {
     uint32_t *d_tile_seg = nullptr, *d_blk_seg = nullptr, *d_deep_count = nullptr;
     unsigned long long *d_item_next = nullptr;
     uint64_t *d_counts = nullptr, *d_geo = nullptr, *d_out = nullptr;
-    unsigned long long *d_nout = nullptr;                 // [0] outputs, [1] rows outside the geometry
+    unsigned long long *d_nout = nullptr;                 // [0] outputs, [1] rows outside the geometry, [2] window pass gave up
+    bool windows = false;                                 // the lists come from an emitting pass that reports in d_nout[2]
+    uint64_t nout_bytes() const { return windows ? 24 : 16; }
     VRec *d_rec = nullptr;
     uint64_t *d_cres = nullptr;
     uint4 *d_bv = nullptr;
@@ -1400,7 +1402,7 @@ int engine_prepare(Engine &E, const pc_tuning *tuning, Scratch &hold) {
     if (!rc) rc = hold.get(&E.d_counts, std::max<uint64_t>(1, E.ntiles * E.stride));
     if (!rc) rc = hold.get(&E.d_geo, std::max<uint64_t>(1, 2 * E.ntiles));
     if (!rc) rc = hold.get(&E.d_out, 2 * std::max<uint64_t>(1, E.out_cap));
-    if (!rc) rc = hold.get(&E.d_nout, 2);
+    if (!rc) rc = hold.get(&E.d_nout, 3);
     if (!rc) rc = hold.get(&E.d_rec, std::max<uint64_t>(1, E.nv));
     if (!rc) rc = hold.get(&E.d_cres, std::max<uint64_t>(1, E.nv));
     if (!rc) rc = hold.get(&E.d_bv, nb1);
@@ -1563,7 +1565,8 @@ int engine_eager(Engine &E, int *launches) {
 
 // Results of a finished run already copied to the host: output count, rows outside the subtile
 // geometry, and the underflow counters of every subtile.
-int engine_check(Engine &E, const unsigned long long nout[2], const uint64_t *counts) {
+int engine_check(Engine &E, const unsigned long long nout[3], const uint64_t *counts) {
+    if (E.windows && nout[2]) return pc_fail(E.ctx, PC_ARITHMETIC, "window pass did not finish");
     if (nout[1]) return pc_fail(E.ctx, PC_INVALID, "v row outside the subtile geometry");
     if (nout[0] > E.out_cap) return pc_fail(E.ctx, PC_OVERFLOW, "output overflow; attempt cannot commit");
     for (uint64_t t = 0; t < E.ntiles; ++t) {
@@ -1576,8 +1579,8 @@ int engine_check(Engine &E, const unsigned long long nout[2], const uint64_t *co
 int engine_collect(Engine &E, uint64_t *counts, uint64_t *geometry, uint64_t *out, uint64_t *n_out) {
     pc_ctx *ctx = E.ctx;
     cudaStream_t st = ctx->stream;
-    unsigned long long nout[2] = {0, 0};
-    PC_CHECK(ctx, pc_copy(ctx, nout, E.d_nout, 16, cudaMemcpyDeviceToHost));
+    unsigned long long nout[3] = {0, 0, 0};
+    PC_CHECK(ctx, pc_copy(ctx, nout, E.d_nout, E.nout_bytes(), cudaMemcpyDeviceToHost));
     if (E.ntiles) {
         PC_CHECK(ctx, pc_copy(ctx, counts, E.d_counts, E.ntiles * E.stride * 8, cudaMemcpyDeviceToHost));
         PC_CHECK(ctx, pc_copy(ctx, geometry, E.d_geo, 2 * E.ntiles * 8, cudaMemcpyDeviceToHost));
@@ -1700,12 +1703,12 @@ extern "C" int pc_run_lease(pc_ctx *ctx, const pc_focus *fa, const pc_focus *fb,
     const pc_focus *foc[2] = {fa, fb};
     const uint64_t lows[2] = {(uint64_t)ulo, first}, highs[2] = {(uint64_t)uhi, end};
     WinBatch wb;
-    int rc = winbatch_plan(ctx, hold, foc, lows, highs, nullptr, 2, (UINT64_C(1) << 32) - 1, wb, &launches);
-    uint64_t *d_lists = nullptr;
-    if (!rc) rc = hold.get(&d_lists, std::max<uint64_t>(1, wb.out_len));
-    if (!rc) rc = winbatch_emit(ctx, wb, d_lists);
+    uint64_t *d_lists = nullptr, list_bytes = 0;
+    int rc = winbatch_run(ctx, hold, foc, lows, highs, 2, UINT64_C(1) << 33, wb, &d_lists, &list_bytes, &launches);
+    if (d_lists) hold.items.emplace_back(d_lists, list_bytes);
     if (rc) return rc;
-    ++launches;
+    for (uint64_t n : wb.total)
+        if (n > (UINT64_C(1) << 32) - 1) return pc_fail(ctx, PC_OVERFLOW, "focus buffer overflow; tile invalid");
     PC_CHECK(ctx, cudaEventRecord(ctx->ev[5], ctx->stream));
     Engine E;
     E.ctx = ctx;
@@ -1898,7 +1901,7 @@ extern "C" int pc_multi_create(pc_ctx *ctx, const pc_focus *const *foci, uint32_
     m->nwin = nwin;
     m->tile_base = tile_base;
     int rc = winbatch_plan(ctx, m->hold, focs.data(), lows.data(), highs.data(), pads.data(), 2 * nwin,
-                           (UINT64_C(1) << 32) - 1, m->wb, nullptr);
+                           (UINT64_C(1) << 32) - 1, m->wb);
     if (!rc) rc = m->hold.get(&m->d_lists, std::max<uint64_t>(1, m->wb.out_len));
     if (rc) {
         delete m;
@@ -1938,7 +1941,11 @@ extern "C" int pc_multi_create(pc_ctx *ctx, const pc_focus *const *foci, uint32_
         m->sizes[2 * i] = g.nu;
         m->sizes[2 * i + 1] = g.nv;
     }
+    E.windows = true;
     rc = engine_prepare(E, tuning, m->hold);
+    // zeroed once: a pass that gave up makes this and every later result of the object an error
+    if (!rc) rc = pc_cuda_status(ctx, cudaMemsetAsync(E.d_nout + 2, 0, 8, ctx->stream), "window flag");
+    m->wb.d_stuck = (uint64_t *)(E.d_nout + 2);
     if (!rc) rc = pc_cuda_status(ctx, cudaStreamSynchronize(ctx->stream), "window batch set-up");
     if (rc) {
         delete m;
@@ -1954,10 +1961,7 @@ int multi_eager(pc_ctx *ctx, pc_multi *m, pc_stats *stats) {
     Engine &E = m->E;
     int launches = 0;
     PC_CHECK(ctx, cudaEventRecord(ctx->ev[4], ctx->stream));
-    // pc_multi_create ran the count pass and its scan to size the lists; the unit counts, offsets
-    // and kept words it left depend only on the windows, so the eager run goes straight to the emit
-    // pass (a graph replay still runs both passes)
-    int rc = winbatch_emit(ctx, m->wb, m->d_lists);
+    int rc = winbatch_emit(ctx, m->wb, m->d_lists, m->wb.out_len);
     if (rc) return rc;
     launches += 1;
     PC_CHECK(ctx, cudaEventRecord(ctx->ev[5], ctx->stream));
@@ -1984,18 +1988,18 @@ int multi_capture(pc_ctx *ctx, pc_multi *m) {
     if (!m->h_counts) {
         PC_CHECK(ctx, cudaMallocHost((void **)&m->h_counts, nc * 8));
         PC_CHECK(ctx, cudaMallocHost((void **)&m->h_geo, ng * 8));
-        PC_CHECK(ctx, cudaMallocHost((void **)&m->h_nout, 16));
+        PC_CHECK(ctx, cudaMallocHost((void **)&m->h_nout, E.nout_bytes()));
         PC_CHECK(ctx, cudaMallocHost((void **)&m->h_deep, (uint64_t)E.grid * 4));
     }
     int rc = engine_match(E, 2);
     if (rc) return rc;
     PC_CHECK(ctx, cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     int launches = 0;
-    rc = winbatch_count(ctx, m->wb);
-    if (!rc) rc = winbatch_emit(ctx, m->wb, m->d_lists);
+    rc = winbatch_emit(ctx, m->wb, m->d_lists, m->wb.out_len);
     if (!rc) rc = engine_front(E, false, true, &launches);
     if (!rc) rc = engine_back(E, false, &launches);
-    if (!rc) rc = pc_cuda_status(ctx, pc_copy(ctx, m->h_nout, E.d_nout, 16, cudaMemcpyDeviceToHost), "capture copy");
+    if (!rc) rc = pc_cuda_status(ctx, pc_copy(ctx, m->h_nout, E.d_nout, E.nout_bytes(), cudaMemcpyDeviceToHost),
+                                    "capture copy");
     if (!rc && E.ntiles) {
         rc = pc_cuda_status(ctx, pc_copy(ctx, m->h_counts, E.d_counts, E.ntiles * E.stride * 8, cudaMemcpyDeviceToHost),
                             "capture copy");
@@ -2016,9 +2020,9 @@ int multi_capture(pc_ctx *ctx, pc_multi *m) {
     }
     m->graph = g;
     PC_CHECK(ctx, cudaGraphInstantiate(&m->exec, g, 0));
-    m->launches = launches + 5;
+    m->launches = launches + 1;
     // the copies recorded into the graph run at every replay, not at capture
-    m->graph_d2h = 16 + (E.ntiles ? E.ntiles * E.stride * 8 + 2 * E.ntiles * 8 : 0) + (uint64_t)E.grid * 4;
+    m->graph_d2h = E.nout_bytes() + (E.ntiles ? E.ntiles * E.stride * 8 + 2 * E.ntiles * 8 : 0) + (uint64_t)E.grid * 4;
     ctx->d2h -= m->graph_d2h;
     return PC_OK;
 }
@@ -2037,7 +2041,7 @@ int multi_replay(pc_ctx *ctx, pc_multi *m, pc_stats *stats) {
         if (m->h_deep[b] > E.deep_cap) return pc_fail(ctx, PC_ARITHMETIC, "deep survivor count changed between runs");
     m->counts.assign(m->h_counts, m->h_counts + E.ntiles * E.stride);
     m->geometry.assign(m->h_geo, m->h_geo + 2 * E.ntiles);
-    const unsigned long long nout[2] = {m->h_nout[0], m->h_nout[1]};
+    const unsigned long long nout[3] = {m->h_nout[0], m->h_nout[1], m->h_nout[2]};
     m->n_out = nout[0];
     rc = engine_check(E, nout, m->counts.data());
     if (!rc && nout[0]) {

@@ -9,35 +9,42 @@
 // (s + w) mod q in R_q; the window for period K is the AND of the rows s = K*M1 mod q.
 //
 // A window [low, high) is therefore walked in (period, wheel index) order, which is ascending
-// value order: a count pass, an exclusive scan and an emit pass produce the sorted values with
-// no sort and no residue set materialised.  Tables are p-independent for p above the largest
-// focus prime.
+// value order: one pass that finds its output positions as it goes (a decoupled look-back over the
+// tiles before it) produces the sorted values with no sort and no residue set materialised.  Tables
+// are p-independent for p above the largest focus prime.
 #include "common.cuh"
 #include <algorithm>
 #include <chrono>
+#include <cmath>
+#include <cstring>
 #include <numeric>
 
 struct pc_focus {
     uint64_t M = 0, M1 = 1, count1 = 0, words1 = 0;
+    uint64_t stride = 0;         // words from one row to the next: words1 rounded up to 16 bytes
     uint32_t nT = 0;
     uint32_t tq[PC_MAX_WHEEL_T] = {};
     uint32_t t_m1mod[PC_MAX_WHEEL_T] = {};
     uint32_t t_row0[PC_MAX_WHEEL_T] = {};
     uint32_t total_rows = 0;
     uint64_t *W1 = nullptr;      // device, sorted wheel
-    uint32_t *rows = nullptr;    // device, total_rows x words1
+    uint32_t *rows = nullptr;    // device, total_rows x stride
     uint64_t W1_bytes = 0, rows_bytes = 0;
     std::vector<uint64_t> W1_host;
     uint64_t count_lo = 0, count_hi = 0;
     double build_ms = 0;
+    double density = 0;          // focus values per coordinate
 };
 
 namespace {
 
 constexpr int WT = 256;          // threads per CTA of the window kernels
 constexpr int SIEVE_WORDS = 64;  // sieve words per thread
-constexpr int WIN_WORDS = 32;    // wheel words per window unit
-constexpr uint64_t WIN_WORDS_BUDGET = UINT64_C(512) << 20;   // kept count-pass words, bytes
+constexpr int WIN_WORDS = 128;   // wheel words per window unit: four per lane, one 16-byte load per row
+constexpr int WIN_WARPS = WT / 32;
+constexpr uint32_t WIN_ROUNDS = 8;    // most units per warp
+constexpr uint32_t WIN_STAGE = 512;   // values of one warp staged in shared memory (a denser warp writes unit by unit)
+constexpr uint32_t WIN_SPINS = 1u << 22;                      // polls of one look-back wait before it gives up
 
 // Periodic bit patterns of the S rings, replicated so any 32-bit window at offset < q is one
 // funnel shift of two consecutive words.
@@ -85,12 +92,12 @@ __global__ void k_sieve(const SieveRings rings, const uint32_t *__restrict__ pat
 
 // rows[row0 + s][w] bit l = R[(s + W1[32w + l] mod q) mod q], via the rotation of the pattern
 // RR (R repeated) by m = W1 mod q and a warp transpose.
-__global__ void k_wheel_rows(const uint64_t *__restrict__ W1, uint64_t count1, uint64_t words1,
+__global__ void k_wheel_rows(const uint64_t *__restrict__ W1, uint64_t count1,
                              const uint32_t *__restrict__ pattern, uint32_t q, ModQ mq,
-                             uint32_t *__restrict__ rows) {
+                             uint32_t *__restrict__ rows, uint64_t stride) {
     const uint32_t lane = threadIdx.x & 31;
     uint64_t w = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-    if (w >= words1) return;
+    if (w >= stride) return;                            // the words that pad a row are zero
     uint64_t j = w * 32 + lane;
     bool valid = j < count1;
     uint32_t m = valid ? mod64(W1[j], mq) : 0;
@@ -100,7 +107,7 @@ __global__ void k_wheel_rows(const uint64_t *__restrict__ W1, uint64_t count1, u
         col = valid ? col : 0u;
         uint32_t row = transpose32(col, lane);
         uint32_t s = 32 * k + lane;
-        if (s < q) rows[(uint64_t)s * words1 + w] = row;
+        if (s < q) rows[(uint64_t)s * stride + w] = row;
     }
 }
 
@@ -108,19 +115,25 @@ struct WindowPlan {
     uint64_t K0, K1, j_lo, j_hi;
     uint64_t wa0, wb0, wa1, wb1;       // word ranges of the first and last period
     uint64_t units_first, units_mid, units_last, units;
+    uint64_t chunks;                   // 32-word chunks, the measure of the refusal of too long windows
 };
 
 // Device view of one focus: the sorted wheel and the bitset rows of its T rings.
 struct FocusDev {
     const uint64_t *W1;
     const uint32_t *rows;
-    uint64_t M1, count1, words1;
+    uint64_t M1, count1, words1, stride;
     uint32_t nT, pad;
     uint32_t tq[PC_MAX_WHEEL_T];
     uint32_t t_m1mod[PC_MAX_WHEEL_T];
     uint32_t t_row0[PC_MAX_WHEEL_T];
     ModQ tmq[PC_MAX_WHEEL_T];
 };
+
+// Bits [a, e) of one 32-bit word.
+__device__ __forceinline__ uint32_t span_bits(int32_t a, int32_t e) {
+    return low_bits((uint32_t)min(max(e, 0), 32)) & ~low_bits((uint32_t)min(max(a, 0), 32));
+}
 
 // One window of a batch: its plan, its first unit in the batch-wide unit numbering and its focus.
 struct WinDesc {
@@ -153,110 +166,270 @@ __device__ __forceinline__ void unit_of(const WindowPlan &p, uint64_t words1, ui
     wb = min(p.wb1, wa + WIN_WORDS);
 }
 
-constexpr int WIN_UNITS_PER_WARP = 16;
+// Device buffers of one emitting pass.
+struct WinOut {
+    unsigned long long *ticket;        // next tile; the words after it are the tile states, all zeroed before the launch
+    unsigned long long *state;         // per tile: values << 2 | 1 (its own) or 2 (its own and all before it)
+    uint64_t *starts;                  // per window: values of the windows before it; the last entry, the total
+    const uint64_t *delta;             // per window: added to its output positions (modulo 2^64), or null
+    uint64_t *out;
+    uint64_t cap;                      // entries of out
+    uint64_t *stuck;                   // set when a look-back wait ran out
+    uint64_t ntiles;
+};
 
-// One warp per WIN_UNITS_PER_WARP consecutive window units of WIN_WORDS = 32 wheel words each, one
-// word per lane, so every row load of the warp is one coalesced 128-byte request.  The warp finds
-// the window of its first unit by a binary search over the windows' first units and steps to the
-// next window when its units cross into it.  The row addresses of a period are computed once and
-// reused while its units stay in that period (a period spans hundreds of units), and the rows of a
-// unit are loaded together before they are combined.  Count pass: per-unit totals, and (words
-// not null) each unit's 32 words kept for the emit pass, which then reads them instead of the
-// rows.  Emit pass: the lane's exclusive prefix inside the warp, plus the unit's offset inside
-// its window, plus the window's base gives ascending output slots.  Both passes wait on L2 (row
-// words, wheel entries), so the kernel is held to 32 registers for 64 resident warps per SM; the
-// few spills sit on the once-per-period row-address path.
-__global__ void __launch_bounds__(WT, 8) k_windows(const WinDesc *__restrict__ desc, uint32_t ndesc, const FocusDev *__restrict__ foci,
-                          uint64_t units, uint64_t *__restrict__ counts, const uint64_t *__restrict__ offsets,
-                          const uint64_t *__restrict__ bases, uint64_t *__restrict__ out, uint32_t *__restrict__ words) {
-    const uint32_t lane = threadIdx.x & 31;
-    const uint64_t u0 = ((blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5) * WIN_UNITS_PER_WARP;
-    if (u0 >= units) return;                            // warp-uniform
-    const uint64_t u1 = umin64(units, u0 + WIN_UNITS_PER_WARP);
-    uint32_t lo = 0, hi = ndesc;                        // last window with unit_base <= u0
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) / 2;
-        if (desc[mid].unit_base <= u0) lo = mid;
-        else hi = mid;
+// Values of the tiles before `tile`, by warp 0: it publishes the tile's own sum, then adds the states of
+// the 32 tiles before it, and of the 32 before those, until one already holds its whole prefix.  Tiles take
+// ascending tickets, so every tile waited for is running or done; a wait that does not end in WIN_SPINS
+// polls sets *stuck and goes on, and the host refuses the result.
+__device__ __forceinline__ uint64_t look_back(const WinOut &o, uint64_t tile, uint64_t own, uint32_t lane) {
+    volatile unsigned long long *state = o.state;
+    if (tile == 0) {
+        if (lane == 0) state[0] = own << 2 | 2;
+        return 0;
     }
-    uint64_t next_base = lo + 1 < ndesc ? desc[lo + 1].unit_base : UINT64_MAX;
-    // The rows of period K, kept while consecutive units stay in the same period and window.
-    const uint32_t *row[PC_MAX_WHEEL_T];
-    uint64_t row_K = UINT64_MAX;
-    uint32_t row_win = UINT32_MAX;
-    for (uint64_t gu = u0; gu < u1; ++gu) {
-        while (gu >= next_base) {                       // the units crossed into the next window
-            ++lo;
-            next_base = lo + 1 < ndesc ? desc[lo + 1].unit_base : UINT64_MAX;
-        }
-        const WindowPlan &p = desc[lo].plan;
-        const uint64_t ubase = desc[lo].unit_base;
-        const FocusDev &f = foci[desc[lo].focus];
-        uint64_t K, wa, wb;
-        unit_of(p, f.words1, gu - ubase, K, wa, wb);
-        const uint64_t w = wa + lane;
-        uint32_t bits = 0;
-        if (offsets && words) {                         // emit pass: the count pass kept the words
-            bits = words[gu * 32 + lane];
-        } else {
-            if (K != row_K || lo != row_win) {             // warp-uniform
-                row_K = K;
-                row_win = lo;
-#pragma unroll
-                for (uint32_t t = 0; t < PC_MAX_WHEEL_T; ++t) {
-                    row[t] = f.rows;                        // rows past nT: a valid address, never read
-                    if (t < f.nT) {
-                        const uint32_t s = fastmod32(mod64(K, f.tmq[t]) * f.t_m1mod[t], f.tmq[t].c, f.tq[t]);   // < q^2 < 2^32
-                        row[t] += (uint64_t)(f.t_row0[t] + s) * f.words1;
-                    }
-                }
+    if (lane == 0) state[tile] = own << 2 | 1;
+    uint64_t before = 0;
+    for (int64_t at = (int64_t)tile - 1 - lane;; at -= 32) {
+        unsigned long long s = at < 0 ? 2 : state[at];
+        for (uint32_t spin = 0; __any_sync(0xffffffffu, (s & 3) == 0); ++spin) {
+            if (spin == WIN_SPINS) {
+                if (lane == 0) *o.stuck = 1;
+                s |= 2;
+            } else if ((s & 3) == 0) {
+                s = state[at];
             }
-            if (w < wb) {
-                bits = 0xffffffffu;
-                if (f.nT) {                                 // all row loads in flight before the first use
-                    uint32_t r[PC_MAX_WHEEL_T];
+        }
+        const uint32_t whole = __ballot_sync(0xffffffffu, (s & 3) == 2);
+        const uint32_t last = whole ? __ffs(whole) - 1 : 31;
+        uint64_t v = lane <= last ? s >> 2 : 0;
 #pragma unroll
-                    for (uint32_t t = 0; t < PC_MAX_WHEEL_T; ++t) r[t] = t < f.nT ? __ldg(row[t] + w) : 0xffffffffu;
-#pragma unroll
-                    for (uint32_t t = 0; t < PC_MAX_WHEEL_T; ++t) bits &= r[t];
-                }
-                const uint64_t jmin = K == p.K0 ? p.j_lo : 0;
-                const uint64_t jmax = K == p.K1 ? p.j_hi : f.count1;
-                const uint64_t j0 = w * 32;
-                if (j0 < jmin) bits &= ~low_bits((uint32_t)(jmin - j0 < 32 ? jmin - j0 : 32));
-                if (j0 + 32 > jmax) bits &= jmax > j0 ? low_bits((uint32_t)(jmax - j0)) : 0u;
-            }
-            if (words) words[gu * 32 + lane] = bits;
-        }
-        const uint32_t n = __popc(bits);
-        if (!offsets) {
-            const uint32_t total = __reduce_add_sync(0xffffffffu, n);
-            if (lane == 0) counts[gu] = total;
-            continue;
-        }
-        uint32_t incl = n;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, d);
-            if (lane >= (uint32_t)d) incl += y;
-        }
-        uint64_t pos = bases[lo] + (offsets[gu] - offsets[ubase]) + incl - n;
-        const uint64_t base = K * f.M1, j0 = w * 32;
-        while (bits) {
-            const uint32_t b = __ffs(bits) - 1;
-            bits &= bits - 1;
-            out[pos++] = base + __ldg(f.W1 + j0 + b);
-        }
+        for (int d = 16; d; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+        before += v;
+        if (whole) break;
     }
+    if (lane == 0) state[tile] = (before + own) << 2 | 2;
+    return before;
 }
 
-// Per window: its value count (offsets hold units + 1 entries, the total last).
-__global__ void k_window_totals(const WinDesc *__restrict__ desc, uint32_t ndesc, const uint64_t *__restrict__ offsets,
-                                uint64_t *__restrict__ totals) {
-    const uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
-    if (w >= ndesc) return;
-    const uint64_t b = desc[w].unit_base;
-    totals[w] = offsets[b + desc[w].plan.units] - offsets[b];
+// Walks a warp's consecutive units.  The first is found by a binary search over the windows' first units
+// and a division; each next one is 128 words on, in the next period or in the next window.  The rows of a
+// period are located by one lane per T ring when the period changes.
+struct UnitWalk {
+    const WinDesc *desc;
+    const FocusDev *foci, *f;
+    uint32_t lane, win, nT;
+    uint32_t row[PC_MAX_WHEEL_T];                       // the period's rows, in 16-byte steps from the table's start
+    uint64_t K, K0, K1, wa, wb;                         // the unit's period and first word, the period's word end
+
+    __device__ __forceinline__ UnitWalk(const WinDesc *d, uint32_t ndesc, const FocusDev *fs, uint64_t u0, uint32_t l)
+        : desc(d), foci(fs), lane(l), win(0) {
+        uint32_t hi = ndesc;                            // last window with unit_base <= u0
+        while (hi - win > 1) {
+            const uint32_t mid = (win + hi) / 2;
+            if (desc[mid].unit_base <= u0) win = mid;
+            else hi = mid;
+        }
+        open();
+        unit_of(desc[win].plan, f->words1, u0 - desc[win].unit_base, K, wa, wb);
+        wb = K == K0 ? desc[win].plan.wb0 : K == K1 ? desc[win].plan.wb1 : f->words1;
+        locate();
+    }
+
+    __device__ __forceinline__ void open() {            // the first period of window `win`
+        const WindowPlan &p = desc[win].plan;
+        f = foci + desc[win].focus;
+        nT = f->nT;
+        K0 = K = p.K0, K1 = p.K1, wa = p.wa0, wb = p.wb0;
+    }
+
+    __device__ __forceinline__ void locate() {
+        uint32_t mine = 0;
+        if (lane < nT) {
+            const ModQ &m = f->tmq[lane];
+            const uint32_t s = fastmod32(mod64(K, m) * f->t_m1mod[lane], m.c, m.q);   // < q^2 < 2^32
+            mine = (uint32_t)((uint64_t)(f->t_row0[lane] + s) * (f->stride / 4));
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < PC_MAX_WHEEL_T; ++k) row[k] = __shfl_sync(0xffffffffu, mine, k);
+    }
+
+    __device__ __forceinline__ void step() {            // only while another unit follows
+        wa += WIN_WORDS;
+        if (wa < wb) return;
+        while (wa >= wb) {
+            if (K < K1) {
+                ++K;
+                wa = 0;
+                wb = K == K1 ? desc[win].plan.wb1 : f->words1;
+            } else {
+                ++win;
+                open();
+            }
+        }
+        locate();
+    }
+
+    // The lane's four words of the unit; w: the first of them.
+    __device__ __forceinline__ uint4 words(uint32_t &w) const {
+        w = (uint32_t)wa + 4 * lane;
+        const uint4 ones = make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu);
+        uint4 t[PC_MAX_WHEEL_T];
+        const bool in = w < wb;
+        const uint4 *rows = (const uint4 *)f->rows + (w >> 2);
+#pragma unroll
+        for (uint32_t k = 0; k < PC_MAX_WHEEL_T; ++k) { // all row loads in flight before the first use
+            t[k] = ones;
+            if (k < nT && in) t[k] = __ldg(rows + row[k]);
+        }
+        uint4 b = in ? ones : make_uint4(0, 0, 0, 0);
+#pragma unroll
+        for (uint32_t k = 0; k < PC_MAX_WHEEL_T; ++k)
+            if (k < nT) b.x &= t[k].x, b.y &= t[k].y, b.z &= t[k].z, b.w &= t[k].w;
+        if (K == K0 || K == K1 || !nT) {                // entries of [jmin, jmax) only (rows end in zero bits)
+            const WindowPlan &p = desc[win].plan;
+            const uint64_t j = (uint64_t)w * 32, jmin = K == K0 ? p.j_lo : 0, jmax = K == K1 ? p.j_hi : f->count1;
+            const int32_t a = j < jmin ? (int32_t)umin64(jmin - j, 128) : 0;
+            const int32_t e = j < jmax ? (int32_t)umin64(jmax - j, 128) : 0;
+            b.x &= span_bits(a, e), b.y &= span_bits(a - 32, e - 32);
+            b.z &= span_bits(a - 64, e - 64), b.w &= span_bits(a - 96, e - 96);
+        }
+        return b;
+    }
+};
+
+__device__ __forceinline__ uint32_t popc128(uint4 b) { return __popc(b.x) + __popc(b.y) + __popc(b.z) + __popc(b.w); }
+
+// The windows' values, in order.  A unit is 128 wheel words: a lane takes four, so each row of the
+// period is one 16-byte load per lane and 512 coalesced bytes per warp, and the unit's address
+// arithmetic, warp scan and window lookup are paid once for 4,096 wheel entries.  A warp takes `rounds`
+// consecutive units.  Without EMIT only the windows' totals are counted.  With EMIT the warp stages
+// its values in shared memory (the wheel indices first, so that the wheel loads are one value per
+// lane) while warp 0 finds the tile's output position by look-back, and then stores them
+// coalesced.  A warp whose units hold more than WIN_STAGE values (a focus without T rings keeps every wheel
+// entry) writes them word by word after the look-back instead, one bit per lane.
+//
+// Bound: L2 (per lease 1.07 GB of row words, one 32-byte sector of W1 for each of 26M values, 0.2 GB of
+// stores) and the look-back's latency.  The two windows of a lease take 0.46 ms; a count pass, a scan and an
+// emit pass with one wheel word per lane took 1.15 ms, and 512 uneven windows 0.86 ms (now 0.35 ms).
+template <bool EMIT>
+__global__ void __launch_bounds__(WT, 4) k_windows(const WinDesc *__restrict__ desc, uint32_t ndesc,
+                                                const FocusDev *__restrict__ foci, uint64_t units, uint32_t rounds,
+                                                unsigned long long *__restrict__ totals, const WinOut o) {
+    __shared__ uint64_t tile_s, before_s;
+    __shared__ uint32_t sum_s[WIN_WARPS];
+    __shared__ uint64_t value_s[EMIT ? WIN_WARPS : 1][EMIT ? WIN_STAGE : 1];
+    __shared__ uint16_t index_s[EMIT ? WIN_WARPS : 1][EMIT ? WIN_STAGE : 1];   // round << 12 | entry of the unit
+    __shared__ struct {
+        uint64_t kbase, delta;                          // K * M1; output position minus values before the window
+        const uint64_t *wheel;                          // the unit's first entry
+        uint32_t before, win;                           // values of the warp's earlier units
+    } unit_s[EMIT ? WIN_WARPS : 1][EMIT ? WIN_ROUNDS : 1];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint64_t tile = blockIdx.x;
+    if (EMIT) {
+        if (threadIdx.x == 0) tile_s = atomicAdd(o.ticket, 1ull);
+        __syncthreads();
+        tile = tile_s;
+    }
+    const uint64_t u0 = (tile * WIN_WARPS + warp) * rounds;
+    const uint32_t mine = u0 < units ? (uint32_t)umin64(units - u0, rounds) : 0;      // warp-uniform
+    uint32_t own = 0;                                   // EMIT: values of the warp; else of the lane
+    if (mine) {
+        UnitWalk walk(desc, ndesc, foci, u0, lane);
+        uint32_t counted = walk.win;
+        for (uint32_t r = 0; r < mine; ++r) {
+            if (r) walk.step();
+            if (!EMIT && walk.win != counted) {
+                const uint32_t sum = __reduce_add_sync(0xffffffffu, own);
+                if (lane == 0 && sum) atomicAdd(totals + counted, (unsigned long long)sum);
+                own = 0;
+                counted = walk.win;
+            }
+            uint32_t w;
+            const uint4 b = walk.words(w);
+            const uint32_t n = popc128(b);
+            if (!EMIT) {
+                own += n;
+                continue;
+            }
+            if (lane == 0) {
+                auto &u = unit_s[warp][r];
+                u.kbase = walk.K * walk.f->M1;
+                u.delta = o.delta ? o.delta[walk.win] : 0;
+                u.wheel = walk.f->W1 + (uint64_t)w * 32;
+                u.before = own;
+                u.win = walk.win;
+            }
+            uint32_t incl = n;
+#pragma unroll
+            for (int s = 1; s < 32; s <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, incl, s);
+                if (lane >= (uint32_t)s) incl += y;
+            }
+            const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+            if (own + total <= WIN_STAGE) {
+                uint16_t *at = index_s[warp] + own + incl - n;
+                const uint32_t e = r << 12 | lane * 128;
+                for (uint64_t x = (uint64_t)b.y << 32 | b.x; x; x &= x - 1) *at++ = (uint16_t)(e + __ffsll(x) - 1);
+                for (uint64_t x = (uint64_t)b.w << 32 | b.z; x; x &= x - 1) *at++ = (uint16_t)(e + 64 + __ffsll(x) - 1);
+            }
+            own += total;
+        }
+        if (!EMIT) {
+            const uint32_t sum = __reduce_add_sync(0xffffffffu, own);
+            if (lane == 0 && sum) atomicAdd(totals + counted, (unsigned long long)sum);
+        }
+    }
+    if (!EMIT) return;
+    if (lane == 0) sum_s[warp] = own;
+    __syncthreads();
+    if (warp == 0) {
+        const uint32_t all = __reduce_add_sync(0xffffffffu, lane < WIN_WARPS ? sum_s[lane] : 0u);
+        const uint64_t before = look_back(o, tile, all, lane);
+        if (lane == 0) {
+            before_s = before;
+            if (tile + 1 == o.ntiles) o.starts[ndesc] = before + all;
+        }
+    }
+    const bool staged = own <= WIN_STAGE;
+    if (staged)
+        for (uint32_t i = lane; i < own; i += 32) {     // the wheel loads overlap the look-back
+            const uint32_t e = index_s[warp][i];
+            const auto &u = unit_s[warp][e >> 12];
+            value_s[warp][i] = u.kbase + __ldg(u.wheel + (e & 0xfffu));
+        }
+    __syncthreads();
+    uint64_t at = before_s;                             // values before the warp's
+    for (uint32_t k = 0; k < warp; ++k) at += sum_s[k];
+    if (lane < mine) {
+        const auto &u = unit_s[warp][lane];
+        if (u0 + lane == desc[u.win].unit_base) o.starts[u.win] = at + u.before;
+    }
+    if (staged) {
+        for (uint32_t i = lane; i < own; i += 32) {
+            const uint64_t pos = at + i + unit_s[warp][index_s[warp][i] >> 12].delta;
+            if (pos < o.cap) o.out[pos] = value_s[warp][i];
+        }
+    } else if (mine) {
+        UnitWalk walk(desc, ndesc, foci, u0, lane);
+        for (uint32_t r = 0; r < mine; ++r) {
+            if (r) walk.step();
+            uint32_t w;
+            const uint4 b = walk.words(w);
+            const auto &u = unit_s[warp][r];
+            uint64_t pos = at + u.before + u.delta;
+            for (uint32_t k = 0; k < 128; ++k) {        // word k of the unit: lane k / 4, component k % 4
+                const uint32_t own_word = (k & 2) ? (k & 1) ? b.w : b.z : (k & 1) ? b.y : b.x;
+                const uint32_t word = __shfl_sync(0xffffffffu, own_word, k >> 2);
+                if (word >> lane & 1) {
+                    const uint64_t slot = pos + __popc(word & ((1u << lane) - 1));
+                    if (slot < o.cap) o.out[slot] = u.kbase + __ldg(u.wheel + k * 32 + lane);
+                }
+                pos += __popc(word);
+            }
+        }
+    }
 }
 
 // 128-bit product of 64-bit counts, host side.
@@ -306,6 +479,8 @@ extern "C" int pc_focus_create(pc_ctx *ctx, uint64_t M, uint32_t nrings, const u
     f->M = M;
     f->count_lo = 1;
     for (auto &r : rings) mul_acc(f->count_lo, f->count_hi, r.n);
+    f->density = 1;
+    for (auto &r : rings) f->density *= (double)r.n / r.q;
     // Choose the T rings: the fewest largest rings whose removal makes the sieve over M1 and
     // the tables fit; among the feasible, the smallest table budget use wins ties.
     uint32_t chosen = UINT32_MAX;
@@ -396,6 +571,7 @@ extern "C" int pc_focus_create(pc_ctx *ctx, uint64_t M, uint32_t nrings, const u
     }
     f->count1 = total;
     f->words1 = (total + 31) / 32;
+    f->stride = (f->words1 + 3) & ~UINT64_C(3);
     f->W1_bytes = std::max<uint64_t>(16, total * 8);
     rc = pc_alloc(ctx, (void **)&f->W1, f->W1_bytes);
     if (rc) {
@@ -413,7 +589,7 @@ extern "C" int pc_focus_create(pc_ctx *ctx, uint64_t M, uint32_t nrings, const u
         f->t_row0[t] = f->total_rows;
         f->total_rows += f->tq[t];
     }
-    f->rows_bytes = std::max<uint64_t>(16, (uint64_t)f->total_rows * f->words1 * 4);
+    f->rows_bytes = std::max<uint64_t>(16, (uint64_t)f->total_rows * f->stride * 4);
     rc = pc_alloc(ctx, (void **)&f->rows, f->rows_bytes);
     if (rc) {
         pc_release(ctx, f->W1, f->W1_bytes);
@@ -432,9 +608,9 @@ extern "C" int pc_focus_create(pc_ctx *ctx, uint64_t M, uint32_t nrings, const u
         rc = s.get(&d_rp, words.size());
         if (rc) break;
         pc_copy(ctx, d_rp, words.data(), words.size() * 4, cudaMemcpyHostToDevice);
-        uint64_t threads = f->words1 * 32;
+        uint64_t threads = f->stride * 32;
         k_wheel_rows<<<(unsigned)((threads + WT - 1) / WT), WT, 0, ctx->stream>>>(
-            f->W1, f->count1, f->words1, d_rp, r.q, make_modq(r.q), f->rows + (uint64_t)f->t_row0[t] * f->words1);
+            f->W1, f->count1, d_rp, r.q, make_modq(r.q), f->rows + (uint64_t)f->t_row0[t] * f->stride, f->stride);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) {
             rc = pc_cuda_fail(ctx, e, "wheel rows");
@@ -503,12 +679,17 @@ int plan_window(pc_ctx *ctx, const pc_focus *f, uint64_t low, uint64_t high, Win
         p.wa1 = 0;
         p.wb1 = (p.j_hi + 31) / 32;
     }
-    p.units_first = (p.wb0 - p.wa0 + WIN_WORDS - 1) / WIN_WORDS;
-    p.units_mid = (f->words1 + WIN_WORDS - 1) / WIN_WORDS;
-    p.units_last = p.K1 > p.K0 ? (p.wb1 - p.wa1 + WIN_WORDS - 1) / WIN_WORDS : 0;
-    uint64_t mid_periods = p.K1 > p.K0 + 1 ? p.K1 - p.K0 - 1 : 0;
-    p.units = p.units_first + mid_periods * p.units_mid + p.units_last;
-    if (p.units >= (UINT64_C(1) << 31)) return pc_fail(ctx, PC_OVERFLOW, "focus window too long");
+    const uint64_t mid_periods = p.K1 > p.K0 + 1 ? p.K1 - p.K0 - 1 : 0;
+    auto units = [&](uint64_t words) {
+        p.units_first = (p.wb0 - p.wa0 + words - 1) / words;
+        p.units_mid = (f->words1 + words - 1) / words;
+        p.units_last = p.K1 > p.K0 ? (p.wb1 - p.wa1 + words - 1) / words : 0;
+        return p.units_first + mid_periods * p.units_mid + p.units_last;
+    };
+    p.chunks = units(32);
+    if (p.chunks >= (UINT64_C(1) << 31)) return pc_fail(ctx, PC_OVERFLOW, "focus window too long");
+    p.wa0 &= ~UINT64_C(3);             // a unit starts on a 16-byte boundary of the rows
+    p.units = units(WIN_WORDS);
     return PC_OK;
 }
 
@@ -519,6 +700,7 @@ FocusDev focus_dev(const pc_focus *f) {
     d.M1 = f->M1;
     d.count1 = f->count1;
     d.words1 = f->words1;
+    d.stride = f->stride;
     d.nT = f->nT;
     for (uint32_t t = 0; t < f->nT; ++t) {
         d.tq[t] = f->tq[t];
@@ -531,138 +713,194 @@ FocusDev focus_dev(const pc_focus *f) {
 
 }  // namespace
 
-int winbatch_count(pc_ctx *ctx, const WinBatch &wb) {
-    if (wb.units) {
-        const uint64_t warps = (wb.units + WIN_UNITS_PER_WARP - 1) / WIN_UNITS_PER_WARP;
-        const unsigned grid = (unsigned)((warps * 32 + WT - 1) / WT);
-        k_windows<<<grid, WT, 0, ctx->stream>>>((const WinDesc *)wb.d_desc, wb.n, (const FocusDev *)wb.d_foci, wb.units,
-                                                wb.d_cnt, nullptr, nullptr, nullptr, wb.d_bits);
-        PC_LAUNCHED(ctx, "window count");
-    }
-    return pc_exclusive_scan_ws(ctx, wb.d_cnt, wb.d_off, wb.units, wb.d_off + wb.units, wb.d_ws);
+namespace {
+
+// Units per warp: enough tiles for four CTAs per SM, then as many units as keep a warp's values well inside
+// its stage (per_unit: expected values of the densest focus's unit), so that there are few tiles to look
+// back over and a window's lookup and a period's rows serve several units.
+uint32_t win_rounds(const pc_ctx *ctx, uint64_t units, double per_unit) {
+    const double most = std::min<double>(WIN_ROUNDS, 0.75 * WIN_STAGE / std::max(per_unit, 1.0));
+    return (uint32_t)std::max(1.0, std::min(most, (double)(units / ((uint64_t)ctx->sm_count * 4 * WIN_WARPS))));
 }
 
-int winbatch_emit(pc_ctx *ctx, const WinBatch &wb, uint64_t *out) {
-    if (!wb.out_len) return PC_OK;
-    PC_CHECK(ctx, cudaMemsetAsync(out, 0, wb.out_len * 8, ctx->stream));   // padding slots read as 0
-    if (wb.units) {
-        const uint64_t warps = (wb.units + WIN_UNITS_PER_WARP - 1) / WIN_UNITS_PER_WARP;
-        const unsigned grid = (unsigned)((warps * 32 + WT - 1) / WT);
-        k_windows<<<grid, WT, 0, ctx->stream>>>((const WinDesc *)wb.d_desc, wb.n, (const FocusDev *)wb.d_foci, wb.units,
-                                                nullptr, wb.d_off, wb.d_base, out, wb.d_bits);
-        PC_LAUNCHED(ctx, "window emit");
-    }
-    return PC_OK;
+uint64_t win_tiles(const WinBatch &wb) {
+    const uint64_t per = (uint64_t)WIN_WARPS * wb.rounds;
+    return (wb.units + per - 1) / per;
 }
 
-int winbatch_plan(pc_ctx *ctx, Scratch &hold, const pc_focus *const *focus, const uint64_t *low, const uint64_t *high,
-                  const uint64_t *pad, uint32_t n, uint64_t cap, WinBatch &wb, int *launches) {
+// Plans of n windows, their descriptors and the foci on the device.
+int winbatch_describe(pc_ctx *ctx, Scratch &hold, const pc_focus *const *focus, const uint64_t *low, const uint64_t *high,
+                      uint32_t n, WinBatch &wb) {
     wb = WinBatch{};
     wb.n = n;
-    if (!n) return PC_OK;
     std::vector<WinDesc> desc(n);
     std::vector<FocusDev> foci;
     std::vector<const pc_focus *> seen;
+    uint64_t chunks = 0;
+    double per_unit = 0;
+    wb.has.resize(n);
     for (uint32_t i = 0; i < n; ++i) {
         int rc = plan_window(ctx, focus[i], low[i], high[i], desc[i].plan);
         if (rc) return rc;
         desc[i].unit_base = wb.units;
+        wb.has[i] = desc[i].plan.units != 0;
         wb.units += desc[i].plan.units;
+        chunks += desc[i].plan.chunks;
         uint32_t k = 0;
         while (k < seen.size() && seen[k] != focus[i]) ++k;
         if (k == seen.size()) {
             seen.push_back(focus[i]);
             foci.push_back(focus_dev(focus[i]));
+            per_unit = std::max(per_unit, focus[i]->density * (double)focus[i]->M1 / (double)focus[i]->count1 * 32 * WIN_WORDS);
         }
         desc[i].focus = k;
     }
-    if (wb.units >= (UINT64_C(1) << 34)) return pc_fail(ctx, PC_OVERFLOW, "focus windows too long");
-    WinDesc *d_desc;
-    FocusDev *d_foci;
-    int rc = hold.get(&d_desc, n);
-    if (!rc) rc = hold.get(&d_foci, foci.size());
-    if (!rc) rc = hold.get(&wb.d_cnt, std::max<uint64_t>(1, wb.units));
-    if (!rc) rc = hold.get(&wb.d_off, wb.units + 1);
-    if (!rc) rc = hold.get(&wb.d_ws, pc_scan_workspace(wb.units));
-    if (!rc) rc = hold.get(&wb.d_tot, n);
-    if (!rc) rc = hold.get(&wb.d_base, n);
-    // keep the count pass's unit words for the emit pass when they fit WIN_WORDS_BUDGET bytes
-    if (!rc && wb.units * WIN_WORDS * 4 <= WIN_WORDS_BUDGET && ctx->in_use + wb.units * WIN_WORDS * 4 <= ctx->cap / 2)
-        rc = hold.get(&wb.d_bits, wb.units * WIN_WORDS);
+    if (chunks >= (UINT64_C(1) << 34)) return pc_fail(ctx, PC_OVERFLOW, "focus windows too long");
+    wb.rounds = win_rounds(ctx, wb.units, per_unit);
+    // one upload: the descriptors, then the foci
+    const uint64_t at = (n * sizeof(WinDesc) + 15) & ~UINT64_C(15), bytes = at + foci.size() * sizeof(FocusDev);
+    wb.staged.resize(bytes);
+    memcpy(wb.staged.data(), desc.data(), n * sizeof(WinDesc));
+    memcpy(wb.staged.data() + at, foci.data(), foci.size() * sizeof(FocusDev));
+    unsigned char *d = nullptr;
+    int rc = hold.get(&d, bytes);
+    // ticket, tile states, starts (one per window and the total), the stuck flag
+    if (!rc) rc = hold.get(&wb.d_scan, 1 + win_tiles(wb) + n + 2);
     if (rc) return rc;
-    wb.d_desc = d_desc;
-    wb.d_foci = d_foci;
-    PC_CHECK(ctx, pc_copy(ctx, d_desc, desc.data(), n * sizeof(WinDesc), cudaMemcpyHostToDevice));
-    PC_CHECK(ctx, pc_copy(ctx, d_foci, foci.data(), foci.size() * sizeof(FocusDev), cudaMemcpyHostToDevice));
-    rc = winbatch_count(ctx, wb);
-    if (rc) return rc;
-    k_window_totals<<<(n + 255) / 256, 256, 0, ctx->stream>>>(d_desc, n, wb.d_off, wb.d_tot);
-    PC_LAUNCHED(ctx, "window totals");
-    wb.total.assign(n, 0);
-    PC_CHECK(ctx, pc_copy(ctx, wb.total.data(), wb.d_tot, n * 8, cudaMemcpyDeviceToHost));
-    PC_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
-    wb.base.assign(n, 0);
-    for (uint32_t i = 0; i < n; ++i) {
-        if (wb.total[i] > cap) return pc_fail(ctx, PC_OVERFLOW, "focus buffer overflow; tile invalid");
-        const uint64_t pd = pad && pad[i] ? pad[i] : 1;
-        wb.base[i] = (wb.out_len + pd - 1) / pd * pd;
-        wb.out_len = wb.base[i] + wb.total[i];
-    }
-    PC_CHECK(ctx, pc_copy(ctx, wb.d_base, wb.base.data(), n * 8, cudaMemcpyHostToDevice));
-    PC_CHECK(ctx, cudaStreamSynchronize(ctx->stream));   // the host vectors above go out of scope
-    if (launches) *launches += 4;
+    wb.d_desc = d;
+    wb.d_foci = d + at;
+    wb.d_stuck = wb.d_scan + 1 + win_tiles(wb) + n + 1;
+    PC_CHECK(ctx, pc_copy(ctx, d, wb.staged.data(), bytes, cudaMemcpyHostToDevice));
     return PC_OK;
 }
 
-// Plan and run one window; out is allocated by the call (out_bytes returned for release).
-// total_host receives the count.
-int pc_window_into(pc_ctx *ctx, const pc_focus *f, uint64_t low, uint64_t high, uint64_t cap,
-                   uint64_t **out, uint64_t *out_bytes, uint64_t *total_host, int *launches) {
+}  // namespace
+
+// Emits every window's values (out_cap entries of out).  Nothing is allocated and nothing waits for the
+// device, so the pass can be recorded into a CUDA graph.
+int winbatch_emit(pc_ctx *ctx, const WinBatch &wb, uint64_t *out, uint64_t out_cap) {
+    if (!wb.units) return PC_OK;
+    const uint64_t tiles = win_tiles(wb);
+    PC_CHECK(ctx, cudaMemsetAsync(wb.d_scan, 0, (1 + tiles + wb.n + 2) * 8, ctx->stream));
+    WinOut o{};
+    o.ticket = (unsigned long long *)wb.d_scan;
+    o.state = o.ticket + 1;
+    o.starts = wb.d_scan + 1 + tiles;
+    o.stuck = wb.d_stuck;
+    o.delta = wb.d_delta;
+    o.out = out;
+    o.cap = out_cap;
+    o.ntiles = tiles;
+    k_windows<true><<<(unsigned)tiles, WT, 0, ctx->stream>>>((const WinDesc *)wb.d_desc, wb.n, (const FocusDev *)wb.d_foci,
+                                                             wb.units, wb.rounds, nullptr, o);
+    PC_LAUNCHED(ctx, "windows");
+    return PC_OK;
+}
+
+// Windows one after another (unpadded) into one buffer allocated here: sized from the foci's densities
+// and filled in one pass; a pass whose values outgrow it reruns once with room for all.  A total above
+// `cap` is an overflow, and no more than `cap` entries are allocated.
+int winbatch_run(pc_ctx *ctx, Scratch &hold, const pc_focus *const *focus, const uint64_t *low, const uint64_t *high,
+                 uint32_t n, uint64_t cap, WinBatch &wb, uint64_t **out, uint64_t *out_bytes, int *launches) {
     *out = nullptr;
     *out_bytes = 0;
-    *total_host = 0;
-    if (high < low) return pc_fail(ctx, PC_INVALID, "invalid bounded focus window");
-    if (high == low) return PC_OK;
-    Scratch s(ctx);
-    WinBatch wb;
-    int rc = winbatch_plan(ctx, s, &f, &low, &high, nullptr, 1, UINT64_MAX, wb, launches);
+    int rc = winbatch_describe(ctx, hold, focus, low, high, n, wb);
     if (rc) return rc;
-    *total_host = wb.total[0];
-    if (wb.total[0] > cap) return pc_fail(ctx, PC_OVERFLOW, "focus buffer overflow; tile invalid");
-    if (!wb.out_len) return PC_OK;
-    const uint64_t bytes = std::max<uint64_t>(16, wb.out_len * 8);
-    rc = pc_alloc(ctx, (void **)out, bytes);
+    wb.total.assign(n, 0);
+    wb.base.assign(n, 0);
+    double expect = 0;
+    uint64_t most = 0;
+    for (uint32_t i = 0; i < n; ++i) {
+        expect += (double)(high[i] - low[i]) * focus[i]->density;
+        most += high[i] - low[i];
+    }
+    uint64_t room = (uint64_t)(expect * 1.01 + 8 * std::sqrt(expect)) + 1024;
+    room = std::min(std::min(room, most), cap);
+    std::vector<uint64_t> got(n + 2);
+    for (int attempt = 0;; ++attempt) {
+        *out_bytes = std::max<uint64_t>(16, room * 8);
+        rc = pc_alloc(ctx, (void **)out, *out_bytes);
+        if (rc) return rc;
+        if (!wb.units) return PC_OK;
+        rc = winbatch_emit(ctx, wb, *out, room);
+        if (launches) ++*launches;
+        if (!rc)
+            rc = pc_cuda_status(ctx, pc_copy(ctx, got.data(), wb.d_scan + 1 + win_tiles(wb), (n + 2) * 8, cudaMemcpyDeviceToHost),
+                                "window totals");
+        if (!rc) rc = pc_cuda_status(ctx, cudaStreamSynchronize(ctx->stream), "window totals");
+        if (!rc && got[n + 1]) rc = pc_fail(ctx, PC_ARITHMETIC, "window pass did not finish");
+        const uint64_t total = got[n];
+        if (!rc && (total <= room || total > cap)) {
+            uint64_t next = total;
+            for (uint32_t i = n; i-- > 0;) {           // a window without units starts where the next one does
+                wb.base[i] = wb.has[i] ? got[i] : next;
+                wb.total[i] = next - wb.base[i];
+                next = wb.base[i];
+            }
+            wb.out_len = total;
+            return PC_OK;
+        }
+        if (!rc && attempt) rc = pc_fail(ctx, PC_ARITHMETIC, "window size changed between attempts");
+        pc_release(ctx, *out, *out_bytes);
+        *out = nullptr;
+        if (rc) return rc;
+        room = total;
+    }
+}
+
+// The windows' sizes by a counting pass, and their places in a shared output: window i starts on a
+// multiple of pad[i].  The emitting passes follow with winbatch_emit.
+int winbatch_plan(pc_ctx *ctx, Scratch &hold, const pc_focus *const *focus, const uint64_t *low, const uint64_t *high,
+                  const uint64_t *pad, uint32_t n, uint64_t cap, WinBatch &wb) {
+    int rc = winbatch_describe(ctx, hold, focus, low, high, n, wb);
+    uint64_t *d_total = nullptr;
+    if (!rc) rc = hold.get(&d_total, n);
+    if (!rc) rc = hold.get(&wb.d_delta, n);
     if (rc) return rc;
-    *out_bytes = bytes;
-    rc = winbatch_emit(ctx, wb, *out);
-    if (launches) *launches += 1;
-    return rc;
+    wb.total.assign(n, 0);
+    wb.base.assign(n, 0);
+    if (wb.units) {
+        PC_CHECK(ctx, cudaMemsetAsync(d_total, 0, n * 8, ctx->stream));
+        k_windows<false><<<(unsigned)win_tiles(wb), WT, 0, ctx->stream>>>((const WinDesc *)wb.d_desc, n,
+                                                                          (const FocusDev *)wb.d_foci, wb.units, wb.rounds,
+                                                                          (unsigned long long *)d_total, WinOut{});
+        PC_LAUNCHED(ctx, "window count");
+        PC_CHECK(ctx, pc_copy(ctx, wb.total.data(), d_total, n * 8, cudaMemcpyDeviceToHost));
+        PC_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
+    }
+    wb.delta.assign(n, 0);
+    uint64_t before = 0;
+    for (uint32_t i = 0; i < n; ++i) {
+        if (wb.total[i] > cap) return pc_fail(ctx, PC_OVERFLOW, "focus buffer overflow; tile invalid");
+        const uint64_t pd = pad[i] ? pad[i] : 1;
+        wb.base[i] = (wb.out_len + pd - 1) / pd * pd;
+        wb.out_len = wb.base[i] + wb.total[i];
+        wb.delta[i] = wb.base[i] - before;
+        before += wb.total[i];
+    }
+    PC_CHECK(ctx, pc_copy(ctx, wb.d_delta, wb.delta.data(), n * 8, cudaMemcpyHostToDevice));
+    return PC_OK;
 }
 
 extern "C" int pc_focus_window(pc_ctx *ctx, const pc_focus *f, uint64_t low, uint64_t high, uint64_t cap,
                                pc_buf **out, uint64_t *count) {
     *out = nullptr;
     *count = 0;
-    uint64_t *d = nullptr, bytes = 0, total = 0;
-    int rc = pc_window_into(ctx, f, low, high, cap, &d, &bytes, &total, nullptr);
-    *count = total;
+    if (high < low) return pc_fail(ctx, PC_INVALID, "invalid bounded focus window");
+    Scratch hold(ctx);
+    WinBatch wb;
+    uint64_t *d = nullptr, bytes = 0;
+    int rc = winbatch_run(ctx, hold, &f, &low, &high, 1, cap, wb, &d, &bytes, nullptr);
+    if (!rc) *count = wb.out_len;
+    if (!rc && wb.out_len > cap) rc = pc_fail(ctx, PC_OVERFLOW, "focus buffer overflow; tile invalid");
     if (rc) {
         pc_release(ctx, d, bytes);
         return rc;
     }
     pc_buf *b = new pc_buf();
     b->d = d;
-    b->n = total;
+    b->n = wb.out_len;
     b->bytes = bytes;
-    if (!d) {
-        rc = pc_alloc(ctx, (void **)&b->d, 16);
-        if (rc) {
-            delete b;
-            return rc;
-        }
-        b->bytes = 16;
-    }
-    PC_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
     *out = b;
     return PC_OK;
 }
