@@ -181,23 +181,8 @@ __device__ __forceinline__ uint32_t low_bits(uint32_t n) {
 
 // ------------------------------------------------------------------------------------------
 // 32x32 bit-matrix transpose across a warp: lane l holds row l (bit i = column i) on entry and
-// column l on exit.  Five exchange rounds of the off-diagonal blocks.
-__device__ __forceinline__ uint32_t transpose32(uint32_t x, uint32_t lane) {
-#pragma unroll
-    for (int j = 16; j >= 1; j >>= 1) {
-        const uint32_t hm = j == 16 ? 0xffff0000u : j == 8 ? 0xff00ff00u : j == 4 ? 0xf0f0f0f0u
-                          : j == 2 ? 0xccccccccu : 0xaaaaaaaau;
-        uint32_t p = __shfl_xor_sync(0xffffffffu, x, j);
-        bool upper = lane & j;
-        uint32_t keep = upper ? hm : ~hm;
-        uint32_t moved = upper ? (p >> j) : (p << j);
-        x = (x & keep) | (moved & ~keep);
-    }
-    return x;
-}
-
-// The same transpose with its per-lane constants computed once: in exchange round r (block size
-// j = 16 >> r) a lane rotates its partner's word by sh[r] (left by j for the lower lane of a pair,
+// column l on exit.  Five exchange rounds of the off-diagonal blocks, with per-lane constants
+// computed once: in exchange round r (block size j = 16 >> r) a lane rotates its partner's word by sh[r] (left by j for the lower lane of a pair,
 // right by j for the upper one) and keeps its own bits where keep[r] is set, one funnel shift and
 // one bit-select per round.
 __device__ __forceinline__ void transpose_consts(uint32_t lane, uint32_t (&sh)[5], uint32_t (&keep)[5]) {
@@ -223,9 +208,47 @@ __device__ __forceinline__ uint32_t transpose32c(uint32_t x, const uint32_t (&sh
 }
 
 // ------------------------------------------------------------------------------------------
+// Exclusive prefix over the tiles of one launch (decoupled look-back).  A tile's state is one word:
+// value << 2 | 1 (its own sum) or 2 (its own and all before it), zeroed before the launch.
+constexpr uint32_t LOOK_BACK_SPINS = 1u << 22;   // polls of one wait before it gives up
+
+// Values of the tiles before `tile`, by warp 0: it publishes the tile's own sum, then adds the states of
+// the 32 tiles before it, and of the 32 before those, until one already holds its whole prefix.  Tiles take
+// ascending tickets, so every tile waited for is running or done; a wait that does not end in LOOK_BACK_SPINS
+// polls sets *stuck and goes on, and the host refuses the result.
+__device__ __forceinline__ uint64_t look_back(volatile unsigned long long *state, uint64_t *stuck, uint64_t tile,
+                                              uint64_t own, uint32_t lane) {
+    if (tile == 0) {
+        if (lane == 0) state[0] = own << 2 | 2;
+        return 0;
+    }
+    if (lane == 0) state[tile] = own << 2 | 1;
+    uint64_t before = 0;
+    for (int64_t at = (int64_t)tile - 1 - lane;; at -= 32) {
+        unsigned long long s = at < 0 ? 2 : state[at];
+        for (uint32_t spin = 0; __any_sync(0xffffffffu, (s & 3) == 0); ++spin) {
+            if (spin == LOOK_BACK_SPINS) {
+                if (lane == 0) *stuck = 1;
+                s |= 2;
+            } else if ((s & 3) == 0) {
+                s = state[at];
+            }
+        }
+        const uint32_t whole = __ballot_sync(0xffffffffu, (s & 3) == 2);
+        const uint32_t last = whole ? __ffs(whole) - 1 : 31;
+        uint64_t v = lane <= last ? s >> 2 : 0;
+#pragma unroll
+        for (int d = 16; d; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+        before += v;
+        if (whole) break;
+    }
+    if (lane == 0) state[tile] = (before + own) << 2 | 2;
+    return before;
+}
+
+// ------------------------------------------------------------------------------------------
 // internal host helpers shared across translation units
 
-int pc_exclusive_scan_u64(pc_ctx *ctx, const uint64_t *in, uint64_t *out, uint64_t n, uint64_t *total_dev);
 uint64_t pc_scan_workspace(uint64_t n);
 int pc_exclusive_scan_ws(pc_ctx *ctx, const uint64_t *in, uint64_t *out, uint64_t n, uint64_t *total_dev,
                          uint64_t *ws);

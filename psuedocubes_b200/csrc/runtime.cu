@@ -332,14 +332,6 @@ int pc_exclusive_scan_ws(pc_ctx *ctx, const uint64_t *in, uint64_t *out, uint64_
     return PC_OK;
 }
 
-int pc_exclusive_scan_u64(pc_ctx *ctx, const uint64_t *in, uint64_t *out, uint64_t n, uint64_t *total_dev) {
-    Scratch s(ctx);
-    uint64_t *ws;
-    int rc = s.get(&ws, pc_scan_workspace(n));
-    if (rc) return rc;
-    return pc_exclusive_scan_ws(ctx, in, out, n, total_dev, ws);
-}
-
 // ------------------------------------------------------------------------------------------
 // limb self-test (kernels/pseudocube.cuh:7-11 semantics)
 

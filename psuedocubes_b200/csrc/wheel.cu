@@ -3,7 +3,7 @@
 // A focus of modulus M is the set of y >= 0 whose residue mod every ring modulus q | M lies in
 // the ring's (coefficient-adjusted) allowed set R_q.  Split the rings into S (small moduli) and
 // T (the largest few).  With M1 = prod(S), the sorted wheel W1 = {w in [0, M1): w mod q in R_q
-// for q in S} is built once by a bitset sieve over [0, M1).  Every y = K*M1 + w (w in W1)
+// for q in S} is built once, from the wheel of its smallest rings up (below).  Every y = K*M1 + w (w in W1)
 // satisfies the S rings; it is in the focus iff (K*M1 + w) mod q in R_q for the T rings.  For
 // each T ring and each s in [0, q), a bitset row over W1's index space marks the w with
 // (s + w) mod q in R_q; the window for period K is the AND of the rows s = K*M1 mod q.
@@ -17,6 +17,7 @@
 #include <chrono>
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <numeric>
 
 struct pc_focus {
@@ -30,7 +31,7 @@ struct pc_focus {
     uint64_t *W1 = nullptr;      // device, sorted wheel
     uint32_t *rows = nullptr;    // device, total_rows x stride
     uint64_t W1_bytes = 0, rows_bytes = 0;
-    std::vector<uint64_t> W1_host;
+    std::vector<uint64_t> sample; // host: every SAMPLE-th wheel entry (window ends are refined on the device)
     uint64_t count_lo = 0, count_hi = 0;
     double build_ms = 0;
     double density = 0;          // focus values per coordinate
@@ -39,80 +40,59 @@ struct pc_focus {
 namespace {
 
 constexpr int WT = 256;          // threads per CTA of the window kernels
-constexpr int SIEVE_WORDS = 64;  // sieve words per thread
+constexpr uint64_t SAMPLE = 128;      // wheel entries per host sample: the 128 entries of a lane's four words
+constexpr uint64_t BASE_STEPS = 1 << 16;   // candidates of one ring's step of the host's base wheel
 constexpr int WIN_WORDS = 128;   // wheel words per window unit: four per lane, one 16-byte load per row
 constexpr int WIN_WARPS = WT / 32;
 constexpr uint32_t WIN_ROUNDS = 8;    // most units per warp
 constexpr uint32_t WIN_STAGE = 512;   // values of one warp staged in shared memory (a denser warp writes unit by unit)
-constexpr uint32_t WIN_SPINS = 1u << 22;                      // polls of one look-back wait before it gives up
 
-// Periodic bit patterns of the S rings, replicated so any 32-bit window at offset < q is one
-// funnel shift of two consecutive words.
-struct SieveRings {
-    uint32_t n;
-    uint32_t q[16];
-    uint32_t off[16];            // word offset of each ring's pattern in the pattern array
-    uint32_t step[16];           // 32 mod q
-    ModQ mq[16];
+// Rings whose rows one launch of k_wheel_rows builds.
+struct RowRings {
+    uint32_t q[PC_MAX_WHEEL_T], off[PC_MAX_WHEEL_T], row0[PC_MAX_WHEEL_T];   // off: first word of the ring's pattern
+    ModQ mq[PC_MAX_WHEEL_T];
 };
 
-__global__ void k_sieve(const SieveRings rings, const uint32_t *__restrict__ patterns, uint64_t M1,
-                        uint64_t nwords, uint64_t *__restrict__ counts, const uint64_t *__restrict__ offsets,
-                        uint64_t *__restrict__ out) {
-    uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    uint64_t w0 = t * SIEVE_WORDS;
-    if (w0 >= nwords) return;
-    uint64_t w1 = min(nwords, w0 + SIEVE_WORDS);
-    uint32_t s[16];
-    for (uint32_t r = 0; r < rings.n; ++r) s[r] = mod64(w0 * 32, rings.mq[r]);
-    uint64_t total = 0, pos = offsets ? offsets[t] : 0;
-    for (uint64_t w = w0; w < w1; ++w) {
-        uint32_t bits = 0xffffffffu;
-        for (uint32_t r = 0; r < rings.n; ++r) {
-            const uint32_t *p = patterns + rings.off[r];
-            uint32_t lo = p[s[r] >> 5], hi = p[(s[r] >> 5) + 1];
-            bits &= __funnelshift_r(lo, hi, s[r] & 31);
-            s[r] += rings.step[r];
-            if (s[r] >= rings.q[r]) s[r] -= rings.q[r];
-        }
-        uint64_t base = w * 32;
-        if (base + 32 > M1) bits &= low_bits((uint32_t)(M1 - base));
-        if (offsets) {
-            while (bits) {
-                uint32_t b = __ffs(bits) - 1;
-                bits &= bits - 1;
-                out[pos++] = base + b;
-            }
-        } else {
-            total += __popc(bits);
-        }
+// rows[row0 + s][w] bit l = R[(s + W1[32w + l] mod q) mod q], via the rotation of the pattern
+// RR (R repeated) by m = W1 mod q and a warp transpose.  A warp builds four consecutive words of every
+// row of one ring (blockIdx.y), so a row's four words are one 16-byte store.
+__global__ void k_wheel_rows(const uint64_t *__restrict__ W1, uint64_t count1, const uint32_t *__restrict__ patterns,
+                             const RowRings rings, uint32_t *__restrict__ rows, uint64_t stride) {
+    const uint32_t lane = threadIdx.x & 31, ring = blockIdx.y, q = rings.q[ring];
+    const uint64_t w = ((blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5) * 4;
+    if (w >= stride) return;                            // the words that pad a row are zero
+    const uint32_t *pattern = patterns + rings.off[ring];
+    uint32_t m[4];
+    bool valid[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const uint64_t j = (w + k) * 32 + lane;
+        valid[k] = j < count1;
+        m[k] = valid[k] ? mod64(W1[j], rings.mq[ring]) : 0;
     }
-    if (!offsets) counts[t] = total;
+    uint32_t sh[5], keep[5];
+    transpose_consts(lane, sh, keep);
+    for (uint32_t g = 0; g * 32 < q; ++g) {
+        uint32_t v[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const uint32_t st = 32 * g + m[k];
+            const uint32_t col = __funnelshift_r(pattern[st >> 5], pattern[(st >> 5) + 1], st & 31);
+            v[k] = transpose32c(valid[k] ? col : 0u, sh, keep);
+        }
+        const uint32_t s = 32 * g + lane;
+        if (s < q) *(uint4 *)(rows + (uint64_t)(rings.row0[ring] + s) * stride + w) = make_uint4(v[0], v[1], v[2], v[3]);
+    }
 }
 
-// rows[row0 + s][w] bit l = R[(s + W1[32w + l] mod q) mod q], via the rotation of the pattern
-// RR (R repeated) by m = W1 mod q and a warp transpose.
-__global__ void k_wheel_rows(const uint64_t *__restrict__ W1, uint64_t count1,
-                             const uint32_t *__restrict__ pattern, uint32_t q, ModQ mq,
-                             uint32_t *__restrict__ rows, uint64_t stride) {
-    const uint32_t lane = threadIdx.x & 31;
-    uint64_t w = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-    if (w >= stride) return;                            // the words that pad a row are zero
-    uint64_t j = w * 32 + lane;
-    bool valid = j < count1;
-    uint32_t m = valid ? mod64(W1[j], mq) : 0;
-    for (uint32_t k = 0; k * 32 < q; ++k) {
-        uint32_t st = 32 * k + m;
-        uint32_t col = __funnelshift_r(pattern[st >> 5], pattern[(st >> 5) + 1], st & 31);
-        col = valid ? col : 0u;
-        uint32_t row = transpose32(col, lane);
-        uint32_t s = 32 * k + lane;
-        if (s < q) rows[(uint64_t)s * stride + w] = row;
-    }
+__global__ void k_sample(const uint64_t *__restrict__ W1, uint64_t n, uint64_t *__restrict__ out) {
+    const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    if (i < n) out[i] = W1[i * SAMPLE];
 }
 
 struct WindowPlan {
-    uint64_t K0, K1, j_lo, j_hi;
+    uint64_t K0, K1, j_lo, j_hi;       // wheel range: j_lo and j_hi are the ends of the 128-entry blocks
+    uint64_t rem_lo, rem_hi;           // that hold the first entry >= rem_lo and the last < rem_hi
     uint64_t wa0, wb0, wa1, wb1;       // word ranges of the first and last period
     uint64_t units_first, units_mid, units_last, units;
     uint64_t chunks;                   // 32-word chunks, the measure of the refusal of too long windows
@@ -178,40 +158,6 @@ struct WinOut {
     uint64_t ntiles;
 };
 
-// Values of the tiles before `tile`, by warp 0: it publishes the tile's own sum, then adds the states of
-// the 32 tiles before it, and of the 32 before those, until one already holds its whole prefix.  Tiles take
-// ascending tickets, so every tile waited for is running or done; a wait that does not end in WIN_SPINS
-// polls sets *stuck and goes on, and the host refuses the result.
-__device__ __forceinline__ uint64_t look_back(const WinOut &o, uint64_t tile, uint64_t own, uint32_t lane) {
-    volatile unsigned long long *state = o.state;
-    if (tile == 0) {
-        if (lane == 0) state[0] = own << 2 | 2;
-        return 0;
-    }
-    if (lane == 0) state[tile] = own << 2 | 1;
-    uint64_t before = 0;
-    for (int64_t at = (int64_t)tile - 1 - lane;; at -= 32) {
-        unsigned long long s = at < 0 ? 2 : state[at];
-        for (uint32_t spin = 0; __any_sync(0xffffffffu, (s & 3) == 0); ++spin) {
-            if (spin == WIN_SPINS) {
-                if (lane == 0) *o.stuck = 1;
-                s |= 2;
-            } else if ((s & 3) == 0) {
-                s = state[at];
-            }
-        }
-        const uint32_t whole = __ballot_sync(0xffffffffu, (s & 3) == 2);
-        const uint32_t last = whole ? __ffs(whole) - 1 : 31;
-        uint64_t v = lane <= last ? s >> 2 : 0;
-#pragma unroll
-        for (int d = 16; d; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
-        before += v;
-        if (whole) break;
-    }
-    if (lane == 0) state[tile] = (before + own) << 2 | 2;
-    return before;
-}
-
 // Walks a warp's consecutive units.  The first is found by a binary search over the windows' first units
 // and a division; each next one is 128 words on, in the next period or in the next window.  The rows of a
 // period are located by one lane per T ring when the period changes.
@@ -270,6 +216,15 @@ struct UnitWalk {
         locate();
     }
 
+    // Entries below x among the 128 wheel entries from j on (the whole warp, for one block).
+    __device__ __forceinline__ uint32_t below(uint64_t j, uint64_t x) const {
+        uint32_t n = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < SAMPLE; k += 32)
+            n += __popc(__ballot_sync(0xffffffffu, j + k + lane < f->count1 && __ldg(f->W1 + j + k + lane) < x));
+        return n;
+    }
+
     // The lane's four words of the unit; w: the first of them.
     __device__ __forceinline__ uint4 words(uint32_t &w) const {
         w = (uint32_t)wa + 4 * lane;
@@ -288,7 +243,13 @@ struct UnitWalk {
             if (k < nT) b.x &= t[k].x, b.y &= t[k].y, b.z &= t[k].z, b.w &= t[k].w;
         if (K == K0 || K == K1 || !nT) {                // entries of [jmin, jmax) only (rows end in zero bits)
             const WindowPlan &p = desc[win].plan;
-            const uint64_t j = (uint64_t)w * 32, jmin = K == K0 ? p.j_lo : 0, jmax = K == K1 ? p.j_hi : f->count1;
+            uint64_t jmin = 0, jmax = f->count1;
+            const uint64_t j = (uint64_t)w * 32, first = wa * 32;
+            if (K == K0) jmin = first <= p.j_lo && p.j_lo < first + 32 * WIN_WORDS ? p.j_lo + below(p.j_lo, p.rem_lo) : p.j_lo;
+            if (K == K1) {
+                const uint64_t block = p.j_hi ? (p.j_hi - 1) & ~(SAMPLE - 1) : 0;
+                jmax = first <= block && block < first + 32 * WIN_WORDS ? block + below(block, p.rem_hi) : p.j_hi;
+            }
             const int32_t a = j < jmin ? (int32_t)umin64(jmin - j, 128) : 0;
             const int32_t e = j < jmax ? (int32_t)umin64(jmax - j, 128) : 0;
             b.x &= span_bits(a, e), b.y &= span_bits(a - 32, e - 32);
@@ -386,7 +347,7 @@ __global__ void __launch_bounds__(WT, 4) k_windows(const WinDesc *__restrict__ d
     __syncthreads();
     if (warp == 0) {
         const uint32_t all = __reduce_add_sync(0xffffffffu, lane < WIN_WARPS ? sum_s[lane] : 0u);
-        const uint64_t before = look_back(o, tile, all, lane);
+        const uint64_t before = look_back(o.state, o.stuck, tile, all, lane);
         if (lane == 0) {
             before_s = before;
             if (tile + 1 == o.ntiles) o.starts[ndesc] = before + all;
@@ -448,6 +409,13 @@ uint64_t gcd64(uint64_t a, uint64_t b) {
     return a;
 }
 
+struct Ring {
+    uint32_t q, n;
+    std::vector<uint32_t> res;
+};
+
+int focus_tables(pc_ctx *ctx, pc_focus *f, const std::vector<Ring> &rings, uint32_t nS);
+
 }  // namespace
 
 extern "C" int pc_focus_create(pc_ctx *ctx, uint64_t M, uint32_t nrings, const uint32_t *q, const uint32_t *counts,
@@ -456,10 +424,6 @@ extern "C" int pc_focus_create(pc_ctx *ctx, uint64_t M, uint32_t nrings, const u
     if (M == 0 || M >= (UINT64_C(1) << 63) || nrings > 16) return pc_fail(ctx, PC_INVALID, "invalid focus modulus");
     auto t_start = std::chrono::steady_clock::now();
     if (!table_budget) table_budget = UINT64_C(256) << 20;
-    struct Ring {
-        uint32_t q, n;
-        std::vector<uint32_t> res;
-    };
     std::vector<Ring> rings;
     uint64_t prodq = 1, off = 0;
     for (uint32_t k = 0; k < nrings; ++k) {
@@ -506,123 +470,8 @@ extern "C" int pc_focus_create(pc_ctx *ctx, uint64_t M, uint32_t nrings, const u
         return pc_fail(ctx, PC_INVALID, "focus wheel does not fit the table budget");
     }
     f->nT = chosen;
-    uint32_t nS = nrings - chosen;
-    f->M1 = 1;
-    for (uint32_t k = 0; k < nS; ++k) f->M1 *= rings[k].q;
-
-    // --- W1: sieve over [0, M1) with the S rings
-    SieveRings sr{};
-    sr.n = nS;
-    std::vector<uint32_t> pat;
-    for (uint32_t k = 0; k < nS; ++k) {
-        const Ring &r = rings[k];
-        sr.q[k] = r.q;
-        sr.off[k] = (uint32_t)pat.size();
-        sr.step[k] = 32 % r.q;
-        sr.mq[k] = make_modq(r.q);
-        uint32_t nbits = r.q + 64;
-        std::vector<uint32_t> words((nbits + 31) / 32 + 1, 0);
-        std::vector<char> ok(r.q, 0);
-        for (uint32_t a : r.res) ok[a] = 1;
-        for (uint32_t b = 0; b < nbits; ++b)
-            if (ok[b % r.q]) words[b / 32] |= 1u << (b % 32);
-        pat.insert(pat.end(), words.begin(), words.end());
-    }
-    Scratch s(ctx);
-    uint32_t *d_pat;
-    int rc = s.get(&d_pat, pat.size() + 1);
-    if (rc) {
-        delete f;
-        return rc;
-    }
-    if (!pat.empty()) pc_copy(ctx, d_pat, pat.data(), pat.size() * 4, cudaMemcpyHostToDevice);
-    uint64_t nwords = (f->M1 + 31) / 32;
-    uint64_t nthreads = (nwords + SIEVE_WORDS - 1) / SIEVE_WORDS;
-    uint64_t *d_cnt, *d_off, *d_total;
-    rc = s.get(&d_cnt, nthreads);
-    if (!rc) rc = s.get(&d_off, nthreads);
-    if (!rc) rc = s.get(&d_total, 1);
-    if (rc) {
-        delete f;
-        return rc;
-    }
-    unsigned grid = (unsigned)((nthreads + WT - 1) / WT);
-    k_sieve<<<grid, WT, 0, ctx->stream>>>(sr, d_pat, f->M1, nwords, d_cnt, nullptr, nullptr);
-    rc = pc_exclusive_scan_u64(ctx, d_cnt, d_off, nthreads, d_total);
-    uint64_t total = 0;
-    if (!rc && pc_copy(ctx, &total, d_total, 8, cudaMemcpyDeviceToHost) == cudaSuccess &&
-        cudaStreamSynchronize(ctx->stream) == cudaSuccess) {
-    } else if (!rc) {
-        rc = pc_cuda_fail(ctx, cudaGetLastError(), "wheel count");
-    }
-    if (rc) {
-        delete f;
-        return rc;
-    }
-    uint64_t expect_lo = f->count_lo, expect_hi = f->count_hi;
-    for (uint32_t k = nS; k < nrings; ++k) {
-        unsigned __int128 c = ((unsigned __int128)expect_hi << 64 | expect_lo) / rings[k].n;
-        expect_lo = (uint64_t)c;
-        expect_hi = (uint64_t)(c >> 64);
-    }
-    if (total != expect_lo || expect_hi) {
-        delete f;
-        return pc_fail(ctx, PC_ARITHMETIC, "wheel size disagrees with the ring counts");
-    }
-    f->count1 = total;
-    f->words1 = (total + 31) / 32;
-    f->stride = (f->words1 + 3) & ~UINT64_C(3);
-    f->W1_bytes = std::max<uint64_t>(16, total * 8);
-    rc = pc_alloc(ctx, (void **)&f->W1, f->W1_bytes);
-    if (rc) {
-        delete f;
-        return rc;
-    }
-    k_sieve<<<grid, WT, 0, ctx->stream>>>(sr, d_pat, f->M1, nwords, nullptr, d_off, f->W1);
-    PC_LAUNCHED(ctx, "wheel sieve");
-
-    // --- rows of the T rings
-    f->total_rows = 0;
-    for (uint32_t t = 0; t < chosen; ++t) {
-        f->tq[t] = rings[nS + t].q;
-        f->t_m1mod[t] = (uint32_t)(f->M1 % f->tq[t]);
-        f->t_row0[t] = f->total_rows;
-        f->total_rows += f->tq[t];
-    }
-    f->rows_bytes = std::max<uint64_t>(16, (uint64_t)f->total_rows * f->stride * 4);
-    rc = pc_alloc(ctx, (void **)&f->rows, f->rows_bytes);
-    if (rc) {
-        pc_release(ctx, f->W1, f->W1_bytes);
-        delete f;
-        return rc;
-    }
-    for (uint32_t t = 0; t < chosen; ++t) {
-        const Ring &r = rings[nS + t];
-        uint32_t nbits = 2 * r.q + 64;
-        std::vector<uint32_t> words((nbits + 31) / 32 + 1, 0);
-        std::vector<char> ok(r.q, 0);
-        for (uint32_t a : r.res) ok[a] = 1;
-        for (uint32_t b = 0; b < nbits; ++b)
-            if (ok[b % r.q]) words[b / 32] |= 1u << (b % 32);
-        uint32_t *d_rp;
-        rc = s.get(&d_rp, words.size());
-        if (rc) break;
-        pc_copy(ctx, d_rp, words.data(), words.size() * 4, cudaMemcpyHostToDevice);
-        uint64_t threads = f->stride * 32;
-        k_wheel_rows<<<(unsigned)((threads + WT - 1) / WT), WT, 0, ctx->stream>>>(
-            f->W1, f->count1, d_rp, r.q, make_modq(r.q), f->rows + (uint64_t)f->t_row0[t] * f->stride, f->stride);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) {
-            rc = pc_cuda_fail(ctx, e, "wheel rows");
-            break;
-        }
-    }
-    if (!rc) {
-        f->W1_host.resize(f->count1);
-        cudaError_t e = pc_copy(ctx, f->W1_host.data(), f->W1, f->count1 * 8, cudaMemcpyDeviceToHost);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-        if (e != cudaSuccess) rc = pc_cuda_fail(ctx, e, "wheel download");
-    }
+    const uint32_t nS = nrings - chosen;
+    const int rc = focus_tables(ctx, f, rings, nS);
     if (rc) {
         pc_release(ctx, f->W1, f->W1_bytes);
         pc_release(ctx, f->rows, f->rows_bytes);
@@ -666,9 +515,16 @@ int plan_window(pc_ctx *ctx, const pc_focus *f, uint64_t low, uint64_t high, Win
     if ((high - 1) / f->M - low / f->M + 1 > 4096) return pc_fail(ctx, PC_OVERFLOW, "focus window exceeds bounded period count");
     p.K0 = low / f->M1;
     p.K1 = (high - 1) / f->M1;
-    const std::vector<uint64_t> &W = f->W1_host;
-    p.j_lo = std::lower_bound(W.begin(), W.end(), low - p.K0 * f->M1) - W.begin();
-    p.j_hi = std::lower_bound(W.begin(), W.end(), high - p.K1 * f->M1) - W.begin();
+    // samples below x: the first entry >= x lies in the block of the last of them, or is its end
+    auto samples_below = [&](uint64_t x) -> uint64_t {
+        if (x == 0 || x >= f->M1) return x ? (f->count1 + SAMPLE - 1) / SAMPLE : 0;
+        return std::lower_bound(f->sample.begin(), f->sample.end(), x) - f->sample.begin();
+    };
+    p.rem_lo = low - p.K0 * f->M1;
+    p.rem_hi = high - p.K1 * f->M1;
+    const uint64_t below_lo = samples_below(p.rem_lo);
+    p.j_lo = below_lo ? (below_lo - 1) * SAMPLE : 0;
+    p.j_hi = std::min(samples_below(p.rem_hi) * SAMPLE, f->count1);
     if (p.K0 == p.K1) {
         p.wa0 = p.j_lo / 32;
         p.wb0 = std::max(p.wa0, (p.j_hi + 31) / 32);
@@ -796,6 +652,161 @@ int winbatch_emit(pc_ctx *ctx, const WinBatch &wb, uint64_t *out, uint64_t out_c
     PC_LAUNCHED(ctx, "windows");
     return PC_OK;
 }
+
+namespace {
+
+// Bitset rows of `rings` over the wheel f->W1 (count1 entries), into f->rows: total_rows x stride words.
+int wheel_rows(pc_ctx *ctx, pc_focus *f, const Ring *rings, uint32_t n, const uint32_t *d_pat, const uint32_t *off) {
+    RowRings rr{};
+    for (uint32_t t = 0; t < n; ++t) {
+        rr.q[t] = rings[t].q;
+        rr.off[t] = off[t];
+        rr.row0[t] = f->t_row0[t];
+        rr.mq[t] = make_modq(rings[t].q);
+    }
+    const uint64_t threads = f->stride / 4 * 32;
+    k_wheel_rows<<<dim3((unsigned)((threads + WT - 1) / WT), n), WT, 0, ctx->stream>>>(f->W1, f->count1, d_pat, rr, f->rows,
+                                                                                     f->stride);
+    PC_LAUNCHED(ctx, "wheel rows");
+    return PC_OK;
+}
+
+// The T rings of f are rings[0..n): moduli, periods mod each, row places.
+void set_rings(pc_focus *f, const Ring *rings, uint32_t n) {
+    f->nT = n;
+    f->total_rows = 0;
+    for (uint32_t t = 0; t < n; ++t) {
+        f->tq[t] = rings[t].q;
+        f->t_m1mod[t] = (uint32_t)(f->M1 % f->tq[t]);
+        f->t_row0[t] = f->total_rows;
+        f->total_rows += f->tq[t];
+    }
+    f->words1 = (f->count1 + 31) / 32;
+    f->stride = (f->words1 + 3) & ~UINT64_C(3);
+    f->rows_bytes = std::max<uint64_t>(16, (uint64_t)f->total_rows * f->stride * 4);
+}
+
+// The wheel W1 over the rings [0, nS) and the bitset rows of the rest.  The wheel of the smallest rings is
+// enumerated on the host (period by period, so in order; a few thousand entries).  Then up to six rings
+// at a time: the sorted values of one whole period of the larger modulus are a window of the smaller wheel
+// with those rings as bitset rows, written by k_windows like any other.  That tests 32 candidates of the
+// smaller wheel per word and ring; a bit sieve over [0, M1), which this replaces, walked all M1
+// positions twice (0.33 and 0.48 ms a pass for the two foci of a (7, 6) split, whose wheels now take
+// 26 and 24 us).  The host keeps one wheel entry in 128 for planning, not the whole wheel (0.27 and 0.82 ms
+// of copies).
+int focus_tables(pc_ctx *ctx, pc_focus *f, const std::vector<Ring> &rings, uint32_t nS) {
+    Scratch hold(ctx);
+    std::vector<std::vector<char>> ok(rings.size());
+    for (size_t k = 0; k < rings.size(); ++k) {
+        ok[k].assign(rings[k].q, 0);
+        for (uint32_t a : rings[k].res) ok[k][a] = 1;
+    }
+    std::vector<uint64_t> base(1, 0), next;
+    uint64_t M = 1, expect = 1;
+    uint32_t k = 0;
+    for (; k < nS && base.size() * rings[k].q <= BASE_STEPS; ++k) {
+        const uint32_t q = rings[k].q;
+        next.clear();
+        for (uint32_t period = 0; period < q; ++period)
+            for (uint64_t w : base)
+                if (ok[k][(period * M + w) % q]) next.push_back(period * M + w);
+        base.swap(next);
+        M *= q;
+        expect *= rings[k].n;
+    }
+    if (base.size() != expect) return pc_fail(ctx, PC_ARITHMETIC, "wheel size disagrees with the ring counts");
+    // patterns of the remaining rings: R repeated, so that any 32 bits from an offset below q are one funnel shift
+    std::vector<uint32_t> pat, off(rings.size(), 0);
+    for (size_t r = k; r < rings.size(); ++r) {
+        off[r] = (uint32_t)pat.size();
+        const uint32_t nbits = 2 * rings[r].q + 64;
+        std::vector<uint32_t> words((nbits + 31) / 32 + 1, 0);
+        for (uint32_t b = 0; b < nbits; ++b)
+            if (ok[r][b % rings[r].q]) words[b / 32] |= 1u << (b % 32);
+        pat.insert(pat.end(), words.begin(), words.end());
+    }
+    uint32_t *d_pat = nullptr;
+    int rc = hold.get(&d_pat, pat.size() + 1);
+    if (rc) return rc;
+    if (!pat.empty()) PC_CHECK(ctx, pc_copy(ctx, d_pat, pat.data(), pat.size() * 4, cudaMemcpyHostToDevice));
+
+    struct Level {                                      // kept until the stream has run it
+        pc_focus wheel;
+        WinBatch wb;
+        uint64_t got[3];                                // start, total, stuck flag
+    };
+    std::vector<std::unique_ptr<Level>> levels;
+    pc_focus small;                                     // the wheel so far
+    small.M1 = M;
+    small.count1 = base.size();
+    uint64_t *d_base = nullptr;
+    auto wheel_buffer = [&](uint64_t entries, bool last) {
+        if (!last) return hold.get(&d_base, entries);
+        f->W1_bytes = std::max<uint64_t>(16, entries * 8);
+        const int rc2 = pc_alloc(ctx, (void **)&f->W1, f->W1_bytes);
+        d_base = f->W1;
+        return rc2;
+    };
+    rc = wheel_buffer(base.size(), k == nS);
+    if (rc) return rc;
+    PC_CHECK(ctx, pc_copy(ctx, d_base, base.data(), base.size() * 8, cudaMemcpyHostToDevice));
+    small.W1 = d_base;
+    while (k < nS) {
+        const uint32_t n = std::min<uint32_t>(PC_MAX_WHEEL_T, nS - k);
+        levels.emplace_back(new Level());
+        Level &l = *levels.back();
+        l.wheel = small;
+        set_rings(&l.wheel, rings.data() + k, n);
+        uint64_t period = small.M1, entries = small.count1;
+        double density = (double)small.count1 / (double)small.M1;
+        for (uint32_t t = 0; t < n; ++t) {
+            period *= rings[k + t].q;
+            entries *= rings[k + t].n;
+            density *= (double)rings[k + t].n / rings[k + t].q;
+        }
+        l.wheel.M = period;
+        l.wheel.density = density;
+        rc = hold.get(&l.wheel.rows, l.wheel.rows_bytes / 4);
+        if (!rc) rc = wheel_rows(ctx, &l.wheel, rings.data() + k, n, d_pat, off.data() + k);
+        const pc_focus *wheel = &l.wheel;
+        const uint64_t low = 0, high = period;
+        if (!rc) rc = winbatch_describe(ctx, hold, &wheel, &low, &high, 1, l.wb);
+        if (!rc) rc = wheel_buffer(entries, k + n == nS);
+        if (!rc) rc = winbatch_emit(ctx, l.wb, d_base, entries);
+        if (rc) return rc;
+        small.M1 = period;
+        small.count1 = entries;
+        small.W1 = d_base;
+        k += n;
+    }
+    f->M1 = small.M1;
+    f->count1 = small.count1;
+    set_rings(f, rings.data() + nS, (uint32_t)rings.size() - nS);
+    rc = pc_alloc(ctx, (void **)&f->rows, f->rows_bytes);
+    if (!rc && f->nT) rc = wheel_rows(ctx, f, rings.data() + nS, f->nT, d_pat, off.data() + nS);
+    uint64_t *d_sample = nullptr;
+    const uint64_t samples = (f->count1 + SAMPLE - 1) / SAMPLE;
+    if (!rc) rc = hold.get(&d_sample, samples);
+    if (rc) return rc;
+    k_sample<<<(unsigned)((samples + WT - 1) / WT), WT, 0, ctx->stream>>>(f->W1, samples, d_sample);
+    PC_LAUNCHED(ctx, "wheel samples");
+    f->sample.resize(samples);
+    PC_CHECK(ctx, pc_copy(ctx, f->sample.data(), d_sample, samples * 8, cudaMemcpyDeviceToHost));
+    for (const auto &l : levels)
+        PC_CHECK(ctx, pc_copy(ctx, l->got, l->wb.d_scan + 1 + win_tiles(l->wb), sizeof(l->got), cudaMemcpyDeviceToHost));
+    PC_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
+    for (const auto &l : levels) {
+        if (l->got[2]) return pc_fail(ctx, PC_ARITHMETIC, "window pass did not finish");
+        uint64_t entries = l->wheel.count1;
+        for (uint32_t t = 0; t < l->wheel.nT; ++t)
+            for (const Ring &r : rings)
+                if (r.q == l->wheel.tq[t]) entries *= r.n;
+        if (l->got[1] != entries) return pc_fail(ctx, PC_ARITHMETIC, "wheel size disagrees with the ring counts");
+    }
+    return PC_OK;
+}
+
+}  // namespace
 
 // Windows one after another (unpadded) into one buffer allocated here: sized from the foci's densities
 // and filled in one pass; a pass whose values outgrow it reruns once with room for all.  A total above
