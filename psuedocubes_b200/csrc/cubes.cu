@@ -7,15 +7,13 @@
 // (review/cube_count.c:12-37) and an odd-only bit sieve (review/cube_count_independent.c:9-34)
 // over inclusive root bounds 1 <= first <= last < 2^32, 2 <= p <= 2000.
 //
-// Device form: the primes <= p are packed into groups whose product P stays <= 2^16; for each
-// group a bit pattern marks the residues r mod P that share a factor with P, stored for r up to
-// P + 33 * 32 so that 33 consecutive words starting at any offset r < P are read without a wrap.
-// A warp owns 32 x 33 consecutive words of the root bitmap (bit i <-> root first + i); lane l
-// holds the 33 words from 33 l on, so its window for word k + 1 shares a pattern word with the
-// window for word k: one shared-memory load, one funnel shift and one OR per group and word.  The
-// lanes start 33 words apart, so (away from the pattern's end) their loads fall in 32 different
-// banks.  The OR over all groups marks the roots with a prime factor <= p; the rest are counted,
-// or, after a scan of per-warp counts, written out in ascending order (lane order is root order).
+// Device form: a = W k + r with W the product of the primes 2, 3, 5 that are <= p and r one of the residues
+// coprime to W, so only 8 of 30 numbers are sieved, one bitmap over k per residue class.  The other
+// primes are packed into groups whose product P stays <= 2^16; q | W k + r exactly when
+// q | k + r W^-1 (mod q), so one bit pattern per group (bit z set when z shares a factor with P) serves
+// every class from the offset (k + r W^-1) mod P.  Patterns are stored past P, so that consecutive words
+// starting at any offset below P are read without a wrap; each CTA marks them in its shared memory from
+// the primes (a few thousand bits), so only the table of groups (a few KB) comes from the host.
 #include "common.cuh"
 #include <algorithm>
 #include <vector>
@@ -23,120 +21,288 @@
 namespace {
 
 constexpr uint32_t ROOT_GROUP_MAX = 1u << 16;   // largest product of one prime group
-constexpr int ROOT_LANE_WORDS = 33;             // consecutive words per lane of one warp chunk
-constexpr uint64_t ROOT_CHUNK_WORDS = 32 * ROOT_LANE_WORDS;
-constexpr int ROOT_THREADS = 256;
+constexpr uint32_t ROOT_GROUPS = 304, ROOT_CLASSES = 8;   // 303 primes below 2000
+constexpr int ROOT_THREADS = 1024, LIST_THREADS = 128;
+constexpr uint32_t LIST_STAGE = 32 * 32 * ROOT_CLASSES;         // a warp's candidates, 16 bits each while staged
 
-struct RootGroup {
+struct __align__(16) RootGroup {
     uint64_t c;                      // fastmod constant of P
-    uint32_t P, P2, two32, off;      // period, 2P, 2^32 mod P, pattern word offset
+    uint32_t P, inv;                 // period; W^-1 mod P
+    uint32_t off, words;             // first word of the pattern, its words
+    uint32_t pad[2];
 };
 
-struct RootTables {
-    std::vector<RootGroup> groups;
-    std::vector<uint32_t> pattern;
+struct RootPrime {
+    uint32_t q, off, bits;           // the prime; its group's pattern: first word, bits
+    uint32_t every;                  // bit i set when q | i, i < 32
 };
 
-RootTables root_tables(uint32_t p) {
+// The table in shared memory and its source: groups, then primes.
+struct RootParams {
+    uint32_t ngroups, nprimes, W, nclass, table_words;
+    uint64_t first, last, k0, nk;    // numbers; k of the first number, k values
+    uint32_t cls[ROOT_CLASSES];      // residues coprime to W, ascending
+    const uint4 *table;
+    __host__ __device__ uint32_t table_bytes() const { return ngroups * sizeof(RootGroup) + nprimes * sizeof(RootPrime); }
+    uint32_t smem() const { return table_bytes() + table_words * 4; }
+};
+
+// The groups and their patterns' places; `run` consecutive words are read from any offset below P.
+void root_params(RootParams &p, std::vector<unsigned char> &table, uint64_t first, uint64_t last, uint32_t bound, uint32_t run) {
+    std::vector<char> composite(bound + 1, 0);
     std::vector<uint32_t> primes;
-    std::vector<char> composite(p + 1, 0);
-    for (uint32_t q = 2; q <= p; ++q) {
+    p.W = 1;
+    for (uint32_t q = 2; q <= bound; ++q) {
         if (composite[q]) continue;
-        primes.push_back(q);
-        for (uint32_t m = q * q; m <= p; m += q) composite[m] = 1;
+        if (q <= 5) p.W *= q;
+        else primes.push_back(q);
+        for (uint32_t m = q * q; m <= bound; m += q) composite[m] = 1;
     }
-    RootTables t;
+    p.nclass = 0;
+    for (uint32_t r = 1; r < p.W; ++r)
+        if ((p.W % 2 || r % 2) && (p.W % 3 || r % 3) && (p.W % 5 || r % 5)) p.cls[p.nclass++] = r;
+    p.first = first;
+    p.last = last;
+    p.k0 = first / p.W;
+    p.nk = last / p.W - p.k0 + 1;
+    p.table_words = 0;
+    std::vector<RootGroup> groups;
+    std::vector<RootPrime> marks;
     for (size_t i = 0; i < primes.size();) {
-        uint32_t P = 1;
-        size_t j = i;
-        while (j < primes.size() && (uint64_t)P * primes[j] <= ROOT_GROUP_MAX) P *= primes[j++];
         RootGroup g{};
-        g.P = P;
-        g.c = fastmod_constant(P);
-        g.P2 = 2 * P;
-        g.two32 = (uint32_t)((UINT64_C(1) << 32) % P);
-        g.off = (uint32_t)t.pattern.size();
-        const uint32_t words = (P - 1) / 32 + ROOT_LANE_WORDS + 1;   // 33 windows from any r < P
-        t.pattern.resize(t.pattern.size() + words, 0);
-        uint32_t *w = t.pattern.data() + g.off;
-        for (size_t k = i; k < j; ++k)                 // q | P, so q | r iff q | (r mod P)
-            for (uint32_t r = 0; r < words * 32; r += primes[k]) w[r >> 5] |= 1u << (r & 31);
-        t.groups.push_back(g);
-        i = j;
+        g.P = 1;
+        const size_t i0 = i;
+        while (i < primes.size() && (uint64_t)g.P * primes[i] <= ROOT_GROUP_MAX) g.P *= primes[i++];
+        g.c = fastmod_constant(g.P);
+        for (uint64_t m = 0; m < p.W; ++m)               // W^-1 = (1 + m P) / W for the m that makes it whole
+            if ((1 + m * g.P) % p.W == 0) {
+                g.inv = (uint32_t)((1 + m * g.P) / p.W % g.P);
+                break;
+            }
+        g.off = p.table_words;
+        g.words = (g.P - 1) / 32 + run + 1;
+        p.table_words += g.words;
+        for (size_t k = i0; k < i; ++k) {
+            RootPrime m{primes[k], g.off, g.words * 32, 0};
+            for (uint32_t b = 0; b < 32; b += m.q) m.every |= 1u << b;
+            marks.push_back(m);
+        }
+        groups.push_back(g);
     }
-    return t;
+    p.table_words = (p.table_words + 3) & ~3u;
+    p.ngroups = (uint32_t)groups.size();
+    p.nprimes = (uint32_t)marks.size();
+    table.resize(p.table_bytes());
+    std::copy((const unsigned char *)groups.data(), (const unsigned char *)(groups.data() + groups.size()), table.begin());
+    std::copy((const unsigned char *)marks.data(), (const unsigned char *)(marks.data() + marks.size()),
+              table.begin() + groups.size() * sizeof(RootGroup));
 }
 
-// Counts (offsets == nullptr) or writes (offsets != nullptr) the roots of each warp chunk.
-// Count mode adds into *total, or stores per-chunk counts when chunk_counts is given.
-__global__ void __launch_bounds__(ROOT_THREADS) k_roots(const uint4 *__restrict__ tables, uint32_t table_words,
-                                                        uint32_t ngroups, uint64_t first, uint64_t n, uint64_t nchunks,
-                                                        unsigned long long *__restrict__ total,
-                                                        uint64_t *__restrict__ chunk_counts,
-                                                        const uint64_t *__restrict__ offsets, uint32_t *__restrict__ out) {
-    extern __shared__ uint4 smem4[];
-    for (uint32_t i = threadIdx.x; i < table_words / 4; i += blockDim.x) smem4[i] = tables[i];
+// The CTA's table and patterns.  A prime below 32 gives each of its group's words whole (32 lanes
+// marking it bit by bit would meet in the same words); larger ones are marked bit by bit.
+__device__ const RootGroup *mark_patterns(const RootParams &p, uint4 *smem, uint32_t *&pattern) {
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5, tw = p.table_bytes() / 16;
+    uint4 *zero = smem + tw;
+    pattern = (uint32_t *)zero;
+    for (uint32_t i = threadIdx.x; i < tw; i += blockDim.x) smem[i] = p.table[i];
+    for (uint32_t i = threadIdx.x; i < p.table_words / 4; i += blockDim.x) zero[i] = make_uint4(0, 0, 0, 0);
     __syncthreads();
-    const RootGroup *groups = (const RootGroup *)smem4;
-    const uint32_t *pattern = (const uint32_t *)(groups + ngroups);
-    const uint32_t lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-    for (uint64_t chunk = blockIdx.x * (uint64_t)warps + (threadIdx.x >> 5); chunk < nchunks;
-         chunk += (uint64_t)gridDim.x * warps) {          // warp-uniform
-        const uint64_t w0 = chunk * ROOT_CHUNK_WORDS + ROOT_LANE_WORDS * lane;   // the lane's first word
-        const uint64_t x0 = first + 32 * w0;                                     // < 2^34
-        const uint32_t xlo = (uint32_t)x0, xhi = (uint32_t)(x0 >> 32);
-        uint32_t acc[ROOT_LANE_WORDS];
-#pragma unroll
-        for (int k = 0; k < ROOT_LANE_WORDS; ++k) acc[k] = 0;
-        for (uint32_t g = 0; g < ngroups; ++g) {
-            const RootGroup G = groups[g];
-            uint32_t s = fastmod32(xlo, G.c, G.P) + xhi * G.two32;   // < 3P, as x0 < 2^34
-            s -= s >= G.P2 ? G.P2 : 0;
-            s -= s >= G.P ? G.P : 0;
-            const uint32_t *pat = pattern + G.off + (s >> 5), sh = s & 31;
-            uint32_t lo = pat[0];
-#pragma unroll
-            for (int k = 0; k < ROOT_LANE_WORDS; ++k) {
-                const uint32_t hi = pat[k + 1];
-                acc[k] |= __funnelshift_r(lo, hi, sh);
-                lo = hi;
+    const RootGroup *groups = (const RootGroup *)smem;
+    const RootPrime *primes = (const RootPrime *)(groups + p.ngroups);
+    for (uint32_t i = warp; i < p.nprimes; i += warps) {
+        const RootPrime m = primes[i];
+        uint32_t *w = pattern + m.off;
+        if (m.q < 32) {
+            for (uint32_t z = lane; z < m.bits / 32; z += 32) {
+                const uint32_t r = 32 * z % m.q;
+                atomicOr(w + z, m.every << (r ? m.q - r : 0));
             }
-        }
-        uint32_t count = 0;
-#pragma unroll
-        for (int k = 0; k < ROOT_LANE_WORDS; ++k) {
-            const uint64_t bit0 = 32 * (w0 + k);
-            const uint32_t valid = bit0 >= n ? 0u : (n - bit0 >= 32 ? 0xffffffffu : low_bits((uint32_t)(n - bit0)));
-            acc[k] = ~acc[k] & valid;
-            count += __popc(acc[k]);
-        }
-        if (!offsets) {
-            const uint32_t sum = __reduce_add_sync(0xffffffffu, count);
-            if (lane == 0) {
-                if (chunk_counts) chunk_counts[chunk] = sum;
-                else atomicAdd(total, (unsigned long long)sum);
-            }
-            continue;
-        }
-        uint32_t incl = count;                            // lanes hold ascending root ranges
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, d);
-            if (lane >= (uint32_t)d) incl += y;
-        }
-        uint64_t slot = offsets[chunk] + incl - count;
-#pragma unroll
-        for (int k = 0; k < ROOT_LANE_WORDS; ++k) {
-            const uint64_t root0 = x0 + 32 * (uint64_t)k;
-            uint32_t bits = acc[k];
-            while (bits) {
-                const uint32_t b = __ffs(bits) - 1;
-                bits &= bits - 1;
-                out[slot++] = (uint32_t)(root0 + b);
-            }
+        } else {
+            for (uint32_t z = m.q * lane; z < m.bits; z += 32 * m.q) atomicOr(w + (z >> 5), 1u << (z & 31));
         }
     }
+    __syncthreads();
+    return groups;
 }
+
+// Bits of the 32 k values from k (relative to k0) on that give numbers of [first, last] in class r.
+__device__ __forceinline__ uint32_t class_bits(const RootParams &p, uint64_t k, uint32_t r) {
+    const uint64_t lo = p.k0 * p.W + r < p.first;                                    // the first k value is too small
+    const uint64_t end = p.nk - ((p.k0 + p.nk - 1) * p.W + r > p.last);              // the last one too large
+    if (k >= end) return 0;
+    uint32_t bits = end - k >= 32 ? 0xffffffffu : low_bits((uint32_t)(end - k));
+    if (k < lo) bits &= ~1u;
+    return bits;
+}
+
+// Counting: a warp owns 32 x RUN consecutive words of one class's bitmap, RUN per lane.  The patterns
+// reach 32 x RUN words past P, so the whole warp reads one window without a wrap: its offset and shift are
+// warp-uniform, a lane's window for one word shares a pattern word with the next (one shared load, one
+// funnel shift and half a three-input OR per group and word), and RUN is odd, so the lanes' loads always
+// fall in 32 different banks.  Bound: those shared loads, one per clock and SM.  With all 30 residues and
+// patterns that wrapped per lane (33 words each, two bank conflicts per load) 4e8 numbers took 201 us, with 8
+// of 30 residues 79 us; now 55 us.
+template <int RUN>
+__global__ void __launch_bounds__(ROOT_THREADS) k_roots(const RootParams p, unsigned long long *__restrict__ total) {
+    extern __shared__ uint4 smem[];
+    __shared__ uint32_t cls_s[ROOT_CLASSES];
+#pragma unroll
+    for (uint32_t i = 0; i < ROOT_CLASSES; ++i)
+        if (threadIdx.x == i) cls_s[i] = p.cls[i];
+    uint32_t *pattern;
+    const RootGroup *groups = mark_patterns(p, smem, pattern);
+    const uint32_t lane = threadIdx.x & 31, warps = ROOT_THREADS / 32;
+    constexpr uint32_t K = 32 * 32 * RUN;                  // k values of one warp task
+    const uint64_t tasks = (p.nk + K - 1) / K * p.nclass;
+    uint32_t count = 0;
+    for (uint64_t task = (threadIdx.x >> 5) * (uint64_t)gridDim.x + blockIdx.x; task < tasks;
+         task += (uint64_t)gridDim.x * warps) {            // warp-uniform; consecutive tasks on different SMs
+        const uint32_t r = cls_s[task % p.nclass];
+        const uint64_t k0 = task / p.nclass * K, k = k0 + lane * (32 * RUN);
+        const uint32_t x = (uint32_t)(p.k0 + k0);          // with any group W = 30, so this is below 2^28
+        uint32_t acc[RUN];
+#pragma unroll
+        for (int w = 0; w < RUN; ++w) acc[w] = 0;
+        const uint32_t *lane_pattern = pattern + lane * RUN;
+        for (uint32_t g0 = 0; g0 < p.ngroups; g0 += 32) {  // lane i finds the window of group g0 + i
+            const uint32_t n = min(p.ngroups - g0, 32u);
+            uint32_t place = 0;                            // pattern word << 5 | shift
+            if (lane < n) {
+                const RootGroup G = groups[g0 + lane];
+                place = G.off * 32 + fastmod32(x + r * G.inv, G.c, G.P);   // x + r inv < 2^28 + 30 2^16
+            }
+            uint32_t i = 0;
+            for (; i + 1 < n; i += 2) {
+                const uint32_t sa = __shfl_sync(0xffffffffu, place, i), sb = __shfl_sync(0xffffffffu, place, i + 1);
+                const uint32_t *pa = lane_pattern + (sa >> 5), *pb = lane_pattern + (sb >> 5);
+                uint32_t la = pa[0], lb = pb[0];
+#pragma unroll
+                for (int w = 0; w < RUN; ++w) {
+                    const uint32_t ha = pa[w + 1], hb = pb[w + 1];
+                    acc[w] |= __funnelshift_r(la, ha, sa) | __funnelshift_r(lb, hb, sb);   // by the low five bits
+                    la = ha, lb = hb;
+                }
+            }
+            if (i < n) {
+                const uint32_t sa = __shfl_sync(0xffffffffu, place, i);
+                const uint32_t *pa = lane_pattern + (sa >> 5);
+                uint32_t la = pa[0];
+#pragma unroll
+                for (int w = 0; w < RUN; ++w) {
+                    const uint32_t ha = pa[w + 1];
+                    acc[w] |= __funnelshift_r(la, ha, sa);
+                    la = ha;
+                }
+            }
+        }
+#pragma unroll
+        for (int w = 0; w < RUN; ++w) count += __popc(~acc[w] & class_bits(p, k + 32 * w, r));
+    }
+    count = __reduce_add_sync(0xffffffffu, count);
+    if (lane == 0 && count) atomicAdd(total, (unsigned long long)count);
+}
+
+// Listing (and counting short ranges, which would leave k_roots a few long warps): a lane owns 32
+// consecutive k values of every class, so number order is lane order, then k, then class.  The tile's place in
+// the list comes from a look-back over the tiles before it (out may be null: count only).  A warp's roots
+// are staged in the patterns' space, which nothing reads any more, and stored coalesced.
+__global__ void __launch_bounds__(LIST_THREADS) k_root_list(const RootParams p,
+                                                            unsigned long long *__restrict__ ticket, uint64_t ntiles,
+                                                            uint64_t *__restrict__ stuck, uint64_t *__restrict__ total,
+                                                            uint32_t *__restrict__ out, uint64_t cap) {
+    extern __shared__ uint4 smem[];
+    __shared__ uint64_t tile_s, before_s;
+    __shared__ uint32_t sum_s[LIST_THREADS / 32];
+    __shared__ uint32_t shift_s[ROOT_GROUPS][ROOT_CLASSES / 2];    // r W^-1 mod P of every class, 16 bits each
+    __shared__ uint32_t cls_s[ROOT_CLASSES];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) tile_s = atomicAdd(ticket, 1ull);
+#pragma unroll
+    for (uint32_t i = 0; i < ROOT_CLASSES; ++i)
+        if (threadIdx.x == i) cls_s[i] = p.cls[i];
+    uint32_t *pattern;
+    const RootGroup *groups = mark_patterns(p, smem, pattern);
+    for (uint32_t i = threadIdx.x; i < p.ngroups * ROOT_CLASSES; i += LIST_THREADS) {
+        const RootGroup &g = groups[i / ROOT_CLASSES];
+        ((uint16_t *)shift_s)[i] = (uint16_t)fastmod32(cls_s[i % ROOT_CLASSES] * g.inv, g.c, g.P);
+    }
+    __syncthreads();
+    const uint64_t tile = tile_s, k = (tile * LIST_THREADS + threadIdx.x) * 32;
+    uint32_t acc[ROOT_CLASSES] = {};
+#pragma unroll 2
+    for (uint32_t g = 0; g < p.ngroups; ++g) {                     // with any group there are eight classes
+        const RootGroup G = groups[g];
+        const uint32_t P = G.P, s0 = fastmod32((uint32_t)(p.k0 + k), G.c, P);
+        const uint32_t *pat = pattern + G.off;
+#pragma unroll
+        for (uint32_t i = 0; i < ROOT_CLASSES; ++i) {
+            uint32_t s = s0 + ((shift_s[g][i / 2] >> (16 * (i & 1))) & 0xffffu);
+            s -= s >= P ? P : 0;
+            acc[i] |= __funnelshift_r(pat[s >> 5], pat[(s >> 5) + 1], s & 31);
+        }
+    }
+    uint32_t n = 0;
+#pragma unroll
+    for (uint32_t i = 0; i < ROOT_CLASSES; ++i) {
+        acc[i] = i < p.nclass ? ~acc[i] & class_bits(p, k, p.cls[i]) : 0u;
+        n += __popc(acc[i]);
+    }
+    uint32_t incl = n;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= (uint32_t)d) incl += y;
+    }
+    if (lane == 31) sum_s[warp] = incl;
+    __syncthreads();
+    if (warp == 0) {
+        const uint32_t all = __reduce_add_sync(0xffffffffu, lane < LIST_THREADS / 32 ? sum_s[lane] : 0u);
+        const uint64_t before = look_back(ticket + 1, stuck, tile, all, lane);
+        if (lane == 0) {
+            before_s = before;
+            if (tile + 1 == ntiles) *total = before + all;
+        }
+    }
+    if (!out) return;
+    uint16_t *stage = (uint16_t *)pattern + warp * LIST_STAGE;
+    uint32_t any = 0, slot = incl - n;
+#pragma unroll
+    for (uint32_t i = 0; i < ROOT_CLASSES; ++i) any |= acc[i];
+    for (; any; any &= any - 1) {                                  // k values with a root, ascending
+        const uint32_t b = __ffs(any) - 1;
+#pragma unroll
+        for (uint32_t i = 0; i < ROOT_CLASSES; ++i)
+            if (acc[i] >> b & 1) stage[slot++] = (uint16_t)((lane * 32 + b) * ROOT_CLASSES + i);
+    }
+    __syncthreads();
+    uint64_t at = before_s;
+    for (uint32_t w = 0; w < warp; ++w) at += sum_s[w];
+    const uint64_t k_warp = p.k0 + k - lane * 32;
+    for (uint32_t i = lane; i < sum_s[warp]; i += 32) {
+        const uint32_t e = stage[i];
+        if (at + i < cap) out[at + i] = (uint32_t)((k_warp + e / ROOT_CLASSES) * p.W) + cls_s[e % ROOT_CLASSES];
+    }
+}
+
+// The share of all numbers that is coprime to every prime.
+double root_density(const RootParams &p, const std::vector<unsigned char> &table) {
+    double d = (double)p.nclass / p.W;
+    const RootPrime *m = (const RootPrime *)(table.data() + p.ngroups * sizeof(RootGroup));
+    for (uint32_t i = 0; i < p.nprimes; ++i) d *= 1.0 - 1.0 / m[i].q;
+    return d;
+}
+
+template <int RUN>
+int launch_roots(pc_ctx *ctx, const RootParams &p, unsigned long long *d_total) {
+    PC_CHECK(ctx, cudaFuncSetAttribute(k_roots<RUN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem()));
+    k_roots<RUN><<<ctx->sm_count, ROOT_THREADS, p.smem(), ctx->stream>>>(p, d_total);
+    PC_LAUNCHED(ctx, "cube roots count");
+    return PC_OK;
+}
+
+// Words per lane of k_roots: the most whose patterns fit shared memory (p = 619: 177 KB at 9; p = 2000: 218 KB
+// at 3).  Fewer words mean more offsets per word; more would not fit.
+constexpr uint32_t RUNS[] = {9, 5, 3}, ROOT_SMEM = 224 * 1024;
 
 }  // namespace
 
@@ -146,80 +312,74 @@ extern "C" int pc_cube_roots(pc_ctx *ctx, uint64_t first, uint64_t last, uint32_
     if (kernel_ms) *kernel_ms = 0;
     if (first < 1 || last < first || last > UINT32_MAX || p < 2 || p > 2000)
         return pc_fail(ctx, PC_INVALID, "cube roots need 1 <= first <= last < 2^32 and 2 <= p <= 2000");
-    const RootTables t = root_tables(p);
-    const uint32_t ngroups = (uint32_t)t.groups.size();
-    std::vector<uint32_t> host(ngroups * sizeof(RootGroup) / 4 + t.pattern.size());
-    std::copy(t.pattern.begin(), t.pattern.end(),
-              std::copy((const uint32_t *)t.groups.data(), (const uint32_t *)(t.groups.data() + ngroups), host.begin()));
-    host.resize((host.size() + 3) & ~size_t(3), 0);
-    const uint32_t table_words = (uint32_t)host.size();
-    const size_t smem = table_words * 4;
-
     const uint64_t n = last - first + 1;
-    const uint64_t nchunks = (n + 32 * ROOT_CHUNK_WORDS - 1) / (32 * ROOT_CHUNK_WORDS);   // bits per chunk
-    Scratch hold(ctx);
-    uint32_t *d_tables = nullptr;
-    unsigned long long *d_total = nullptr;
-    int rc = hold.get(&d_tables, table_words);
-    if (!rc) rc = hold.get(&d_total, 1);
-    if (rc) return rc;
-    PC_CHECK(ctx, cudaFuncSetAttribute(k_roots, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int per_sm = 0;
-    PC_CHECK(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_roots, ROOT_THREADS, smem));
-    const uint64_t warps = ROOT_THREADS / 32;
-    const unsigned grid = (unsigned)std::max<uint64_t>(
-        1, std::min<uint64_t>((nchunks + warps - 1) / warps, (uint64_t)ctx->sm_count * std::max(1, per_sm)));
-    PC_CHECK(ctx, pc_copy(ctx, d_tables, host.data(), smem, cudaMemcpyHostToDevice));
-    PC_CHECK(ctx, cudaMemsetAsync(d_total, 0, 8, ctx->stream));
-    auto elapsed = [&](float &ms) { return cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]); };
-    if (!roots) {
-        PC_CHECK(ctx, cudaEventRecord(ctx->ev[0], ctx->stream));
-        k_roots<<<grid, ROOT_THREADS, smem, ctx->stream>>>((const uint4 *)d_tables, table_words, ngroups, first, n, nchunks,
-                                                           d_total, nullptr, nullptr, nullptr);
-        PC_LAUNCHED(ctx, "cube roots count");
-        PC_CHECK(ctx, cudaEventRecord(ctx->ev[1], ctx->stream));
-        unsigned long long total = 0;
-        PC_CHECK(ctx, pc_copy(ctx, &total, d_total, 8, cudaMemcpyDeviceToHost));
-        PC_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
-        float ms = 0;
-        PC_CHECK(ctx, elapsed(ms));
-        if (kernel_ms) *kernel_ms = ms;
-        *count = total;
-        return PC_OK;
+    RootParams rp{};
+    std::vector<unsigned char> table;
+    // counts take k_roots from one warp task per SM on (4e6 numbers): its fixed cost, marking the
+    // longer patterns, is then below what the list kernel's three times as many shared loads cost
+    uint32_t run = 0;
+    for (uint32_t r : RUNS) {
+        root_params(rp, table, first, last, p, 32 * r);
+        if (!roots && rp.smem() <= ROOT_SMEM) {
+            if ((rp.nk + 1024 * r - 1) / (1024 * r) * rp.nclass >= (uint64_t)ctx->sm_count) run = r;
+            break;
+        }
     }
-    uint64_t *d_counts = nullptr, *d_offsets = nullptr, *d_ws = nullptr;
-    rc = hold.get(&d_counts, nchunks + 1);
-    if (!rc) rc = hold.get(&d_offsets, nchunks + 1);
-    if (!rc) rc = hold.get(&d_ws, pc_scan_workspace(nchunks));
+    const bool longer = run != 0;
+    if (!longer) root_params(rp, table, first, last, p, 1);
+    const uint64_t ntiles = (rp.nk + LIST_THREADS * 32 - 1) / (LIST_THREADS * 32);
+    Scratch hold(ctx);
+    uint64_t *d_scan = nullptr;                            // total, stuck flag, ticket, tile states
+    const uint64_t words = 3 + (longer ? 0 : ntiles);
+    uint4 *d_table = nullptr;
+    int rc = hold.get(&d_scan, words);
+    if (!rc) rc = hold.get(&d_table, std::max<size_t>(1, table.size() / 16));
     if (rc) return rc;
-    PC_CHECK(ctx, cudaEventRecord(ctx->ev[0], ctx->stream));
-    k_roots<<<grid, ROOT_THREADS, smem, ctx->stream>>>((const uint4 *)d_tables, table_words, ngroups, first, n, nchunks,
-                                                       nullptr, d_counts, nullptr, nullptr);
-    PC_LAUNCHED(ctx, "cube roots chunk counts");
-    PC_CHECK(ctx, cudaEventRecord(ctx->ev[1], ctx->stream));
-    rc = pc_exclusive_scan_ws(ctx, d_counts, d_offsets, nchunks, d_offsets + nchunks, d_ws);
-    if (rc) return rc;
-    uint64_t total = 0;
-    PC_CHECK(ctx, pc_copy(ctx, &total, d_offsets + nchunks, 8, cudaMemcpyDeviceToHost));
-    PC_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
-    float ms = 0;
-    PC_CHECK(ctx, elapsed(ms));
-    if (kernel_ms) *kernel_ms = ms;
-    *count = total;
-    if (total > cap) return pc_fail(ctx, PC_OVERFLOW, "more cube roots than the output capacity");
-    if (!total) return PC_OK;
-    uint32_t *d_out = nullptr;
-    rc = hold.get(&d_out, total);
-    if (rc) return rc;
-    PC_CHECK(ctx, cudaEventRecord(ctx->ev[0], ctx->stream));
-    k_roots<<<grid, ROOT_THREADS, smem, ctx->stream>>>((const uint4 *)d_tables, table_words, ngroups, first, n, nchunks,
-                                                       nullptr, nullptr, d_offsets, d_out);
-    PC_LAUNCHED(ctx, "cube roots emit");
-    PC_CHECK(ctx, cudaEventRecord(ctx->ev[1], ctx->stream));
-    PC_CHECK(ctx, pc_copy(ctx, roots, d_out, total * 4, cudaMemcpyDeviceToHost));
-    PC_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
-    float emit_ms = 0;
-    PC_CHECK(ctx, elapsed(emit_ms));
-    if (kernel_ms) *kernel_ms += emit_ms;
-    return PC_OK;
+    rp.table = d_table;
+    if (!table.empty()) PC_CHECK(ctx, pc_copy(ctx, d_table, table.data(), table.size(), cudaMemcpyHostToDevice));
+    auto elapsed = [&](double &ms) {
+        float f = 0;
+        PC_CHECK(ctx, cudaEventElapsedTime(&f, ctx->ev[0], ctx->ev[1]));
+        ms += f;
+        return (int)PC_OK;
+    };
+    // a listing pass is sized by the density; a list that outgrows it (never seen) is written again
+    uint64_t room = roots ? std::min(std::min(n, cap), (uint64_t)(root_density(rp, table) * n * 1.02) + 4096) : 0;
+    double ms = 0;
+    uint64_t got[2] = {0, 0};
+    for (int attempt = 0;; ++attempt) {
+        Scratch list(ctx);
+        uint32_t *d_out = nullptr;
+        if (roots && (rc = list.get(&d_out, std::max<uint64_t>(1, room)))) return rc;
+        PC_CHECK(ctx, cudaMemsetAsync(d_scan, 0, words * 8, ctx->stream));
+        PC_CHECK(ctx, cudaEventRecord(ctx->ev[0], ctx->stream));
+        if (longer) {
+            unsigned long long *d_total = (unsigned long long *)d_scan;
+            rc = run == 9 ? launch_roots<9>(ctx, rp, d_total) : run == 5 ? launch_roots<5>(ctx, rp, d_total) : launch_roots<3>(ctx, rp, d_total);
+            if (rc) return rc;
+        } else {
+            const size_t smem = rp.table_bytes() + std::max(rp.table_words * 4, LIST_THREADS / 32 * LIST_STAGE * 2);
+            PC_CHECK(ctx, cudaFuncSetAttribute(k_root_list, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            k_root_list<<<(unsigned)ntiles, LIST_THREADS, smem, ctx->stream>>>(
+                rp, (unsigned long long *)d_scan + 2, ntiles, d_scan + 1, d_scan, d_out, room);
+            PC_LAUNCHED(ctx, "cube root list");
+        }
+        PC_CHECK(ctx, cudaEventRecord(ctx->ev[1], ctx->stream));
+        PC_CHECK(ctx, pc_copy(ctx, got, d_scan, sizeof(got), cudaMemcpyDeviceToHost));
+        PC_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
+        if ((rc = elapsed(ms))) return rc;
+        if (kernel_ms) *kernel_ms = ms;
+        if (got[1]) return pc_fail(ctx, PC_ARITHMETIC, "cube root pass did not finish");
+        *count = got[0];
+        if (!roots) return PC_OK;
+        if (got[0] > cap) return pc_fail(ctx, PC_OVERFLOW, "more cube roots than the output capacity");
+        if (got[0] <= room) {
+            if (!got[0]) return PC_OK;
+            PC_CHECK(ctx, pc_copy(ctx, roots, d_out, got[0] * 4, cudaMemcpyDeviceToHost));
+            PC_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
+            return PC_OK;
+        }
+        if (attempt) return pc_fail(ctx, PC_ARITHMETIC, "cube root count changed between attempts");
+        room = got[0];
+    }
 }
