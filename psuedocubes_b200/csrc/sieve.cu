@@ -178,13 +178,26 @@ __device__ __forceinline__ uint32_t seg_of_u(const SegDev *__restrict__ seg, uin
     return lo;
 }
 
+// What k_vprep needs of a segment and of a family, beside SegDev.
+struct SegPrep {
+    uint64_t ia, fa, am;             // A / B: whole part and 64 fraction bits; A mod B
+    uint64_t ilo, ihi;               // floor(lo / B), floor(hi / B)
+    uint64_t wr;                     // floor(2^64 / subtile width) (2^64 - 1 for width 1)
+    uint64_t fast;                   // B < 2^62 and every bound fits 64 bits
+};
+
+struct FamPrep {
+    uint4 f[PC_MAX_BITSET + PC_MAX_CHEAP];   // 2^16 | 2^32 << 16, 2^48 | q << 16 (all mod q), floor(2^32 / q), row0 or A mod q
+};
+
 struct PrepArgs {
     const uint64_t *us;
     const uint64_t *vs;
     uint64_t nv;
     const SegDev *seg;
+    const SegPrep *segp;
     uint32_t nseg;
-    const FamDev *fam;
+    const FamPrep *fam;
     uint32_t nb, stride;
     VRec *rec;
     uint64_t *cres;                  // per v: v*A mod q of the cheap-tier filters, 16 bits each
@@ -193,89 +206,262 @@ struct PrepArgs {
     unsigned long long *bad;
 };
 
-// Per v row: exact u interval as list indices (batch_experiment.py:209-215), bitset row
-// indices, the residues v*A mod q of the cheap-tier filters, and the focused-position count of
-// its subtile.  A thread owns PREP_RUN consecutive v
-// rows: one binary search per bound for the first row of each segment, then the monotone bounds
-// advance linearly (about N_u/N_v < 1 step per row).
-constexpr int PREP_RUN = 16;
+constexpr uint32_t PREP_T = 256;       // threads per CTA; a CTA takes PREP_T x ROWS consecutive v rows
 
-// Monotone advance of a bound from its previous position: a few linear steps, then a galloping
-// search (strides 8, 16, 32, ...) that brackets the answer, then a binary search inside the
-// bracket, so a row whose bound moved by g entries costs O(log g) loads near the previous bound.
-__device__ __forceinline__ uint64_t advance_le(const uint64_t *__restrict__ us, uint64_t n, uint64_t B, u128 key,
-                                               uint64_t from) {
-    for (int step = 0; step < 4; ++step) {
-        if (from >= n || less128(key, mul_wide(__ldg(us + from), B))) return from;
-        ++from;
-    }
-    uint64_t lo = from, stride = 8;                      // us[lo - 1] * B <= key
-    for (;;) {
-        const uint64_t probe = lo + stride;
-        if (probe >= n) return lo + count_le(us + lo, n - lo, B, key);
-        if (less128(key, mul_wide(__ldg(us + probe), B))) return lo + count_le(us + lo, probe - lo, B, key);
-        lo = probe + 1;
-        stride *= 2;
-    }
+// x mod q for x < 2^32, m = floor(2^32 / q): the quotient estimate is at most one too small.
+__device__ __forceinline__ uint32_t mod_short(uint32_t x, uint32_t m, uint32_t q) {
+    const uint32_t r = x - __umulhi(x, m) * q;
+    return __viaddmin_u32(r, 0u - q, r);
 }
 
-__global__ void k_vprep(const PrepArgs a) {
-    const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    const uint64_t j0 = t * PREP_RUN;
-    if (j0 >= a.nv) return;
-    const uint64_t j1 = umin64(a.nv, j0 + PREP_RUN);
-    uint32_t s = seg_of_v(a.seg, a.nseg, j0);
-    uint64_t left = 0, right = 0, tile = UINT64_MAX, t_lo = 1, t_hi = 0, pop = 0;
-    bool fresh = true;
-    for (uint64_t j = j0; j < j1; ++j) {
-        while (s + 1 < a.nseg && j >= (uint64_t)a.seg[s].v_off + a.seg[s].nv) {
-            ++s;
-            fresh = true;
+// U = floor((v A + lo) / B) or, for the upper bound, floor((v A + hi) / B), and its remainder: the number of
+// u with u B <= v A + lo is the number of u <= U.  The fixed-point estimate is at most two too small, and the
+// remainder that corrects it stays below 3 B < 2^64, so 64-bit arithmetic is exact.
+__device__ __forceinline__ uint64_t u_bound(const SegDev &g, const SegPrep &p, uint64_t v, bool upper, uint64_t &rem) {
+    uint64_t u = v * p.ia + __umul64hi(v, p.fa) + (upper ? p.ihi : p.ilo);
+    rem = v * g.A + (upper ? g.hi.lo : g.lo.lo) - u * g.B;
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+        if (rem >= g.B) ++u, rem -= g.B;
+    return u;
+}
+
+// The subtile of v, or UINT64_MAX outside the segment's subtiles: the quotient by the fixed-point reciprocal is
+// at most one too small.
+__device__ __forceinline__ uint64_t tile_of(const SegDev &g, const SegPrep &p, uint64_t v) {
+    const uint64_t d = v - g.v_first;
+    uint64_t t = __umul64hi(d, p.wr);
+    if (d - t * g.width >= g.width) ++t;
+    return v >= g.v_first && t < g.ntiles ? g.tile_base + t : UINT64_MAX;
+}
+
+// entries of the sorted list a[0, n) that are <= x
+__device__ __forceinline__ uint64_t count_le64(const uint64_t *__restrict__ a, uint64_t n, uint64_t x) {
+    uint64_t lo = 0, hi = n;
+    while (lo < hi) {
+        const uint64_t mid = lo + (hi - lo) / 2;
+        if (__ldg(a + mid) <= x) lo = mid + 1;
+        else hi = mid;
+    }
+    return lo;
+}
+
+// The same by 2^LOG lanes of a warp (all 32 lanes call it, each group with its own list and x): 32 probes a step
+// need five dependent loads for ten million entries.
+template <int LOG>
+__device__ __forceinline__ uint64_t group_count_le64(const uint64_t *__restrict__ a, uint64_t n, uint64_t x, uint32_t lane) {
+    constexpr uint32_t L = 1u << LOG;
+    const uint32_t part = lane & (L - 1), group = lane >> LOG << LOG;
+    uint64_t lo = 0, len = n;                             // the answer is in [lo, lo + len]
+    while (__any_sync(0xffffffffu, len != 0)) {
+        const uint64_t step = (len + L - 1) >> LOG, at = lo + umin64((part + 1) * step, len) - 1;   // last entry of the part
+        const uint32_t votes = __ballot_sync(0xffffffffu, part * step < len && __ldg(a + at) <= x);
+        const uint32_t below = __popc(LOG == 5 ? votes : votes >> group & ((1u << (L & 31)) - 1));
+        const uint64_t done = umin64(below * step, len);
+        lo += done;
+        len = len ? umin64(step - 1, len - done) : 0;
+    }
+    return lo;
+}
+
+// entries <= x of a sorted shared list padded with 0xffffffff to 2 top - 1 entries (top: a power of two <= 2048)
+__device__ __forceinline__ uint32_t stage_count_le(const uint32_t *a, uint32_t top, uint32_t x) {
+    uint32_t pos = 0;
+#define PC_STEP(S) case S: if (a[pos + S - 1] <= x) pos += S; [[fallthrough]];
+    switch (top) {
+        PC_STEP(2048) PC_STEP(1024) PC_STEP(512) PC_STEP(256) PC_STEP(128) PC_STEP(64) PC_STEP(32) PC_STEP(16) PC_STEP(8) PC_STEP(4) PC_STEP(2)
+        case 1: if (a[pos] <= x) pos += 1;
+    }
+#undef PC_STEP
+    return pos;
+}
+
+// Per v row: exact u interval as list indices (batch_experiment.py:209-215), bitset row indices, the
+// residues v*A mod q of the cheap-tier filters, and the focused-position count of its subtile.
+//
+// A CTA's rows lie in one segment except at a segment's ends.  Its first row's bounds U, their remainders and the
+// residues are computed once; a row then adds what its distance d < 2^32 from the first row adds, in 32-bit
+// arithmetic but for two 64-bit remainders.  Four warps find the list index of both bounds of the first and last row;
+// the u entries between them (about 0.65 per row) are staged in shared memory as 32-bit offsets, and each row's
+// bounds are two searches there (or, where they are too many to stage, in that part of the list).  In a CTA that
+// spans segments each warp does the same for its own 32 rows in the list, and a row on its own where even these
+// span segments or the moduli are too large for 64-bit bounds.
+//
+// Bound: instruction issue.  Sixteen rows per thread whose bounds advanced through the list in global memory
+// waited on L2: 0.81 ms for a lease's 1.6e7 rows and 50 us for a batch's 6e4, which gave work to 30 SMs; now
+// 0.41 ms and 7 us.
+template <int ROWS>
+__global__ void __launch_bounds__(PREP_T) k_vprep(const PrepArgs a) {
+    constexpr uint32_t PREP_STAGE = ROWS > 4 ? 2048 : 1024;      // u entries staged per bound
+    __shared__ uint32_t stage_s[2][2 * PREP_STAGE];
+    __shared__ uint64_t end_s[4], u_s[4], rem_s[2];              // per bound: first and last row's index and U; remainders
+    __shared__ uint4 res_s[PC_MAX_BITSET + PC_MAX_CHEAP];        // q, floor(2^32 / q), first row's v mod q, row0 or A mod q
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint64_t j0 = blockIdx.x * (uint64_t)(PREP_T * ROWS), j1 = umin64(a.nv, j0 + PREP_T * ROWS);
+    const uint32_t s0 = seg_of_v(a.seg, a.nseg, j0);
+    const SegDev &g0 = a.seg[s0];
+    const SegPrep &p0 = a.segp[s0];
+    auto residue = [](const uint4 f, uint64_t v) {        // v mod q of a FamPrep entry
+        const uint32_t lo = (uint32_t)v, hi = (uint32_t)(v >> 32);
+        return mod_short((lo & 0xffffu) + (lo >> 16) * (f.x & 0xffffu) + (hi & 0xffffu) * (f.x >> 16) + (hi >> 16) * (f.y & 0xffffu),
+                         f.z, f.y >> 16);
+    };
+    bool near = j1 <= (uint64_t)g0.v_off + g0.nv && p0.fast;      // rows as distances from the first; CTA-uniform
+    bool staged = false;
+    uint64_t v_first = 0, first[2] = {}, count[2] = {};
+    uint32_t ahead[2] = {}, top[2] = {};                  // first staged entry minus the first row's U
+    if (near) {
+        const uint64_t *us = a.us + g0.u_off;
+        v_first = a.vs[j0];
+        const uint64_t v_last = a.vs[j1 - 1];
+        if (warp < 4) {                                   // warp: bound * 2 + (first, last row)
+            uint64_t rem;
+            const uint64_t u = u_bound(g0, p0, warp & 1 ? v_last : v_first, warp >= 2, rem);
+            const uint64_t n = group_count_le64<5>(us, g0.nu, u, lane);
+            if (lane == 0) {
+                end_s[warp] = n;
+                u_s[warp] = u;
+                if (!(warp & 1)) rem_s[warp >> 1] = rem;
+            }
+        } else if (warp == 4 && lane < PC_MAX_BITSET + PC_MAX_CHEAP) {
+            const uint4 f = a.fam[g0.fam].f[lane];
+            res_s[lane] = make_uint4(f.y >> 16, f.z, residue(f, v_first), f.w);
         }
-        const SegDev &g = a.seg[s];
-        const FamDev &F = a.fam[g.fam];
-        const uint64_t u0 = g.u_off, u1 = u0 + g.nu;
-        const uint64_t v = a.vs[j];
-        const u128 shift = mul_wide(v, g.A);
-        const u128 klo = add128(shift, g.lo), khi = add128(shift, g.hi);
-        if (fresh) {
-            left = u0 + count_le(a.us + u0, g.nu, g.B, klo);
-            right = umax64(left, u0 + count_le(a.us + u0, g.nu, g.B, khi));
-            t_lo = 1, t_hi = 0;                           // force a subtile lookup
-            fresh = false;
+        __syncthreads();
+        // distances stay below 2^32, also with a residue added
+        near = v_last - v_first < 0xffff0000u && u_s[1] - u_s[0] < 0xffff0000u && u_s[3] - u_s[2] < 0xffff0000u;
+        staged = near;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            first[k] = end_s[2 * k];
+            count[k] = end_s[2 * k + 1] - first[k];
+            const bool some = count[k] && first[k] < g0.nu;       // (an unsorted v list leaves count meaningless)
+            ahead[k] = some ? (uint32_t)(us[first[k]] - u_s[2 * k]) : 0xffffffffu;
+            staged = staged && count[k] <= PREP_STAGE;
+            top[k] = some ? 1u << (31 - __clz((uint32_t)umin64(count[k], PREP_STAGE))) : 0u;
+        }
+        if (staged)
+#pragma unroll
+            for (int k = 0; k < 2; ++k)
+                for (uint32_t i = threadIdx.x; i < 2 * top[k]; i += PREP_T)
+                    stage_s[k][i] = i < count[k] ? (uint32_t)(us[first[k] + i] - u_s[2 * k]) - ahead[k] : 0xffffffffu;
+        __syncthreads();
+    }
+    uint64_t tile = UINT64_MAX, pop = 0;                  // warp-uniform: the subtile being summed
+#pragma unroll 1
+    for (int m = 0; m < ROWS; ++m) {
+        const uint64_t j = j0 + m * PREP_T + threadIdx.x;
+        const bool active = j < j1;
+        uint64_t mine = UINT64_MAX, v = 0, cr = 0;        // the row's subtile
+        uint32_t left = 0, right = 0, row[PC_MAX_BITSET] = {};
+        if (near) {
+            if (active) {
+                v = a.vs[j];
+                const uint32_t d = (uint32_t)(v - v_first);
+                // U grows by d (A / B): floor by the 64 fraction bits, the rest by the remainders (below 3 B)
+                const uint32_t e = (uint32_t)__umul64hi(d, p0.fa);
+                const uint64_t t = d * p0.am - e * g0.B, B2 = 2 * g0.B;
+                uint32_t at[2];
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    const uint64_t r = rem_s[k] + t;
+                    const uint32_t grown = d * (uint32_t)p0.ia + e + (r >= g0.B) + (r >= B2);
+                    uint64_t n = 0;
+                    if (grown >= ahead[k]) {
+                        if (staged) n = stage_count_le(stage_s[k], top[k], grown - ahead[k]);
+                        else n = count_le64(a.us + g0.u_off + first[k], umin64(count[k], g0.nu - first[k]), u_s[2 * k] + grown);
+                    }
+                    at[k] = g0.u_off + (uint32_t)(first[k] + n);
+                }
+                left = at[0];
+                right = max(at[0], at[1]);
+#pragma unroll
+                for (int f = 0; f < PC_MAX_BITSET; ++f)
+                    if (f < (int)a.nb) {
+                        const uint4 c = res_s[f];
+                        row[f] = c.w + mod_short(d + c.z, c.y, c.x);
+                    }
+#pragma unroll
+                for (int f = 0; f < PC_MAX_CHEAP; ++f)
+                    if (f < (int)a.nch) {
+                        const uint4 c = res_s[PC_MAX_BITSET + f];
+                        cr |= (uint64_t)mod_short(mod_short(d + c.z, c.y, c.x) * c.w, c.y, c.x) << (16 * f);
+                    }
+                mine = tile_of(g0, p0, v);
+            }
         } else {
-            left = advance_le(a.us, u1, g.B, klo, left);
-            right = advance_le(a.us, u1, g.B, khi, umax64(left, right));
-        }
-        if (v < t_lo || v >= t_hi) {
-            if (tile != UINT64_MAX && pop) atomicAdd((unsigned long long *)&a.counts[tile * a.stride], (unsigned long long)pop);
-            pop = 0;
-            const uint64_t lt = local_tile(v, g.v_first, g.width, g.ntiles);
-            if (lt >= g.ntiles) {
-                atomicAdd(a.bad, 1ull);
-                tile = UINT64_MAX, t_lo = 1, t_hi = 0;
-            } else {
-                tile = g.tile_base + lt;
-                t_lo = g.v_first + lt * g.width;
-                t_hi = t_lo + g.width;
+            const uint32_t s = active ? seg_of_v(a.seg, a.nseg, j) : s0;
+            const SegDev &g = a.seg[s];
+            const SegPrep &p = a.segp[s];
+            const uint32_t rows = __ballot_sync(0xffffffffu, active);
+            // the warp's rows in one segment with 64-bit bounds: eight lanes for each bound of its first and last row
+            const uint32_t lead = __shfl_sync(0xffffffffu, s, 0);
+            const bool together = rows && __all_sync(0xffffffffu, !active || (s == lead && p.fast));
+            const uint64_t *us = a.us + g.u_off;
+            uint64_t rem, lo[2] = {0, 0}, n[2] = {g.nu, g.nu};
+            if (active) v = a.vs[j];
+            if (together) {
+                const uint64_t v_end = __shfl_sync(0xffffffffu, v, lane & 8 ? 31 - __clz(rows) : 0);
+                const SegDev &gw = a.seg[lead];
+                const uint64_t u = u_bound(gw, a.segp[lead], v_end, lane >= 16, rem);
+                const uint64_t at = group_count_le64<3>(a.us + gw.u_off, gw.nu, u, lane);
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    lo[k] = __shfl_sync(0xffffffffu, at, 16 * k);
+                    const uint64_t end = __shfl_sync(0xffffffffu, at, 16 * k + 8);
+                    n[k] = end > lo[k] ? end - lo[k] : 0;
+                }
+            }
+            if (active) {
+                uint64_t at[2];
+                if (p.fast) {
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) at[k] = lo[k] + count_le64(us + lo[k], n[k], u_bound(g, p, v, k, rem));
+                } else {
+                    const u128 shift = mul_wide(v, g.A);
+                    at[0] = count_le(us, g.nu, g.B, add128(shift, g.lo));
+                    at[1] = count_le(us, g.nu, g.B, add128(shift, g.hi));
+                }
+                left = g.u_off + (uint32_t)at[0];
+                right = g.u_off + (uint32_t)umax64(at[0], at[1]);
+                const FamPrep &F = a.fam[g.fam];
+#pragma unroll
+                for (int f = 0; f < PC_MAX_BITSET; ++f)
+                    if (f < (int)a.nb) {
+                        const uint4 c = F.f[f];
+                        row[f] = c.w + residue(c, v);
+                    }
+#pragma unroll
+                for (int f = 0; f < PC_MAX_CHEAP; ++f)
+                    if (f < (int)a.nch) {
+                        const uint4 c = F.f[PC_MAX_BITSET + f];
+                        cr |= (uint64_t)mod_short(residue(c, v) * c.w, c.z, c.y >> 16) << (16 * f);
+                    }
+                mine = tile_of(g, p, v);
             }
         }
-        VRec r;
-        r.left = (uint32_t)left;
-        r.right = (uint32_t)right;
-        r.v = v;
-#pragma unroll
-        for (int f = 0; f < PC_MAX_BITSET; ++f)
-            r.row[f] = f < (int)a.nb ? (uint16_t)(F.row0[f] + mod64(v, F.mq[f])) : (uint16_t)0;
-        a.rec[j] = r;
-        uint64_t cr = 0;
-#pragma unroll
-        for (int t = 0; t < PC_MAX_CHEAP; ++t)
-            if (t < (int)a.nch) cr |= (uint64_t)fastmod32(mod64(v, F.cmq[t]) * F.caq[t], F.cmq[t].c, F.cq[t]) << (16 * t);
-        a.cres[j] = cr;
-        pop += right - left;
+        if (active) {
+            if (mine == UINT64_MAX) atomicAdd(a.bad, 1ull);
+            uint4 *out = (uint4 *)(a.rec + j);
+            out[0] = make_uint4(left, right, (uint32_t)v, (uint32_t)(v >> 32));
+            out[1] = make_uint4(row[0] | row[1] << 16, row[2] | row[3] << 16, row[4] | row[5] << 16, row[6] | row[7] << 16);
+            a.cres[j] = cr;
+        }
+        // a warp's rows mostly share one subtile, which is summed over the warp's rounds
+        const uint32_t width = right - left;
+        const uint64_t common = __shfl_sync(0xffffffffu, mine, 0);
+        if (__all_sync(0xffffffffu, mine == common)) {
+            if (common != tile) {
+                if (lane == 0 && tile != UINT64_MAX && pop) atomicAdd((unsigned long long *)&a.counts[tile * a.stride], (unsigned long long)pop);
+                tile = common;
+                pop = 0;
+            }
+            pop += __reduce_add_sync(0xffffffffu, width & 0xffffu) + ((uint64_t)__reduce_add_sync(0xffffffffu, width >> 16) << 16);
+        } else if (mine != UINT64_MAX && width) {
+            atomicAdd((unsigned long long *)&a.counts[mine * a.stride], (unsigned long long)width);
+        }
     }
-    if (tile != UINT64_MAX && pop) atomicAdd((unsigned long long *)&a.counts[tile * a.stride], (unsigned long long)pop);
+    if (lane == 0 && tile != UINT64_MAX && pop) atomicAdd((unsigned long long *)&a.counts[tile * a.stride], (unsigned long long)pop);
 }
 
 // Per subtile: u count and v count of its envelope (searchsorted bounds of
@@ -1332,6 +1518,31 @@ FamDev fam_dev(const pc_filters *f, uint32_t nb, uint32_t nch) {
     return d;
 }
 
+FamPrep fam_prep(const FamDev &d, uint32_t nb, uint32_t nch) {
+    FamPrep p{};
+    auto pack = [](const ModQ &m, uint32_t w) {
+        return make_uint4(m.r16[0] | m.r16[1] << 16, m.r16[2] | m.q << 16, (uint32_t)(m.c >> 32), w);
+    };
+    for (uint32_t t = 0; t < nb; ++t) p.f[t] = pack(d.mq[t], d.row0[t]);
+    for (uint32_t t = 0; t < nch; ++t) p.f[PC_MAX_BITSET + t] = pack(d.cmq[t], d.caq[t]);
+    return p;
+}
+
+// Fixed-point A / B and the whole parts of the interval's ends over B.
+SegPrep seg_prep(const SegDev &g) {
+    typedef unsigned __int128 w128;
+    const w128 lo = (w128)g.lo.hi << 64 | g.lo.lo, hi = (w128)g.hi.hi << 64 | g.hi.lo, last = (w128)(g.v_end ? g.v_end - 1 : 0) * g.A;
+    SegPrep p{};
+    p.ia = g.A / g.B;
+    p.am = g.A % g.B;
+    p.fa = (uint64_t)(((w128)p.am << 64) / g.B);
+    p.ilo = (uint64_t)(lo / g.B);
+    p.ihi = (uint64_t)(hi / g.B);
+    p.wr = g.width > 1 ? (uint64_t)(((w128)1 << 64) / g.width) : UINT64_MAX;
+    p.fast = g.B < (UINT64_C(1) << 62) && hi + last >= last && !((hi + last) / g.B >> 64);
+    return p;
+}
+
 // The device half of stages 2 and 3 over a set of segments whose u and v lists are already on
 // the device.  Every buffer is sized once by engine_prepare, so the launch sequence (front + back)
 // can be recorded into a CUDA graph and replayed.
@@ -1352,6 +1563,10 @@ struct Engine {
     uint32_t deep_cap = 1u << 15, deep_max = 0;
     SegDev *d_seg = nullptr;
     FamDev *d_fam = nullptr;
+    SegPrep *d_segp = nullptr;
+    FamPrep *d_famp = nullptr;
+    std::vector<SegPrep> segprep;
+    std::vector<FamPrep> famprep;
     uint32_t *d_tile_seg = nullptr, *d_blk_seg = nullptr, *d_deep_count = nullptr;
     unsigned long long *d_item_next = nullptr;
     uint64_t *d_counts = nullptr, *d_geo = nullptr, *d_out = nullptr;
@@ -1390,7 +1605,13 @@ int engine_prepare(Engine &E, const pc_tuning *tuning, Scratch &hold) {
     for (const pc_filters *f : E.fams) E.ngmax = std::max(E.ngmax, f->ng);
     E.stride = E.ngmax + 3;
     E.famdev.clear();
-    for (const pc_filters *f : E.fams) E.famdev.push_back(fam_dev(f, E.tn.nb, E.tn.nch));
+    E.famprep.clear();
+    E.segprep.clear();
+    for (const pc_filters *f : E.fams) {
+        E.famdev.push_back(fam_dev(f, E.tn.nb, E.tn.nch));
+        E.famprep.push_back(fam_prep(E.famdev.back(), E.tn.nb, E.tn.nch));
+    }
+    for (const SegDev &g : E.segs) E.segprep.push_back(seg_prep(g));
     E.grid = ctx->sm_count;
     if (tuning && tuning->deep_records) E.deep_cap = tuning->deep_records;
     const uint32_t UB = E.tn.K * 32;
@@ -1398,6 +1619,8 @@ int engine_prepare(Engine &E, const pc_tuning *tuning, Scratch &hold) {
     const uint64_t nb1 = std::max<uint64_t>(1, E.nblocks);
     rc = hold.get(&E.d_seg, E.segs.size());
     if (!rc) rc = hold.get(&E.d_fam, E.famdev.size());
+    if (!rc) rc = hold.get(&E.d_segp, E.segs.size());
+    if (!rc) rc = hold.get(&E.d_famp, E.famdev.size());
     if (!rc) rc = hold.get(&E.d_tile_seg, std::max<uint64_t>(1, E.ntiles));
     if (!rc) rc = hold.get(&E.d_counts, std::max<uint64_t>(1, E.ntiles * E.stride));
     if (!rc) rc = hold.get(&E.d_geo, std::max<uint64_t>(1, 2 * E.ntiles));
@@ -1419,6 +1642,8 @@ int engine_prepare(Engine &E, const pc_tuning *tuning, Scratch &hold) {
     if (rc) return rc;
     PC_CHECK(ctx, pc_copy(ctx, E.d_seg, E.segs.data(), E.segs.size() * sizeof(SegDev), cudaMemcpyHostToDevice));
     PC_CHECK(ctx, pc_copy(ctx, E.d_fam, E.famdev.data(), E.famdev.size() * sizeof(FamDev), cudaMemcpyHostToDevice));
+    PC_CHECK(ctx, pc_copy(ctx, E.d_segp, E.segprep.data(), E.segprep.size() * sizeof(SegPrep), cudaMemcpyHostToDevice));
+    PC_CHECK(ctx, pc_copy(ctx, E.d_famp, E.famprep.data(), E.famprep.size() * sizeof(FamPrep), cudaMemcpyHostToDevice));
     if (E.ntiles)
         PC_CHECK(ctx, pc_copy(ctx, E.d_tile_seg, E.tile_seg.data(), E.ntiles * 4, cudaMemcpyHostToDevice));
     return PC_OK;
@@ -1470,7 +1695,8 @@ int engine_front(Engine &E, bool events, bool capturing, int *launches) {
         pa.nv = E.nv;
         pa.seg = E.d_seg;
         pa.nseg = (uint32_t)E.segs.size();
-        pa.fam = E.d_fam;
+        pa.segp = E.d_segp;
+        pa.fam = E.d_famp;
         pa.nb = E.tn.nb;
         pa.stride = E.stride;
         pa.rec = E.d_rec;
@@ -1478,8 +1704,16 @@ int engine_front(Engine &E, bool events, bool capturing, int *launches) {
         pa.nch = E.tn.nch;
         pa.counts = E.d_counts;
         pa.bad = E.d_nout + 1;
-        const uint64_t runs = (E.nv + PREP_RUN - 1) / PREP_RUN;
-        k_vprep<<<(unsigned)((runs + 127) / 128), 128, 0, st>>>(pa);
+        // 8 or 4 rows per thread share a CTA's end searches where that still leaves every SM that many CTAs and
+        // most CTAs lie in one segment; else one (a lease's 1.6e7 rows: 0.41 ms at 8, 0.44 at 4; 24 batches'
+        // 1.5e6 rows: 54 us at 8, 47 at 4)
+        uint32_t rows = 1;
+        for (uint32_t r : {8u, 4u}) {
+            const uint64_t ctas = E.nv / (r * PREP_T);
+            if (rows == 1 && ctas >= (uint64_t)E.grid * r && ctas >= 4 * E.segs.size()) rows = r;
+        }
+        auto kern = rows == 8 ? k_vprep<8> : rows == 4 ? k_vprep<4> : k_vprep<1>;
+        kern<<<(unsigned)((E.nv + rows * PREP_T - 1) / (rows * PREP_T)), PREP_T, 0, st>>>(pa);
         PC_LAUNCHED(ctx, "vprep");
         ++*launches;
     }
