@@ -22,6 +22,7 @@ struct pc_ctx {
     uint64_t cap = 0, in_use = 0, peak = 0;
     uint64_t h2d = 0, d2h = 0;       // bytes the library has copied to and from the host
     int sm_count = 0, cc_major = 0, cc_minor = 0;
+    uint64_t *stage = nullptr;       // PC_STAGE_BYTES of page-locked memory for results, from the first use on
     char name[256] = {};
     std::string err;
 };
@@ -34,6 +35,10 @@ struct pc_buf {
 
 int pc_fail(pc_ctx *ctx, int code, const std::string &msg);
 int pc_cuda_fail(pc_ctx *ctx, cudaError_t e, const char *what);
+constexpr uint64_t PC_STAGE_BYTES = UINT64_C(512) << 10;
+// The context's page-locked stage, or null when `bytes` do not fit it or it cannot be had.  Its content is the
+// caller's until the next library call on the context.
+uint64_t *pc_stage(pc_ctx *ctx, uint64_t bytes);
 int pc_alloc(pc_ctx *ctx, void **ptr, uint64_t bytes);
 void pc_release(pc_ctx *ctx, void *ptr, uint64_t bytes);
 
@@ -78,6 +83,24 @@ struct Scratch {
         items.emplace_back(q, bytes);
         *p = (T *)q;
         return PC_OK;
+    }
+};
+
+// Several device arrays in one allocation, each 256-byte aligned, in the order added.
+struct Carve {
+    std::vector<std::pair<void **, uint64_t>> parts;     // pointer to set, byte offset
+    uint64_t bytes = 0;
+    template <class T>
+    void add(T **p, uint64_t count) {
+        parts.emplace_back((void **)p, bytes);
+        bytes = (bytes + count * sizeof(T) + 255) & ~UINT64_C(255);
+    }
+    int get(Scratch &s) {
+        unsigned char *base = nullptr;
+        const int rc = s.get(&base, bytes);
+        if (!rc)
+            for (auto &p : parts) *p.first = base + p.second;
+        return rc;
     }
 };
 
@@ -207,6 +230,24 @@ __device__ __forceinline__ uint32_t transpose32c(uint32_t x, const uint32_t (&sh
     return x;
 }
 
+// Entries of a sorted range of n for which `below(index)` holds (a prefix of it), by each group of eight lanes of a
+// warp for its own range: three bits a step, where a thread alone takes one dependent load per bit.
+template <class F>
+__device__ __forceinline__ uint64_t group_prefix(uint64_t n, uint32_t lane, F below) {
+    const uint32_t part = lane & 7, group = lane & 24;
+    uint64_t lo = 0, len = n;                             // the answer is in [lo, lo + len]
+    while (__any_sync(0xffffffffu, len != 0)) {
+        const uint64_t step = (len + 7) / 8, at = lo + umin64((part + 1) * step, len) - 1;   // last entry of the part
+        bool hit = false;
+        if (part * step < len) hit = below(at);
+        const uint32_t parts = __popc(__ballot_sync(0xffffffffu, hit) >> group & 0xffu);
+        const uint64_t done = umin64(parts * step, len);
+        lo += done;
+        len = len ? umin64(step - 1, len - done) : 0;
+    }
+    return lo;
+}
+
 // ------------------------------------------------------------------------------------------
 // Exclusive prefix over the tiles of one launch (decoupled look-back).  A tile's state is one word:
 // value << 2 | 1 (its own sum) or 2 (its own and all before it), zeroed before the launch.
@@ -248,10 +289,6 @@ __device__ __forceinline__ uint64_t look_back(volatile unsigned long long *state
 
 // ------------------------------------------------------------------------------------------
 // internal host helpers shared across translation units
-
-uint64_t pc_scan_workspace(uint64_t n);
-int pc_exclusive_scan_ws(pc_ctx *ctx, const uint64_t *in, uint64_t *out, uint64_t n, uint64_t *total_dev,
-                         uint64_t *ws);
 
 // Many sorted focus windows generated together by one launch.  winbatch_run writes them one after another
 // into a buffer it sizes; winbatch_plan counts them first and gives window i a place that starts on a

@@ -34,6 +34,15 @@ void pc_release(pc_ctx *ctx, void *ptr, uint64_t bytes) {
     ctx->in_use -= std::min(ctx->in_use, bytes);
 }
 
+uint64_t *pc_stage(pc_ctx *ctx, uint64_t bytes) {
+    if (bytes > PC_STAGE_BYTES) return nullptr;
+    if (!ctx->stage && cudaHostAlloc((void **)&ctx->stage, PC_STAGE_BYTES, cudaHostAllocDefault) != cudaSuccess) {
+        cudaGetLastError();
+        ctx->stage = nullptr;
+    }
+    return ctx->stage;
+}
+
 extern "C" int pc_version(void) { return 1; }
 
 extern "C" int pc_device_count(int *count) {
@@ -117,6 +126,7 @@ extern "C" int pc_free(pc_ctx *ctx) {
     for (auto &ev : ctx->marks)
         if (ev) cudaEventDestroy(ev);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
+    if (ctx->stage) cudaFreeHost(ctx->stage);
     delete ctx;
     return PC_OK;
 }
@@ -212,123 +222,32 @@ extern "C" int pc_buf_free(pc_ctx *ctx, pc_buf *buf) {
     return PC_OK;
 }
 
-__global__ void k_searchsorted(const uint64_t *__restrict__ a, uint64_t n, const uint64_t *__restrict__ q,
-                               uint64_t nq, uint64_t *__restrict__ out) {
-    uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (i >= nq) return;
-    uint64_t key = q[i], lo = 0, hi = n;
-    while (lo < hi) {
-        uint64_t mid = lo + (hi - lo) / 2;
-        if (a[mid] < key) lo = mid + 1;
-        else hi = mid;
-    }
-    out[i] = lo;
+// Eight lanes per query (group_prefix): a dependent load for every three bits of the list's length.
+__global__ void __launch_bounds__(256) k_searchsorted(const uint64_t *__restrict__ a, uint64_t n, const uint64_t *__restrict__ q,
+                                                      uint64_t nq, uint64_t *__restrict__ out) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t i = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) / 8;
+    const uint64_t key = i < nq ? q[i] : 0;
+    const uint64_t at = group_prefix(i < nq ? n : 0, lane, [&](uint64_t j) { return __ldg(a + j) < key; });
+    if (i < nq && (lane & 7) == 0) out[i] = at;
 }
 
 extern "C" int pc_buf_searchsorted(pc_ctx *ctx, const pc_buf *buf, const uint64_t *queries, uint64_t n, uint64_t *positions) {
     if (!n) return PC_OK;
     Scratch s(ctx);
     uint64_t *dq, *dp;
-    int rc = s.get(&dq, n);
-    if (!rc) rc = s.get(&dp, n);
+    Carve both;
+    both.add(&dq, n);
+    both.add(&dp, n);
+    const int rc = both.get(s);
     if (rc) return rc;
     PC_CHECK(ctx, pc_copy(ctx, dq, queries, n * 8, cudaMemcpyHostToDevice));
-    k_searchsorted<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(buf->d, buf->n, dq, n, dp);
+    k_searchsorted<<<(unsigned)((n + 31) / 32), 256, 0, ctx->stream>>>(buf->d, buf->n, dq, n, dp);
     PC_LAUNCHED(ctx, "searchsorted");
-    PC_CHECK(ctx, pc_copy(ctx, positions, dp, n * 8, cudaMemcpyDeviceToHost));
+    uint64_t *stage = pc_stage(ctx, n * 8);
+    PC_CHECK(ctx, pc_copy(ctx, stage ? stage : positions, dp, n * 8, cudaMemcpyDeviceToHost));
     PC_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
-    return PC_OK;
-}
-
-// ------------------------------------------------------------------------------------------
-// Exclusive scan of uint64 (three phases: per-block sums, scan of the block sums, add back).
-
-static constexpr int SCAN_T = 512, SCAN_ITEMS = 4, SCAN_TILE = SCAN_T * SCAN_ITEMS;
-
-__device__ __forceinline__ uint64_t block_exclusive_scan(uint64_t v, uint64_t *warp_sums, uint64_t *total) {
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint64_t x = v;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        uint64_t y = __shfl_up_sync(0xffffffffu, x, d);
-        if (lane >= (uint32_t)d) x += y;
-    }
-    if (lane == 31) warp_sums[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-        uint64_t w = lane < blockDim.x / 32 ? warp_sums[lane] : 0;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            uint64_t y = __shfl_up_sync(0xffffffffu, w, d);
-            if (lane >= (uint32_t)d) w += y;
-        }
-        warp_sums[lane] = w;
-    }
-    __syncthreads();
-    uint64_t before = warp ? warp_sums[warp - 1] : 0;
-    if (total) *total = warp_sums[blockDim.x / 32 - 1];
-    return before + x - v;
-}
-
-__global__ void k_scan_tiles(const uint64_t *__restrict__ in, uint64_t *__restrict__ out, uint64_t n,
-                             uint64_t *__restrict__ tile_sums) {
-    __shared__ uint64_t warp_sums[32];
-    uint64_t base = blockIdx.x * (uint64_t)SCAN_TILE + threadIdx.x * (uint64_t)SCAN_ITEMS;
-    uint64_t v[SCAN_ITEMS], sum = 0;
-#pragma unroll
-    for (int k = 0; k < SCAN_ITEMS; ++k) {
-        v[k] = base + k < n ? in[base + k] : 0;
-        sum += v[k];
-    }
-    uint64_t total;
-    uint64_t run = block_exclusive_scan(sum, warp_sums, &total);
-#pragma unroll
-    for (int k = 0; k < SCAN_ITEMS; ++k) {
-        if (base + k < n) out[base + k] = run;
-        run += v[k];
-    }
-    if (threadIdx.x == 0) tile_sums[blockIdx.x] = total;
-}
-
-__global__ void k_scan_add(uint64_t *__restrict__ out, uint64_t n, const uint64_t *__restrict__ offsets) {
-    uint64_t i = blockIdx.x * (uint64_t)SCAN_TILE + threadIdx.x;
-    uint64_t add = offsets[blockIdx.x];
-    for (int k = 0; k < SCAN_ITEMS; ++k, i += SCAN_T)
-        if (i < n) out[i] += add;
-}
-
-// Words of scratch the scan of n values needs (two arrays of tile sums per level).
-uint64_t pc_scan_workspace(uint64_t n) {
-    uint64_t words = 0;
-    for (;;) {
-        const uint64_t tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
-        words += 2 * (tiles + 1);
-        if (tiles <= 1) return words;
-        n = tiles;
-    }
-}
-
-// out[i] = sum in[0..i); *total_dev = sum of all (device pointer, may be null).  in may alias out.
-// ws holds pc_scan_workspace(n) words; nothing is allocated and nothing waits for the device, so
-// the scan can be recorded into a CUDA graph.
-int pc_exclusive_scan_ws(pc_ctx *ctx, const uint64_t *in, uint64_t *out, uint64_t n, uint64_t *total_dev,
-                         uint64_t *ws) {
-    if (n == 0) {
-        if (total_dev) PC_CHECK(ctx, cudaMemsetAsync(total_dev, 0, 8, ctx->stream));
-        return PC_OK;
-    }
-    const uint64_t tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
-    uint64_t *sums = ws, *sums_scan = ws + tiles + 1;
-    k_scan_tiles<<<(unsigned)tiles, SCAN_T, 0, ctx->stream>>>(in, out, n, sums);
-    PC_LAUNCHED(ctx, "scan tiles");
-    if (tiles > 1) {
-        int rc = pc_exclusive_scan_ws(ctx, sums, sums_scan, tiles, total_dev, ws + 2 * (tiles + 1));
-        if (rc) return rc;
-        k_scan_add<<<(unsigned)tiles, SCAN_T, 0, ctx->stream>>>(out, n, sums_scan);
-        PC_LAUNCHED(ctx, "scan add");
-    } else if (total_dev) {
-        PC_CHECK(ctx, cudaMemcpyAsync(total_dev, sums, 8, cudaMemcpyDeviceToDevice, ctx->stream));
-    }
+    if (stage) memcpy(positions, stage, n * 8);
     return PC_OK;
 }
 

@@ -465,85 +465,125 @@ __global__ void __launch_bounds__(PREP_T) k_vprep(const PrepArgs a) {
 }
 
 // Per subtile: u count and v count of its envelope (searchsorted bounds of
-// batch_experiment.py:37-43, as list-independent differences).
-__global__ void k_geometry(const uint64_t *__restrict__ us, const uint64_t *__restrict__ vs, const SegDev *__restrict__ seg,
-                           const uint32_t *__restrict__ tile_seg, uint64_t ntiles, uint64_t *__restrict__ geometry) {
-    const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (t >= ntiles) return;
+// batch_experiment.py:37-43, as list-independent differences).  A warp per subtile, eight lanes per bound.  Bound:
+// the latency of the searches' dependent loads (a thread per subtile with four searches in turn: 13 us for a
+// batch, now 5 us; 37 us for a lease's 16,384 subtiles either way).
+__global__ void __launch_bounds__(256) k_geometry(const uint64_t *__restrict__ us, const uint64_t *__restrict__ vs,
+                                                  const SegDev *__restrict__ seg, const uint32_t *__restrict__ tile_seg,
+                                                  uint64_t ntiles, uint64_t *__restrict__ geometry) {
+    const uint32_t lane = threadIdx.x & 31, which = lane >> 3;
+    const uint64_t t = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+    if (t >= ntiles) return;                              // warp-uniform
     const SegDev &g = seg[tile_seg[t]];
     const uint64_t first = g.v_first + (t - g.tile_base) * g.width;
     const uint64_t end = umin64(first + g.width, g.v_end);
     const uint64_t *su = us + g.u_off, *sv = vs + g.v_off;
-    const uint64_t ua = count_le(su, g.nu, g.B, add128(mul_wide(first, g.A), g.lo));
-    const uint64_t ub = count_le(su, g.nu, g.B, add128(mul_wide(end - 1, g.A), g.hi));
-    const uint64_t va = lower_bound64(sv, g.nv, first), vb = lower_bound64(sv, g.nv, end);
-    geometry[2 * t] = ub > ua ? ub - ua : 0;
-    geometry[2 * t + 1] = vb - va;
+    // groups 0 and 1: u B <= first A + lo, (end - 1) A + hi; groups 2 and 3: v < first, end
+    const u128 key = which == 0 ? add128(mul_wide(first, g.A), g.lo) : add128(mul_wide(end - 1, g.A), g.hi);
+    const uint64_t vkey = which == 2 ? first : end;
+    const uint64_t n = group_prefix(which < 2 ? g.nu : g.nv, lane, [&](uint64_t i) {
+        return which < 2 ? !less128(key, mul_wide(__ldg(su + i), g.B)) : __ldg(sv + i) < vkey;
+    });
+    const uint64_t ua = __shfl_sync(0xffffffffu, n, 0), ub = __shfl_sync(0xffffffffu, n, 8);
+    const uint64_t va = __shfl_sync(0xffffffffu, n, 16), vb = __shfl_sync(0xffffffffu, n, 24);
+    if (lane == 0) {
+        geometry[2 * t] = ub > ua ? ub - ua : 0;
+        geometry[2 * t + 1] = vb - va;
+    }
 }
 
 // Per u block of UB entries: [va, vb) of v rows whose [left, right) meets the block, and the
 // sub-range [f0, f1) of rows covering the whole block (left <= start and right >= stop); left and
-// right are monotone in the row index within a segment, so all four are binary searches.
-__device__ __forceinline__ uint64_t first_right_ge(const VRec *__restrict__ rec, uint64_t lo, uint64_t hi, uint64_t x) {
-    while (lo < hi) {
-        uint64_t mid = lo + (hi - lo) / 2;
-        if (rec[mid].right >= x) hi = mid;
-        else lo = mid + 1;
+// right are monotone in the row index within a segment, so all four are searches: a warp per block, eight lanes
+// each (a thread per block with four searches in turn: 24 us for a batch, 57 us for a lease; now 5 and 18 us).
+// The blocks' rows are also summed (the pieces from which k_items sizes work items).
+__global__ void __launch_bounds__(256) k_blocks(const VRec *__restrict__ rec, const SegDev *__restrict__ seg, uint32_t nseg,
+                                                uint32_t UB, uint64_t nblocks, uint4 *__restrict__ bv,
+                                                uint32_t *__restrict__ blk_seg, unsigned long long *__restrict__ pieces) {
+    __shared__ unsigned long long sum_s;
+    if (threadIdx.x == 0) sum_s = 0;
+    __syncthreads();
+    const uint32_t lane = threadIdx.x & 31, which = lane >> 3;
+    const uint64_t b = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+    if (b < nblocks) {                                    // warp-uniform
+        const uint64_t start = b * UB;
+        const uint32_t s = seg_of_u(seg, nseg, start);
+        const SegDev &g = seg[s];
+        const uint64_t u_end = (uint64_t)g.u_off + g.nu;
+        uint4 range = make_uint4(0, 0, 0, 0);             // also for the padding between segments
+        if (start < u_end) {
+            const uint64_t stop = umin64(u_end, start + UB);
+            // groups: va (right > start), vb (left >= stop), f0 (right >= stop), f1 (left > start)
+            const uint64_t x = which == 0 || which == 3 ? start + 1 : stop;
+            const uint32_t n = (uint32_t)group_prefix(g.nv, lane, [&](uint64_t i) {
+                const VRec &r = rec[g.v_off + i];
+                return (which & 1 ? r.left : r.right) < x;
+            });
+            const uint32_t va = __shfl_sync(0xffffffffu, n, 0), vb = max(va, __shfl_sync(0xffffffffu, n, 8));
+            const uint32_t f0 = min(max(__shfl_sync(0xffffffffu, n, 16), va), vb), f1 = min(__shfl_sync(0xffffffffu, n, 24), vb);
+            range = make_uint4(g.v_off + va, g.v_off + vb, g.v_off + f0, g.v_off + max(f0, f1));
+        }
+        if (lane == 0) {
+            bv[b] = range;
+            blk_seg[b] = s;
+            if (range.y != range.x) atomicAdd(&sum_s, (unsigned long long)(range.y - range.x));
+        }
     }
-    return lo;
-}
-
-__device__ __forceinline__ uint64_t first_left_ge(const VRec *__restrict__ rec, uint64_t lo, uint64_t hi, uint64_t x) {
-    while (lo < hi) {
-        uint64_t mid = lo + (hi - lo) / 2;
-        if (rec[mid].left >= x) hi = mid;
-        else lo = mid + 1;
-    }
-    return lo;
-}
-
-__global__ void k_blocks(const VRec *__restrict__ rec, const SegDev *__restrict__ seg, uint32_t nseg, uint32_t UB,
-                         uint64_t nblocks, uint4 *__restrict__ bv, uint32_t *__restrict__ blk_seg,
-                         uint64_t *__restrict__ pieces) {
-    const uint64_t b = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (b >= nblocks) return;
-    const uint64_t start = b * UB;
-    const uint32_t s = seg_of_u(seg, nseg, start);
-    const SegDev &g = seg[s];
-    const uint64_t u_end = (uint64_t)g.u_off + g.nu;
-    blk_seg[b] = s;
-    if (start >= u_end) {                                 // padding between segments
-        bv[b] = make_uint4(0, 0, 0, 0);
-        pieces[b] = 0;
-        return;
-    }
-    const uint64_t stop = umin64(u_end, start + UB);
-    const uint64_t r0 = g.v_off, r1 = r0 + g.nv;
-    const uint64_t va = first_right_ge(rec, r0, r1, start + 1);
-    const uint64_t vb = first_left_ge(rec, va, r1, stop);
-    uint64_t f0 = umax64(va, first_right_ge(rec, va, vb, stop));
-    uint64_t f1 = umin64(vb, first_left_ge(rec, va, vb, start + 1));
-    if (f1 < f0) f1 = f0;
-    bv[b] = make_uint4((uint32_t)va, (uint32_t)vb, (uint32_t)f0, (uint32_t)f1);
-    pieces[b] = vb > va ? vb - va : 0;
+    __syncthreads();
+    if (threadIdx.x == 0 && sum_s) atomicAdd(pieces, sum_s);
 }
 
 // v chunk per work item: fixed, or total pieces / target items, at least min_chunk (four rounds of
 // 32 rows for every warp of a k_match CTA, so a small launch keeps every warp busy and pays the
-// per-item set-up over enough rows) and at most 2^20.
-__global__ void k_chunk(const uint64_t *__restrict__ total_pieces, uint64_t fixed_chunk, uint64_t target_items,
-                        uint64_t min_chunk, uint64_t *__restrict__ vchunk) {
-    uint64_t c = fixed_chunk;
-    if (!c) c = umax64((*total_pieces + target_items - 1) / umax64(1, target_items), min_chunk);
-    *vchunk = umin64(c, UINT64_C(1) << 20);
-}
+// per-item set-up over enough rows) and at most 2^20; and the items before each block (prefix[nblocks]: all).
+// One CTA: a lease has 1e4 blocks, two turns of 8,192.
+constexpr uint32_t ITEMS_T = 1024, ITEMS_PER = 8;
 
-__global__ void k_item_counts(const uint64_t *__restrict__ pieces, uint64_t nblocks,
-                              const uint64_t *__restrict__ vchunk, uint64_t *__restrict__ items) {
-    uint64_t b = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (b >= nblocks) return;
-    uint64_t c = *vchunk;
-    items[b] = (pieces[b] + c - 1) / c;
+__global__ void __launch_bounds__(ITEMS_T) k_items(const uint4 *__restrict__ bv, uint64_t nblocks,
+                                                   const unsigned long long *__restrict__ pieces, uint64_t fixed_chunk,
+                                                   uint64_t target_items, uint64_t min_chunk, uint64_t *__restrict__ vchunk,
+                                                   uint64_t *__restrict__ prefix) {
+    __shared__ uint64_t warp_s[ITEMS_T / 32];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint64_t c = fixed_chunk;
+    if (!c) c = umax64((*pieces + target_items - 1) / umax64(1, target_items), min_chunk);
+    c = umin64(c, UINT64_C(1) << 20);
+    if (threadIdx.x == 0) *vchunk = c;
+    uint64_t before = 0;                                  // items of the blocks of earlier turns
+    for (uint64_t base = 0; base < nblocks; base += ITEMS_T * ITEMS_PER) {
+        const uint64_t b0 = base + threadIdx.x * ITEMS_PER;
+        uint32_t items[ITEMS_PER];
+        uint64_t own = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < ITEMS_PER; ++k) {
+            items[k] = 0;
+            if (b0 + k < nblocks) {
+                const uint4 r = bv[b0 + k];
+                items[k] = (r.y - r.x + (uint32_t)c - 1) / (uint32_t)c;
+            }
+            own += items[k];
+        }
+        uint64_t incl = own;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint64_t y = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= (uint32_t)d) incl += y;
+        }
+        __syncthreads();                                  // the previous turn's sums have been read
+        if (lane == 31) warp_s[warp] = incl;
+        __syncthreads();
+        uint64_t at = before + incl - own;
+        for (uint32_t w = 0; w < ITEMS_T / 32; ++w) {
+            if (w < warp) at += warp_s[w];
+            before += warp_s[w];
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < ITEMS_PER; ++k) {
+            if (b0 + k < nblocks) prefix[b0 + k] = at;
+            at += items[k];
+        }
+    }
+    if (threadIdx.x == 0) prefix[nblocks] = before;
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1050,11 +1090,14 @@ __device__ __forceinline__ uint32_t mod_limbs(const uint32_t h[6], const FiltC &
 }
 
 // Exact later filters on every deep record: x = uB - vA in two 64-bit limbs, filters first..nres-1
-// of the record's family with group counters, then the output record.  One record per thread;
-// outputs are appended with one atomic per warp.
+// of the record's family with group counters, then the output record.  A lane tests the next DEEP_ALONE
+// filters on its own record; the few records that pass them (1 in 6,000 where each keeps a third) are then
+// tested one by one by the whole warp, a filter per lane, so none waits for eighty dependent table loads (a lane
+// per record to the end: 32 us for a batch, most of it one record's chain; now 8 us).
+constexpr uint32_t DEEP_ALONE = 8;
+
 __global__ void __launch_bounds__(256) k_deep(const DeepArgs a) {
     const uint32_t lane = threadIdx.x & 31;
-    const uint32_t lanes_below = (1u << lane) - 1u;
     const uint32_t slice = blockIdx.y;
     const uint32_t count = min(a.deep_count[slice], a.deep_cap);
     for (uint32_t base = blockIdx.x * blockDim.x; base < count; base += gridDim.x * blockDim.x) {
@@ -1062,55 +1105,70 @@ __global__ void __launch_bounds__(256) k_deep(const DeepArgs a) {
         const uint64_t i = (uint64_t)slice * a.deep_cap + at;
         bool pass = false;
         u128 x{0, 0};
-        uint64_t tile = 0;
-        uint32_t ng = 0;
+        uint32_t tile = 0, fam = 0;
+        auto limbs = [](const u128 &y, uint32_t (&h)[6]) {
+            h[0] = (uint32_t)y.lo & 0xffffu, h[1] = (uint32_t)(y.lo >> 16) & 0xffffu;
+            h[2] = (uint32_t)(y.lo >> 32) & 0xffffu, h[3] = (uint32_t)(y.lo >> 48);
+            h[4] = (uint32_t)y.hi & 0xffffu, h[5] = (uint32_t)(y.hi >> 16) & 0xffffu;
+        };
+        auto allowed = [](const FamDev &F, uint32_t idx, const uint32_t (&h)[6]) {
+            const FiltC f = F.fcs[idx];
+            const uint32_t m = mod_limbs(h, f);
+            return (__ldg(F.bits + f.tab_off + (m >> 5)) >> (m & 31)) & 1u;
+        };
         if (at < count) {
             const uint4 r = a.deep[i];
             const uint64_t v = (uint64_t)r.y << 32 | r.x;
             tile = r.w;
             if (tile < a.ntiles) {
                 const SegDev &g = a.seg[a.tile_seg[tile]];
-                const FamDev &F = a.fam[g.fam];
-                ng = F.ng;
+                fam = g.fam;
+                const FamDev &F = a.fam[fam];
                 const u128 pos = mul_wide(__ldg(a.us + r.z), g.B), shift = mul_wide(v, g.A);
                 if (less128(pos, shift)) {
-                    atomicAdd((unsigned long long *)&a.counts[tile * a.stride + ng + 2], 1ull);
+                    atomicAdd((unsigned long long *)&a.counts[(uint64_t)tile * a.stride + F.ng + 2], 1ull);
                 } else {
                     x = sub128(pos, shift);
-                    const uint32_t h[6] = {(uint32_t)x.lo & 0xffffu, (uint32_t)(x.lo >> 16) & 0xffffu,
-                                           (uint32_t)(x.lo >> 32) & 0xffffu, (uint32_t)(x.lo >> 48),
-                                           (uint32_t)x.hi & 0xffffu, (uint32_t)(x.hi >> 16) & 0xffffu};
+                    uint32_t h[6];
+                    limbs(x, h);
                     pass = true;
-                    const uint32_t nres = F.nres;
-                    const FiltC *fcs = F.fcs;
-                    const uint32_t *bits = F.bits;
-                    for (uint32_t idx = a.first; idx < nres; ++idx) {
-                        const FiltC f = fcs[idx];
-                        const uint32_t m = mod_limbs(h, f);
-                        if (!((__ldg(bits + f.tab_off + (m >> 5)) >> (m & 31)) & 1u)) {
+                    const uint32_t stop = min(F.nres, a.first + DEEP_ALONE);
+                    for (uint32_t idx = a.first; idx < stop; ++idx) {
+                        if (!allowed(F, idx, h)) {
                             pass = false;
                             break;
                         }
-                        if ((idx & 3) == 3 || idx + 1 == nres)
-                            atomicAdd((unsigned long long *)&a.counts[tile * a.stride + idx / 4 + 1], 1ull);
+                        if ((idx & 3) == 3 || idx + 1 == F.nres)
+                            atomicAdd((unsigned long long *)&a.counts[(uint64_t)tile * a.stride + idx / 4 + 1], 1ull);
                     }
                 }
             }
         }
-        const uint32_t won = __ballot_sync(0xffffffffu, pass);
-        if (won) {
-            const uint32_t leader = __ffs(won) - 1;
-            unsigned long long first = 0;
-            if (lane == leader) first = atomicAdd(a.n_out, (unsigned long long)__popc(won));
-            first = __shfl_sync(0xffffffffu, first, leader);
-            if (pass) {
-                const uint32_t same = __match_any_sync(won, tile);
-                if (lane == (uint32_t)(__ffs(same) - 1))
-                    atomicAdd((unsigned long long *)&a.counts[tile * a.stride + ng + 1], (unsigned long long)__popc(same));
-                const unsigned long long o = first + __popc(won & lanes_below);
+        for (uint32_t left = __ballot_sync(0xffffffffu, pass); left; left &= left - 1) {
+            const uint32_t src = __ffs(left) - 1;
+            const u128 y{__shfl_sync(0xffffffffu, x.lo, src), __shfl_sync(0xffffffffu, x.hi, src)};
+            const uint64_t t = __shfl_sync(0xffffffffu, tile, src);
+            const FamDev &F = a.fam[__shfl_sync(0xffffffffu, fam, src)];
+            uint64_t *counts = a.counts + t * a.stride;
+            uint32_t h[6];
+            limbs(y, h);
+            const uint32_t nres = F.nres;
+            bool ok = true;
+            for (uint32_t idx0 = a.first + DEEP_ALONE; ok && idx0 < nres; idx0 += 32) {
+                const uint32_t idx = idx0 + lane;
+                const bool fails = idx < nres && !allowed(F, idx, h);
+                const uint32_t failed = __ballot_sync(0xffffffffu, fails);
+                const uint32_t until = failed ? idx0 + __ffs(failed) - 1 : idx0 + 32;    // filters below it have passed
+                if (idx < until && ((idx & 3) == 3 || idx + 1 == nres) && idx < nres)
+                    atomicAdd((unsigned long long *)&counts[idx / 4 + 1], 1ull);
+                ok = !failed;
+            }
+            if (ok && lane == 0) {
+                atomicAdd((unsigned long long *)&counts[F.ng + 1], 1ull);
+                const unsigned long long o = atomicAdd(a.n_out, 1ull);
                 if (o < a.out_cap) {
-                    a.out[2 * o] = x.lo;
-                    a.out[2 * o + 1] = x.hi | (tile << 32);
+                    a.out[2 * o] = y.lo;
+                    a.out[2 * o + 1] = y.hi | (t << 32);
                 }
             }
         }
@@ -1567,17 +1625,25 @@ struct Engine {
     FamPrep *d_famp = nullptr;
     std::vector<SegPrep> segprep;
     std::vector<FamPrep> famprep;
-    uint32_t *d_tile_seg = nullptr, *d_blk_seg = nullptr, *d_deep_count = nullptr;
-    unsigned long long *d_item_next = nullptr;
-    uint64_t *d_counts = nullptr, *d_geo = nullptr, *d_out = nullptr;
-    unsigned long long *d_nout = nullptr;                 // [0] outputs, [1] rows outside the geometry, [2] window pass gave up
-    bool windows = false;                                 // the lists come from an emitting pass that reports in d_nout[2]
-    uint64_t nout_bytes() const { return windows ? 24 : 16; }
+    std::vector<unsigned char> upload;                    // the descriptors as copied to the device
+    uint32_t *d_tile_seg = nullptr, *d_blk_seg = nullptr;
     VRec *d_rec = nullptr;
     uint64_t *d_cres = nullptr;
     uint4 *d_bv = nullptr;
-    uint64_t *d_pieces = nullptr, *d_tmp = nullptr, *d_items = nullptr, *d_prefix = nullptr, *d_vchunk = nullptr;
-    uint64_t *d_ws = nullptr;
+    uint64_t *d_prefix = nullptr;
+    // Everything a run reports lies together, in this order, so that one fill resets it and one copy fetches it:
+    // scalars, deep survivors per CTA, counters, envelopes, output records.
+    enum { STUCK, NOUT, BAD, ITEM_NEXT, PIECES, VCHUNK, SCALARS = 8 };    // STUCK: the window pass gave up
+    bool windows = false;                                 // the window pass is the owner's: STUCK is not reset
+    uint64_t *d_report = nullptr;
+    uint64_t o_deep = 0, o_counts = 0, o_geo = 0, o_out = 0;   // word offsets
+    unsigned long long *scalar(int k) const { return (unsigned long long *)d_report + k; }
+    uint32_t *d_deep_count() const { return (uint32_t *)(d_report + o_deep); }
+    uint64_t *d_counts() const { return d_report + o_counts; }
+    uint64_t *d_geo() const { return d_report + o_geo; }
+    uint64_t *d_out() const { return d_report + o_out; }
+    uint64_t fetch_words() const { return o_out + 2 * std::min<uint64_t>(out_cap, FETCH_RECORDS); }
+    static constexpr uint64_t FETCH_RECORDS = 256;        // output records fetched with the counters
     uint4 *d_deep = nullptr;
     uint64_t deep_bytes = 0;
     ~Engine() {
@@ -1617,35 +1683,37 @@ int engine_prepare(Engine &E, const pc_tuning *tuning, Scratch &hold) {
     const uint32_t UB = E.tn.K * 32;
     E.nblocks = (E.nu + UB - 1) / UB;
     const uint64_t nb1 = std::max<uint64_t>(1, E.nblocks);
-    rc = hold.get(&E.d_seg, E.segs.size());
-    if (!rc) rc = hold.get(&E.d_fam, E.famdev.size());
-    if (!rc) rc = hold.get(&E.d_segp, E.segs.size());
-    if (!rc) rc = hold.get(&E.d_famp, E.famdev.size());
-    if (!rc) rc = hold.get(&E.d_tile_seg, std::max<uint64_t>(1, E.ntiles));
-    if (!rc) rc = hold.get(&E.d_counts, std::max<uint64_t>(1, E.ntiles * E.stride));
-    if (!rc) rc = hold.get(&E.d_geo, std::max<uint64_t>(1, 2 * E.ntiles));
-    if (!rc) rc = hold.get(&E.d_out, 2 * std::max<uint64_t>(1, E.out_cap));
-    if (!rc) rc = hold.get(&E.d_nout, 3);
-    if (!rc) rc = hold.get(&E.d_rec, std::max<uint64_t>(1, E.nv));
-    if (!rc) rc = hold.get(&E.d_cres, std::max<uint64_t>(1, E.nv));
-    if (!rc) rc = hold.get(&E.d_bv, nb1);
-    if (!rc) rc = hold.get(&E.d_blk_seg, nb1);
-    if (!rc) rc = hold.get(&E.d_pieces, nb1);
-    if (!rc) rc = hold.get(&E.d_tmp, E.nblocks + 1);
-    if (!rc) rc = hold.get(&E.d_items, nb1);
-    if (!rc) rc = hold.get(&E.d_prefix, E.nblocks + 1);
-    if (!rc) rc = hold.get(&E.d_vchunk, 1);
-    if (!rc) rc = hold.get(&E.d_ws, pc_scan_workspace(E.nblocks));
-    if (!rc) rc = hold.get(&E.d_deep_count, E.grid);
-    if (!rc) rc = hold.get(&E.d_item_next, 1);
+    E.o_deep = Engine::SCALARS;
+    E.o_counts = E.o_deep + (E.grid + 1) / 2;
+    E.o_geo = E.o_counts + E.ntiles * E.stride;
+    E.o_out = E.o_geo + 2 * E.ntiles;
+    // one allocation for the descriptors (one upload) and one for the scratch
+    Carve in, work;
+    in.add(&E.d_seg, E.segs.size());
+    in.add(&E.d_fam, E.famdev.size());
+    in.add(&E.d_segp, E.segs.size());
+    in.add(&E.d_famp, E.famdev.size());
+    in.add(&E.d_tile_seg, std::max<uint64_t>(1, E.ntiles));
+    work.add(&E.d_report, E.o_out + 2 * std::max<uint64_t>(1, E.out_cap));
+    work.add(&E.d_rec, std::max<uint64_t>(1, E.nv));
+    work.add(&E.d_cres, std::max<uint64_t>(1, E.nv));
+    work.add(&E.d_bv, nb1);
+    work.add(&E.d_blk_seg, nb1);
+    work.add(&E.d_prefix, E.nblocks + 1);
+    rc = in.get(hold);
+    if (!rc) rc = work.get(hold);
     if (!rc) rc = engine_deep_alloc(E, E.deep_cap);
     if (rc) return rc;
-    PC_CHECK(ctx, pc_copy(ctx, E.d_seg, E.segs.data(), E.segs.size() * sizeof(SegDev), cudaMemcpyHostToDevice));
-    PC_CHECK(ctx, pc_copy(ctx, E.d_fam, E.famdev.data(), E.famdev.size() * sizeof(FamDev), cudaMemcpyHostToDevice));
-    PC_CHECK(ctx, pc_copy(ctx, E.d_segp, E.segprep.data(), E.segprep.size() * sizeof(SegPrep), cudaMemcpyHostToDevice));
-    PC_CHECK(ctx, pc_copy(ctx, E.d_famp, E.famprep.data(), E.famprep.size() * sizeof(FamPrep), cudaMemcpyHostToDevice));
-    if (E.ntiles)
-        PC_CHECK(ctx, pc_copy(ctx, E.d_tile_seg, E.tile_seg.data(), E.ntiles * 4, cudaMemcpyHostToDevice));
+    E.upload.resize(in.bytes);
+    auto put = [&](const void *dev, const void *src, uint64_t bytes) {
+        memcpy(E.upload.data() + ((const unsigned char *)dev - (const unsigned char *)E.d_seg), src, bytes);
+    };
+    put(E.d_seg, E.segs.data(), E.segs.size() * sizeof(SegDev));
+    put(E.d_fam, E.famdev.data(), E.famdev.size() * sizeof(FamDev));
+    put(E.d_segp, E.segprep.data(), E.segprep.size() * sizeof(SegPrep));
+    put(E.d_famp, E.famprep.data(), E.famprep.size() * sizeof(FamPrep));
+    put(E.d_tile_seg, E.tile_seg.data(), E.ntiles * 4);
+    PC_CHECK(ctx, pc_copy(ctx, E.d_seg, E.upload.data(), in.bytes, cudaMemcpyHostToDevice));
     return PC_OK;
 }
 
@@ -1664,29 +1732,28 @@ int engine_match(Engine &E, int mode) {
     ma.stride = E.stride;
     ma.total_rows = 0;
     for (const FamDev &d : E.famdev) ma.total_rows = std::max(ma.total_rows, d.total_rows);
-    ma.counts = E.d_counts;
+    ma.counts = E.d_counts();
     ma.bv = E.d_bv;
     ma.item_prefix = E.d_prefix;
     ma.nblocks = E.nblocks;
-    ma.vchunk = E.d_vchunk;
+    ma.vchunk = E.d_report + Engine::VCHUNK;
     ma.deep = E.d_deep;
     ma.deep_cap = E.deep_cap;
-    ma.deep_count = E.d_deep_count;
-    ma.item_next = E.d_item_next;
+    ma.deep_count = E.d_deep_count();
+    ma.item_next = E.scalar(Engine::ITEM_NEXT);
     if (E.tn.threads == 1024) return launch_match_n<1024>(E.ctx, ma, E.tn.nb, E.tn.K, E.smem, E.grid, mode);
     if (E.tn.threads == 896) return launch_match_n<896>(E.ctx, ma, E.tn.nb, E.tn.K, E.smem, E.grid, mode);
     if (E.tn.threads == 768) return launch_match_n<768>(E.ctx, ma, E.tn.nb, E.tn.K, E.smem, E.grid, mode);
     return launch_match_n<512>(E.ctx, ma, E.tn.nb, E.tn.K, E.smem, E.grid, mode);
 }
 
-// Counters reset, per-v bounds, subtile envelopes, block ranges, work items and the fused match.
-int engine_front(Engine &E, bool events, bool capturing, int *launches) {
+// Counters reset, per-v bounds, subtile envelopes, block ranges, work items, the fused match and the exact
+// later filters on its deep survivors (as many as the slices hold).  Nothing waits for the device.
+int engine_launch(Engine &E, bool events, bool capturing, int *launches) {
     pc_ctx *ctx = E.ctx;
     cudaStream_t st = ctx->stream;
-    if (E.ntiles) PC_CHECK(ctx, cudaMemsetAsync(E.d_counts, 0, E.ntiles * E.stride * 8, st));
-    PC_CHECK(ctx, cudaMemsetAsync(E.d_nout, 0, 16, st));
-    PC_CHECK(ctx, cudaMemsetAsync(E.d_deep_count, 0, (uint64_t)E.grid * 4, st));
-    PC_CHECK(ctx, cudaMemsetAsync(E.d_item_next, 0, 8, st));
+    const uint64_t from = E.windows ? Engine::NOUT : Engine::STUCK;
+    PC_CHECK(ctx, cudaMemsetAsync(E.d_report + from, 0, (E.o_geo - from) * 8, st));
     if (events) PC_CHECK(ctx, cudaEventRecord(ctx->ev[0], st));
     if (E.nv) {
         PrepArgs pa{};
@@ -1702,8 +1769,8 @@ int engine_front(Engine &E, bool events, bool capturing, int *launches) {
         pa.rec = E.d_rec;
         pa.cres = E.d_cres;
         pa.nch = E.tn.nch;
-        pa.counts = E.d_counts;
-        pa.bad = E.d_nout + 1;
+        pa.counts = E.d_counts();
+        pa.bad = E.scalar(Engine::BAD);
         // 8 or 4 rows per thread share a CTA's end searches where that still leaves every SM that many CTAs and
         // most CTAs lie in one segment; else one (a lease's 1.6e7 rows: 0.41 ms at 8, 0.44 at 4; 24 batches'
         // 1.5e6 rows: 54 us at 8, 47 at 4)
@@ -1718,41 +1785,25 @@ int engine_front(Engine &E, bool events, bool capturing, int *launches) {
         ++*launches;
     }
     if (E.ntiles) {
-        k_geometry<<<(unsigned)((E.ntiles + 127) / 128), 128, 0, st>>>(E.us, E.vs, E.d_seg, E.d_tile_seg, E.ntiles, E.d_geo);
+        k_geometry<<<(unsigned)((E.ntiles + 7) / 8), 256, 0, st>>>(E.us, E.vs, E.d_seg, E.d_tile_seg, E.ntiles, E.d_geo());
         PC_LAUNCHED(ctx, "geometry");
         ++*launches;
     }
     if (events) PC_CHECK(ctx, cudaEventRecord(ctx->ev[1], st));
-    if (!E.nu || !E.nv) return PC_OK;
-    const uint32_t UB = E.tn.K * 32;
-    k_blocks<<<(unsigned)((E.nblocks + 255) / 256), 256, 0, st>>>(E.d_rec, E.d_seg, (uint32_t)E.segs.size(), UB,
-                                                                 E.nblocks, E.d_bv, E.d_blk_seg, E.d_pieces);
-    PC_LAUNCHED(ctx, "blocks");
-    int rc = pc_exclusive_scan_ws(ctx, E.d_pieces, E.d_tmp, E.nblocks, E.d_tmp + E.nblocks, E.d_ws);
-    if (rc) return rc;
-    k_chunk<<<1, 1, 0, st>>>(E.d_tmp + E.nblocks, E.tn.v_chunk, (uint64_t)E.grid * 32, 4 * (uint64_t)E.tn.threads,
-                             E.d_vchunk);
-    PC_LAUNCHED(ctx, "chunk");
-    k_item_counts<<<(unsigned)((E.nblocks + 255) / 256), 256, 0, st>>>(E.d_pieces, E.nblocks, E.d_vchunk, E.d_items);
-    PC_LAUNCHED(ctx, "item counts");
-    rc = pc_exclusive_scan_ws(ctx, E.d_items, E.d_prefix, E.nblocks, E.d_prefix + E.nblocks, E.d_ws);
-    if (rc) return rc;
-    *launches += 7;
-    if (events) PC_CHECK(ctx, cudaEventRecord(ctx->ev[2], st));
-    rc = engine_match(E, capturing ? 1 : 0);
-    if (rc) return rc;
-    ++*launches;
-    return PC_OK;
-}
-
-// The exact later filters on the deep survivors.
-int engine_back(Engine &E, bool events, int *launches) {
-    pc_ctx *ctx = E.ctx;
-    if (E.nu && E.nv && E.deep_max) {
+    if (E.nu && E.nv) {
+        k_blocks<<<(unsigned)((E.nblocks + 7) / 8), 256, 0, st>>>(E.d_rec, E.d_seg, (uint32_t)E.segs.size(), E.tn.K * 32,
+                                                                E.nblocks, E.d_bv, E.d_blk_seg, E.scalar(Engine::PIECES));
+        PC_LAUNCHED(ctx, "blocks");
+        k_items<<<1, ITEMS_T, 0, st>>>(E.d_bv, E.nblocks, E.scalar(Engine::PIECES), E.tn.v_chunk, (uint64_t)E.grid * 32,
+                                       4 * (uint64_t)E.tn.threads, E.d_report + Engine::VCHUNK, E.d_prefix);
+        PC_LAUNCHED(ctx, "items");
+        if (events) PC_CHECK(ctx, cudaEventRecord(ctx->ev[2], st));
+        const int rc = engine_match(E, capturing ? 1 : 0);
+        if (rc) return rc;
         DeepArgs da{};
         da.us = E.us;
         da.deep = E.d_deep;
-        da.deep_count = E.d_deep_count;
+        da.deep_count = E.d_deep_count();
         da.deep_cap = E.deep_cap;
         da.first = E.tn.nb + E.tn.nch;
         da.stride = E.stride;
@@ -1760,49 +1811,31 @@ int engine_back(Engine &E, bool events, int *launches) {
         da.seg = E.d_seg;
         da.fam = E.d_fam;
         da.tile_seg = E.d_tile_seg;
-        da.counts = E.d_counts;
-        da.out = E.d_out;
+        da.counts = E.d_counts();
+        da.out = E.d_out();
         da.out_cap = E.out_cap;
-        da.n_out = E.d_nout;
-        dim3 dg((unsigned)std::min<uint64_t>((E.deep_max + 255) / 256, 64), (unsigned)E.grid);
-        k_deep<<<dg, 256, 0, ctx->stream>>>(da);
+        da.n_out = E.scalar(Engine::NOUT);
+        k_deep<<<dim3(std::min<uint32_t>((E.deep_cap + 255) / 256, 8), (unsigned)E.grid), 256, 0, st>>>(da);
         PC_LAUNCHED(ctx, "deep");
-        ++*launches;
+        *launches += 4;
     }
-    if (events) PC_CHECK(ctx, cudaEventRecord(ctx->ev[3], ctx->stream));
+    if (events) PC_CHECK(ctx, cudaEventRecord(ctx->ev[3], st));
     return PC_OK;
 }
 
-// Eager run: the match, the deep-survivor counts on the host (a rerun with room for every deep
-// survivor when a slice overflowed), then the deep tier.
-int engine_eager(Engine &E, int *launches) {
-    pc_ctx *ctx = E.ctx;
-    for (int attempt = 0;; ++attempt) {
-        int rc = engine_front(E, true, false, launches);
-        if (rc) return rc;
-        E.deep_max = 0;
-        if (E.nu && E.nv) {
-            std::vector<uint32_t> deep_counts(E.grid);
-            PC_CHECK(ctx, pc_copy(ctx, deep_counts.data(), E.d_deep_count, (uint64_t)E.grid * 4, cudaMemcpyDeviceToHost));
-            PC_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
-            for (uint32_t c : deep_counts) E.deep_max = std::max(E.deep_max, c);
-            if (E.deep_max > E.deep_cap) {
-                if (attempt) return pc_fail(ctx, PC_ARITHMETIC, "deep survivor count changed between attempts");
-                rc = engine_deep_alloc(E, E.deep_max + 1024);
-                if (rc) return rc;
-                continue;
-            }
-        }
-        return engine_back(E, true, launches);
-    }
-}
-
-// Results of a finished run already copied to the host: output count, rows outside the subtile
-// geometry, and the underflow counters of every subtile.
-int engine_check(Engine &E, const unsigned long long nout[3], const uint64_t *counts) {
-    if (E.windows && nout[2]) return pc_fail(E.ctx, PC_ARITHMETIC, "window pass did not finish");
-    if (nout[1]) return pc_fail(E.ctx, PC_INVALID, "v row outside the subtile geometry");
-    if (nout[0] > E.out_cap) return pc_fail(E.ctx, PC_OVERFLOW, "output overflow; attempt cannot commit");
+// A finished run's report, already on the host (head: its scalars and deep counts): whether the deep slices held
+// every survivor, whether a window pass gave up, rows outside the subtile geometry, outputs that did not fit
+// and underflows.
+int engine_check(Engine &E, const uint64_t *head, const uint64_t *counts, bool &outgrown) {
+    const uint32_t *deep = (const uint32_t *)(head + E.o_deep);
+    E.deep_max = 0;
+    if (E.nu && E.nv)
+        for (int b = 0; b < E.grid; ++b) E.deep_max = std::max(E.deep_max, deep[b]);
+    outgrown = E.deep_max > E.deep_cap;
+    if (outgrown) return PC_OK;
+    if (head[Engine::STUCK]) return pc_fail(E.ctx, PC_ARITHMETIC, "window pass did not finish");
+    if (head[Engine::BAD]) return pc_fail(E.ctx, PC_INVALID, "v row outside the subtile geometry");
+    if (head[Engine::NOUT] > E.out_cap) return pc_fail(E.ctx, PC_OVERFLOW, "output overflow; attempt cannot commit");
     for (uint64_t t = 0; t < E.ntiles; ++t) {
         const uint32_t ng = E.fams[E.segs[E.tile_seg[t]].fam]->ng;
         if (counts[t * E.stride + ng + 2]) return pc_fail(E.ctx, PC_ARITHMETIC, "unsigned underflow flagged");
@@ -1810,24 +1843,67 @@ int engine_check(Engine &E, const unsigned long long nout[3], const uint64_t *co
     return PC_OK;
 }
 
-int engine_collect(Engine &E, uint64_t *counts, uint64_t *geometry, uint64_t *out, uint64_t *n_out) {
+// The report of the run just launched: in one copy through the context's page-locked stage where it fits that
+// (a copy to pageable memory costs the host 12 us and a wait each), else straight to the caller's arrays.
+// got: the first records, which the copy brought along.
+int engine_fetch(Engine &E, uint64_t *counts, uint64_t *geometry, std::vector<uint64_t> &head, const uint64_t *&records, uint64_t &got) {
     pc_ctx *ctx = E.ctx;
-    cudaStream_t st = ctx->stream;
-    unsigned long long nout[3] = {0, 0, 0};
-    PC_CHECK(ctx, pc_copy(ctx, nout, E.d_nout, E.nout_bytes(), cudaMemcpyDeviceToHost));
-    if (E.ntiles) {
-        PC_CHECK(ctx, pc_copy(ctx, counts, E.d_counts, E.ntiles * E.stride * 8, cudaMemcpyDeviceToHost));
-        PC_CHECK(ctx, pc_copy(ctx, geometry, E.d_geo, 2 * E.ntiles * 8, cudaMemcpyDeviceToHost));
+    const uint64_t words = E.fetch_words();
+    head.resize(E.o_counts);
+    got = 0;
+    if (uint64_t *stage = pc_stage(ctx, words * 8)) {
+        PC_CHECK(ctx, pc_copy(ctx, stage, E.d_report, words * 8, cudaMemcpyDeviceToHost));
+        PC_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
+        memcpy(head.data(), stage, E.o_counts * 8);
+        if (E.ntiles) {
+            memcpy(counts, stage + E.o_counts, E.ntiles * E.stride * 8);
+            memcpy(geometry, stage + E.o_geo, 2 * E.ntiles * 8);
+        }
+        records = stage + E.o_out;
+        got = (words - E.o_out) / 2;
+        return PC_OK;
     }
-    PC_CHECK(ctx, cudaStreamSynchronize(st));
-    *n_out = nout[0];
-    int rc = engine_check(E, nout, counts);
-    if (rc) return rc;
-    if (nout[0]) {
-        PC_CHECK(ctx, pc_copy(ctx, out, E.d_out, 2 * nout[0] * 8, cudaMemcpyDeviceToHost));
-        PC_CHECK(ctx, cudaStreamSynchronize(st));
+    PC_CHECK(ctx, pc_copy(ctx, head.data(), E.d_report, E.o_counts * 8, cudaMemcpyDeviceToHost));
+    PC_CHECK(ctx, pc_copy(ctx, counts, E.d_counts(), E.ntiles * E.stride * 8, cudaMemcpyDeviceToHost));
+    PC_CHECK(ctx, pc_copy(ctx, geometry, E.d_geo(), 2 * E.ntiles * 8, cudaMemcpyDeviceToHost));
+    PC_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
+    return PC_OK;
+}
+
+// Output records 0..n-1 to out, the first `got` of them from host memory.
+int engine_records(Engine &E, const uint64_t *records, uint64_t got, uint64_t n, uint64_t *out) {
+    got = std::min(got, n);
+    if (got) memcpy(out, records, 16 * got);
+    if (n > got) {
+        PC_CHECK(E.ctx, pc_copy(E.ctx, out + 2 * got, E.d_out() + 2 * got, 16 * (n - got), cudaMemcpyDeviceToHost));
+        PC_CHECK(E.ctx, cudaStreamSynchronize(E.ctx->stream));
     }
     return PC_OK;
+}
+
+// Eager run with its results on the host; once more, with room for every deep survivor, when a slice overflowed.
+// `place` gives the array for the output records once their number is known.
+template <class F>
+int engine_run(Engine &E, uint64_t *counts, uint64_t *geometry, uint64_t *n_out, int *launches, F place) {
+    for (int attempt = 0;; ++attempt) {
+        int rc = engine_launch(E, true, false, launches);
+        std::vector<uint64_t> head;
+        const uint64_t *records = nullptr;
+        uint64_t got = 0;
+        if (!rc) rc = engine_fetch(E, counts, geometry, head, records, got);
+        if (rc) return rc;
+        bool outgrown = false;
+        rc = engine_check(E, head.data(), counts, outgrown);
+        if (outgrown) {
+            if (attempt) return pc_fail(E.ctx, PC_ARITHMETIC, "deep survivor count changed between attempts");
+            rc = engine_deep_alloc(E, E.deep_max + 1024);
+            if (rc) return rc;
+            continue;
+        }
+        *n_out = head[Engine::NOUT];
+        if (rc) return rc;
+        return engine_records(E, records, got, *n_out, place(*n_out));
+    }
 }
 
 void engine_stats(Engine &E, pc_stats *stats, int launches, uint64_t n_out) {
@@ -1904,8 +1980,7 @@ extern "C" int pc_run_batch(pc_ctx *ctx, const pc_filters *f, const pc_tuning *t
     Scratch hold(ctx);
     int launches = 0;
     int rc = engine_prepare(E, tuning, hold);
-    if (!rc) rc = engine_eager(E, &launches);
-    if (!rc) rc = engine_collect(E, counts, geometry, out, n_out);
+    if (!rc) rc = engine_run(E, counts, geometry, n_out, &launches, [&](uint64_t) { return out; });
     if (!rc || rc == PC_OVERFLOW || rc == PC_ARITHMETIC) engine_stats(E, stats, launches, *n_out);
     if (stats) {
         stats->total_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
@@ -1956,8 +2031,7 @@ extern "C" int pc_run_lease(pc_ctx *ctx, const pc_focus *fa, const pc_focus *fb,
     E.ntiles = ntiles64;
     E.out_cap = out_cap;
     rc = engine_prepare(E, tuning, hold);
-    if (!rc) rc = engine_eager(E, &launches);
-    if (!rc) rc = engine_collect(E, counts, geometry, out, n_out);
+    if (!rc) rc = engine_run(E, counts, geometry, n_out, &launches, [&](uint64_t) { return out; });
     if (!rc || rc == PC_OVERFLOW || rc == PC_ARITHMETIC) {
         engine_stats(E, stats, launches, *n_out);
         if (stats) stats->window_ms = elapsed_ms(ctx->ev[4], ctx->ev[5]);
@@ -1999,10 +2073,10 @@ extern "C" int pc_run_plain(pc_ctx *ctx, const pc_filters *f, const pc_buf *us, 
     if (stats) memset(stats, 0, sizeof(*stats));
     const uint32_t ng = f->ng;
     Scratch s(ctx);
-    uint64_t *d_counts, *d_out;
-    int rc = s.get(&d_counts, ng + 3);
-    if (!rc) rc = s.get(&d_out, 2 * std::max<uint64_t>(1, out_cap));
+    uint64_t *d_counts;                                   // then the output records
+    int rc = s.get(&d_counts, ng + 3 + 2 * std::max<uint64_t>(1, out_cap));
     if (rc) return rc;
+    uint64_t *d_out = d_counts + ng + 3;
     cudaStream_t st = ctx->stream;
     PC_CHECK(ctx, cudaMemsetAsync(d_counts, 0, (ng + 3) * 8, st));
     PC_CHECK(ctx, cudaEventRecord(ctx->ev[6], st));
@@ -2032,17 +2106,22 @@ extern "C" int pc_run_plain(pc_ctx *ctx, const pc_filters *f, const pc_buf *us, 
         PC_LAUNCHED(ctx, "plain match");
     }
     PC_CHECK(ctx, cudaEventRecord(ctx->ev[7], st));
-    PC_CHECK(ctx, pc_copy(ctx, counts, d_counts, (ng + 3) * 8, cudaMemcpyDeviceToHost));
+    // the counters and the first records in one copy
+    const uint64_t first = std::min<uint64_t>(out_cap, Engine::FETCH_RECORDS), words = ng + 3 + 2 * first;
+    uint64_t *stage = pc_stage(ctx, words * 8);
+    PC_CHECK(ctx, pc_copy(ctx, stage ? stage : counts, d_counts, (stage ? words : ng + 3) * 8, cudaMemcpyDeviceToHost));
     PC_CHECK(ctx, cudaStreamSynchronize(st));
+    if (stage) memcpy(counts, stage, (ng + 3) * 8);
     uint64_t n = counts[ng + 1];
     if (stats) {
         stats->kernel_ms = elapsed_ms(ctx->ev[6], ctx->ev[7]);
         stats->outputs = n;
         stats->launches = nu && nv ? 1 : 0;
     }
-    uint64_t copy = std::min(n, out_cap);
-    if (copy) {
-        PC_CHECK(ctx, pc_copy(ctx, out, d_out, 2 * copy * 8, cudaMemcpyDeviceToHost));
+    const uint64_t copy = std::min(n, out_cap), got = stage ? std::min(copy, first) : 0;
+    if (got) memcpy(out, stage + ng + 3, 16 * got);
+    if (copy > got) {
+        PC_CHECK(ctx, pc_copy(ctx, out + 2 * got, d_out + 2 * got, 16 * (copy - got), cudaMemcpyDeviceToHost));
         PC_CHECK(ctx, cudaStreamSynchronize(st));
     }
     return PC_OK;
@@ -2073,17 +2152,13 @@ struct pc_multi {
     bool ran = false;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
-    uint64_t *h_counts = nullptr, *h_geo = nullptr;   // pinned copies written by the graph
-    unsigned long long *h_nout = nullptr;
-    uint32_t *h_deep = nullptr;
+    uint64_t *h_report = nullptr;                     // the engine's report, page-locked, written by the graph
+    const uint64_t *from = nullptr, *geo_from = nullptr;   // counters and envelopes of the last run
     explicit pc_multi(pc_ctx *c) : ctx(c), hold(c) { E.ctx = c; }
     ~pc_multi() {
         if (exec) cudaGraphExecDestroy(exec);
         if (graph) cudaGraphDestroy(graph);
-        if (h_counts) cudaFreeHost(h_counts);
-        if (h_geo) cudaFreeHost(h_geo);
-        if (h_nout) cudaFreeHost(h_nout);
-        if (h_deep) cudaFreeHost(h_deep);
+        if (h_report) cudaFreeHost(h_report);
     }
 };
 
@@ -2178,8 +2253,8 @@ extern "C" int pc_multi_create(pc_ctx *ctx, const pc_focus *const *foci, uint32_
     E.windows = true;
     rc = engine_prepare(E, tuning, m->hold);
     // zeroed once: a pass that gave up makes this and every later result of the object an error
-    if (!rc) rc = pc_cuda_status(ctx, cudaMemsetAsync(E.d_nout + 2, 0, 8, ctx->stream), "window flag");
-    m->wb.d_stuck = (uint64_t *)(E.d_nout + 2);
+    if (!rc) rc = pc_cuda_status(ctx, cudaMemsetAsync(E.d_report, 0, 8, ctx->stream), "window flag");
+    m->wb.d_stuck = E.d_report + Engine::STUCK;
     if (!rc) rc = pc_cuda_status(ctx, cudaStreamSynchronize(ctx->stream), "window batch set-up");
     if (rc) {
         delete m;
@@ -2199,12 +2274,14 @@ int multi_eager(pc_ctx *ctx, pc_multi *m, pc_stats *stats) {
     if (rc) return rc;
     launches += 1;
     PC_CHECK(ctx, cudaEventRecord(ctx->ev[5], ctx->stream));
-    rc = engine_eager(E, &launches);
-    if (rc) return rc;
-    m->counts.assign(E.ntiles * E.stride, 0);
-    m->geometry.assign(2 * E.ntiles, 0);
-    m->out.assign(2 * std::max<uint64_t>(1, E.out_cap), 0);
-    rc = engine_collect(E, m->counts.data(), m->geometry.data(), m->out.data(), &m->n_out);
+    m->counts.resize(E.ntiles * E.stride);
+    m->geometry.resize(2 * E.ntiles);
+    rc = engine_run(E, m->counts.data(), m->geometry.data(), &m->n_out, &launches, [&](uint64_t n) {
+        m->out.resize(2 * n);
+        return m->out.data();
+    });
+    m->from = m->counts.data();
+    m->geo_from = m->geometry.data();
     m->launches = launches;
     if (!rc || rc == PC_OVERFLOW || rc == PC_ARITHMETIC) {
         engine_stats(E, stats, launches, m->n_out);
@@ -2218,32 +2295,15 @@ int multi_eager(pc_ctx *ctx, pc_multi *m, pc_stats *stats) {
 int multi_capture(pc_ctx *ctx, pc_multi *m) {
     Engine &E = m->E;
     cudaStream_t st = ctx->stream;
-    const uint64_t nc = std::max<uint64_t>(1, E.ntiles * E.stride), ng = std::max<uint64_t>(1, 2 * E.ntiles);
-    if (!m->h_counts) {
-        PC_CHECK(ctx, cudaMallocHost((void **)&m->h_counts, nc * 8));
-        PC_CHECK(ctx, cudaMallocHost((void **)&m->h_geo, ng * 8));
-        PC_CHECK(ctx, cudaMallocHost((void **)&m->h_nout, E.nout_bytes()));
-        PC_CHECK(ctx, cudaMallocHost((void **)&m->h_deep, (uint64_t)E.grid * 4));
-    }
+    const uint64_t bytes = E.fetch_words() * 8;
+    if (!m->h_report) PC_CHECK(ctx, cudaMallocHost((void **)&m->h_report, bytes));
     int rc = engine_match(E, 2);
     if (rc) return rc;
     PC_CHECK(ctx, cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     int launches = 0;
     rc = winbatch_emit(ctx, m->wb, m->d_lists, m->wb.out_len);
-    if (!rc) rc = engine_front(E, false, true, &launches);
-    if (!rc) rc = engine_back(E, false, &launches);
-    if (!rc) rc = pc_cuda_status(ctx, pc_copy(ctx, m->h_nout, E.d_nout, E.nout_bytes(), cudaMemcpyDeviceToHost),
-                                    "capture copy");
-    if (!rc && E.ntiles) {
-        rc = pc_cuda_status(ctx, pc_copy(ctx, m->h_counts, E.d_counts, E.ntiles * E.stride * 8, cudaMemcpyDeviceToHost),
-                            "capture copy");
-        if (!rc)
-            rc = pc_cuda_status(ctx, pc_copy(ctx, m->h_geo, E.d_geo, 2 * E.ntiles * 8, cudaMemcpyDeviceToHost),
-                                "capture copy");
-    }
-    if (!rc)
-        rc = pc_cuda_status(ctx, pc_copy(ctx, m->h_deep, E.d_deep_count, (uint64_t)E.grid * 4, cudaMemcpyDeviceToHost),
-                            "capture copy");
+    if (!rc) rc = engine_launch(E, false, true, &launches);
+    if (!rc) rc = pc_cuda_status(ctx, pc_copy(ctx, m->h_report, E.d_report, bytes, cudaMemcpyDeviceToHost), "capture copy");
     cudaGraph_t g = nullptr;
     const cudaError_t e = cudaStreamEndCapture(st, &g);       // always leave capture mode
     if (!rc && e != cudaSuccess) rc = pc_cuda_fail(ctx, e, "end capture");
@@ -2256,7 +2316,7 @@ int multi_capture(pc_ctx *ctx, pc_multi *m) {
     PC_CHECK(ctx, cudaGraphInstantiate(&m->exec, g, 0));
     m->launches = launches + 1;
     // the copies recorded into the graph run at every replay, not at capture
-    m->graph_d2h = E.nout_bytes() + (E.ntiles ? E.ntiles * E.stride * 8 + 2 * E.ntiles * 8 : 0) + (uint64_t)E.grid * 4;
+    m->graph_d2h = bytes;
     ctx->d2h -= m->graph_d2h;
     return PC_OK;
 }
@@ -2271,16 +2331,16 @@ int multi_replay(pc_ctx *ctx, pc_multi *m, pc_stats *stats) {
     ctx->d2h += m->graph_d2h;
     PC_CHECK(ctx, cudaEventRecord(ctx->ev[1], st));
     PC_CHECK(ctx, cudaStreamSynchronize(st));
-    for (int b = 0; b < E.grid; ++b)
-        if (m->h_deep[b] > E.deep_cap) return pc_fail(ctx, PC_ARITHMETIC, "deep survivor count changed between runs");
-    m->counts.assign(m->h_counts, m->h_counts + E.ntiles * E.stride);
-    m->geometry.assign(m->h_geo, m->h_geo + 2 * E.ntiles);
-    const unsigned long long nout[3] = {m->h_nout[0], m->h_nout[1], m->h_nout[2]};
-    m->n_out = nout[0];
-    rc = engine_check(E, nout, m->counts.data());
-    if (!rc && nout[0]) {
-        PC_CHECK(ctx, pc_copy(ctx, m->out.data(), E.d_out, 2 * nout[0] * 8, cudaMemcpyDeviceToHost));
-        PC_CHECK(ctx, cudaStreamSynchronize(st));
+    const uint64_t *counts = m->h_report + E.o_counts;
+    bool outgrown = false;
+    rc = engine_check(E, m->h_report, counts, outgrown);
+    if (outgrown) return pc_fail(ctx, PC_ARITHMETIC, "deep survivor count changed between runs");
+    m->from = counts;
+    m->geo_from = m->h_report + E.o_geo;
+    m->n_out = m->h_report[Engine::NOUT];
+    if (!rc) {
+        m->out.resize(2 * m->n_out);
+        rc = engine_records(E, m->h_report + E.o_out, (E.fetch_words() - E.o_out) / 2, m->n_out, m->out.data());
     }
     if (stats) {
         stats->kernel_ms = elapsed_ms(ctx->ev[0], ctx->ev[1]);
@@ -2341,8 +2401,8 @@ extern "C" int pc_multi_layout(const pc_multi *m, uint32_t *tile_base, uint64_t 
 extern "C" int pc_multi_results(pc_ctx *ctx, const pc_multi *m, uint64_t *counts, uint64_t *geometry, uint64_t *out,
                                 uint64_t out_cap, uint64_t *n_out) {
     if (!m || !m->ran) return pc_fail(ctx, PC_INVALID, "window batch has not run");
-    if (counts) std::copy(m->counts.begin(), m->counts.end(), counts);
-    if (geometry) std::copy(m->geometry.begin(), m->geometry.end(), geometry);
+    if (counts) std::copy(m->from, m->from + m->E.ntiles * m->E.stride, counts);
+    if (geometry) std::copy(m->geo_from, m->geo_from + 2 * m->E.ntiles, geometry);
     *n_out = m->n_out;
     if (out) std::copy(m->out.begin(), m->out.begin() + 2 * std::min(m->n_out, out_cap), out);
     return PC_OK;

@@ -827,7 +827,12 @@ int winbatch_run(pc_ctx *ctx, Scratch &hold, const pc_focus *const *focus, const
     }
     uint64_t room = (uint64_t)(expect * 1.01 + 8 * std::sqrt(expect)) + 1024;
     room = std::min(std::min(room, most), cap);
-    std::vector<uint64_t> got(n + 2);
+    std::vector<uint64_t> pageable;
+    uint64_t *got = pc_stage(ctx, (n + 2) * 8);
+    if (!got) {
+        pageable.resize(n + 2);
+        got = pageable.data();
+    }
     for (int attempt = 0;; ++attempt) {
         *out_bytes = std::max<uint64_t>(16, room * 8);
         rc = pc_alloc(ctx, (void **)out, *out_bytes);
@@ -836,7 +841,7 @@ int winbatch_run(pc_ctx *ctx, Scratch &hold, const pc_focus *const *focus, const
         rc = winbatch_emit(ctx, wb, *out, room);
         if (launches) ++*launches;
         if (!rc)
-            rc = pc_cuda_status(ctx, pc_copy(ctx, got.data(), wb.d_scan + 1 + win_tiles(wb), (n + 2) * 8, cudaMemcpyDeviceToHost),
+            rc = pc_cuda_status(ctx, pc_copy(ctx, got, wb.d_scan + 1 + win_tiles(wb), (n + 2) * 8, cudaMemcpyDeviceToHost),
                                 "window totals");
         if (!rc) rc = pc_cuda_status(ctx, cudaStreamSynchronize(ctx->stream), "window totals");
         if (!rc && got[n + 1]) rc = pc_fail(ctx, PC_ARITHMETIC, "window pass did not finish");
