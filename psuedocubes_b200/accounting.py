@@ -34,6 +34,13 @@ def digest(value: Any) -> str:
     return hashlib.sha256(encoded(value)).hexdigest()
 
 
+def digest_decimals(values: list[str]) -> str:
+    """digest() of a list of decimal strings."""
+    if not values:
+        return EMPTY_DIGEST
+    return hashlib.sha256(('["' + '","'.join(values) + '"]\n').encode()).hexdigest()
+
+
 EMPTY_DIGEST = hashlib.sha256(encoded([])).hexdigest()
 _SAFE = 1 << 53
 

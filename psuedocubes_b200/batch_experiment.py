@@ -17,11 +17,11 @@ from typing import Any
 import numpy as np
 
 from . import _native as N
-from .accounting import EMPTY_DIGEST, digest, scope_list
+from .accounting import EMPTY_DIGEST, digest_decimals, scope_list
 from .focus import Config, Tile
 from .gpu import MASK, DeviceArray, Filters, GPUFocus, Matcher, Runtime, launch_plan
 from .predicate import is_perfect_cube, local3
-from .verify import MATERIALISE_MAX, VECTOR_MIN, verify, verify_many
+from .verify import MATERIALISE_MAX, SMALL_VECTOR_MIN, VECTOR_MIN, local_and_cubes, verify, verify_many
 
 
 @dataclass
@@ -40,10 +40,23 @@ def tile_ranges(config: Config, first: int, end: int, width: int) -> list[tuple[
     Tile(first, end).validate(config)
     if width <= 0 or (end - first + width - 1) // width > 64:
         raise ValueError('experiment allows at most 64 bounded subtiles')
+    # floor((lo + vA) / B) + 1 at the subtiles' first v and floor((hi + vA) / B) + 1 at their last: quotient and
+    # remainder step by those of width A from one subtile to the next (a short last one is divided anew)
+    A, B = config.A, config.B
+    dq, dr = divmod(width * A, B)
+    q0, r0 = divmod(config.lo + first * A, B)
+    q1, r1 = divmod(config.hi + (first + width - 1) * A, B)
     rows = []
     for v in range(first, end, width):
-        stop = min(v + width, end)
-        rows.append((v, stop, config.u_interval(v)[0], config.u_interval(stop - 1)[1]))
+        stop = v + width
+        if stop > end:
+            stop, q1 = end, (config.hi + (end - 1) * A) // B
+        rows.append((v, stop, q0 + 1, q1 + 1))
+        q0, r0, q1, r1 = q0 + dq, r0 + dr, q1 + dq, r1 + dr
+        if r0 >= B:
+            q0, r0 = q0 + 1, r0 - B
+        if r1 >= B:
+            q1, r1 = q1 + 1, r1 - B
     return rows
 
 
@@ -89,17 +102,25 @@ class CachedMatcher(Matcher):
         return result
 
 
-def split_outputs(records: np.ndarray, ntiles: int) -> list[list[int]]:
-    """Device output records (x limb 0, x limb 1 | subtile << 32) grouped by subtile, each sorted."""
-    per: list[list[int]] = [[] for _ in range(ntiles)]
+def outputs_by_tile(records: np.ndarray) -> dict[int, list[int]]:
+    """Device output records (x limb 0, x limb 1 | subtile << 32) of the subtiles that have any, each sorted."""
+    per: dict[int, list[int]] = {}
     if len(records):
         lo = records[:, 0]
         hi = records[:, 1] & np.uint64(0xFFFFFFFF)
         tile = (records[:, 1] >> np.uint64(32)).astype(np.int64)
         for t, a, b in zip(tile.tolist(), lo.tolist(), hi.tolist()):
-            per[t].append(a | (b << 64))
-        for t in set(tile.tolist()):
-            per[t].sort()
+            per.setdefault(t, []).append(a | (b << 64))
+        for values in per.values():
+            values.sort()
+    return per
+
+
+def split_outputs(records: np.ndarray, ntiles: int) -> list[list[int]]:
+    """The same as one list per subtile."""
+    per: list[list[int]] = [[] for _ in range(ntiles)]
+    for t, values in outputs_by_tile(records).items():
+        per[t] = values
     return per
 
 
@@ -119,9 +140,17 @@ def verify_values(config: Config, values: list[int]) -> Sequence[dict[str, Any]]
         if not hits.all_valid:
             raise ArithmeticError('independent witness verification failed')
         return list(hits) if len(hits) <= MATERIALISE_MAX else hits
-    if any(not config.lo < n <= config.hi or not local3(n, config.p) for n in values):
-        raise ArithmeticError('GPU/CPU disagreement')
-    hits = [verify(n, config.p) for n in values if not is_perfect_cube(n)]
+    if len(values) >= SMALL_VECTOR_MIN and config.hi < 1 << 96:
+        if any(not config.lo < n <= config.hi for n in (min(values), max(values))):
+            raise ArithmeticError('GPU/CPU disagreement')
+        ok, cubes = local_and_cubes(values, config.p)
+        if not ok.all():
+            raise ArithmeticError('GPU/CPU disagreement')
+        hits = [verify(n, config.p) for n, cube in zip(values, cubes.tolist()) if not cube]
+    else:
+        if any(not config.lo < n <= config.hi or not local3(n, config.p) for n in values):
+            raise ArithmeticError('GPU/CPU disagreement')
+        hits = [verify(n, config.p) for n in values if not is_perfect_cube(n)]
     if any(not row['valid_pseudocube'] for row in hits):
         raise ArithmeticError('independent witness verification failed')
     return hits
@@ -147,7 +176,7 @@ def batch_result(config: Config, ranges: list[tuple[int, int, int, int]], pops: 
             if any(not first <= config.canonical(n)[1] < end for n in values):
                 raise ArithmeticError('output assigned to wrong subtile')
             all_values.extend(values)
-            digests.append(digest([str(n) for n in values]))
+            digests.append(digest_decimals([str(n) for n in values]))
         else:
             digests.append(EMPTY_DIGEST)
     scopes = scope_list([r[0] for r in ranges], [r[1] for r in ranges], pops[:, 0].tolist(),
@@ -190,7 +219,7 @@ class FusedMatcher:
         counts = np.zeros(nt * (ng + 3), dtype=np.uint64)
         geometry = np.zeros(2 * nt, dtype=np.uint64)
         capacity = nt * output_cap
-        records = np.zeros(2 * capacity, dtype=np.uint64)
+        records = np.empty(2 * capacity, dtype=np.uint64)    # as many records are read as were written
         n_out = ctypes.c_uint64()
         stats = N.Stats()
         c = self.config
@@ -254,7 +283,7 @@ class MaskedMatcher(FusedMatcher):
         c = self.config
         capacity = min(nt * output_cap, self.lease_output_records)
         for attempt in range(2):
-            records = np.zeros(2 * max(1, capacity), dtype=np.uint64)
+            records = np.empty(2 * max(1, capacity), dtype=np.uint64)
             self.runtime.check()
             code = self.runtime.lib.pc_run_lease(
                 self.runtime.ctx, af.handle, bf.handle, self.filters.handle, ctypes.byref(self.tuning), first,

@@ -34,7 +34,7 @@ from typing import Any, Iterable, Iterator
 import numpy as np
 
 from . import _native as N
-from .accounting import EMPTY_DIGEST, digest
+from .accounting import EMPTY_DIGEST, digest_decimals
 from .batch_experiment import verify_values
 from .focus import A619, B619, Config
 from .gpu import MASK, Filters, GPUFocus, Runtime
@@ -321,7 +321,7 @@ class WindowBatch:
             c, first, end = self.configs[i], first_l[t], end_l[t]
             if any(not first <= c.canonical(x)[1] < end for x in tile_values):
                 raise ArithmeticError('output assigned to wrong subtile')
-            digests[t] = digest([str(x) for x in tile_values])
+            digests[t] = digest_decimals([str(x) for x in tile_values])
             values_of.setdefault(i, []).extend(tile_values)
         scopes = [{'first': a, 'end': b, 'valid_focused_candidates': v, 'group_survivors': g, 'local_survivors': e,
                    'output_sha256': d}

@@ -47,7 +47,7 @@ def list_roots(runtime: Runtime, first: int, last: int, p: int, cap: int | None 
     roots raise OverflowError; by default ``cap`` admits every root of the range."""
     _check(first, last, p)
     cap = last - first + 1 if cap is None else cap
-    out = np.zeros(max(1, cap), dtype=np.uint32)
+    out = np.empty(max(1, cap), dtype=np.uint32)         # only the roots written are returned
     count = ctypes.c_uint64()
     runtime.call(runtime.lib.pc_cube_roots(runtime.ctx, first, last, p, out.ctypes.data, cap, ctypes.byref(count), None),
                  'cube roots')

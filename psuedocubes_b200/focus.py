@@ -188,10 +188,13 @@ class Config:
         v_rings = tuple((q, _adjusted(q, -self.A)) for q in factors(self.B, self.p))
         return Focus(self.A, u_rings), Focus(self.B, v_rings)
 
+    @cached_property
+    def _inverse(self) -> int:
+        return pow(self.A, -1, self.B) if self.B > 1 else 0
+
     def canonical(self, n: int) -> tuple[int, int]:
         """The canonical pair (u, v) of n, 0 <= v < B."""
-        inverse = pow(self.A, -1, self.B) if self.B > 1 else 0
-        v = -n * inverse % self.B
+        v = -n * self._inverse % self.B
         return (n + v * self.A) // self.B, v
 
     def u_interval(self, v: int) -> tuple[int, int]:

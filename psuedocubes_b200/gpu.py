@@ -15,7 +15,7 @@ import numpy as np
 from . import _native as N
 from .focus import Config, Focus, Tile
 from .predicate import is_perfect_cube, local3
-from .tables import allowed
+from .tables import ring_bytes
 
 MASK = (1 << 64) - 1
 
@@ -115,7 +115,7 @@ class DeviceArray:
         return DeviceArray(self.runtime, self.handle, self.offset + start, stop - start, self._owner or self)
 
     def get(self) -> np.ndarray:
-        out = np.zeros(self.size, dtype=np.uint64)
+        out = np.empty(self.size, dtype=np.uint64)
         if self.size:
             self.runtime.call(self.runtime.lib.pc_buf_download(self.runtime.ctx, self.handle, self.offset,
                                                                self.size, out))
@@ -202,12 +202,7 @@ class Filters:
         self.filter_groups = [order[i:i + 4] for i in range(0, len(order), 4)]
         self.ng = len(self.filter_groups)
         if table is None:
-            table = []
-            for q in order:
-                ring = [0] * q
-                for a in allowed(q):
-                    ring[a] = 1
-                table.extend(ring)
+            table = np.frombuffer(b''.join([ring_bytes(q) for q in order]), dtype=np.uint8)
         elif len(table) != sum(order):
             raise ValueError('residue table must hold one byte per residue of every filter')
         handle = ctypes.c_void_p()
@@ -270,7 +265,7 @@ class Matcher:
             raise ValueError('negative output capacity')
         blocks, stripes = launch_plan(us.size, vs.size, self.sm_count, self.layout, self.blocks_per_sm)
         counts = np.zeros(ng + 3, dtype=np.uint64)
-        out = np.zeros(max(2, 2 * cap), dtype=np.uint64)
+        out = np.empty(max(2, 2 * cap), dtype=np.uint64)     # as many records are read as were written
         stats = N.Stats()
         c = self.config
         self.runtime.check()

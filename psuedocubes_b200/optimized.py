@@ -17,9 +17,9 @@ from typing import Any, Callable, Iterable, Iterator
 
 import numpy as np
 
-from .accounting import EMPTY_DIGEST, digest, encoded_scopes
+from .accounting import EMPTY_DIGEST, digest, digest_decimals, encoded_scopes
 from . import _native as N
-from .batch_experiment import MaskedMatcher, batch_result, prepare, split_outputs, verify_values
+from .batch_experiment import MaskedMatcher, batch_result, outputs_by_tile, prepare, verify_values
 from .focus import Tile
 from .gpu import MASK, GPUFocus
 from .multi import validate_result
@@ -146,13 +146,13 @@ def lease_receipt(matcher: MaskedMatcher, raw: dict[str, Any], first: int, end: 
     values: list[int] = []
     emitted = counts[:, ng + 1].tolist()
     for t in np.nonzero(counts[:, ng + 1])[0].tolist():
-        tile_values = per_tile[t]
+        tile_values = per_tile.get(t, []) if isinstance(per_tile, dict) else per_tile[t]
         lo = first + t * width
         if len(tile_values) != emitted[t]:
             raise ArithmeticError('device output count disagrees with its records')
         if any(not lo <= config.canonical(n)[1] < min(lo + width, end) for n in tile_values):
             raise ArithmeticError('output assigned to wrong subtile')
-        digests[t] = digest([str(n) for n in tile_values])
+        digests[t] = digest_decimals([str(n) for n in tile_values])
         values.extend(tile_values)
     if sum(emitted) != len(values):
         raise ArithmeticError('device output count disagrees with its records')
@@ -267,7 +267,7 @@ class _LeaseChunk:
         m.last_stats = self.stats[i].as_dict()
         return dict(counts=self.counts[i][:nt * self.stride].reshape(nt, self.stride),
                     geometry=self.geometry[i][:2 * nt].reshape(nt, 2),
-                    per_tile=split_outputs(self.out[i][:2 * n].reshape(-1, 2), nt), stats=m.last_stats)
+                    per_tile=outputs_by_tile(self.out[i][:2 * n].reshape(-1, 2)), stats=m.last_stats)
 
     def finish(self) -> None:
         self.future.result()

@@ -39,7 +39,7 @@ from .cubes import genuine_cube_count
 from .focus import Config, Tile
 from .gpu import Matcher, Runtime
 from .tables import allowed
-from .verify import MATERIALISE_MAX, VECTOR_MIN, cube_limbs, icbrt_many, verify, verify_many
+from .verify import MATERIALISE_MAX, VECTOR_MIN, cube_limbs, icbrt_many, local_test, verify, verify_many
 
 A_RINGS = (2, 7, 13, 31, 43, 73, 79, 127, 139, 157, 181)   # the rings of A619, ascending
 B_RINGS = (9, 19, 37, 61, 67, 97, 103, 109, 151, 163)      # the rings of B619, ascending
@@ -86,23 +86,28 @@ def _count(q: int) -> int:
     return len(allowed(q))
 
 
+def _prefixes(rings: tuple[int, ...]) -> list[tuple[int, int, int, int]]:
+    """(length, product, focus count, largest ring) of every prefix of a ring list."""
+    return [(k, math.prod(rings[:k]), math.prod(_count(q) for q in rings[:k]), max(rings[:k]))
+            for k in range(1, len(rings) + 1)]
+
+
+_A_PREFIXES, _B_PREFIXES = _prefixes(A_RINGS), _prefixes(B_RINGS)
+
+
 def plan_request(p: int, lo: int, hi: int) -> Plan:
     """The focus split of least modelled device time for (lo, hi] (deterministic)."""
     if not 0 <= lo < hi <= X_MAX:
         raise ValueError('invalid interval')
     span = hi - lo
     best: Plan | None = None
-    for a in range(1, len(A_RINGS) + 1):
-        A = math.prod(A_RINGS[:a])
-        ca = math.prod(_count(q) for q in A_RINGS[:a])
-        for b in range(1, len(B_RINGS) + 1):
-            B = math.prod(B_RINGS[:b])
-            if A >= 1 << 63 or B >= 1 << 63 or max(A_RINGS[:a] + B_RINGS[:b]) > p:
+    for a, A, ca, top_a in _A_PREFIXES:
+        for b, B, cb, top_b in _B_PREFIXES:
+            if A >= 1 << 63 or B >= 1 << 63 or max(top_a, top_b) > p:
                 continue
             max_u = (hi + (B - 1) * A) // B
             if max_u >= 1 << 64 or max_u * B >= 1 << 128:
                 continue
-            cb = math.prod(_count(q) for q in B_RINGS[:b])
             positions = span * (ca / A) * (cb / B)
             sweeps = max(1, math.ceil(span * ca / A / B / (U_WINDOW / 2)))   # x sub-ranges (request_windows)
             u_entries = sweeps * ca + ca * span / (A * B)
@@ -206,13 +211,16 @@ def verify_outputs(records: np.ndarray, lo: int, hi: int, p: int) -> tuple[list[
     first, last = int(xh[0]) << 64 | int(xl[0]), int(xh[-1]) << 64 | int(xl[-1])
     if not lo < first or not last <= hi:
         raise ArithmeticError('GPU/CPU disagreement: value outside the interval')
-    ok = np.isin(_residues(xl, xh, 9), np.array([1, 8], dtype=np.uint64))
-    for q in primes_upto(p):
-        if q == 3:
-            continue
-        table = np.zeros(q, dtype=bool)
-        table[list(allowed(q))] = True
-        ok &= table[_residues(xl, xh, q).astype(np.int64)]
+    if len(xl) < VECTOR_MIN:
+        ok = local_test(xl, xh, p)
+    else:                                                # prime by prime: the columns of one stay in cache
+        ok = np.isin(_residues(xl, xh, 9), np.array([1, 8], dtype=np.uint64))
+        for q in primes_upto(p):
+            if q == 3:
+                continue
+            table = np.zeros(q, dtype=bool)
+            table[list(allowed(q))] = True
+            ok &= table[_residues(xl, xh, q).astype(np.int64)]
     if not ok.all():
         raise ArithmeticError('GPU/CPU disagreement: local test failed')
     values = [h << 64 | l for h, l in zip(xh.tolist(), xl.tolist())]

@@ -15,13 +15,18 @@ from typing import Any
 
 def sieve_primes(p: int) -> list[int]:
     """Primes <= p by Eratosthenes (pseudocube/tables.py:9-15)."""
+    return list(_primes(p))
+
+
+@lru_cache(maxsize=256)
+def _primes(p: int) -> tuple[int, ...]:
     if p < 2:
-        return []
+        return ()
     composite = bytearray(p + 1)
     for q in range(2, isqrt(p) + 1):
         if not composite[q]:
             composite[q * q::q] = b'\x01' * len(range(q * q, p + 1, q))
-    return [q for q in range(2, p + 1) if not composite[q]]
+    return tuple(q for q in range(2, p + 1) if not composite[q])
 
 
 @lru_cache(maxsize=None)
@@ -32,6 +37,15 @@ def allowed(q: int) -> tuple[int, ...]:
     if q % 3 == 1:
         return tuple(sorted({pow(a, 3, q) for a in range(1, q)}))
     return tuple(range(1, q))
+
+
+@lru_cache(maxsize=None)
+def ring_bytes(q: int) -> bytes:
+    """One byte per residue r of q: 1 when r is allowed."""
+    ring = bytearray(q)
+    for a in allowed(q):
+        ring[a] = 1
+    return bytes(ring)
 
 
 def packed(q: int) -> list[int]:

@@ -8,6 +8,7 @@ millions of survivors) and gives the same rows.
 from __future__ import annotations
 
 from collections.abc import Sequence
+from functools import lru_cache
 from math import isqrt
 from typing import Any
 
@@ -40,6 +41,7 @@ def verify(n: int, p: int) -> dict[str, Any]:
 # the interpreter lock inside its array operations).
 
 VECTOR_MIN = 2048          # fewer values: verify() one by one
+SMALL_VECTOR_MIN = 4       # fewer values: the scalar predicate one by one
 MATERIALISE_MAX = 1 << 20  # more non-cubes than this: the rows are built when read
 
 
@@ -75,6 +77,46 @@ def icbrt_many(lo: np.ndarray, hi: np.ndarray) -> np.ndarray:
         h, l = cube_limbs(np.minimum(a + np.uint64(1), top))
         a = np.where((a < top) & _le(h, l, hi, lo), a + np.uint64(1), a)
     return a
+
+
+@lru_cache(maxsize=None)
+def _fails(q: int) -> np.ndarray:
+    """Per residue r of a prime q: r fails verify()'s test (r = 0, or r^((q-1)/3) != 1 when q = 1 mod 3)."""
+    r = np.arange(q, dtype=np.int64)
+    if q % 3 != 1:
+        return r == 0
+    power, base, e = np.ones(q, dtype=np.int64), r, (q - 1) // 3
+    while e:
+        if e & 1:
+            power = power * base % q
+        base, e = base * base % q, e >> 1
+    return power != 1
+
+
+@lru_cache(maxsize=32)
+def _local_tables(p: int) -> tuple[np.ndarray, np.ndarray, np.ndarray, np.ndarray]:
+    """9 and the primes <= p other than 3, 2^64 mod each, where each one's table starts, and the tables of the
+    residues that fail local3."""
+    moduli = [9] + [q for q in range(2, p + 1) if q != 3 and all(q % d for d in range(2, isqrt(q) + 1))]
+    fails = [np.array([r not in (1, 8) for r in range(9)])] + [_fails(q) for q in moduli[1:]]
+    return (np.array(moduli, dtype=np.uint64), np.array([(1 << 64) % q for q in moduli], dtype=np.uint64),
+            np.cumsum([0] + moduli[:-1]), np.concatenate(fails))
+
+
+def local_test(lo: np.ndarray, hi: np.ndarray, p: int) -> np.ndarray:
+    """local3 of x = hi 2^64 + lo < 2^96 for some values at once: every residue of every value in one array."""
+    q, r64, starts, fails = _local_tables(p)
+    r = ((hi[:, None] % q) * r64 + lo[:, None] % q) % q
+    return ~fails[starts + r.astype(np.int64)].any(axis=1) & ((lo != 0) | (hi != 0))
+
+
+def local_and_cubes(values: list[int], p: int) -> tuple[np.ndarray, np.ndarray]:
+    """Per value 0 <= n < 2^96: local3(n, p), and whether n is a perfect cube."""
+    mask = (1 << 64) - 1
+    lo = np.array([n & mask for n in values], dtype=np.uint64)
+    hi = np.array([n >> 64 for n in values], dtype=np.uint64)
+    h, l = cube_limbs(icbrt_many(lo, hi))
+    return local_test(lo, hi, p), (h == hi) & (l == lo)
 
 
 class Witnesses(Sequence):
@@ -142,9 +184,7 @@ def verify_many(lo: np.ndarray, hi: np.ndarray, p: int, threads: int | None = No
     hi = np.ascontiguousarray(hi, dtype=np.uint64)
     if len(hi) and int(hi.max()) >> 32:
         raise ValueError('values must be below 2^96')
-    tables = {}
-    for q in primes:                                     # failure table of verify(): r = 0, or r^((q-1)/3) != 1
-        tables[q] = np.array([r == 0 or (q % 3 == 1 and pow(r, (q - 1) // 3, q) != 1) for r in range(q)], dtype=bool)
+    tables = {q: _fails(q) for q in primes}
     n = len(lo)
     step = max(1 << 16, -(-n // (4 * (threads or os.cpu_count() or 1))))
     spans = [(a, min(n, a + step)) for a in range(0, n, step)] or [(0, 0)]
