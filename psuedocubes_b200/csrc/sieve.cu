@@ -98,13 +98,14 @@ struct MatchArgs {
     uint32_t total_rows;             // largest over the families
     uint64_t *counts;                // ntiles x stride
     const uint4 *bv;                 // per u block: v rows meeting it, v rows covering it
-    const uint64_t *item_prefix;     // nblocks + 1
+    const uint64_t *prefix;          // work of the blocks before each block; the last entry, all
     uint64_t nblocks;
-    const uint64_t *vchunk;          // device scalar
+    uint32_t shares, whole, pairs;   // shares: even parts of all work, or (whole) blocks, the first `pairs` of them two
+    uint32_t block_cost, v_chunk;    // a block's fixed work in v rows; most rows per work item
     uint4 *deep;                     // (v lo, v hi, u index, subtile) records
     uint32_t deep_cap;               // records per CTA slice
     uint32_t *deep_count;            // per CTA (may exceed deep_cap: the caller retries larger)
-    unsigned long long *item_next;   // next unclaimed work item (zeroed before the launch)
+    unsigned long long *share_next;  // shares claimed beyond each CTA's first (zeroed before the launch)
 };
 
 struct DeepArgs {
@@ -496,13 +497,9 @@ __global__ void __launch_bounds__(256) k_geometry(const uint64_t *__restrict__ u
 // sub-range [f0, f1) of rows covering the whole block (left <= start and right >= stop); left and
 // right are monotone in the row index within a segment, so all four are searches: a warp per block, eight lanes
 // each (a thread per block with four searches in turn: 24 us for a batch, 57 us for a lease; now 5 and 18 us).
-// The blocks' rows are also summed (the pieces from which k_items sizes work items).
 __global__ void __launch_bounds__(256) k_blocks(const VRec *__restrict__ rec, const SegDev *__restrict__ seg, uint32_t nseg,
                                                 uint32_t UB, uint64_t nblocks, uint4 *__restrict__ bv,
-                                                uint32_t *__restrict__ blk_seg, unsigned long long *__restrict__ pieces) {
-    __shared__ unsigned long long sum_s;
-    if (threadIdx.x == 0) sum_s = 0;
-    __syncthreads();
+                                                uint32_t *__restrict__ blk_seg) {
     const uint32_t lane = threadIdx.x & 31, which = lane >> 3;
     const uint64_t b = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
     if (b < nblocks) {                                    // warp-uniform
@@ -526,42 +523,27 @@ __global__ void __launch_bounds__(256) k_blocks(const VRec *__restrict__ rec, co
         if (lane == 0) {
             bv[b] = range;
             blk_seg[b] = s;
-            if (range.y != range.x) atomicAdd(&sum_s, (unsigned long long)(range.y - range.x));
         }
     }
-    __syncthreads();
-    if (threadIdx.x == 0 && sum_s) atomicAdd(pieces, sum_s);
 }
 
-// v chunk per work item: fixed, or total pieces / target items, at least min_chunk (four rounds of
-// 32 rows for every warp of a k_match CTA, so a small launch keeps every warp busy and pays the
-// per-item set-up over enough rows) and at most 2^20; and the items before each block (prefix[nblocks]: all).
+// Work of the blocks before each block: its v rows and, where it has any, the fixed cost of a block in rows.
 // One CTA: a lease has 1e4 blocks, two turns of 8,192.
-constexpr uint32_t ITEMS_T = 1024, ITEMS_PER = 8;
+constexpr uint32_t PIECES_T = 1024, PIECES_PER = 8;
 
-__global__ void __launch_bounds__(ITEMS_T) k_items(const uint4 *__restrict__ bv, uint64_t nblocks,
-                                                   const unsigned long long *__restrict__ pieces, uint64_t fixed_chunk,
-                                                   uint64_t target_items, uint64_t min_chunk, uint64_t *__restrict__ vchunk,
-                                                   uint64_t *__restrict__ prefix) {
-    __shared__ uint64_t warp_s[ITEMS_T / 32];
+__global__ void __launch_bounds__(PIECES_T) k_pieces(const uint4 *__restrict__ bv, uint64_t nblocks, uint32_t block_cost,
+                                                     uint64_t *__restrict__ prefix) {
+    __shared__ uint64_t warp_s[PIECES_T / 32];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint64_t c = fixed_chunk;
-    if (!c) c = umax64((*pieces + target_items - 1) / umax64(1, target_items), min_chunk);
-    c = umin64(c, UINT64_C(1) << 20);
-    if (threadIdx.x == 0) *vchunk = c;
-    uint64_t before = 0;                                  // items of the blocks of earlier turns
-    for (uint64_t base = 0; base < nblocks; base += ITEMS_T * ITEMS_PER) {
-        const uint64_t b0 = base + threadIdx.x * ITEMS_PER;
-        uint32_t items[ITEMS_PER];
+    uint64_t before = 0;                                  // work of the blocks of earlier turns
+    for (uint64_t base = 0; base < nblocks; base += PIECES_T * PIECES_PER) {
+        const uint64_t b0 = base + threadIdx.x * PIECES_PER;
+        uint32_t rows[PIECES_PER];
         uint64_t own = 0;
 #pragma unroll
-        for (uint32_t k = 0; k < ITEMS_PER; ++k) {
-            items[k] = 0;
-            if (b0 + k < nblocks) {
-                const uint4 r = bv[b0 + k];
-                items[k] = (r.y - r.x + (uint32_t)c - 1) / (uint32_t)c;
-            }
-            own += items[k];
+        for (uint32_t k = 0; k < PIECES_PER; ++k) {
+            const uint4 r = b0 + k < nblocks ? bv[b0 + k] : make_uint4(0, 0, 0, 0);
+            own += rows[k] = r.y != r.x ? r.y - r.x + block_cost : 0;
         }
         uint64_t incl = own;
 #pragma unroll
@@ -573,14 +555,14 @@ __global__ void __launch_bounds__(ITEMS_T) k_items(const uint4 *__restrict__ bv,
         if (lane == 31) warp_s[warp] = incl;
         __syncthreads();
         uint64_t at = before + incl - own;
-        for (uint32_t w = 0; w < ITEMS_T / 32; ++w) {
+        for (uint32_t w = 0; w < PIECES_T / 32; ++w) {
             if (w < warp) at += warp_s[w];
             before += warp_s[w];
         }
 #pragma unroll
-        for (uint32_t k = 0; k < ITEMS_PER; ++k) {
+        for (uint32_t k = 0; k < PIECES_PER; ++k) {
             if (b0 + k < nblocks) prefix[b0 + k] = at;
-            at += items[k];
+            at += rows[k];
         }
     }
     if (threadIdx.x == 0) prefix[nblocks] = before;
@@ -649,7 +631,7 @@ __device__ void build_rows(const uint64_t *__restrict__ us, const FamDev &F, uin
 }
 
 constexpr int CBW = 64;                 // bitmap words per cheap-tier filter (q <= 2047)
-constexpr uint64_t ITEM_GRAB = 2;       // fewest work items a CTA claims at a time
+constexpr uint32_t ITEM_ROWS = 1u << 20;   // most v rows of a work item (a ring entry holds the row in 20 bits)
 // Survivor ring per warp (pending < 64 by construction).  An entry is one word pair: the record's
 // index in the work item (< 2^20) | the bit's position in the block (< 2^12) << 20, and the
 // survivor's subtile slot; the drain reads the v row's cheap-tier residues by the record index.
@@ -665,7 +647,7 @@ __host__ __device__ constexpr uint32_t round16(uint32_t x) { return (x + 15) & ~
 // residue-row patterns are only read while rows are built, when every survivor ring is empty,
 // so they share the rings' space.
 struct MatchSmem {
-    uint32_t rows, ures, ring, lq, pat, cbits, cnt, fam, seg, misc, total;
+    uint32_t rows, ures, ring, lq, pat, cbits, cnt, fam, seg, misc, place, total;
     __host__ __device__ MatchSmem(uint32_t total_rows, uint32_t K, uint32_t nb, uint32_t nch, uint32_t tmax,
                                   uint32_t ng, uint32_t warps) {
         rows = 0;
@@ -679,8 +661,9 @@ struct MatchSmem {
         fam = cnt + round16(tmax * (ng + 2) * 4);
         seg = fam + round16(sizeof(FamDev));
         misc = seg + round16(sizeof(SegDev));
-        total = misc + 32;   // deep counter (4 B), the item grab (8 B at +8), the item's first subtile and
-                             // its segment's subtile end (8 B each at +16 and +24)
+        place = misc + 32;   // after the deep counter (4 B), the item's first subtile and its segment's subtile end
+                             // (8 B each at +16 and +24)
+        total = place + 48;
     }
 };
 
@@ -773,51 +756,75 @@ __global__ void __launch_bounds__(NT, 1) k_match(const MatchArgs a) {
     if (threadIdx.x == 0) *deep_ctr = 0;
     uint4 *deep_slice = a.deep + (size_t)blockIdx.x * a.deep_cap;
 
-    const uint64_t n_items = a.item_prefix[a.nblocks];
-    const uint64_t vch = *a.vchunk;
-    uint64_t cur = UINT64_MAX, bsearch = 0;
+    uint64_t cur = UINT64_MAX;
     uint32_t cur_seg = UINT32_MAX, cur_fam = UINT32_MAX;
     const uint32_t nch = a.nch;
-    unsigned long long *grab_s = (unsigned long long *)(base + L.misc + 8);
 
-    // Items are handed out in ascending order from one device counter, so the CTAs work on
-    // neighbouring blocks together: the per-v records of those blocks stay in L2, and the CTAs
-    // finish within one grab of each other.  A grab takes as many items as a block averages (at
-    // least ITEM_GRAB), so a block cut into several items is mostly built by one CTA once, but
-    // never more than a quarter of an even share, so every CTA gets work.  A launch of fewer than
-    // eight items per CTA (one batch) gives each CTA one even share of consecutive items, which
-    // mostly lie in one block, so the rows of a block are built about once per CTA that meets it.
-    const uint64_t ncta = gridDim.x;
-    const uint64_t grab = n_items >= 8 * ncta
-                              ? umax64(ITEM_GRAB, umin64(n_items / umax64(1, a.nblocks), n_items / (4 * ncta)))
-                              : umax64(1, (n_items + ncta - 1) / ncta);
-    uint64_t it = 0, it_end = 0;
+    // A CTA works through shares: its first is its own number, further ones are claimed in ascending order, so the
+    // CTAs work on neighbouring blocks and the per-v records of those blocks stay in L2.  In a launch of many blocks
+    // per CTA a share is two whole blocks, at the end one.  In others all work, in block order, is cut
+    // into one even part per CTA: a block's fixed cost (building its rows, draining its survivors) and its v rows; the
+    // CTAs then finish together whatever the blocks' sizes, and a block is built by one CTA or two.  (Equal numbers of
+    // equally long items per CTA, 3,584 rows or more, left 33 SMs of a batch idle and drained 5,289 items of 24
+    // batches: batch 128 -> 85 us, 24 batches 1.59 -> 1.04 ms, 48 windows 0.93 -> 0.59 ms.)
+    // The place in the share stays in shared memory (place): no register holds it through the unit loop.
+    struct Place {
+        uint64_t share, b, b_end, at, at_end;             // next share; next block, end of the share's blocks, its work
+        uint32_t row, first;                              // rows of block b that are done; b is the share's first
+    };
+    volatile Place &place = *(volatile Place *)(base + L.place);
+    if (threadIdx.x == 0) place.share = blockIdx.x, place.b = place.b_end = 0;
+    __syncthreads();
     for (;;) {
-        if (it == it_end) {
-            __syncthreads();                              // every thread has read the previous grab
-            if (threadIdx.x == 0) *grab_s = atomicAdd(a.item_next, (unsigned long long)grab);
-            __syncthreads();
-            it = *grab_s;
-            if (it >= n_items) break;
-            it_end = umin64(it + grab, n_items);
-            uint64_t lo = 0, hi = a.nblocks;              // block of item it: last b with prefix[b] <= it
-            while (hi - lo > 1) {
-                const uint64_t mid = (lo + hi) / 2;
-                if (a.item_prefix[mid] <= it) lo = mid;
-                else hi = mid;
+        uint64_t b = place.b;
+        uint32_t row = place.row;
+        if (b >= place.b_end) {
+            const uint64_t share = place.share;
+            if (share >= a.shares) break;
+            uint64_t b_end, at = 0, at_end = 0;
+            if (a.whole) {
+                b = share < a.pairs ? 2 * share : a.pairs + share;
+                b_end = b + (share < a.pairs ? 2 : 1);
+            } else {
+                const uint64_t work = a.prefix[a.nblocks];
+                at = work * share / a.shares;
+                at_end = work * (share + 1) / a.shares;
+                b_end = b = group_count_le64<5>(a.prefix, a.nblocks, at, lane) - 1;     // last block that starts at or before it
+                if (at != at_end) b_end = group_count_le64<5>(a.prefix, a.nblocks, at_end - 1, lane);
             }
-            bsearch = lo;
+            __syncthreads();                              // every thread has read the place
+            if (threadIdx.x == 0) {
+                place.b = b, place.b_end = b_end, place.at = at, place.at_end = at_end;
+                place.row = 0, place.first = 1;
+                place.share = gridDim.x + atomicAdd(a.share_next, 1ull);
+            }
+            __syncthreads();
+            continue;
         }
-        while (a.item_prefix[bsearch + 1] <= it) ++bsearch;  // items of one grab are consecutive
-        const uint64_t b = bsearch;
         const uint4 range = a.bv[b];
-        const uint64_t va = range.x + (it - a.item_prefix[b]) * vch;
-        const uint32_t nv_item = (uint32_t)(umin64(range.y, va + vch) - va);   // <= 2^20
+        uint32_t rows_end = range.y - range.x;            // rows of the block in this share
+        if (!a.whole) {
+            const uint64_t start = a.prefix[b] + a.block_cost, at = place.at, at_end = place.at_end;
+            if (at_end < start + rows_end) rows_end = at_end > start ? (uint32_t)(at_end - start) : 0;
+            if (place.first && row == 0 && at > start) row = (uint32_t)umin64(at - start, rows_end);
+        }
+        const uint64_t va = range.x + row;
+        const uint32_t nv_item = min(rows_end - row, a.v_chunk);   // <= 2^20
+        __syncthreads();                                  // every thread has read the place
+        if (threadIdx.x == 0) {                           // the next item (the item's syncs come before its use)
+            const bool done = row + nv_item == rows_end;
+            place.b = done ? b + 1 : b;
+            place.row = done ? 0 : row + nv_item;
+            if (done) place.first = 0;
+        }
+        if (!nv_item) {
+            __syncthreads();
+            continue;
+        }
         // rows of this item covering the whole block, relative to va
         const uint32_t full_lo = (uint32_t)(range.z > va ? umin64(range.z - va, nv_item) : 0);
         const uint32_t full_hi = (uint32_t)(range.w > va ? umin64(range.w - va, nv_item) : 0);
         const uint32_t block_u0 = (uint32_t)(b * G::UB);
-        __syncthreads();                                  // previous item finished with shared memory
         if (b != cur) {
             const uint32_t sg = a.blk_seg[b];
             if (sg != cur_seg) {
@@ -1076,7 +1083,6 @@ __global__ void __launch_bounds__(NT, 1) k_match(const MatchArgs a) {
                     atomicAdd((unsigned long long *)&a.counts[tile * a.stride + g], (unsigned long long)cv);
             }
         }
-        ++it;
     }
     __syncthreads();
     if (threadIdx.x == 0) a.deep_count[blockIdx.x] = *deep_ctr;
@@ -1633,7 +1639,7 @@ struct Engine {
     uint64_t *d_prefix = nullptr;
     // Everything a run reports lies together, in this order, so that one fill resets it and one copy fetches it:
     // scalars, deep survivors per CTA, counters, envelopes, output records.
-    enum { STUCK, NOUT, BAD, ITEM_NEXT, PIECES, VCHUNK, SCALARS = 8 };    // STUCK: the window pass gave up
+    enum { STUCK, NOUT, BAD, SHARE_NEXT, SCALARS };    // STUCK: the window pass gave up
     bool windows = false;                                 // the window pass is the owner's: STUCK is not reset
     uint64_t *d_report = nullptr;
     uint64_t o_deep = 0, o_counts = 0, o_geo = 0, o_out = 0;   // word offsets
@@ -1717,6 +1723,14 @@ int engine_prepare(Engine &E, const pc_tuning *tuning, Scratch &hold) {
     return PC_OK;
 }
 
+// What a block costs beyond its v rows, in rows: building sum(q) rows and the ends of its item took 26 us where
+// 215 v rows of seven filters take a microsecond (p = 619: sum(q) = 1567).
+uint32_t block_cost(const Engine &E) {
+    uint32_t rows = 0;
+    for (const FamDev &d : E.famdev) rows = std::max(rows, d.total_rows);
+    return rows * 25 / E.tn.nb;
+}
+
 // mode 0: set the shared-memory attribute and launch; 1: launch only (inside a capture);
 // 2: set the attribute only.
 int engine_match(Engine &E, int mode) {
@@ -1734,13 +1748,20 @@ int engine_match(Engine &E, int mode) {
     for (const FamDev &d : E.famdev) ma.total_rows = std::max(ma.total_rows, d.total_rows);
     ma.counts = E.d_counts();
     ma.bv = E.d_bv;
-    ma.item_prefix = E.d_prefix;
+    ma.prefix = E.d_prefix;
     ma.nblocks = E.nblocks;
-    ma.vchunk = E.d_report + Engine::VCHUNK;
+    // Whole blocks from 16 blocks per CTA on: the CTAs then end within a block of each other, which costs less than
+    // the second building of the blocks that a cut divides.
+    const uint64_t grid = E.grid;
+    ma.whole = E.nblocks >= 16 * grid;
+    ma.pairs = ma.whole ? (uint32_t)((E.nblocks - 2 * grid) / 2) : 0;
+    ma.shares = ma.whole ? (uint32_t)E.nblocks - ma.pairs : (uint32_t)grid;
+    ma.block_cost = block_cost(E);
+    ma.v_chunk = (uint32_t)std::min<uint64_t>(E.tn.v_chunk ? E.tn.v_chunk : ITEM_ROWS, ITEM_ROWS);
     ma.deep = E.d_deep;
     ma.deep_cap = E.deep_cap;
     ma.deep_count = E.d_deep_count();
-    ma.item_next = E.scalar(Engine::ITEM_NEXT);
+    ma.share_next = E.scalar(Engine::SHARE_NEXT);
     if (E.tn.threads == 1024) return launch_match_n<1024>(E.ctx, ma, E.tn.nb, E.tn.K, E.smem, E.grid, mode);
     if (E.tn.threads == 896) return launch_match_n<896>(E.ctx, ma, E.tn.nb, E.tn.K, E.smem, E.grid, mode);
     if (E.tn.threads == 768) return launch_match_n<768>(E.ctx, ma, E.tn.nb, E.tn.K, E.smem, E.grid, mode);
@@ -1792,11 +1813,10 @@ int engine_launch(Engine &E, bool events, bool capturing, int *launches) {
     if (events) PC_CHECK(ctx, cudaEventRecord(ctx->ev[1], st));
     if (E.nu && E.nv) {
         k_blocks<<<(unsigned)((E.nblocks + 7) / 8), 256, 0, st>>>(E.d_rec, E.d_seg, (uint32_t)E.segs.size(), E.tn.K * 32,
-                                                                E.nblocks, E.d_bv, E.d_blk_seg, E.scalar(Engine::PIECES));
+                                                                E.nblocks, E.d_bv, E.d_blk_seg);
         PC_LAUNCHED(ctx, "blocks");
-        k_items<<<1, ITEMS_T, 0, st>>>(E.d_bv, E.nblocks, E.scalar(Engine::PIECES), E.tn.v_chunk, (uint64_t)E.grid * 32,
-                                       4 * (uint64_t)E.tn.threads, E.d_report + Engine::VCHUNK, E.d_prefix);
-        PC_LAUNCHED(ctx, "items");
+        k_pieces<<<1, PIECES_T, 0, st>>>(E.d_bv, E.nblocks, block_cost(E), E.d_prefix);
+        PC_LAUNCHED(ctx, "pieces");
         if (events) PC_CHECK(ctx, cudaEventRecord(ctx->ev[2], st));
         const int rc = engine_match(E, capturing ? 1 : 0);
         if (rc) return rc;
