@@ -230,6 +230,54 @@ __device__ __forceinline__ uint32_t transpose32c(uint32_t x, const uint32_t (&sh
     return x;
 }
 
+// The same for two matrices at once.  Every exchange moves half of each word, so one shuffle carries the halves
+// of both: five shuffles instead of ten, which share the load/store pipe with everything around them.
+struct TransposePair {
+    uint32_t send[2], a[2], b[2];                        // byte selectors of the rounds of 16 and 8
+    uint32_t up[3], keep[3];                             // shift and kept bits of the rounds of 4, 2 and 1
+    __device__ __forceinline__ explicit TransposePair(uint32_t lane) {
+        const bool u16 = lane & 16, u8 = lane & 8;
+        send[0] = u16 ? 0x5410u : 0x7632u, a[0] = u16 ? 0x3254u : 0x5410u, b[0] = u16 ? 0x3276u : 0x7610u;
+        send[1] = u8 ? 0x6420u : 0x7531u, a[1] = u8 ? 0x3514u : 0x5240u, b[1] = u8 ? 0x3716u : 0x7260u;
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            up[r] = ~lane & (4u >> r);                   // j for the lower lane of a pair, 0 for the upper
+            keep[r] = up[r] ? ~half(r) : half(r);
+        }
+    }
+    __device__ static __forceinline__ constexpr uint32_t half(int r) {
+        return r == 0 ? 0xf0f0f0f0u : r == 1 ? 0xccccccccu : 0xaaaaaaaau;
+    }
+    // N pairs v[0], v[1]; v[2], v[3]; ... round by round, so that their shuffles overlap.
+    template <int N>
+    __device__ __forceinline__ void operator()(uint32_t *v) const {
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            uint32_t p[N];
+#pragma unroll
+            for (int i = 0; i < N; ++i) p[i] = __shfl_xor_sync(0xffffffffu, __byte_perm(v[2 * i], v[2 * i + 1], send[r]), 16u >> r);
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+                v[2 * i] = __byte_perm(v[2 * i], p[i], a[r]);
+                v[2 * i + 1] = __byte_perm(v[2 * i + 1], p[i], b[r]);
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {                    // the upper lane sends its lower half, the lower lane its upper
+            const uint32_t h = half(r), j = 4u >> r, u = up[r], d = j - u;
+            uint32_t p[N];
+#pragma unroll
+            for (int i = 0; i < N; ++i)
+                p[i] = __shfl_xor_sync(0xffffffffu, ((v[2 * i] >> u) & ~h) | ((v[2 * i + 1] << d) & h), j);
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+                v[2 * i] = (v[2 * i] & keep[r]) | ((p[i] << u) & ~keep[r]);
+                v[2 * i + 1] = (v[2 * i + 1] & keep[r]) | ((p[i] >> d) & ~keep[r]);
+            }
+        }
+    }
+};
+
 // Entries of a sorted range of n for which `below(index)` holds (a prefix of it), by each group of eight lanes of a
 // warp for its own range: three bits a step, where a thread alone takes one dependent load per bit.
 template <class F>

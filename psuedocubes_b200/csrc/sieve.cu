@@ -76,10 +76,9 @@ struct SegDev {
 // filters 0..NB-1, cheap-tier filters NB..NB+nch-1, the rest in k_deep.
 struct FamDev {
     uint32_t nres, ng, total_rows, c2_live;   // c2_live: group 2 ends at the last bitset filter
-    uint32_t q[PC_MAX_BITSET], row0[PC_MAX_BITSET], ainvb[PC_MAX_BITSET];
-    ModQ mq[PC_MAX_BITSET];
-    uint32_t cq[PC_MAX_CHEAP], caq[PC_MAX_CHEAP], cbq[PC_MAX_CHEAP], cbits_off[PC_MAX_CHEAP];
-    ModQ cmq[PC_MAX_CHEAP];
+    uint32_t q[PC_MAX_BITSET], row0[PC_MAX_BITSET];
+    uint32_t cq[PC_MAX_CHEAP], cbits_off[PC_MAX_CHEAP];
+    uint4 umod[PC_MAX_BITSET + PC_MAX_CHEAP];   // pack_mod of the bitset filters with B A^-1 mod q, of the cheap tier with B mod q
     uint8_t bgroup[16];              // group ended by filter idx (0 = none), idx < NB + nch
     uint32_t cqg[PC_MAX_CHEAP];      // cheap-tier filter t: q | the group it ends (bgroup[NB + t]) << 16
     const uint32_t *pat;
@@ -134,16 +133,6 @@ __device__ __forceinline__ uint64_t count_le(const uint64_t *__restrict__ us, ui
     return lo;
 }
 
-__device__ __forceinline__ uint64_t lower_bound64(const uint64_t *__restrict__ a, uint64_t n, uint64_t key) {
-    uint64_t lo = 0, hi = n;
-    while (lo < hi) {
-        uint64_t mid = lo + (hi - lo) / 2;
-        if (__ldg(a + mid) < key) lo = mid + 1;
-        else hi = mid;
-    }
-    return lo;
-}
-
 // Subtile of v inside a segment, floor((v - v_first) / width), or ntiles when v lies outside.
 // The double estimate is within one of the quotient (quotients are below 2^31), and the host
 // guarantees ntiles * width < 2^64.
@@ -188,7 +177,7 @@ struct SegPrep {
 };
 
 struct FamPrep {
-    uint4 f[PC_MAX_BITSET + PC_MAX_CHEAP];   // 2^16 | 2^32 << 16, 2^48 | q << 16 (all mod q), floor(2^32 / q), row0 or A mod q
+    uint4 f[PC_MAX_BITSET + PC_MAX_CHEAP];   // pack_mod of the bitset filters with row0, of the cheap tier with A mod q
 };
 
 struct PrepArgs {
@@ -213,6 +202,13 @@ constexpr uint32_t PREP_T = 256;       // threads per CTA; a CTA takes PREP_T x 
 __device__ __forceinline__ uint32_t mod_short(uint32_t x, uint32_t m, uint32_t q) {
     const uint32_t r = x - __umulhi(x, m) * q;
     return __viaddmin_u32(r, 0u - q, r);
+}
+
+// v mod q for a pack_mod entry: 2^16 | 2^32 << 16, 2^48 | q << 16 (all mod q), floor(2^32 / q), a factor.
+__device__ __forceinline__ uint32_t residue(const uint4 f, uint64_t v) {
+    const uint32_t lo = (uint32_t)v, hi = (uint32_t)(v >> 32);
+    return mod_short((lo & 0xffffu) + (lo >> 16) * (f.x & 0xffffu) + (hi & 0xffffu) * (f.x >> 16) + (hi >> 16) * (f.y & 0xffffu),
+                     f.z, f.y >> 16);
 }
 
 // U = floor((v A + lo) / B) or, for the upper bound, floor((v A + hi) / B), and its remainder: the number of
@@ -302,11 +298,6 @@ __global__ void __launch_bounds__(PREP_T) k_vprep(const PrepArgs a) {
     const uint32_t s0 = seg_of_v(a.seg, a.nseg, j0);
     const SegDev &g0 = a.seg[s0];
     const SegPrep &p0 = a.segp[s0];
-    auto residue = [](const uint4 f, uint64_t v) {        // v mod q of a FamPrep entry
-        const uint32_t lo = (uint32_t)v, hi = (uint32_t)(v >> 32);
-        return mod_short((lo & 0xffffu) + (lo >> 16) * (f.x & 0xffffu) + (hi & 0xffffu) * (f.x >> 16) + (hi >> 16) * (f.y & 0xffffu),
-                         f.z, f.y >> 16);
-    };
     bool near = j1 <= (uint64_t)g0.v_off + g0.nv && p0.fast;      // rows as distances from the first; CTA-uniform
     bool staged = false;
     uint64_t v_first = 0, first[2] = {}, count[2] = {};
@@ -578,53 +569,94 @@ struct Geo {
     __device__ static __forceinline__ uint32_t unit(uint32_t row, uint32_t c) { return row * U + c; }
 };
 
-// Residue rows of the family's first NB filters for one block (entries >= n_valid are zero), and
-// the residues u*B mod q of its cheap-tier filters.
+// Residues of the block's u entries: t = u B A^-1 mod q of the bitset filters (t_s) and u B mod q of the cheap tier
+// (ures).  A warp takes 32 entries and every other filter.
 template <int NB, int K>
-__device__ void build_rows(const uint64_t *__restrict__ us, const FamDev &F, uint32_t nch, uint4 *__restrict__ rows,
-                           uint16_t *__restrict__ ures, const uint32_t *__restrict__ pat_s, uint32_t block_u0,
-                           uint32_t n_valid, uint32_t lane, uint32_t warp, uint32_t nwarps) {
-    using G = Geo<K>;
-    const uint64_t *ub = us + block_u0;
-    for (uint32_t k = threadIdx.x; k < G::UB; k += blockDim.x) {
-        const uint64_t u = k < n_valid ? __ldg(ub + k) : 0;
-        for (uint32_t t = 0; t < nch; ++t)
-            ures[t * G::UB + k] = (uint16_t)fastmod32(mod64(u, F.cmq[t]) * F.cbq[t], F.cmq[t].c, F.cq[t]);
-    }
-    // A warp builds all q rows of one filter for two 16-byte units, c and c + U/2 (4 words = 128 u
-    // each).  Its lanes store the two units in two steps, half the lanes writing each unit, so a
-    // quarter-warp store meets two bank groups instead of one.
-    uint32_t sh[5], keep[5];                              // per-lane transpose constants
-    transpose_consts(lane, sh, keep);
-    constexpr uint32_t HU = G::U / 2;
-    const bool hi_first = lane & 4;
-    for (uint32_t item = warp; item < NB * HU; item += nwarps) {
-        const uint32_t f = item / HU, c = item % HU;
-        const uint32_t q = F.q[f];
-        uint32_t t[8];
-        bool valid[8];
+__device__ __forceinline__ void block_residues(const uint64_t *__restrict__ us, const FamDev &F, uint32_t nch,
+                                               uint16_t *__restrict__ t_s, uint16_t *__restrict__ ures, uint32_t block_u0,
+                                               uint32_t n_valid, uint32_t lane, uint32_t warp, uint32_t nwarps) {
+    constexpr uint32_t UB = Geo<K>::UB;
+    for (uint32_t task0 = warp; task0 < 2 * K; task0 += 3 * nwarps) {
+        uint64_t u[3];                                    // loaded together: 64 tasks are three turns of 28 warps
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const uint32_t local = ((c + (k >> 2) * HU) * 4 + (k & 3)) * 32 + lane;
-            valid[k] = local < n_valid;
-            const uint32_t um = valid[k] ? mod64(__ldg(ub + local), F.mq[f]) : 0;
-            t[k] = fastmod32(um * F.ainvb[f], F.mq[f].c, q);
+        for (uint32_t i = 0; i < 3; ++i) {
+            const uint32_t task = task0 + i * nwarps, k = task / 2 * 32 + lane;
+            u[i] = task < 2 * K && k < n_valid ? __ldg(us + block_u0 + k) : 0;
         }
-        const uint32_t *p = pat_s + f * PATW;
-        const uint32_t row0 = F.row0[f];
-        for (uint32_t g = 0; g * 32 < q; ++g) {
-            uint32_t w[8];
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const uint32_t st = 32 * g + q - t[k];
-                const uint32_t col = __funnelshift_r(p[st >> 5], p[(st >> 5) + 1], st & 31);
-                w[k] = transpose32c(valid[k] ? col : 0u, sh, keep);
+        for (uint32_t i = 0; i < 3; ++i) {
+            const uint32_t task = task0 + i * nwarps, k = task / 2 * 32 + lane, odd = task & 1;
+            if (task >= 2 * K) break;
+            auto put = [&](uint32_t f, uint16_t *to) {
+                const uint4 m = F.umod[f];
+                to[k] = (uint16_t)mod_short(residue(m, u[i]) * m.w, m.z, m.y >> 16);
+            };
+#pragma unroll
+            for (uint32_t h = 0; h < (NB + 1) / 2; ++h) {
+                const uint32_t f = 2 * h + odd;
+                if (f < NB) put(f, t_s + f * UB);
             }
-            const uint32_t r = 32 * g + lane;
+#pragma unroll
+            for (uint32_t h = 0; h < PC_MAX_CHEAP / 2; ++h) {
+                const uint32_t c = 2 * h + odd;
+                if (c < nch) put(PC_MAX_BITSET + c, ures + c * UB);
+            }
+        }
+    }
+}
+
+// Residue rows of the family's first NB filters for one block (entries >= n_valid are zero).  A warp builds 32 rows
+// of one filter, four 16-byte units at a time: a lane's column of a word is the filter's
+// pattern from offset 32 g + q - t on, one funnel shift, and a warp transpose turns 32 columns into 32 rows' words.
+// Before they are stored the lanes rotate their units, so that at each store eight neighbouring lanes, whose rows
+// lie a multiple of the banks apart, write four different units.  (Two units per warp and filter, stored from two
+// lane halves, met four bank conflicts a store and ten shuffles per word pair: 15.5 us of a block's 18; now 11 of 16.5.
+// Eight units at a time have no conflicts, but their 32 words spill: 13.4.)
+template <int NB, int K>
+__device__ __forceinline__ void build_rows(const FamDev &F, uint4 *__restrict__ rows, const uint16_t *__restrict__ t_s,
+                                           const uint32_t *__restrict__ pat_s, uint32_t n_valid, uint32_t lane, uint32_t warp,
+                                           uint32_t nwarps) {
+    using G = Geo<K>;
+    constexpr uint32_t UN = 4;                            // units at a time
+    const TransposePair transpose(lane);
+    const uint32_t turn = G::U == 4 ? (lane >> 1) & 3 : lane & 3;
+    uint32_t f = 0, g = warp;                             // 32-row group g of filter f
+    for (;; g += nwarps) {
+        while (f < NB && g >= (F.q[f] + 31) / 32) g -= (F.q[f] + 31) / 32, ++f;
+        if (f >= NB) return;
+        const uint32_t q = F.q[f], r = 32 * g + lane;
+        const uint32_t *p = pat_s + f * PATW;
+        const uint16_t *t = t_s + f * G::UB + lane;
+#pragma unroll 1
+        for (uint32_t u0 = 0; u0 < G::U; u0 += UN) {
+            uint32_t w[4 * UN];
+#pragma unroll
+            for (uint32_t k = 0; k < 4 * UN; ++k) {
+                const uint32_t st = 32 * g + q - t[u0 * 128 + k * 32];
+                w[k] = __funnelshift_r(p[st >> 5], p[(st >> 5) + 1], st & 31);
+            }
+            transpose.operator()<UN>(w);
+            transpose.operator()<UN>(w + 2 * UN);
+            if (n_valid < G::UB) {
+#pragma unroll
+                for (uint32_t k = 0; k < 4 * UN; ++k) {
+                    const uint32_t first = u0 * 128 + k * 32;
+                    w[k] &= low_bits(n_valid > first ? min(n_valid - first, 32u) : 0u);
+                }
+            }
+#pragma unroll
+            for (uint32_t s = 1; s < UN; s *= 2) {        // unit u becomes unit (u + turn) % UN
+                uint32_t x[4 * UN];
+#pragma unroll
+                for (uint32_t k = 0; k < 4 * UN; ++k) x[k] = turn & s ? w[(k + 4 * s) % (4 * UN)] : w[k];
+#pragma unroll
+                for (uint32_t k = 0; k < 4 * UN; ++k) w[k] = x[k];
+            }
             if (r < q) {
-                const uint4 lo = make_uint4(w[0], w[1], w[2], w[3]), hi = make_uint4(w[4], w[5], w[6], w[7]);
-                rows[G::unit(row0 + r, hi_first ? c + HU : c)] = hi_first ? hi : lo;
-                rows[G::unit(row0 + r, hi_first ? c : c + HU)] = hi_first ? lo : hi;
+                uint4 *row = rows + G::unit(F.row0[f] + r, u0);
+#pragma unroll
+                for (uint32_t u = 0; u < UN; ++u)
+                    row[(u + turn) & (UN - 1)] = make_uint4(w[4 * u], w[4 * u + 1], w[4 * u + 2], w[4 * u + 3]);
             }
         }
     }
@@ -643,18 +675,19 @@ constexpr int LCAP = 32;
 
 __host__ __device__ constexpr uint32_t round16(uint32_t x) { return (x + 15) & ~15u; }
 
-// Shared-memory layout of k_match (byte offsets); every region starts 16-byte aligned.  The
-// residue-row patterns are only read while rows are built, when every survivor ring is empty,
+// Shared-memory layout of k_match (byte offsets); every region starts 16-byte aligned.  The u entries' residues t and
+// the residue-row patterns are only read while rows are built, when every survivor ring is empty,
 // so they share the rings' space.
 struct MatchSmem {
-    uint32_t rows, ures, ring, lq, pat, cbits, cnt, fam, seg, misc, place, total;
+    uint32_t rows, ures, ring, lq, t, pat, cbits, cnt, fam, seg, misc, place, total;
     __host__ __device__ MatchSmem(uint32_t total_rows, uint32_t K, uint32_t nb, uint32_t nch, uint32_t tmax,
                                   uint32_t ng, uint32_t warps) {
         rows = 0;
         ures = rows + total_rows * (K / 4) * 16;
         ring = ures + round16(nch * K * 32 * 2);
         lq = ring + warps * QCAP * 8;
-        pat = ring;
+        t = ring;
+        pat = t + nb * K * 32 * 2;
         const uint32_t ring_end = lq + warps * LCAP * 4, pat_end = pat + nb * PATW * 4;
         cbits = round16(ring_end > pat_end ? ring_end : pat_end);
         cnt = cbits + nch * CBW * 4;
@@ -841,11 +874,12 @@ __global__ void __launch_bounds__(NT, 1) k_match(const MatchArgs a) {
                 cur_seg = sg;
                 cur_fam = fm;
             }
-            for (uint32_t i = threadIdx.x; i < NB * PATW; i += blockDim.x) pat_s[i] = F.pat[i];
-            __syncthreads();
             const uint32_t u_end = S.u_off + S.nu;
             const uint32_t n_valid = u_end > block_u0 ? min(u_end - block_u0, (uint32_t)G::UB) : 0u;
-            build_rows<NB, K>(a.us, F, nch, (uint4 *)rows, ures, pat_s, block_u0, n_valid, lane, warp, nwarps);
+            for (uint32_t i = threadIdx.x; i < NB * PATW; i += blockDim.x) pat_s[i] = F.pat[i];
+            block_residues<NB, K>(a.us, F, nch, (uint16_t *)(base + L.t), ures, block_u0, n_valid, lane, warp, nwarps);
+            __syncthreads();
+            build_rows<NB, K>(F, (uint4 *)rows, (const uint16_t *)(base + L.t), pat_s, n_valid, lane, warp, nwarps);
             cur = b;
         }
         for (uint32_t k = threadIdx.x; k < a.tmax * cstride; k += blockDim.x) cnt_s[k] = 0;
@@ -990,10 +1024,17 @@ __global__ void __launch_bounds__(NT, 1) k_match(const MatchArgs a) {
             queue_bits(acc, u, rel, slot);
         };
 
-        // a warp takes consecutive rounds, so its lanes stay in one subtile for many rounds
-        const uint32_t nrounds = (nv_item + 31) / 32, per_warp = (nrounds + nwarps - 1) / nwarps;
-        const uint32_t r_end = min(nrounds, (warp + 1) * per_warp);
-        for (uint32_t r = warp * per_warp; r < r_end; ++r) {
+        // a warp takes consecutive rounds, so its lanes stay in one subtile for many rounds; a round whose rows cover
+        // only part of the block (the item's first and last ones) counts 9, a full one 8 (a lease: 10.51 ms, 10.53 at
+        // 17 : 16, 10.59 at 1 : 1 and 10.79 with equal runs rounded up)
+        const uint32_t nrounds = (nv_item + 31) / 32;
+        const uint32_t fr = min((full_lo + 31) / 32, nrounds), lr = max(fr, full_hi / 32);    // the full rounds
+        const uint32_t w1 = 9 * fr, w2 = w1 + 8 * (lr - fr), weight = w2 + 9 * (nrounds - lr);
+        auto round_at = [&](uint32_t x) {
+            return x <= w1 ? (x + 8) / 9 : x <= w2 ? fr + (x - w1 + 7) / 8 : lr + (x - w2 + 8) / 9;
+        };
+        const uint32_t r_end = round_at((warp + 1) * weight / nwarps);
+        for (uint32_t r = round_at(warp * weight / nwarps); r < r_end; ++r) {
             const uint32_t rel = r * 32 + lane;
             const bool active = rel < nv_item;
             VRec rec{};
@@ -1553,6 +1594,12 @@ int resolve_tuning(pc_ctx *ctx, const std::vector<const pc_filters *> &fams, con
     }
 }
 
+// q < 2^11 and a factor below q as residue() and mod_short() use them.
+uint4 pack_mod(uint32_t q, uint32_t factor) {
+    const ModQ m = make_modq(q);
+    return make_uint4(m.r16[0] | m.r16[1] << 16, m.r16[2] | q << 16, (uint32_t)(m.c >> 32), factor);
+}
+
 FamDev fam_dev(const pc_filters *f, uint32_t nb, uint32_t nch) {
     FamDev d{};
     d.nres = f->nres;
@@ -1562,15 +1609,12 @@ FamDev fam_dev(const pc_filters *f, uint32_t nb, uint32_t nch) {
     for (uint32_t i = 0; i < nb; ++i) {
         d.q[i] = f->primes[i];
         d.row0[i] = f->rows_sum[i];
-        d.ainvb[i] = f->ainvb[i];
-        d.mq[i] = make_modq(f->primes[i]);
+        d.umod[i] = pack_mod(f->primes[i], f->ainvb[i]);
     }
     for (uint32_t t = 0; t < nch; ++t) {
         const uint32_t q = f->primes[nb + t];
         d.cq[t] = q;
-        d.caq[t] = (uint32_t)(f->A % q);
-        d.cbq[t] = (uint32_t)(f->B % q);
-        d.cmq[t] = make_modq(q);
+        d.umod[PC_MAX_BITSET + t] = pack_mod(q, (uint32_t)(f->B % q));
         d.cbits_off[t] = f->fcs[nb + t].tab_off;
     }
     for (uint32_t idx = 0; idx < 16; ++idx)
@@ -1582,13 +1626,10 @@ FamDev fam_dev(const pc_filters *f, uint32_t nb, uint32_t nch) {
     return d;
 }
 
-FamPrep fam_prep(const FamDev &d, uint32_t nb, uint32_t nch) {
+FamPrep fam_prep(const pc_filters *f, const FamDev &d, uint32_t nb, uint32_t nch) {
     FamPrep p{};
-    auto pack = [](const ModQ &m, uint32_t w) {
-        return make_uint4(m.r16[0] | m.r16[1] << 16, m.r16[2] | m.q << 16, (uint32_t)(m.c >> 32), w);
-    };
-    for (uint32_t t = 0; t < nb; ++t) p.f[t] = pack(d.mq[t], d.row0[t]);
-    for (uint32_t t = 0; t < nch; ++t) p.f[PC_MAX_BITSET + t] = pack(d.cmq[t], d.caq[t]);
+    for (uint32_t t = 0; t < nb; ++t) p.f[t] = pack_mod(d.q[t], d.row0[t]);
+    for (uint32_t t = 0; t < nch; ++t) p.f[PC_MAX_BITSET + t] = pack_mod(d.cq[t], (uint32_t)(f->A % d.cq[t]));
     return p;
 }
 
@@ -1681,7 +1722,7 @@ int engine_prepare(Engine &E, const pc_tuning *tuning, Scratch &hold) {
     E.segprep.clear();
     for (const pc_filters *f : E.fams) {
         E.famdev.push_back(fam_dev(f, E.tn.nb, E.tn.nch));
-        E.famprep.push_back(fam_prep(E.famdev.back(), E.tn.nb, E.tn.nch));
+        E.famprep.push_back(fam_prep(f, E.famdev.back(), E.tn.nb, E.tn.nch));
     }
     for (const SegDev &g : E.segs) E.segprep.push_back(seg_prep(g));
     E.grid = ctx->sm_count;
