@@ -35,7 +35,7 @@ struct pc_buf {
 
 int pc_fail(pc_ctx *ctx, int code, const std::string &msg);
 int pc_cuda_fail(pc_ctx *ctx, cudaError_t e, const char *what);
-constexpr uint64_t PC_STAGE_BYTES = UINT64_C(512) << 10;
+constexpr uint64_t PC_STAGE_BYTES = UINT64_C(4) << 20;   // a lease's counters and envelopes: 3.8 MB
 // The context's page-locked stage, or null when `bytes` do not fit it or it cannot be had.  Its content is the
 // caller's until the next library call on the context.
 uint64_t *pc_stage(pc_ctx *ctx, uint64_t bytes);

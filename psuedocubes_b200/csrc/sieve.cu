@@ -284,11 +284,12 @@ __device__ __forceinline__ uint32_t stage_count_le(const uint32_t *a, uint32_t t
 // spans segments each warp does the same for its own 32 rows in the list, and a row on its own where even these
 // span segments or the moduli are too large for 64-bit bounds.
 //
-// Bound: instruction issue.  Sixteen rows per thread whose bounds advanced through the list in global memory
-// waited on L2: 0.81 ms for a lease's 1.6e7 rows and 50 us for a batch's 6e4, which gave work to 30 SMs; now
-// 0.41 ms and 7 us.
+// Bound: the latency of its dependent loads and instruction issue (0.5 per cycle); 48 registers, for 40 warps per SM,
+// took a lease's launch from 0.46 to 0.41 ms (40 registers spill: 0.41, and slower for fewer rows).  Sixteen rows per
+// thread whose bounds advanced through the list in global memory waited on L2: 0.85 ms for a lease's 1.6e7 rows and 50
+// us for a batch's 6e4, which gave work to 30 SMs (now 7 us).
 template <int ROWS>
-__global__ void __launch_bounds__(PREP_T) k_vprep(const PrepArgs a) {
+__global__ void __launch_bounds__(PREP_T, 5) k_vprep(const PrepArgs a) {
     constexpr uint32_t PREP_STAGE = ROWS > 4 ? 2048 : 1024;      // u entries staged per bound
     __shared__ uint32_t stage_s[2][2 * PREP_STAGE];
     __shared__ uint64_t end_s[4], u_s[4], rem_s[2];              // per bound: first and last row's index and U; remainders
@@ -1904,6 +1905,8 @@ int engine_check(Engine &E, const uint64_t *head, const uint64_t *counts, bool &
     return PC_OK;
 }
 
+constexpr uint64_t SMALL_REPORT = 1 << 14;                // words
+
 // The report of the run just launched: in one copy through the context's page-locked stage where it fits that
 // (a copy to pageable memory costs the host 12 us and a wait each), else straight to the caller's arrays.
 // got: the first records, which the copy brought along.
@@ -1912,7 +1915,11 @@ int engine_fetch(Engine &E, uint64_t *counts, uint64_t *geometry, std::vector<ui
     const uint64_t words = E.fetch_words();
     head.resize(E.o_counts);
     got = 0;
-    if (uint64_t *stage = pc_stage(ctx, words * 8)) {
+    // a large report goes straight to page-locked arrays, where the caller has them: no second copy on the host
+    cudaPointerAttributes at{};
+    const bool direct = words > SMALL_REPORT && cudaPointerGetAttributes(&at, counts) == cudaSuccess && at.type == cudaMemoryTypeHost;
+    if (words > SMALL_REPORT) cudaGetLastError();
+    if (uint64_t *stage = direct ? nullptr : pc_stage(ctx, words * 8)) {
         PC_CHECK(ctx, pc_copy(ctx, stage, E.d_report, words * 8, cudaMemcpyDeviceToHost));
         PC_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
         memcpy(head.data(), stage, E.o_counts * 8);
