@@ -58,3 +58,24 @@ def test_masked_equals_plain_at_other_moduli(runtime, A, B, width):
     assert masked['valid_focused_candidates'] > 1000
     for key in FIELDS[:5]:
         assert masked[key] == plain[key], key
+
+
+@pytest.mark.parametrize('tuning', [{}, dict(bitset_filters=4, block_words=16, threads=512), dict(bitset_filters=5, block_words=64, threads=512)],
+                         ids=['default', '4x16', '5x64'])
+def test_few_rows_per_block_equal_plain(runtime, tuning):
+    """Windows of one to forty v rows (blocks whose rows are made for them alone, and whole blocks) against the
+    plain per-tile loop."""
+    rng = random.Random(len(tuning))
+    engine = BatchedEngine(runtime)
+    windows = []
+    for rows in (1, 2, 5, 9, 12, 14, 16, 17, 18, 19, 20, 24, 30, 40):
+        first = rng.randrange(0, B619 - 10**9)
+        windows.append(Window(rng.choice((499, 547, 619)), first, first + rows_span(rows)))
+    batch = engine.plan(windows, width=10**6, tuning=tuning)
+    batch.run()
+    for w, row in zip(windows, batch.results()):
+        c = w.config()
+        want = compute_batch(Matcher(runtime, c), *engine.focus_pair(c), w.first, w.end, 10**8)
+        assert all(row[k] == want[k] for k in FIELDS[:4]), w
+        assert sorted(row['all_values']) == sorted(want['all_values']), w
+    batch.close()
