@@ -344,13 +344,14 @@ __device__ __forceinline__ uint64_t look_back(volatile unsigned long long *state
 struct WinBatch {
     uint32_t n = 0, rounds = 1;
     uint64_t units = 0;
-    void *d_desc = nullptr, *d_foci = nullptr;
+    void *d_desc = nullptr, *d_foci = nullptr;   // null for a few windows: launch parameters
     uint64_t *d_scan = nullptr;      // ticket, tile states, window starts and total, stuck flag
+    uint64_t *d_starts = nullptr;    // window starts and total (in d_scan, or where the owner reads them)
     uint64_t *d_stuck = nullptr;     // set by an emitting pass that gave up (in d_scan, or where the owner reads it)
     uint64_t *d_delta = nullptr;     // per window: output position minus values before it (null: 0)
     std::vector<uint64_t> total, base, delta;
     std::vector<char> has;           // windows with any unit
-    std::vector<unsigned char> staged;   // descriptors as uploaded (kept until the copy has run)
+    std::vector<unsigned char> staged;   // descriptors and foci, as uploaded or passed (kept until the copy has run)
     uint64_t out_len = 0;
 };
 struct pc_focus;

@@ -9,6 +9,7 @@ import random
 import numpy as np
 import pytest
 
+from psuedocubes_b200.batched import BatchedEngine, Window
 from psuedocubes_b200.focus import Config
 from psuedocubes_b200.gpu import GPUFocus
 from psuedocubes_b200.served import A_RINGS, B_RINGS
@@ -71,3 +72,37 @@ def test_many_units_per_warp_match_oracle(focuses619, oracle619):
     _, ofa, ofb = oracle619
     for focus, of, low, span in ((focuses619[0], ofa, 123456789012345678, 3 * 10**11), (focuses619[1], ofb, 400000000000000001, 10**11)):
         assert np.array_equal(focus.window(low, low + span, cap=1 << 24).get(), of.window(low, low + span, cap=1 << 24))
+
+
+@pytest.mark.parametrize('n', [1, 31, 32, 33, 255, 256, 257, 1000])
+def test_searchsorted_queries_at_the_launch_limit(runtime, focuses619, n):
+    """Queries passed with the launch (up to 256) and uploaded, on a whole list and on a slice of it."""
+    low = 10**17
+    array = focuses619[0].window(low, low + 10**10, cap=1 << 22)
+    host = array.get()
+    rng = np.random.default_rng(n)
+    q = rng.integers(low - 10**9, low + 11 * 10**9, size=n).astype(np.uint64)
+    q[::3] = host[rng.integers(0, len(host), size=len(q[::3]))]
+    assert np.array_equal(array.searchsorted(q), np.searchsorted(host, q))
+    part = slice(len(host) // 3, len(host) // 2)
+    assert np.array_equal(array[part].searchsorted(q), np.searchsorted(host[part], q))
+
+
+@pytest.mark.parametrize('graph', [False, True], ids=['eager', 'graph'])
+def test_one_window_and_several_agree(runtime, graph):
+    """A plan of one window passes its descriptors with the launch, a plan of more uploads them."""
+    engine = BatchedEngine(runtime)
+    windows = [Window(p, 10**17 + k * 10**12, 10**17 + k * 10**12 + span)
+               for k, (p, span) in enumerate(((619, 10**6), (547, 3 * 10**8), (619, 10**9)))]
+    every = engine.plan(windows, width=10**8)
+    for _ in range(3):                                   # with a graph: eager, capture, replay
+        every.run(graph=graph)
+    for w, row in zip(windows, every.results()):
+        alone = engine.plan([w], width=10**8)
+        for _ in range(3):
+            alone.run(graph=graph)
+        mine = alone.results()[0]
+        for key in ('focus_u', 'focus_v', 'valid_focused_candidates', 'group_survivors', 'all_values'):
+            assert mine[key] == row[key], (w, key)
+        alone.close()
+    every.close()
