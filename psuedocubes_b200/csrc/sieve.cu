@@ -1265,8 +1265,9 @@ __global__ void __launch_bounds__(256) k_deep(const DeepArgs a) {
 // costs one subtraction and one bitmap lookup per filter (x mod q = (uB - vA) mod q).  The 1 in 81
 // positions that pass are queued per warp and finished 32 at a time in 128-bit arithmetic, filter by
 // filter.  The work is split over u chunks and v runs, so a tile of ten v rows fills the device: with a
-// warp per v row such a tile, and one of 964 rows, took 570 us, bound by the one warp that walked 17,400
-// u entries of a row; now 11 us and 57 us (the latter bound by instruction issue, 0.61 per cycle).
+// warp per v row such a tile took 570 us, bound by the one warp that walked 17,400 u entries of a row; now
+// 11 us.  It takes 275 instructions of a warp for 128 positions, so from 64 v rows on (a tile of 7 10^6 positions)
+// k_plain_rows takes over.
 
 constexpr uint32_t PLAIN_T = 256, PLAIN_PER = 4, PLAIN_U = PLAIN_T * PLAIN_PER;   // threads, u entries per thread, per CTA
 constexpr uint32_t PLAIN_V = 64;                  // v rows staged at a time
@@ -1289,6 +1290,21 @@ struct PlainArgs {
     uint64_t run;                                 // v rows per CTA
     uint32_t aq[PLAIN_FIRST], bq[PLAIN_FIRST];    // A mod q, B mod q of the first filters
 };
+
+// A position that passed the first nf filters: the others on x = uB - vA in two limbs.
+__device__ __forceinline__ void plain_rest(const PlainArgs &a, const u128 x, uint32_t nf, unsigned long long *cnt) {
+    for (uint32_t idx = nf; idx < a.nres; ++idx) {
+        const FiltConst fc = a.fc[idx];
+        const uint32_t m = mod128(x, fc.m);
+        if (!((__ldg(a.bits + fc.tab_off + (m >> 5)) >> (m & 31)) & 1u)) return;
+        if ((idx & 3) == 3 || idx + 1 == a.nres) atomicAdd(&cnt[idx / 4 + 1], 1ull);
+    }
+    const unsigned long long slot = atomicAdd((unsigned long long *)&a.counts[a.ng + 1], 1ull);
+    if (slot < a.out_cap) {
+        a.out[2 * slot] = x.lo;
+        a.out[2 * slot + 1] = x.hi;
+    }
+}
 
 __global__ void __launch_bounds__(PLAIN_T) k_plain(const PlainArgs a) {
     __shared__ unsigned long long cnt[PC_MAX_RES / 4 + 4];
@@ -1333,18 +1349,7 @@ __global__ void __launch_bounds__(PLAIN_T) k_plain(const PlainArgs a) {
         __syncwarp();
         qhead += n;
         if (!mine) return;
-        const u128 x = sub128(mul_wide(__ldg(us + (ent & (PLAIN_U - 1))), a.B), mul_wide(__ldg(a.vs + j0 + ent / PLAIN_U), a.A));
-        for (uint32_t idx = nf; idx < a.nres; ++idx) {
-            const FiltConst fc = a.fc[idx];
-            const uint32_t m = mod128(x, fc.m);
-            if (!((__ldg(a.bits + fc.tab_off + (m >> 5)) >> (m & 31)) & 1u)) return;
-            if ((idx & 3) == 3 || idx + 1 == a.nres) atomicAdd(&cnt[idx / 4 + 1], 1ull);
-        }
-        const unsigned long long slot = atomicAdd((unsigned long long *)&a.counts[a.ng + 1], 1ull);
-        if (slot < a.out_cap) {
-            a.out[2 * slot] = x.lo;
-            a.out[2 * slot + 1] = x.hi;
-        }
+        plain_rest(a, sub128(mul_wide(__ldg(us + (ent & (PLAIN_U - 1))), a.B), mul_wide(__ldg(a.vs + j0 + ent / PLAIN_U), a.A)), nf, cnt);
     };
 
     for (uint64_t base = j0; base < j1; base += PLAIN_V) {
@@ -1410,13 +1415,172 @@ __global__ void __launch_bounds__(PLAIN_T) k_plain(const PlainArgs a) {
         if (k != a.ng + 1 && cnt[k]) atomicAdd((unsigned long long *)&a.counts[k], cnt[k]);
 }
 
-// Grid of a plain launch: every u chunk, times as many v runs as one wave of four CTAs per SM (64 registers)
-// holds.  More, shorter runs only repeat the staging of rows and leave fuller last waves.
-dim3 plain_grid(PlainArgs &a, int sm_count) {
-    const uint64_t chunks = (a.nu + PLAIN_U - 1) / PLAIN_U, want = (uint64_t)sm_count * 4;
-    const uint64_t runs = std::max(std::min(a.nv, std::max<uint64_t>(1, want / chunks)), (a.nv + PLAIN_RUN_MAX - 1) / PLAIN_RUN_MAX);
+// The same with more v rows.  A CTA owns 128 u entries and a run of v rows and first makes, for every residue r of
+// the first four filters, the 128 bits allowed[(uB - r) mod q]: a warp takes one filter's word of 32 entries, a lane
+// reads 32 residues of its entry as one word of the filter's pattern, and five exchanges transpose the warp's words.
+// Then a v row is four words per filter: a lane loads one word of each of the four rows that vA mod q names, four
+// lanes to a v row, and 128 positions take some 8 instructions of a warp where the lookups of k_plain take 275.  The
+// rest (interval searches in the entries' products, one v row per lane; the queue of the 1 in 81) is as there.
+// Bound: latency, of the prologue, the rows and the 128-bit tail, each a few us long with 16 warps on an SM.
+// Times with their events, k_plain -> here, by v rows (17,400 u entries): 55 19.2 -> 20, 91 20.7 -> 20.0, 193 26 -> 21,
+// 474 39 -> 23, 997 62 -> 25.6, 1,988 108 -> 34 us.
+constexpr uint32_t PR_T = 512, PR_U = 128;        // threads, u entries per CTA
+static_assert(PR_T / 32 == 4 * PLAIN_FIRST && PR_U == 4 * 32, "a warp per filter and word");
+constexpr uint32_t PR_QUEUE = 64;                 // queued positions per warp (31 left over and 32 fit)
+constexpr uint32_t PR_ROWS = 2048;                // most rows of the first four filters (32 KB)
+constexpr uint32_t PR_PAT = (2 * PR_ROWS + PLAIN_FIRST * 96) / 32;   // pattern words
+constexpr uint64_t PLAIN_ROWS_MIN = 64;           // v rows of a launch and of a run from which the rows are worth making
+constexpr uint64_t PR_RUN_MAX = UINT64_C(1) << 25;   // v rows per CTA (a queue entry holds the row in 25 bits)
+
+__global__ void __launch_bounds__(PR_T) k_plain_rows(const PlainArgs a) {
+    extern __shared__ uint4 rows_s[];             // 128 bits per row
+    __shared__ unsigned long long cnt[PC_MAX_RES / 4 + 4];
+    __shared__ u128 prod_s[PR_U];                 // uB
+    __shared__ FiltConst fc_s[PLAIN_FIRST];
+    __shared__ uint32_t pat_s[PR_PAT];
+    __shared__ uint32_t queue_s[PR_T / 32][PR_QUEUE];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lanes_below = (1u << lane) - 1u;
+    const uint32_t nf = min(a.nres, PLAIN_FIRST);
+    const uint64_t c0 = blockIdx.x * (uint64_t)PR_U;
+    const uint32_t n_here = (uint32_t)umin64(a.nu - c0, PR_U);
+    const uint64_t j0 = blockIdx.y * a.run, j1 = umin64(a.nv, j0 + a.run);
+    const uint64_t *us = a.us + c0;
+    for (uint32_t k = threadIdx.x; k < a.ng + 3; k += PR_T) cnt[k] = 0;
+    if (threadIdx.x < n_here) prod_s[threadIdx.x] = mul_wide(__ldg(us + threadIdx.x), a.B);
+    if (warp < nf && lane < sizeof(FiltConst) / 4) ((uint32_t *)(fc_s + warp))[lane] = ((const uint32_t *)(a.fc + warp))[lane];
+    __syncthreads();
+    uint32_t row0[PLAIN_FIRST], rows = 0, words = 0, my_row0 = 0, my_pat = 0;
+#pragma unroll
+    for (uint32_t f = 0; f < PLAIN_FIRST; ++f) {
+        const uint32_t q = f < nf ? fc_s[f].m.q : 0;
+        row0[f] = rows;
+        if (f == warp / 4) my_row0 = rows, my_pat = words;
+        rows += q, words += (2 * q + 63) / 32 + 1;
+    }
+    const uint32_t filt = warp / 4, part = warp % 4;   // a filter's pattern and rows are made by four warps
+    if (filt < nf) {
+        // pattern bit b: residue b - 31 mod q, for a window of 32 that ends at any residue below 2q
+        const FiltConst &fc = fc_s[filt];
+        const uint32_t q = fc.m.q;
+        for (uint32_t w = part; w < (2 * q + 63) / 32; w += 4) {
+            const uint32_t m = fastmod32(w * 32 + lane + 31 * (q - 1), fc.m.c, q);
+            const uint32_t word = __ballot_sync(0xffffffffu, __ldg(a.bits + fc.tab_off + (m >> 5)) >> (m & 31) & 1u);
+            if (lane == 0) pat_s[my_pat + w] = word;
+        }
+    }
+    __syncthreads();
+    if (filt < nf) {                              // word `part` of the CTA's entries
+        const FiltConst &fc = fc_s[filt];
+        const uint32_t q = fc.m.q, i = part * 32 + lane;
+        const uint32_t ru = fastmod32(mod64(i < n_here ? __ldg(us + i) : 0, fc.m) * a.bq[filt], fc.m.c, q);
+        for (uint32_t r0 = 0; r0 < q; r0 += 32) {
+            const uint32_t at = ru + q - r0;      // bits 31 - i of the window: residue ru - r0 - i
+            const uint32_t *p = pat_s + my_pat + (at >> 5);
+            uint32_t x = __brev(__funnelshift_r(p[0], p[1], at));
+#pragma unroll
+            for (uint32_t d = 16; d; d >>= 1) {   // lane = entry, bit = row -> lane = row, bit = entry
+                const uint32_t keep = d == 16 ? 0x0000ffffu : d == 8 ? 0x00ff00ffu : d == 4 ? 0x0f0f0f0fu : d == 2 ? 0x33333333u : 0x55555555u;
+                const uint32_t y = __shfl_xor_sync(0xffffffffu, x, d);
+                x = lane & d ? (x & ~keep) | (y >> d & keep) : (x & keep) | (y << d & ~keep);
+            }
+            if (r0 + lane < q) ((uint32_t *)(rows_s + my_row0 + r0 + lane))[part] = x;
+        }
+    }
+    __syncthreads();
+    uint32_t passed = 0, qhead = 0, qtail = 0;    // group-1 positions of the lane; warp-uniform queue positions
+    uint32_t tested = 0;                          // at most 128 of each of the lane's 2^16 v rows
+    auto drain = [&](uint32_t n) {
+        __syncwarp();
+        const bool mine = lane < n;
+        const uint32_t ent = mine ? queue_s[warp][(qhead + lane) & (PR_QUEUE - 1)] : 0u;
+        __syncwarp();
+        qhead += n;
+        if (mine) plain_rest(a, sub128(prod_s[ent & (PR_U - 1)], mul_wide(__ldg(a.vs + j0 + ent / PR_U), a.A)), nf, cnt);
+    };
+    auto count = [&](u128 key) {                  // entries with uB <= key
+        uint32_t lo = 0, hi = n_here;
+        if (less128(key, prod_s[0])) hi = 0;
+        else if (!less128(key, prod_s[n_here - 1])) lo = n_here;
+        while (lo < hi) {
+            const uint32_t mid = (lo + hi) / 2;
+            if (less128(key, prod_s[mid])) hi = mid;
+            else lo = mid + 1;
+        }
+        return lo;
+    };
+    for (uint64_t base = j0 + warp * 32; base < j1; base += PR_T) {
+        uint32_t span = 0, at01 = 0, at23 = 0;    // the lane's v row: interval start | end << 16, its rows
+        if (base + lane < j1) {
+            const uint64_t v = __ldg(a.vs + base + lane);
+            const u128 shift = mul_wide(v, a.A), above = add128(shift, a.lo);
+            uint32_t left = count(above);
+            const uint32_t right = max(left, count(add128(shift, a.hi)));
+            if (less128(above, shift)) {          // vA + lo wrapped: positions below vA are flagged, not tested
+                uint32_t first = left;
+                while (first < right && less128(prod_s[first], shift)) ++first;
+                if (first > left) atomicAdd(&cnt[a.ng + 2], (unsigned long long)(first - left));
+                left = first;
+            }
+            tested += right - left;
+            span = left | right << 16;
+            uint32_t row[PLAIN_FIRST];
+#pragma unroll
+            for (uint32_t f = 0; f < PLAIN_FIRST; ++f)
+                row[f] = f < nf ? row0[f] + fastmod32(mod64(v, fc_s[f].m) * a.aq[f], fc_s[f].m.c, fc_s[f].m.q) : 0;
+            at01 = row[0] | row[1] << 16, at23 = row[2] | row[3] << 16;
+        }
+        for (uint32_t k = 0; k < 32 && base + k < j1; k += 8) {     // eight v rows, four lanes each
+            const uint32_t src = k + (lane >> 2), w = lane & 3;
+            const uint32_t sp = __shfl_sync(0xffffffffu, span, src);
+            const uint32_t r01 = __shfl_sync(0xffffffffu, at01, src), r23 = __shfl_sync(0xffffffffu, at23, src);
+            uint32_t x = unit_mask((int32_t)(sp & 0xffffu) - 32 * (int32_t)w, (int32_t)(sp >> 16) - 32 * (int32_t)w);
+            const uint32_t *rw = (const uint32_t *)rows_s + w;
+            if (x) {
+                x &= rw[4 * (r01 & 0xffffu)];
+                if (nf > 1) x &= rw[4 * (r01 >> 16)];
+                if (nf > 2) x &= rw[4 * (r23 & 0xffffu)];
+                if (nf > 3) x &= rw[4 * (r23 >> 16)];
+            }
+            passed += __popc(x);
+            for (uint32_t won; (won = __ballot_sync(0xffffffffu, x != 0)) != 0;) {
+                if (x) {
+                    queue_s[warp][(qtail + __popc(won & lanes_below)) & (PR_QUEUE - 1)] =
+                        (w * 32 + __ffs(x) - 1) | (uint32_t)(base - j0 + src) * PR_U;
+                    x &= x - 1;
+                }
+                qtail += __popc(won);
+                if (qtail - qhead >= 32) drain(32);
+            }
+        }
+    }
+    if (qtail != qhead) drain(qtail - qhead);
+    passed = __reduce_add_sync(0xffffffffu, passed);
+    if (lane == 0 && passed) atomicAdd(&cnt[1], (unsigned long long)passed);
+    tested = __reduce_add_sync(0xffffffffu, tested);
+    if (lane == 0 && tested) atomicAdd(&cnt[0], (unsigned long long)tested);
+    __syncthreads();
+    for (uint32_t k = threadIdx.x; k < a.ng + 3; k += PR_T)
+        if (k != a.ng + 1 && cnt[k]) atomicAdd((unsigned long long *)&a.counts[k], cnt[k]);
+}
+
+// A plain launch: every u chunk, times as many v runs as fill the device.  k_plain: one wave of four CTAs per SM
+// (64 registers); more, shorter runs only repeat the staging of rows and leave fuller last waves.  k_plain_rows from
+// PLAIN_ROWS_MIN v rows on, two CTAs per SM with at least that many rows each, unless the first filters' rows are too many.
+void plain_launch(PlainArgs &a, const uint32_t *primes, int sm_count, cudaStream_t st) {
+    uint32_t rows = 0;
+    for (uint32_t k = 0; k < std::min(a.nres, PLAIN_FIRST); ++k) {
+        a.aq[k] = (uint32_t)(a.A % primes[k]);
+        a.bq[k] = (uint32_t)(a.B % primes[k]);
+        rows += primes[k];
+    }
+    const bool by_rows = a.nv >= PLAIN_ROWS_MIN && rows <= PR_ROWS;
+    const uint64_t per = by_rows ? PR_U : PLAIN_U, chunks = (a.nu + per - 1) / per, want = (uint64_t)sm_count * (by_rows ? 2 : 4);
+    const uint64_t most = by_rows ? PR_RUN_MAX : PLAIN_RUN_MAX, least = by_rows ? a.nv / PLAIN_ROWS_MIN : a.nv;
+    const uint64_t runs = std::max(std::min(least, std::max<uint64_t>(1, want / chunks)), (a.nv + most - 1) / most);
     a.run = (a.nv + runs - 1) / runs;
-    return dim3((unsigned)chunks, (unsigned)((a.nv + a.run - 1) / a.run));
+    const dim3 grid((unsigned)chunks, (unsigned)((a.nv + a.run - 1) / a.run));
+    if (by_rows) k_plain_rows<<<grid, PR_T, rows * 16, st>>>(a);
+    else k_plain<<<grid, PLAIN_T, 0, st>>>(a);
 }
 
 template <int NB, int K, int NT>
@@ -2198,12 +2362,7 @@ extern "C" int pc_run_plain(pc_ctx *ctx, const pc_filters *f, const pc_buf *us, 
         a.counts = d_counts;
         a.out = d_out;
         a.out_cap = out_cap;
-        for (uint32_t k = 0; k < std::min(f->nres, PLAIN_FIRST); ++k) {
-            a.aq[k] = (uint32_t)(f->A % f->primes[k]);
-            a.bq[k] = (uint32_t)(f->B % f->primes[k]);
-        }
-        const dim3 grid = plain_grid(a, ctx->sm_count);
-        k_plain<<<grid, PLAIN_T, 0, st>>>(a);
+        plain_launch(a, f->primes.data(), ctx->sm_count, st);
         PC_LAUNCHED(ctx, "plain match");
     }
     PC_CHECK(ctx, cudaEventRecord(ctx->ev[7], st));
@@ -2681,12 +2840,7 @@ static int plain_static_on(int device, const uint64_t *us, uint64_t nu, const ui
         a.counts = (uint64_t *)(base + o_counts);
         a.out = (uint64_t *)(base + o_out);
         a.out_cap = out_cap;
-        for (uint32_t k = 0; k < std::min(nres, PLAIN_FIRST); ++k) {
-            a.aq[k] = (uint32_t)(A % primes[k]);
-            a.bq[k] = (uint32_t)(B % primes[k]);
-        }
-        const dim3 grid = plain_grid(a, std::max(sm, 1));
-        k_plain<<<grid, PLAIN_T, 0, st>>>(a);
+        plain_launch(a, primes, std::max(sm, 1), st);
         e = cudaGetLastError();
         if (e != cudaSuccess) return static_cuda(err, err_len, e, "plain match launch");
     }

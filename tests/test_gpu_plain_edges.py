@@ -63,3 +63,44 @@ def test_plain_split_edges(runtime, config, size):
     want, values = brute(config, us, vs)
     assert [int(n) for n in counts] == want
     assert sorted(int(a) | int(b) << 64 for a, b in out[:2 * len(values)].reshape(-1, 2)) == values
+
+
+@pytest.mark.parametrize('config', CONFIGS, ids=lambda c: f'p{c.p}')
+@pytest.mark.parametrize('size', [(127, 64), (128, 65), (129, 63), (257, 511), (1, 512), (130, 513), (40, 2100)],
+                         ids=lambda s: f'{s[0]}x{s[1]}')
+def test_plain_rows_edges(runtime, config, size):
+    """The kernel for 64 and more v rows: chunks of 128 u entries, 32 v rows per warp, eight at a time."""
+    test_plain_split_edges(runtime, config, size)
+
+
+@pytest.mark.parametrize('nv', [63, 64, 200])
+@pytest.mark.parametrize('primes', [(1021, 1019, 7, 2, 5), (1021, 1019, 7, 5, 3), (4093, 8191, 13), (1999, 47), (2039,)],
+                         ids=lambda q: '-'.join(map(str, q)))
+def test_plain_many_rows(runtime, primes, nv):
+    """First filters whose residues are 2,048 and fewer rows, or more (the lookup kernel for every v list), with
+    arbitrary residue tables, through the entry point that takes them."""
+    rng = random.Random(sum(primes) + nv)
+    A, B, nu = 11 * 17, 19 * 23, 300
+    tables = [[int(rng.random() < 0.6) for _ in range(q)] for q in primes]
+    vs = sorted(rng.randrange(10**9, 10**9 + 4 * nv) for _ in range(nv))
+    us = sorted(rng.randrange(vs[0] * A // B, vs[-1] * A // B + 900) for _ in range(nu))
+    lo, hi, ng, cap = 1000, 300_000, (len(primes) + 3) // 4, nu * nv
+    counts, out, err = np.zeros(ng + 3, dtype=np.uint64), np.zeros(2 * cap, dtype=np.uint64), ctypes.create_string_buffer(256)
+    code = runtime.lib.pc_run_plain_static(0, N.u64(us), nu, N.u64(vs), nv, A, B, lo, 0, hi, 0,
+                                           np.array(primes, dtype=np.uint32), len(primes),
+                                           np.array([b for t in tables for b in t], dtype=np.uint8), counts, out, cap, err, 256)
+    assert code == 0, err.value
+    want, values = [0] * (ng + 3), []
+    for x in (u * B - v * A for v in vs for u in us):
+        if lo < x <= hi:
+            want[0] += 1
+            for i, (q, table) in enumerate(zip(primes, tables)):
+                if not table[x % q]:
+                    break
+                if i % 4 == 3 or i + 1 == len(primes):
+                    want[i // 4 + 1] += 1
+            else:
+                values.append(x)
+    want[ng + 1] = len(values)
+    assert values and [int(n) for n in counts] == want
+    assert sorted(out[:2 * len(values):2].tolist()) == sorted(values)
