@@ -526,16 +526,20 @@ CUBE_ROOTS = (1000000001, 1442249570, 619)   # cube roots of (10^27, 3*10^27], t
 CUBE_METRIC = 'cube roots checked/s (genuine-cube control, p=619, roots of (1e27, 3e27])'
 
 
-def cube_groups(p: int) -> int:
-    """Prime groups of the device sieve (products <= 2^16), as pc_cube_roots forms them."""
-    primes = [q for q in range(2, p + 1) if all(q % d for d in range(2, int(q ** 0.5) + 1))]
+def cube_ops_per_root(p: int) -> tuple[float, int]:
+    """Lane operations per number of the device sieve and its prime groups, as pc_cube_roots forms them: 8 of 30
+    numbers are sieved, 32 to a word; a word takes a pattern load, a funnel shift and an OR per group of primes
+    (products <= 2^16) up to 256, and five operations per multiple of a larger prime."""
+    primes = [q for q in range(7, p + 1) if all(q % d for d in range(2, int(q**0.5) + 1))]
     groups, product = 0, None
     for q in primes:
+        if q > 256:
+            break
         if product is None or product * q > 1 << 16:
             groups, product = groups + 1, q
         else:
             product *= q
-    return groups
+    return (3 * groups + 5 * sum(32 / q for q in primes if q > 256)) * 8 / 30 / 32, groups
 
 
 def reference_cube_count(first: int, last: int, p: int) -> tuple[int, float]:
@@ -585,8 +589,7 @@ def run_cubes(args) -> None:
         clock = clocks.summary()
         sm_mhz = clock['sm_max_mhz'] or 1965.0
         peak = runtime.sm_count * 4 * 32 * sm_mhz * 1e6 / 1e12
-        groups = cube_groups(p)
-        ops_per_root = 3 * groups / 32     # per (prime group, 32-root word): pattern load, funnel shift, OR
+        ops_per_root, groups = cube_ops_per_root(p)
         mean_ms = statistics.mean(kernel_ms)
         achieved = ops_per_root * n / (mean_ms / 1000) / 1e12
         line = dict(metric=CUBE_METRIC, value=n * args.steps * world / seconds, unit='roots/s', n_gpus=world,
@@ -595,7 +598,7 @@ def run_cubes(args) -> None:
                     config=dict(workload='genuine-cube control: roots [1000000001, 1442249570] coprime to every '
                                          'prime <= 619 (tools/check_cpu.py --full-cube-count)',
                                 first=first, last=last, p=p, count=38322775, parallelism=f'replicas{world}',
-                                l2='no input beyond 85 KB of prime patterns per CTA, staged in shared memory (compute bound)'),
+                                l2='no input beyond a few KB of primes, from which each CTA marks 100 KB of patterns in shared memory (compute bound)'),
                     roofline=dict(bound='int_alu', achieved=achieved, peak=peak, unit='Tlaneop/s', frac=achieved / peak,
                                   traffic=None, kernel='k_roots (count)', ops_per_root=ops_per_root, prime_groups=groups,
                                   kernel_ms=mean_ms,

@@ -37,18 +37,34 @@ struct RootPrime {
     uint32_t every;                  // bit i set when q | i, i < 32
 };
 
-// The table in shared memory and its source: groups, then primes.
+// A prime that k_roots strikes out multiple by multiple.
+struct __align__(16) RootStrike {
+    uint64_t c;                      // fastmod constant of q
+    uint32_t q, inv;                 // the prime; W^-1 mod q
+};
+
+// The table in shared memory and its source: groups, primes, then strikes.
 struct RootParams {
-    uint32_t ngroups, nprimes, W, nclass, table_words;
+    uint32_t ngroups, nprimes, nstrikes, W, nclass, table_words;
     uint64_t first, last, k0, nk;    // numbers; k of the first number, k values
     uint32_t cls[ROOT_CLASSES];      // residues coprime to W, ascending
     const uint4 *table;
-    __host__ __device__ uint32_t table_bytes() const { return ngroups * sizeof(RootGroup) + nprimes * sizeof(RootPrime); }
-    uint32_t smem() const { return table_bytes() + table_words * 4; }
+    __host__ __device__ uint32_t table_bytes() const {
+        return ngroups * sizeof(RootGroup) + nprimes * sizeof(RootPrime) + nstrikes * sizeof(RootStrike);
+    }
 };
 
-// The groups and their patterns' places; `run` consecutive words are read from any offset below P.
-void root_params(RootParams &p, std::vector<unsigned char> &table, uint64_t first, uint64_t last, uint32_t bound, uint32_t run) {
+// W^-1 mod P = (1 + m P) / W for the m that makes it whole
+uint32_t inverse_w(uint64_t P, uint64_t W) {
+    uint64_t m = 0;
+    while ((1 + m * P) % W) ++m;
+    return (uint32_t)((1 + m * P) / W % P);
+}
+
+// The groups and their patterns' places; `run` consecutive words are read from any offset below P.  Primes above
+// `strike` have no pattern but a RootStrike.
+void root_params(RootParams &p, std::vector<unsigned char> &table, uint64_t first, uint64_t last, uint32_t bound, uint32_t run,
+                 uint32_t strike) {
     std::vector<char> composite(bound + 1, 0);
     std::vector<uint32_t> primes;
     p.W = 1;
@@ -68,17 +84,16 @@ void root_params(RootParams &p, std::vector<unsigned char> &table, uint64_t firs
     p.table_words = 0;
     std::vector<RootGroup> groups;
     std::vector<RootPrime> marks;
+    std::vector<RootStrike> strikes;
+    for (; !primes.empty() && primes.back() > strike; primes.pop_back())
+        strikes.push_back(RootStrike{fastmod_constant(primes.back()), primes.back(), inverse_w(primes.back(), p.W)});
     for (size_t i = 0; i < primes.size();) {
         RootGroup g{};
         g.P = 1;
         const size_t i0 = i;
         while (i < primes.size() && (uint64_t)g.P * primes[i] <= ROOT_GROUP_MAX) g.P *= primes[i++];
         g.c = fastmod_constant(g.P);
-        for (uint64_t m = 0; m < p.W; ++m)               // W^-1 = (1 + m P) / W for the m that makes it whole
-            if ((1 + m * g.P) % p.W == 0) {
-                g.inv = (uint32_t)((1 + m * g.P) / p.W % g.P);
-                break;
-            }
+        g.inv = inverse_w(g.P, p.W);
         g.off = p.table_words;
         g.words = (g.P - 1) / 32 + run + 1;
         p.table_words += g.words;
@@ -92,10 +107,13 @@ void root_params(RootParams &p, std::vector<unsigned char> &table, uint64_t firs
     p.table_words = (p.table_words + 3) & ~3u;
     p.ngroups = (uint32_t)groups.size();
     p.nprimes = (uint32_t)marks.size();
+    p.nstrikes = (uint32_t)strikes.size();
     table.resize(p.table_bytes());
     std::copy((const unsigned char *)groups.data(), (const unsigned char *)(groups.data() + groups.size()), table.begin());
     std::copy((const unsigned char *)marks.data(), (const unsigned char *)(marks.data() + marks.size()),
               table.begin() + groups.size() * sizeof(RootGroup));
+    std::copy((const unsigned char *)strikes.data(), (const unsigned char *)(strikes.data() + strikes.size()),
+              table.end() - strikes.size() * sizeof(RootStrike));
 }
 
 // The CTA's table and patterns.  A prime below 32 gives each of its group's words whole (32 lanes
@@ -139,9 +157,13 @@ __device__ __forceinline__ uint32_t class_bits(const RootParams &p, uint64_t k, 
 // reach 32 x RUN words past P, so the whole warp reads one window without a wrap: its offset and shift are
 // warp-uniform, a lane's window for one word shares a pattern word with the next (one shared load, one
 // funnel shift and half a three-input OR per group and word), and RUN is odd, so the lanes' loads always
-// fall in 32 different banks.  Bound: those shared loads, one per clock and SM.  With all 30 residues and
-// patterns that wrapped per lane (33 words each, two bank conflicts per load) 4e8 numbers took 201 us, with 8
-// of 30 residues 79 us; now 55 us.
+// fall in 32 different banks.  A prime above STRIKE hits a word in eight at most and would have a pattern to
+// itself: it is struck out instead, multiple by multiple in the warp's bitmap in shared memory, a lane per prime
+// (about one shared OR of a warp per prime where the pattern takes RUN + 1 loads and 1.5 RUN operations).
+// Bound: the patterns' marking (some 15 us whatever the range) and those loads and ORs, one per clock and SM.  4e8 numbers
+// with p = 619: 201 us with all 30 residues and patterns that wrapped per lane, 61 us with a pattern for every prime, 39 us
+// now (primes above 128 struck out: 41); all below 2^32 with p = 1999, whose patterns left room for 3 words: 2,052 -> 359.
+constexpr uint32_t STRIKE = 256;   // the square root of ROOT_GROUP_MAX: no two larger primes share a pattern
 template <int RUN>
 __global__ void __launch_bounds__(ROOT_THREADS) k_roots(const RootParams p, unsigned long long *__restrict__ total) {
     extern __shared__ uint4 smem[];
@@ -151,7 +173,11 @@ __global__ void __launch_bounds__(ROOT_THREADS) k_roots(const RootParams p, unsi
         if (threadIdx.x == i) cls_s[i] = p.cls[i];
     uint32_t *pattern;
     const RootGroup *groups = mark_patterns(p, smem, pattern);
+    const RootStrike *strikes = (const RootStrike *)((const RootPrime *)(groups + p.ngroups) + p.nprimes);
     const uint32_t lane = threadIdx.x & 31, warps = ROOT_THREADS / 32;
+    uint32_t *struck = pattern + p.table_words + (threadIdx.x >> 5) * (32 * RUN);   // the warp's bitmap
+#pragma unroll
+    for (int w = 0; w < RUN; ++w) struck[lane * RUN + w] = 0;
     constexpr uint32_t K = 32 * 32 * RUN;                  // k values of one warp task
     const uint64_t tasks = (p.nk + K - 1) / K * p.nclass;
     uint32_t count = 0;
@@ -160,6 +186,12 @@ __global__ void __launch_bounds__(ROOT_THREADS) k_roots(const RootParams p, unsi
         const uint32_t r = cls_s[task % p.nclass];
         const uint64_t k0 = task / p.nclass * K, k = k0 + lane * (32 * RUN);
         const uint32_t x = (uint32_t)(p.k0 + k0);          // with any group W = 30, so this is below 2^28
+        __syncwarp();
+        for (uint32_t i = lane; i < p.nstrikes; i += 32) {
+            const RootStrike S = strikes[i];
+            const uint32_t at = fastmod32(x + r * S.inv, S.c, S.q);   // x + r inv < 2^28 + 30 2^11
+            for (uint32_t z = at ? S.q - at : 0; z < K; z += S.q) atomicOr(struck + (z >> 5), 1u << (z & 31));
+        }
         uint32_t acc[RUN];
 #pragma unroll
         for (int w = 0; w < RUN; ++w) acc[w] = 0;
@@ -195,8 +227,13 @@ __global__ void __launch_bounds__(ROOT_THREADS) k_roots(const RootParams p, unsi
                 }
             }
         }
+        __syncwarp();
 #pragma unroll
-        for (int w = 0; w < RUN; ++w) count += __popc(~acc[w] & class_bits(p, k + 32 * w, r));
+        for (int w = 0; w < RUN; ++w) {
+            acc[w] |= struck[lane * RUN + w];
+            struck[lane * RUN + w] = 0;
+            count += __popc(~acc[w] & class_bits(p, k + 32 * w, r));
+        }
     }
     count = __reduce_add_sync(0xffffffffu, count);
     if (lane == 0 && count) atomicAdd(total, (unsigned long long)count);
@@ -292,17 +329,10 @@ double root_density(const RootParams &p, const std::vector<unsigned char> &table
     return d;
 }
 
-template <int RUN>
-int launch_roots(pc_ctx *ctx, const RootParams &p, unsigned long long *d_total) {
-    PC_CHECK(ctx, cudaFuncSetAttribute(k_roots<RUN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem()));
-    k_roots<RUN><<<ctx->sm_count, ROOT_THREADS, p.smem(), ctx->stream>>>(p, d_total);
-    PC_LAUNCHED(ctx, "cube roots count");
-    return PC_OK;
-}
-
-// Words per lane of k_roots: the most whose patterns fit shared memory (p = 619: 177 KB at 9; p = 2000: 218 KB
-// at 3).  Fewer words mean more offsets per word; more would not fit.
-constexpr uint32_t RUNS[] = {9, 5, 3}, ROOT_SMEM = 224 * 1024;
+// Words per lane of k_roots: patterns and bitmaps take 135 KB of shared memory at p = 619.  Fewer words mean more
+// offsets per word; more words, longer tasks that short ranges have too few of (5, 9, 13, 17 words: 4e8 numbers 41.6, 39.5, 38,
+// 39.4 us; 6e6 numbers 17, 19, 27, 27 us).
+constexpr uint32_t ROOT_RUN = 9;
 
 }  // namespace
 
@@ -317,16 +347,9 @@ extern "C" int pc_cube_roots(pc_ctx *ctx, uint64_t first, uint64_t last, uint32_
     std::vector<unsigned char> table;
     // counts take k_roots from one warp task per SM on (4e6 numbers): its fixed cost, marking the
     // longer patterns, is then below what the list kernel's three times as many shared loads cost
-    uint32_t run = 0;
-    for (uint32_t r : RUNS) {
-        root_params(rp, table, first, last, p, 32 * r);
-        if (!roots && rp.smem() <= ROOT_SMEM) {
-            if ((rp.nk + 1024 * r - 1) / (1024 * r) * rp.nclass >= (uint64_t)ctx->sm_count) run = r;
-            break;
-        }
-    }
-    const bool longer = run != 0;
-    if (!longer) root_params(rp, table, first, last, p, 1);
+    root_params(rp, table, first, last, p, 32 * ROOT_RUN, STRIKE);
+    const bool longer = !roots && (rp.nk + 1024 * ROOT_RUN - 1) / (1024 * ROOT_RUN) * rp.nclass >= (uint64_t)ctx->sm_count;
+    if (!longer) root_params(rp, table, first, last, p, 1, UINT32_MAX);
     const uint64_t ntiles = (rp.nk + LIST_THREADS * 32 - 1) / (LIST_THREADS * 32);
     Scratch hold(ctx);
     uint64_t *d_scan = nullptr;                            // total, stuck flag, ticket, tile states
@@ -354,9 +377,10 @@ extern "C" int pc_cube_roots(pc_ctx *ctx, uint64_t first, uint64_t last, uint32_
         PC_CHECK(ctx, cudaMemsetAsync(d_scan, 0, words * 8, ctx->stream));
         PC_CHECK(ctx, cudaEventRecord(ctx->ev[0], ctx->stream));
         if (longer) {
-            unsigned long long *d_total = (unsigned long long *)d_scan;
-            rc = run == 9 ? launch_roots<9>(ctx, rp, d_total) : run == 5 ? launch_roots<5>(ctx, rp, d_total) : launch_roots<3>(ctx, rp, d_total);
-            if (rc) return rc;
+            const uint32_t smem = rp.table_bytes() + rp.table_words * 4 + (ROOT_THREADS / 32) * (32 * ROOT_RUN) * 4;
+            PC_CHECK(ctx, cudaFuncSetAttribute(k_roots<ROOT_RUN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            k_roots<ROOT_RUN><<<ctx->sm_count, ROOT_THREADS, smem, ctx->stream>>>(rp, (unsigned long long *)d_scan);
+            PC_LAUNCHED(ctx, "cube roots count");
         } else {
             const size_t smem = rp.table_bytes() + std::max(rp.table_words * 4, LIST_THREADS / 32 * LIST_STAGE * 2);
             PC_CHECK(ctx, cudaFuncSetAttribute(k_root_list, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));

@@ -35,3 +35,12 @@ def test_long_counts_match_oracle(runtime, oracle, p):
 def test_whole_range_count_matches_oracle(runtime, oracle):
     for p in (31, 619):
         assert cubes.count_roots(runtime, 1, 2**32 - 1, p) == oracle.cube_roots(1, 2**32 - 1, p, threads=8)
+
+
+@pytest.mark.parametrize('p', [251, 257, 263, 443, 449, 1999])
+def test_struck_primes_match_oracle(runtime, oracle, p):
+    """No, one, two, 32 and 33 primes above the largest with a pattern, around whole tasks of 9,216 k values."""
+    task = 30 * 9216
+    for first, n in ((1, 20 * task), (30 * 10**6 + 1, 19 * task + 31), (2**32 - 21 * task + 1, 21 * task - 1)):
+        want = oracle.cube_roots(first, first + n - 1, p, threads=8)
+        assert cubes.count_roots(runtime, first, first + n - 1, p) == want, (first, n)
