@@ -16,6 +16,7 @@
 // the primes (a few thousand bits), so only the table of groups (a few KB) comes from the host.
 #include "common.cuh"
 #include <algorithm>
+#include <cstring>
 #include <vector>
 
 namespace {
@@ -343,13 +344,13 @@ extern "C" int pc_cube_roots(pc_ctx *ctx, uint64_t first, uint64_t last, uint32_
     if (first < 1 || last < first || last > UINT32_MAX || p < 2 || p > 2000)
         return pc_fail(ctx, PC_INVALID, "cube roots need 1 <= first <= last < 2^32 and 2 <= p <= 2000");
     const uint64_t n = last - first + 1;
-    RootParams rp{};
-    std::vector<unsigned char> table;
     // counts take k_roots from one warp task per SM on (4e6 numbers): its fixed cost, marking the
     // longer patterns, is then below what the list kernel's three times as many shared loads cost
-    root_params(rp, table, first, last, p, 32 * ROOT_RUN, STRIKE);
-    const bool longer = !roots && (rp.nk + 1024 * ROOT_RUN - 1) / (1024 * ROOT_RUN) * rp.nclass >= (uint64_t)ctx->sm_count;
-    if (!longer) root_params(rp, table, first, last, p, 1, UINT32_MAX);
+    const uint64_t W = p < 3 ? 2 : p < 5 ? 6 : 30, classes = p < 3 ? 1 : p < 5 ? 2 : 8, nk = last / W - first / W + 1;
+    const bool longer = !roots && (nk + 1024 * ROOT_RUN - 1) / (1024 * ROOT_RUN) * classes >= (uint64_t)ctx->sm_count;
+    RootParams rp{};
+    std::vector<unsigned char> table;
+    root_params(rp, table, first, last, p, longer ? 32 * ROOT_RUN : 1, longer ? STRIKE : UINT32_MAX);
     const uint64_t ntiles = (rp.nk + LIST_THREADS * 32 - 1) / (LIST_THREADS * 32);
     Scratch hold(ctx);
     uint64_t *d_scan = nullptr;                            // total, stuck flag, ticket, tile states
@@ -389,8 +390,13 @@ extern "C" int pc_cube_roots(pc_ctx *ctx, uint64_t first, uint64_t last, uint32_
             PC_LAUNCHED(ctx, "cube root list");
         }
         PC_CHECK(ctx, cudaEventRecord(ctx->ev[1], ctx->stream));
-        PC_CHECK(ctx, pc_copy(ctx, got, d_scan, sizeof(got), cudaMemcpyDeviceToHost));
+        // the sums, and a list with them, through the page-locked stage: one wait, and no copy in pieces to pageable
+        // memory
+        uint64_t *stage = pc_stage(ctx, sizeof(got) + room * 4);
+        PC_CHECK(ctx, pc_copy(ctx, stage ? stage : got, d_scan, sizeof(got), cudaMemcpyDeviceToHost));
+        if (stage && room) PC_CHECK(ctx, pc_copy(ctx, stage + 2, d_out, room * 4, cudaMemcpyDeviceToHost));
         PC_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
+        if (stage) memcpy(got, stage, sizeof(got));
         if ((rc = elapsed(ms))) return rc;
         if (kernel_ms) *kernel_ms = ms;
         if (got[1]) return pc_fail(ctx, PC_ARITHMETIC, "cube root pass did not finish");
@@ -399,6 +405,10 @@ extern "C" int pc_cube_roots(pc_ctx *ctx, uint64_t first, uint64_t last, uint32_
         if (got[0] > cap) return pc_fail(ctx, PC_OVERFLOW, "more cube roots than the output capacity");
         if (got[0] <= room) {
             if (!got[0]) return PC_OK;
+            if (stage) {
+                memcpy(roots, stage + 2, got[0] * 4);
+                return PC_OK;
+            }
             PC_CHECK(ctx, pc_copy(ctx, roots, d_out, got[0] * 4, cudaMemcpyDeviceToHost));
             PC_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
             return PC_OK;
