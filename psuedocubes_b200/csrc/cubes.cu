@@ -23,7 +23,8 @@ namespace {
 
 constexpr uint32_t ROOT_GROUP_MAX = 1u << 16;   // largest product of one prime group
 constexpr uint32_t ROOT_GROUPS = 304, ROOT_CLASSES = 8;   // 303 primes below 2000
-constexpr int ROOT_THREADS = 1024, LIST_THREADS = 128;
+constexpr int ROOT_THREADS = 1024, LIST_THREADS = 512;
+constexpr uint32_t LIST_K = LIST_THREADS * 2 / ROOT_CLASSES;   // words of every class in a tile of k_root_list: a thread, two classes
 constexpr uint32_t LIST_STAGE = 32 * 32 * ROOT_CLASSES;         // a warp's candidates, 16 bits each while staged
 
 struct __align__(16) RootGroup {
@@ -240,17 +241,21 @@ __global__ void __launch_bounds__(ROOT_THREADS) k_roots(const RootParams p, unsi
     if (lane == 0 && count) atomicAdd(total, (unsigned long long)count);
 }
 
-// Listing (and counting short ranges, which would leave k_roots a few long warps): a lane owns 32
-// consecutive k values of every class, so number order is lane order, then k, then class.  The tile's place in
+// Listing (and counting short ranges, which would leave k_roots a few long warps): a tile is LIST_K words of 32
+// consecutive k values in every class, a thread sieves one word of two classes.  Then one thread per word takes all
+// its classes, so number order is lane order, then k, then class.  The tile's place in
 // the list comes from a look-back over the tiles before it (out may be null: count only).  A warp's roots
-// are staged in the patterns' space, which nothing reads any more, and stored coalesced.
+// are staged in the patterns' space, which nothing reads any more, and stored coalesced.  Bound: latency, of marking the
+// patterns and of a thread's way through all groups.  With a thread per word, 128 of them, sieving all eight classes a
+// list over 1e6 numbers took 33 us, now 29.5 (p = 1999: 59.5 -> 52; 2e7 numbers, where every SM has work: 41.5 -> 43.5).
 __global__ void __launch_bounds__(LIST_THREADS) k_root_list(const RootParams p,
                                                             unsigned long long *__restrict__ ticket, uint64_t ntiles,
                                                             uint64_t *__restrict__ stuck, uint64_t *__restrict__ total,
                                                             uint32_t *__restrict__ out, uint64_t cap) {
     extern __shared__ uint4 smem[];
     __shared__ uint64_t tile_s, before_s;
-    __shared__ uint32_t sum_s[LIST_THREADS / 32];
+    __shared__ uint32_t sum_s[LIST_K / 32];
+    __shared__ uint32_t acc_s[ROOT_CLASSES][LIST_K];
     __shared__ uint32_t shift_s[ROOT_GROUPS][ROOT_CLASSES / 2];    // r W^-1 mod P of every class, 16 bits each
     __shared__ uint32_t cls_s[ROOT_CLASSES];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -265,24 +270,32 @@ __global__ void __launch_bounds__(LIST_THREADS) k_root_list(const RootParams p,
         ((uint16_t *)shift_s)[i] = (uint16_t)fastmod32(cls_s[i % ROOT_CLASSES] * g.inv, g.c, g.P);
     }
     __syncthreads();
-    const uint64_t tile = tile_s, k = (tile * LIST_THREADS + threadIdx.x) * 32;
-    uint32_t acc[ROOT_CLASSES] = {};
+    const uint32_t word = threadIdx.x % LIST_K, two = threadIdx.x / LIST_K;   // `two` is warp-uniform
+    const uint64_t tile = tile_s, k = (tile * LIST_K + word) * 32;
+    uint32_t both[2] = {};
 #pragma unroll 2
     for (uint32_t g = 0; g < p.ngroups; ++g) {                     // with any group there are eight classes
         const RootGroup G = groups[g];
-        const uint32_t P = G.P, s0 = fastmod32((uint32_t)(p.k0 + k), G.c, P);
+        const uint32_t P = G.P, s0 = fastmod32((uint32_t)(p.k0 + k), G.c, P), shift = shift_s[g][two];
         const uint32_t *pat = pattern + G.off;
 #pragma unroll
-        for (uint32_t i = 0; i < ROOT_CLASSES; ++i) {
-            uint32_t s = s0 + ((shift_s[g][i / 2] >> (16 * (i & 1))) & 0xffffu);
+        for (uint32_t i = 0; i < 2; ++i) {
+            uint32_t s = s0 + (shift >> (16 * i) & 0xffffu);
             s -= s >= P ? P : 0;
-            acc[i] |= __funnelshift_r(pat[s >> 5], pat[(s >> 5) + 1], s & 31);
+            both[i] |= __funnelshift_r(pat[s >> 5], pat[(s >> 5) + 1], s & 31);
         }
     }
-    uint32_t n = 0;
+#pragma unroll
+    for (uint32_t i = 0; i < 2; ++i) {
+        const uint32_t c = 2 * two + i;
+        acc_s[c][word] = c < p.nclass ? ~both[i] & class_bits(p, k, cls_s[c]) : 0u;
+    }
+    __syncthreads();
+    const bool mine = threadIdx.x < LIST_K;                        // warp-uniform
+    uint32_t acc[ROOT_CLASSES], n = 0;
 #pragma unroll
     for (uint32_t i = 0; i < ROOT_CLASSES; ++i) {
-        acc[i] = i < p.nclass ? ~acc[i] & class_bits(p, k, p.cls[i]) : 0u;
+        acc[i] = mine ? acc_s[i][word] : 0u;
         n += __popc(acc[i]);
     }
     uint32_t incl = n;
@@ -291,10 +304,10 @@ __global__ void __launch_bounds__(LIST_THREADS) k_root_list(const RootParams p,
         const uint32_t y = __shfl_up_sync(0xffffffffu, incl, d);
         if (lane >= (uint32_t)d) incl += y;
     }
-    if (lane == 31) sum_s[warp] = incl;
+    if (lane == 31 && mine) sum_s[warp] = incl;
     __syncthreads();
     if (warp == 0) {
-        const uint32_t all = __reduce_add_sync(0xffffffffu, lane < LIST_THREADS / 32 ? sum_s[lane] : 0u);
+        const uint32_t all = __reduce_add_sync(0xffffffffu, lane < LIST_K / 32 ? sum_s[lane] : 0u);
         const uint64_t before = look_back(ticket + 1, stuck, tile, all, lane);
         if (lane == 0) {
             before_s = before;
@@ -313,6 +326,7 @@ __global__ void __launch_bounds__(LIST_THREADS) k_root_list(const RootParams p,
             if (acc[i] >> b & 1) stage[slot++] = (uint16_t)((lane * 32 + b) * ROOT_CLASSES + i);
     }
     __syncthreads();
+    if (!mine) return;
     uint64_t at = before_s;
     for (uint32_t w = 0; w < warp; ++w) at += sum_s[w];
     const uint64_t k_warp = p.k0 + k - lane * 32;
@@ -351,7 +365,7 @@ extern "C" int pc_cube_roots(pc_ctx *ctx, uint64_t first, uint64_t last, uint32_
     RootParams rp{};
     std::vector<unsigned char> table;
     root_params(rp, table, first, last, p, longer ? 32 * ROOT_RUN : 1, longer ? STRIKE : UINT32_MAX);
-    const uint64_t ntiles = (rp.nk + LIST_THREADS * 32 - 1) / (LIST_THREADS * 32);
+    const uint64_t ntiles = (rp.nk + LIST_K * 32 - 1) / (LIST_K * 32);
     Scratch hold(ctx);
     uint64_t *d_scan = nullptr;                            // total, stuck flag, ticket, tile states
     const uint64_t words = 3 + (longer ? 0 : ntiles);
@@ -383,7 +397,7 @@ extern "C" int pc_cube_roots(pc_ctx *ctx, uint64_t first, uint64_t last, uint32_
             k_roots<ROOT_RUN><<<ctx->sm_count, ROOT_THREADS, smem, ctx->stream>>>(rp, (unsigned long long *)d_scan);
             PC_LAUNCHED(ctx, "cube roots count");
         } else {
-            const size_t smem = rp.table_bytes() + std::max(rp.table_words * 4, LIST_THREADS / 32 * LIST_STAGE * 2);
+            const size_t smem = rp.table_bytes() + std::max(rp.table_words * 4, LIST_K / 32 * LIST_STAGE * 2);
             PC_CHECK(ctx, cudaFuncSetAttribute(k_root_list, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             k_root_list<<<(unsigned)ntiles, LIST_THREADS, smem, ctx->stream>>>(
                 rp, (unsigned long long *)d_scan + 2, ntiles, d_scan + 1, d_scan, d_out, room);
