@@ -205,9 +205,9 @@ __device__ __forceinline__ uint32_t low_bits(uint32_t n) {
 // ------------------------------------------------------------------------------------------
 // 32x32 bit-matrix transpose across a warp: lane l holds row l (bit i = column i) on entry and
 // column l on exit.  Five exchange rounds of the off-diagonal blocks, with per-lane constants
-// computed once: in exchange round r (block size j = 16 >> r) a lane rotates its partner's word by sh[r] (left by j for the lower lane of a pair,
-// right by j for the upper one) and keeps its own bits where keep[r] is set, one funnel shift and
-// one bit-select per round.
+// computed once: in exchange round r (block size j = 16 >> r) a lane rotates its partner's word by sh[r]
+// (left by j for the lower lane of a pair, right by j for the upper one) and keeps its own bits where
+// keep[r] is set, one funnel shift and one bit-select per round.
 __device__ __forceinline__ void transpose_consts(uint32_t lane, uint32_t (&sh)[5], uint32_t (&keep)[5]) {
 #pragma unroll
     for (int r = 0; r < 5; ++r) {

@@ -1,4 +1,4 @@
-// Context, memory accounting, device buffers, device-wide scan and the limb self-test.
+// Context, memory accounting, device buffers, the page-locked stage, sorted searches and the limb self-test.
 #include "common.cuh"
 #include <algorithm>
 #include <cstring>
