@@ -5,6 +5,7 @@
 #include <string>
 #include <vector>
 #include "../../include/pcube.h"
+#include "stage.cuh"
 
 #define PC_MAX_BITSET 8        // residual filters intersected as bitsets
 #define PC_MAX_RES 1024        // residual filters per (p, A, B)
@@ -22,7 +23,7 @@ struct pc_ctx {
     uint64_t cap = 0, in_use = 0, peak = 0;
     uint64_t h2d = 0, d2h = 0;       // bytes the library has copied to and from the host
     int sm_count = 0, cc_major = 0, cc_minor = 0;
-    uint64_t *stage = nullptr;       // PC_STAGE_BYTES of page-locked memory for results, from the first use on
+    StageBuffer stage;               // PC_STAGE_BYTES of page-locked memory for results
     char name[256] = {};
     std::string err;
 };
@@ -36,9 +37,9 @@ struct pc_buf {
 int pc_fail(pc_ctx *ctx, int code, const std::string &msg);
 int pc_cuda_fail(pc_ctx *ctx, cudaError_t e, const char *what);
 constexpr uint64_t PC_STAGE_BYTES = UINT64_C(4) << 20;   // a lease's counters and envelopes: 3.8 MB
-// The context's page-locked stage, or null when `bytes` do not fit it or it cannot be had.  Its content is the
-// caller's until the next library call on the context.
-uint64_t *pc_stage(pc_ctx *ctx, uint64_t bytes);
+// The context's page-locked stage for as long as the loan lasts; none when `bytes` do not fit it, it cannot be had or
+// another call has it.  A loan ends after the stream has finished all that writes to the stage.
+StageLoan pc_stage(pc_ctx *ctx, uint64_t bytes);
 int pc_alloc(pc_ctx *ctx, void **ptr, uint64_t bytes);
 void pc_release(pc_ctx *ctx, void *ptr, uint64_t bytes);
 

@@ -390,7 +390,7 @@ extern "C" int pc_cube_roots(pc_ctx *ctx, uint64_t first, uint64_t last, uint32_
         uint32_t *d_out = nullptr;
         if (roots && (rc = list.get(&d_out, std::max<uint64_t>(1, room)))) return rc;
         PC_CHECK(ctx, cudaMemsetAsync(d_scan, 0, words * 8, ctx->stream));
-        PC_CHECK(ctx, cudaEventRecord(ctx->ev[0], ctx->stream));
+        if (kernel_ms) PC_CHECK(ctx, cudaEventRecord(ctx->ev[0], ctx->stream));
         if (longer) {
             const uint32_t smem = rp.table_bytes() + rp.table_words * 4 + (ROOT_THREADS / 32) * (32 * ROOT_RUN) * 4;
             PC_CHECK(ctx, cudaFuncSetAttribute(k_roots<ROOT_RUN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -403,16 +403,19 @@ extern "C" int pc_cube_roots(pc_ctx *ctx, uint64_t first, uint64_t last, uint32_
                 rp, (unsigned long long *)d_scan + 2, ntiles, d_scan + 1, d_scan, d_out, room);
             PC_LAUNCHED(ctx, "cube root list");
         }
-        PC_CHECK(ctx, cudaEventRecord(ctx->ev[1], ctx->stream));
+        if (kernel_ms) PC_CHECK(ctx, cudaEventRecord(ctx->ev[1], ctx->stream));
         // the sums, and a list with them, through the page-locked stage: one wait, and no copy in pieces to pageable
         // memory
-        uint64_t *stage = pc_stage(ctx, sizeof(got) + room * 4);
+        const StageLoan loan = pc_stage(ctx, sizeof(got) + room * 4);
+        uint64_t *stage = loan.get();
         PC_CHECK(ctx, pc_copy(ctx, stage ? stage : got, d_scan, sizeof(got), cudaMemcpyDeviceToHost));
         if (stage && room) PC_CHECK(ctx, pc_copy(ctx, stage + 2, d_out, room * 4, cudaMemcpyDeviceToHost));
         PC_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
         if (stage) memcpy(got, stage, sizeof(got));
-        if ((rc = elapsed(ms))) return rc;
-        if (kernel_ms) *kernel_ms = ms;
+        if (kernel_ms) {
+            if ((rc = elapsed(ms))) return rc;
+            *kernel_ms = ms;
+        }
         if (got[1]) return pc_fail(ctx, PC_ARITHMETIC, "cube root pass did not finish");
         *count = got[0];
         if (!roots) return PC_OK;

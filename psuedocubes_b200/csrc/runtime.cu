@@ -34,13 +34,16 @@ void pc_release(pc_ctx *ctx, void *ptr, uint64_t bytes) {
     ctx->in_use -= std::min(ctx->in_use, bytes);
 }
 
-uint64_t *pc_stage(pc_ctx *ctx, uint64_t bytes) {
-    if (bytes > PC_STAGE_BYTES) return nullptr;
-    if (!ctx->stage && cudaHostAlloc((void **)&ctx->stage, PC_STAGE_BYTES, cudaHostAllocDefault) != cudaSuccess) {
-        cudaGetLastError();
-        ctx->stage = nullptr;
-    }
-    return ctx->stage;
+StageLoan pc_stage(pc_ctx *ctx, uint64_t bytes) {
+    if (bytes > PC_STAGE_BYTES) return {};
+    return StageLoan(ctx->stage, [] {
+        void *words = nullptr;
+        if (cudaHostAlloc(&words, PC_STAGE_BYTES, cudaHostAllocDefault) != cudaSuccess) {
+            cudaGetLastError();
+            words = nullptr;
+        }
+        return (uint64_t *)words;
+    });
 }
 
 extern "C" int pc_version(void) { return 1; }
@@ -126,7 +129,7 @@ extern "C" int pc_free(pc_ctx *ctx) {
     for (auto &ev : ctx->marks)
         if (ev) cudaEventDestroy(ev);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
-    if (ctx->stage) cudaFreeHost(ctx->stage);
+    if (ctx->stage.words) cudaFreeHost(ctx->stage.words);
     delete ctx;
     return PC_OK;
 }
@@ -244,7 +247,9 @@ extern "C" int pc_buf_searchsorted(pc_ctx *ctx, const pc_buf *buf, const uint64_
     if (!n) return PC_OK;
     const unsigned blocks = (unsigned)((n + 31) / 32);
     SearchFew few;
-    if (uint64_t *stage = n <= SEARCH_FEW ? pc_stage(ctx, n * 8) : nullptr) {
+    const StageLoan loan = pc_stage(ctx, n * 8);
+    uint64_t *stage = loan.get();
+    if (stage && n <= SEARCH_FEW) {
         memcpy(few.q, queries, n * 8);
         k_searchsorted<<<blocks, 256, 0, ctx->stream>>>(buf->d, buf->n, nullptr, n, stage, few);
         PC_LAUNCHED(ctx, "searchsorted");
@@ -263,7 +268,6 @@ extern "C" int pc_buf_searchsorted(pc_ctx *ctx, const pc_buf *buf, const uint64_
     PC_CHECK(ctx, pc_copy(ctx, dq, queries, n * 8, cudaMemcpyHostToDevice));
     k_searchsorted<<<blocks, 256, 0, ctx->stream>>>(buf->d, buf->n, dq, n, dp, few);
     PC_LAUNCHED(ctx, "searchsorted");
-    uint64_t *stage = pc_stage(ctx, n * 8);
     PC_CHECK(ctx, pc_copy(ctx, stage ? stage : positions, dp, n * 8, cudaMemcpyDeviceToHost));
     PC_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
     if (stage) memcpy(positions, stage, n * 8);

@@ -1631,7 +1631,7 @@ uint32_t inv_mod(uint32_t a, uint32_t q) {
 
 double elapsed_ms(cudaEvent_t a, cudaEvent_t b) {
     float ms = 0;
-    cudaEventElapsedTime(&ms, a, b);
+    if (cudaEventElapsedTime(&ms, a, b) != cudaSuccess) cudaGetLastError();   // recorded anew by another thread's call
     return ms;
 }
 
@@ -2106,8 +2106,9 @@ constexpr uint64_t SMALL_REPORT = 1 << 14;                // words
 
 // The report of the run just launched: in one copy through the context's page-locked stage where it fits that
 // (a copy to pageable memory costs the host 12 us and a wait each), else straight to the caller's arrays.
-// got: the first records, which the copy brought along.
-int engine_fetch(Engine &E, uint64_t *counts, uint64_t *geometry, std::vector<uint64_t> &head, const uint64_t *&records, uint64_t &got) {
+// got: the first records, which the copy brought along; they lie in the stage, which `loan` holds.
+int engine_fetch(Engine &E, uint64_t *counts, uint64_t *geometry, std::vector<uint64_t> &head, StageLoan &loan,
+                 const uint64_t *&records, uint64_t &got) {
     pc_ctx *ctx = E.ctx;
     const uint64_t words = E.fetch_words();
     head.resize(E.o_counts);
@@ -2116,7 +2117,8 @@ int engine_fetch(Engine &E, uint64_t *counts, uint64_t *geometry, std::vector<ui
     cudaPointerAttributes at{};
     const bool direct = words > SMALL_REPORT && cudaPointerGetAttributes(&at, counts) == cudaSuccess && at.type == cudaMemoryTypeHost;
     if (words > SMALL_REPORT) cudaGetLastError();
-    if (uint64_t *stage = direct ? nullptr : pc_stage(ctx, words * 8)) {
+    if (!direct) loan = pc_stage(ctx, words * 8);
+    if (uint64_t *stage = loan.get()) {
         PC_CHECK(ctx, pc_copy(ctx, stage, E.d_report, words * 8, cudaMemcpyDeviceToHost));
         PC_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
         memcpy(head.data(), stage, E.o_counts * 8);
@@ -2153,9 +2155,10 @@ int engine_run(Engine &E, uint64_t *counts, uint64_t *geometry, uint64_t *n_out,
     for (int attempt = 0;; ++attempt) {
         int rc = engine_launch(E, true, false, launches);
         std::vector<uint64_t> head;
+        StageLoan loan;
         const uint64_t *records = nullptr;
         uint64_t got = 0;
-        if (!rc) rc = engine_fetch(E, counts, geometry, head, records, got);
+        if (!rc) rc = engine_fetch(E, counts, geometry, head, loan, records, got);
         if (rc) return rc;
         bool outgrown = false;
         rc = engine_check(E, head.data(), counts, outgrown);
@@ -2368,7 +2371,8 @@ extern "C" int pc_run_plain(pc_ctx *ctx, const pc_filters *f, const pc_buf *us, 
     PC_CHECK(ctx, cudaEventRecord(ctx->ev[7], st));
     // the counters and the first records in one copy
     const uint64_t first = std::min<uint64_t>(out_cap, Engine::FETCH_RECORDS), words = ng + 3 + 2 * first;
-    uint64_t *stage = pc_stage(ctx, words * 8);
+    const StageLoan loan = pc_stage(ctx, words * 8);
+    uint64_t *stage = loan.get();
     PC_CHECK(ctx, pc_copy(ctx, stage ? stage : counts, d_counts, (stage ? words : ng + 3) * 8, cudaMemcpyDeviceToHost));
     PC_CHECK(ctx, cudaStreamSynchronize(st));
     if (stage) memcpy(counts, stage, (ng + 3) * 8);

@@ -857,7 +857,8 @@ int winbatch_run(pc_ctx *ctx, Scratch &hold, const pc_focus *const *focus, const
     // A few words: the kernel writes them to the page-locked stage itself.  With the descriptors as parameters
     // that saves an allocation, an upload and a copy a call: a tile of 10^6 positions (two window calls) 160 -> 137 us.
     std::vector<uint64_t> pageable;
-    uint64_t *got = pc_stage(ctx, (n + 2) * 8);
+    const StageLoan stage = pc_stage(ctx, (n + 2) * 8);
+    uint64_t *got = stage.get();
     const bool direct = got && n <= WIN_FEW;
     if (direct) {
         wb.d_starts = got;
