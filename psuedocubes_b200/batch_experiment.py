@@ -12,6 +12,7 @@ import ctypes
 import time
 from collections.abc import Sequence
 from dataclasses import dataclass
+from operator import index
 from typing import Any
 
 import numpy as np
@@ -41,8 +42,10 @@ def tile_ranges(config: Config, first: int, end: int, width: int) -> list[tuple[
     if width <= 0 or (end - first + width - 1) // width > 64:
         raise ValueError('experiment allows at most 64 bounded subtiles')
     # floor((lo + vA) / B) + 1 at the subtiles' first v and floor((hi + vA) / B) + 1 at their last: quotient and
-    # remainder step by those of width A from one subtile to the next (a short last one is divided anew)
+    # remainder step by those of width A from one subtile to the next (a short last one is divided anew); in Python
+    # integers, as the products pass 2^64
     A, B = config.A, config.B
+    first, end, width = index(first), index(end), index(width)
     dq, dr = divmod(width * A, B)
     q0, r0 = divmod(config.lo + first * A, B)
     q1, r1 = divmod(config.hi + (first + width - 1) * A, B)
