@@ -14,7 +14,7 @@ from psuedocubes_b200.focus import A619, B619, Config
 def test_numpy_bounds_give_the_same_ranges(config, kind):
     first = config.B // 3
     span = min(config.B // 2, 10**10)
-    for width in (span, span // 7, max(1, span // 63)):
+    for width in (span, -(-span // 7), -(-span // 63)):   # 64 subtiles at most
         want = [(v, min(v + width, first + span)) for v in range(first, first + span, width)]
         want = [(v, e, config.u_interval(v)[0], config.u_interval(e - 1)[1]) for v, e in want]
         for bounds in ((kind(first), first + span, width), (kind(first), kind(first + span), kind(width))):
