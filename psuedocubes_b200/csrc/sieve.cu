@@ -1831,7 +1831,8 @@ FamPrep fam_prep(const pc_filters *f, const FamDev &d, uint32_t nb, uint32_t nch
     return p;
 }
 
-// Fixed-point A / B and the whole parts of the interval's ends over B.
+// Fixed-point A / B and the whole parts of the interval's ends over B.  64-bit bounds need lo <= hi: `fast` is decided by
+// hi alone, and floor(lo / B) of a larger lo need not fit 64 bits.
 SegPrep seg_prep(const SegDev &g) {
     typedef unsigned __int128 w128;
     const w128 lo = (w128)g.lo.hi << 64 | g.lo.lo, hi = (w128)g.hi.hi << 64 | g.hi.lo, last = (w128)(g.v_end ? g.v_end - 1 : 0) * g.A;
@@ -1842,7 +1843,7 @@ SegPrep seg_prep(const SegDev &g) {
     p.ilo = (uint64_t)(lo / g.B);
     p.ihi = (uint64_t)(hi / g.B);
     p.wr = g.width > 1 ? (uint64_t)(((w128)1 << 64) / g.width) : UINT64_MAX;
-    p.fast = g.B < (UINT64_C(1) << 62) && hi + last >= last && !((hi + last) / g.B >> 64);
+    p.fast = g.B < (UINT64_C(1) << 62) && lo <= hi && hi + last >= last && !((hi + last) / g.B >> 64);
     return p;
 }
 
