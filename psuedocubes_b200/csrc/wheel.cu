@@ -835,9 +835,25 @@ int focus_tables(pc_ctx *ctx, pc_focus *f, const std::vector<Ring> &rings, uint3
 
 }  // namespace
 
+namespace {
+
+// The windows' sizes by a counting pass (d_total: a word per window), into wb.total.
+int windows_count(pc_ctx *ctx, WinBatch &wb, uint64_t *d_total) {
+    if (!wb.units) return PC_OK;
+    PC_CHECK(ctx, cudaMemsetAsync(d_total, 0, wb.n * 8, ctx->stream));
+    const int rc = windows_launch<false>(ctx, wb, d_total, WinOut{});
+    if (rc) return rc;
+    PC_CHECK(ctx, pc_copy(ctx, wb.total.data(), d_total, wb.n * 8, cudaMemcpyDeviceToHost));
+    PC_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
+    return PC_OK;
+}
+
+}  // namespace
+
 // Windows one after another (unpadded) into one buffer allocated here: sized from the foci's densities
-// and filled in one pass; a pass whose values outgrow it reruns once with room for all.  A total above
-// `cap` is an overflow, and no more than `cap` entries are allocated.
+// and filled in one pass; a pass whose values outgrow it reruns once with room for all.  Where the memory cap has no
+// room for the estimate (1 % and some 1,000 entries above the need), the values are counted first and given exactly their
+// room.  A total above `cap` is an overflow (with no buffer, if it was counted), and no more than `cap` entries are allocated.
 int winbatch_run(pc_ctx *ctx, Scratch &hold, const pc_focus *const *focus, const uint64_t *low, const uint64_t *high,
                  uint32_t n, uint64_t cap, WinBatch &wb, uint64_t **out, uint64_t *out_bytes, int *launches) {
     *out = nullptr;
@@ -871,6 +887,15 @@ int winbatch_run(pc_ctx *ctx, Scratch &hold, const pc_focus *const *focus, const
     for (int attempt = 0;; ++attempt) {
         *out_bytes = std::max<uint64_t>(16, room * 8);
         rc = pc_alloc(ctx, (void **)out, *out_bytes);
+        if (rc == PC_NOMEM && wb.units && !attempt) {
+            *out = nullptr;
+            rc = windows_count(ctx, wb, wb.d_scan + 1 + win_tiles(wb));    // the words the emitting pass resets
+            if (rc) return rc;
+            wb.out_len = std::accumulate(wb.total.begin(), wb.total.end(), UINT64_C(0));
+            if (wb.out_len > cap) return PC_OK;
+            room = wb.out_len;
+            continue;
+        }
         if (rc) return rc;
         if (!wb.units) return PC_OK;
         if (direct) {
@@ -914,13 +939,8 @@ int winbatch_plan(pc_ctx *ctx, Scratch &hold, const pc_focus *const *focus, cons
     if (rc) return rc;
     wb.total.assign(n, 0);
     wb.base.assign(n, 0);
-    if (wb.units) {
-        PC_CHECK(ctx, cudaMemsetAsync(d_total, 0, n * 8, ctx->stream));
-        rc = windows_launch<false>(ctx, wb, d_total, WinOut{});
-        if (rc) return rc;
-        PC_CHECK(ctx, pc_copy(ctx, wb.total.data(), d_total, n * 8, cudaMemcpyDeviceToHost));
-        PC_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
-    }
+    rc = windows_count(ctx, wb, d_total);
+    if (rc) return rc;
     wb.delta.assign(n, 0);
     uint64_t before = 0;
     for (uint32_t i = 0; i < n; ++i) {

@@ -22,7 +22,7 @@ def test_no_position_between_lo_and_a_smaller_hi(runtime, config, nv):
     filters = Filters(runtime, config)
     first = config.B // 5
     span = min(config.B - first, 10**9)
-    vs = np.unique(np.linspace(first, first + span - 1, nv).astype(np.uint64))
+    vs = np.unique(np.array([first + (span - 1) * k // (nv - 1) for k in range(nv)], dtype=np.uint64))
     low, high = config.u_interval(first)[0], config.u_interval(first + span - 1)[1]
     us = np.unique(np.array([low + (high - low) * k // 2500 for k in range(2500)], dtype=np.uint64))
     du, dv = (DeviceArray.from_host(runtime, x) for x in (us, vs))
