@@ -381,14 +381,18 @@ extern "C" int pc_cube_roots(pc_ctx *ctx, uint64_t first, uint64_t last, uint32_
         ms += f;
         return (int)PC_OK;
     };
-    // a listing pass is sized by the density; a list that outgrows it (never seen) is written again
+    // a listing pass is sized by the density; a list that outgrows it (never seen) is written again.  Where the memory cap
+    // has no room for the estimate, the first pass only counts.
     uint64_t room = roots ? std::min(std::min(n, cap), (uint64_t)(root_density(rp, table) * n * 1.02) + 4096) : 0;
     double ms = 0;
     uint64_t got[2] = {0, 0};
     for (int attempt = 0;; ++attempt) {
         Scratch list(ctx);
         uint32_t *d_out = nullptr;
-        if (roots && (rc = list.get(&d_out, std::max<uint64_t>(1, room)))) return rc;
+        if (roots) rc = list.get(&d_out, std::max<uint64_t>(1, room));
+        const bool counting = rc == PC_NOMEM && !attempt;
+        if (counting) rc = PC_OK, room = 0;
+        if (rc) return rc;
         PC_CHECK(ctx, cudaMemsetAsync(d_scan, 0, words * 8, ctx->stream));
         if (kernel_ms) PC_CHECK(ctx, cudaEventRecord(ctx->ev[0], ctx->stream));
         if (longer) {
@@ -430,7 +434,7 @@ extern "C" int pc_cube_roots(pc_ctx *ctx, uint64_t first, uint64_t last, uint32_
             PC_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
             return PC_OK;
         }
-        if (attempt) return pc_fail(ctx, PC_ARITHMETIC, "cube root count changed between attempts");
+        if (attempt) return pc_fail(ctx, PC_ARITHMETIC, "cube root count changed between attempts");   // counted or written before
         room = got[0];
     }
 }

@@ -1,4 +1,4 @@
-"""Focus windows in a context whose memory cap has room for their values and little else."""
+"""Focus windows and root lists in a context whose memory cap has room for their values and little else."""
 from __future__ import annotations
 
 import ctypes
@@ -8,6 +8,7 @@ import time
 import numpy as np
 import pytest
 
+from psuedocubes_b200.cubes import count_roots, list_roots
 from psuedocubes_b200.focus import Config
 from psuedocubes_b200.gpu import DeviceArray, GPUFocus, Runtime
 from psuedocubes_b200.served import A_RINGS, B_RINGS
@@ -73,3 +74,25 @@ def test_refusals_without_room(tight):
         assert count.value == total and left(runtime) == SPARE
     del taken
     assert len(focus.window(low, high, cap=total)) == total
+
+
+@pytest.mark.parametrize('p, n', [(5, 2_000_000), (619, 1_000_003), (2, 5000)])
+def test_root_list_that_just_fits(tight, p, n):
+    """8 KB beside the roots: the table of primes, the tile states and their rounding to 256 bytes."""
+    runtime, _ = tight
+    first = 10**9 + 1
+    want = list_roots(runtime, first, first + n - 1, p)
+    exact = (4 * len(want) + 255) // 256 * 256
+    taken = fill(runtime, exact + 2 * SPARE)
+    assert np.array_equal(list_roots(runtime, first, first + n - 1, p), want)
+    assert count_roots(runtime, first, first + n - 1, p) == len(want)
+    with pytest.raises(OverflowError):
+        list_roots(runtime, first, first + n - 1, p, cap=len(want) - 1)
+    del taken
+    taken = fill(runtime, 2 * SPARE)
+    with pytest.raises(OverflowError):
+        list_roots(runtime, first, first + n - 1, p, cap=100)
+    if exact > 2 * SPARE:
+        with pytest.raises(MemoryError):
+            list_roots(runtime, first, first + n - 1, p)
+    del taken
