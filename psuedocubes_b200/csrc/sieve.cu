@@ -16,6 +16,7 @@
 // Rows are stored unswizzled, K/4 16-byte units per row; lane l reads unit (l + p) mod (K/4) at
 // step p, so the 32 lanes of a warp spread evenly over the bank groups whatever rows they read.
 #include "common.cuh"
+#include "shares.cuh"
 #include <algorithm>
 #include <chrono>
 #include <cstring>
@@ -97,9 +98,8 @@ struct MatchArgs {
     uint32_t total_rows;             // largest over the families
     uint64_t *counts;                // ntiles x stride
     const uint4 *bv;                 // per u block: v rows meeting it, v rows covering it
-    const uint64_t *prefix;          // work of the blocks before each block; the last entry, all
+    const uint64_t *prefix;          // work of the blocks before each block; then all work; then its division (Shares)
     uint64_t nblocks;
-    uint32_t shares, whole, pairs;   // shares: even parts of all work, or (whole) blocks, the first `pairs` of them two
     uint32_t block_cost, v_chunk;    // a block's fixed work in v rows; most rows per work item
     uint4 *deep;                     // (v lo, v hi, u index, subtile) records
     uint32_t deep_cap;               // records per CTA slice
@@ -519,15 +519,17 @@ __global__ void __launch_bounds__(256) k_blocks(const VRec *__restrict__ rec, co
     }
 }
 
-// Work of the blocks before each block: its v rows and, where it has any, the fixed cost of a block in rows.
-// One CTA: a lease has 1e4 blocks, two turns of 8,192.
+// Work of the blocks before each block: its v rows and, where it has any, the fixed cost of a block in rows.  Then all
+// work, and its division among `grid` CTAs.  One CTA: a lease has 1e4 blocks, two turns of 8,192.
 constexpr uint32_t PIECES_T = 1024, PIECES_PER = 8;
 
 __global__ void __launch_bounds__(PIECES_T) k_pieces(const uint4 *__restrict__ bv, uint64_t nblocks, uint32_t block_cost,
-                                                     uint64_t *__restrict__ prefix) {
+                                                     uint32_t grid, uint64_t *__restrict__ prefix) {
     __shared__ uint64_t warp_s[PIECES_T / 32];
+    __shared__ uint32_t most_s[PIECES_T / 32];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint64_t before = 0;                                  // work of the blocks of earlier turns
+    uint32_t most = 0;                                    // of the thread's largest block
     for (uint64_t base = 0; base < nblocks; base += PIECES_T * PIECES_PER) {
         const uint64_t b0 = base + threadIdx.x * PIECES_PER;
         uint32_t rows[PIECES_PER];
@@ -536,6 +538,7 @@ __global__ void __launch_bounds__(PIECES_T) k_pieces(const uint4 *__restrict__ b
         for (uint32_t k = 0; k < PIECES_PER; ++k) {
             const uint4 r = b0 + k < nblocks ? bv[b0 + k] : make_uint4(0, 0, 0, 0);
             own += rows[k] = r.y != r.x ? r.y - r.x + block_cost : 0;
+            most = max(most, rows[k]);
         }
         uint64_t incl = own;
 #pragma unroll
@@ -557,7 +560,17 @@ __global__ void __launch_bounds__(PIECES_T) k_pieces(const uint4 *__restrict__ b
             at += rows[k];
         }
     }
-    if (threadIdx.x == 0) prefix[nblocks] = before;
+    most = __reduce_max_sync(0xffffffffu, most);
+    if (lane == 0) most_s[warp] = most;
+    __syncthreads();
+    if (warp == 0) {
+        most = __reduce_max_sync(0xffffffffu, most_s[lane]);
+        const Shares shares = divide_work(before, most, nblocks, grid, block_cost);
+        if (lane == 0) {
+            prefix[nblocks] = before;
+            prefix[nblocks + 1] = (uint64_t)shares.pairs << 32 | shares.n;
+        }
+    }
 }
 
 // ------------------------------------------------------------------------------------------
@@ -719,8 +732,8 @@ struct MatchSmem {
         fam = cnt + round16(tmax * (ng + 2) * 4);
         seg = fam + round16(sizeof(FamDev));
         misc = seg + round16(sizeof(SegDev));
-        place = misc + 32;   // after the deep counter (4 B), the item's first subtile and its segment's subtile end
-                             // (8 B each at +16 and +24)
+        place = misc + 32;   // after the deep counter (4 B), the division of the work (8 B at +8), the item's first
+                             // subtile and its segment's subtile end (8 B each at +16 and +24)
         total = place + 48;
     }
 };
@@ -818,35 +831,36 @@ __global__ void __launch_bounds__(NT, 1) k_match(const MatchArgs a) {
     uint32_t cur_seg = UINT32_MAX, cur_fam = UINT32_MAX;
     const uint32_t nch = a.nch;
 
-    // A CTA works through shares: its first is its own number, further ones are claimed in ascending order, so the
-    // CTAs work on neighbouring blocks and the per-v records of those blocks stay in L2.  In a launch of many blocks
-    // per CTA a share is two whole blocks, at the end one.  In others all work, in block order, is cut
-    // into one even part per CTA: a block's fixed cost (building its rows, draining its survivors) and its v rows; the
-    // CTAs then finish together whatever the blocks' sizes, and a block is built by one CTA or two.  (Equal numbers of
-    // equally long items per CTA, 3,584 rows or more, left 33 SMs of a batch idle and drained 5,289 items of 24
-    // batches: batch 128 -> 85 us, 24 batches 1.59 -> 1.04 ms, 48 windows 0.93 -> 0.59 ms.)
-    // The place in the share stays in shared memory (place): no register holds it through the unit loop.
+    // A CTA works through shares (divide_work); claimed in ascending order, they keep the CTAs on neighbouring blocks, whose
+    // per-v records then stay in L2.  The division and the place in the share stay in shared memory (shares, place): no
+    // register holds them through the unit loop.
     struct Place {
         uint64_t share, b, b_end, at, at_end;             // next share; next block, end of the share's blocks, its work
         uint32_t row, first;                              // rows of block b that are done; b is the share's first
     };
     volatile Place &place = *(volatile Place *)(base + L.place);
-    if (threadIdx.x == 0) place.share = blockIdx.x, place.b = place.b_end = 0;
+    volatile Shares &shares = *(volatile Shares *)(base + L.misc + 8);
+    if (threadIdx.x == 0) {
+        place.share = blockIdx.x, place.b = place.b_end = 0;
+        const uint64_t division = a.prefix[a.nblocks + 1];
+        shares.n = (uint32_t)division, shares.pairs = (uint32_t)(division >> 32);
+    }
     __syncthreads();
     for (;;) {
         uint64_t b = place.b;
         uint32_t row = place.row;
         if (b >= place.b_end) {
             const uint64_t share = place.share;
-            if (share >= a.shares) break;
+            const uint32_t nshares = shares.n, pairs = shares.pairs;
+            if (share >= nshares) break;
             uint64_t b_end, at = 0, at_end = 0;
-            if (a.whole) {
-                b = share < a.pairs ? 2 * share : a.pairs + share;
-                b_end = b + (share < a.pairs ? 2 : 1);
+            if (pairs) {
+                b = share < pairs ? 2 * share : pairs + share;
+                b_end = b + (share < pairs ? 2 : 1);
             } else {
                 const uint64_t work = a.prefix[a.nblocks];
-                at = work * share / a.shares;
-                at_end = work * (share + 1) / a.shares;
+                at = work * share / nshares;
+                at_end = work * (share + 1) / nshares;
                 b_end = b = group_count_le64<5>(a.prefix, a.nblocks, at, lane) - 1;     // last block that starts at or before it
                 if (at != at_end) b_end = group_count_le64<5>(a.prefix, a.nblocks, at_end - 1, lane);
             }
@@ -861,11 +875,7 @@ __global__ void __launch_bounds__(NT, 1) k_match(const MatchArgs a) {
         }
         const uint4 range = a.bv[b];
         uint32_t rows_end = range.y - range.x;            // rows of the block in this share
-        if (!a.whole) {
-            const uint64_t start = a.prefix[b] + a.block_cost, at = place.at, at_end = place.at_end;
-            if (at_end < start + rows_end) rows_end = at_end > start ? (uint32_t)(at_end - start) : 0;
-            if (place.first && row == 0 && at > start) row = (uint32_t)umin64(at - start, rows_end);
-        }
+        if (!shares.pairs) cut_rows(a.prefix[b] + a.block_cost, place.first ? place.at : 0, place.at_end, row, rows_end);
         const uint64_t va = range.x + row;
         const uint32_t nv_item = min(rows_end - row, a.v_chunk);   // <= 2^20
         __syncthreads();                                  // every thread has read the place
@@ -1945,7 +1955,7 @@ int engine_prepare(Engine &E, const pc_tuning *tuning, Scratch &hold) {
     work.add(&E.d_cres, std::max<uint64_t>(1, E.nv));
     work.add(&E.d_bv, nb1);
     work.add(&E.d_blk_seg, nb1);
-    work.add(&E.d_prefix, E.nblocks + 1);
+    work.add(&E.d_prefix, E.nblocks + 2);
     rc = in.get(hold);
     if (!rc) rc = work.get(hold);
     if (!rc) rc = engine_deep_alloc(E, E.deep_cap);
@@ -1990,12 +2000,6 @@ int engine_match(Engine &E, int mode) {
     ma.bv = E.d_bv;
     ma.prefix = E.d_prefix;
     ma.nblocks = E.nblocks;
-    // Whole blocks from 16 blocks per CTA on: the CTAs then end within a block of each other, which costs less than
-    // the second building of the blocks that a cut divides.
-    const uint64_t grid = E.grid;
-    ma.whole = E.nblocks >= 16 * grid;
-    ma.pairs = ma.whole ? (uint32_t)((E.nblocks - 2 * grid) / 2) : 0;
-    ma.shares = ma.whole ? (uint32_t)E.nblocks - ma.pairs : (uint32_t)grid;
     ma.block_cost = block_cost(E);
     ma.v_chunk = (uint32_t)std::min<uint64_t>(E.tn.v_chunk ? E.tn.v_chunk : ITEM_ROWS, ITEM_ROWS);
     ma.deep = E.d_deep;
@@ -2055,7 +2059,7 @@ int engine_launch(Engine &E, bool events, bool capturing, int *launches) {
         k_blocks<<<(unsigned)((E.nblocks + 7) / 8), 256, 0, st>>>(E.d_rec, E.d_seg, (uint32_t)E.segs.size(), E.tn.K * 32,
                                                                 E.nblocks, E.d_bv, E.d_blk_seg);
         PC_LAUNCHED(ctx, "blocks");
-        k_pieces<<<1, PIECES_T, 0, st>>>(E.d_bv, E.nblocks, block_cost(E), E.d_prefix);
+        k_pieces<<<1, PIECES_T, 0, st>>>(E.d_bv, E.nblocks, block_cost(E), (uint32_t)E.grid, E.d_prefix);
         PC_LAUNCHED(ctx, "pieces");
         if (events) PC_CHECK(ctx, cudaEventRecord(ctx->ev[2], st));
         const int rc = engine_match(E, capturing ? 1 : 0);
