@@ -1298,6 +1298,8 @@ struct PlainArgs {
     uint64_t *out;
     uint64_t out_cap;
     uint64_t run;                                 // v rows per CTA
+    bool ordered;                                 // the v rows may be in order: a CTA looks for those it shares positions with
+    const uint64_t *disorder;                     // where the device found whether they are: 0 (null: they are)
     uint32_t aq[PLAIN_FIRST], bq[PLAIN_FIRST];    // A mod q, B mod q of the first filters
 };
 
@@ -1316,6 +1318,35 @@ __device__ __forceinline__ void plain_rest(const PlainArgs &a, const u128 x, uin
     }
 }
 
+// Sets *disorder when a v row is below the one before it.
+__global__ void __launch_bounds__(256) k_order(const uint64_t *__restrict__ vs, uint64_t nv, uint64_t *__restrict__ disorder) {
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x + 1; i < nv; i += (uint64_t)gridDim.x * blockDim.x)
+        if (vs[i] < vs[i - 1]) *disorder = 1;
+}
+
+// Narrows the CTA's v rows [j0, j1) to those whose interval meets its entries us[0, n), which are consecutive when the rows
+// are in order and no v A + hi or v A + lo wraps.  Without it each CTA looks at every row of its run: 4.3e5 u entries and
+// 6.8e5 v rows that meet one entry each, or 87, take 32.8 ms, with it 0.17 and 0.21; 6e4 and 6.7e4, where a row meets a third of
+// the entries, 0.92 and 0.52 ms.
+constexpr uint64_t PLAIN_ORDERED_MIN = UINT64_C(1) << 28;   // (u, v) pairs: some 0.1 ms where every CTA looks at every row,
+                                                            // against 3 us for k_order and the search; a tile has 5 10^7 at most
+__device__ __forceinline__ void plain_band(const PlainArgs &a, const uint64_t *us, uint32_t n, uint64_t &j0, uint64_t &j1) {
+    __shared__ uint64_t band_s[2];
+    if (a.disorder && *a.disorder) return;
+    if (threadIdx.x < 32) {                       // eight lanes each: rows that end below the entries, that start below the last
+        const uint32_t lane = threadIdx.x, which = lane >> 3 & 1;
+        const u128 edge = mul_wide(__ldg(us + (which ? n - 1 : 0)), a.B), bound = which ? a.lo : a.hi;
+        const uint64_t rows = group_prefix(j1 - j0, lane, [&](uint64_t i) {
+            return less128(add128(mul_wide(__ldg(a.vs + j0 + i), a.A), bound), edge);
+        });
+        if (lane == 0 || lane == 8) band_s[which] = rows;
+    }
+    __syncthreads();
+    j1 = j0 + band_s[1];
+    j0 += band_s[0];
+}
+
+template <bool ORDERED>
 __global__ void __launch_bounds__(PLAIN_T) k_plain(const PlainArgs a) {
     __shared__ unsigned long long cnt[PC_MAX_RES / 4 + 4];
     __shared__ uint32_t bits_s[PLAIN_FIRST][PLAIN_WORDS];
@@ -1325,8 +1356,12 @@ __global__ void __launch_bounds__(PLAIN_T) k_plain(const PlainArgs a) {
     const uint32_t nf = min(a.nres, PLAIN_FIRST);
     const uint64_t c0 = blockIdx.x * (uint64_t)PLAIN_U;
     const uint32_t n_here = (uint32_t)umin64(a.nu - c0, PLAIN_U);
-    const uint64_t j0 = blockIdx.y * a.run, j1 = umin64(a.nv, j0 + a.run);
+    uint64_t j0 = blockIdx.y * a.run, j1 = umin64(a.nv, j0 + a.run);
     const uint64_t *us = a.us + c0;
+    if (ORDERED) {
+        plain_band(a, us, n_here, j0, j1);
+        if (j0 >= j1) return;
+    }
     for (uint32_t k = threadIdx.x; k < a.ng + 3; k += PLAIN_T) cnt[k] = 0;
     uint32_t q[PLAIN_FIRST], ru[PLAIN_PER][PLAIN_FIRST];
     // entry (warp, k, lane) of the chunk: a warp owns 128 consecutive entries
@@ -1442,6 +1477,7 @@ constexpr uint32_t PR_PAT = (2 * PR_ROWS + PLAIN_FIRST * 96) / 32;   // pattern 
 constexpr uint64_t PLAIN_ROWS_MIN = 64;           // v rows of a launch and of a run from which the rows are worth making
 constexpr uint64_t PR_RUN_MAX = UINT64_C(1) << 25;   // v rows per CTA (a queue entry holds the row in 25 bits)
 
+template <bool ORDERED>
 __global__ void __launch_bounds__(PR_T) k_plain_rows(const PlainArgs a) {
     extern __shared__ uint4 rows_s[];             // 128 bits per row
     __shared__ unsigned long long cnt[PC_MAX_RES / 4 + 4];
@@ -1453,8 +1489,12 @@ __global__ void __launch_bounds__(PR_T) k_plain_rows(const PlainArgs a) {
     const uint32_t nf = min(a.nres, PLAIN_FIRST);
     const uint64_t c0 = blockIdx.x * (uint64_t)PR_U;
     const uint32_t n_here = (uint32_t)umin64(a.nu - c0, PR_U);
-    const uint64_t j0 = blockIdx.y * a.run, j1 = umin64(a.nv, j0 + a.run);
+    uint64_t j0 = blockIdx.y * a.run, j1 = umin64(a.nv, j0 + a.run);
     const uint64_t *us = a.us + c0;
+    if (ORDERED) {
+        plain_band(a, us, n_here, j0, j1);
+        if (j0 >= j1) return;
+    }
     for (uint32_t k = threadIdx.x; k < a.ng + 3; k += PR_T) cnt[k] = 0;
     if (threadIdx.x < n_here) prod_s[threadIdx.x] = mul_wide(__ldg(us + threadIdx.x), a.B);
     if (warp < nf && lane < sizeof(FiltConst) / 4) ((uint32_t *)(fc_s + warp))[lane] = ((const uint32_t *)(a.fc + warp))[lane];
@@ -1589,8 +1629,13 @@ void plain_launch(PlainArgs &a, const uint32_t *primes, int sm_count, cudaStream
     const uint64_t runs = std::max(std::min(least, std::max<uint64_t>(1, want / chunks)), (a.nv + most - 1) / most);
     a.run = (a.nv + runs - 1) / runs;
     const dim3 grid((unsigned)chunks, (unsigned)((a.nv + a.run - 1) / a.run));
-    if (by_rows) k_plain_rows<<<grid, PR_T, rows * 16, st>>>(a);
-    else k_plain<<<grid, PLAIN_T, 0, st>>>(a);
+    if (by_rows) (a.ordered ? k_plain_rows<true> : k_plain_rows<false>)<<<grid, PR_T, rows * 16, st>>>(a);
+    else (a.ordered ? k_plain<true> : k_plain<false>)<<<grid, PLAIN_T, 0, st>>>(a);
+}
+
+// Whether the CTAs of a launch may look for their v rows, should these be in order (u entries always are).
+bool plain_ordered(const PlainArgs &a) {
+    return (unsigned __int128)a.nu * a.nv >= PLAIN_ORDERED_MIN && a.lo.hi <= UINT64_MAX - a.A && a.hi.hi <= UINT64_MAX - a.A;
 }
 
 template <int NB, int K, int NT>
@@ -2351,6 +2396,7 @@ extern "C" int pc_run_plain(pc_ctx *ctx, const pc_filters *f, const pc_buf *us, 
     if (rc) return rc;
     uint64_t *d_out = d_counts + ng + 3;
     cudaStream_t st = ctx->stream;
+    int launches = 0;
     PC_CHECK(ctx, cudaMemsetAsync(d_counts, 0, (ng + 3) * 8, st));
     PC_CHECK(ctx, cudaEventRecord(ctx->ev[6], st));
     if (nu && nv) {
@@ -2370,8 +2416,18 @@ extern "C" int pc_run_plain(pc_ctx *ctx, const pc_filters *f, const pc_buf *us, 
         a.counts = d_counts;
         a.out = d_out;
         a.out_cap = out_cap;
+        uint64_t *d_disorder = nullptr;
+        if (plain_ordered(a) && s.get(&d_disorder, 1) == PC_OK) {   // without it, should it not fit, rows count as unordered
+            PC_CHECK(ctx, cudaMemsetAsync(d_disorder, 0, 8, st));
+            k_order<<<(unsigned)std::min<uint64_t>((nv + 1023) / 1024, (uint64_t)ctx->sm_count * 4), 256, 0, st>>>(a.vs, nv, d_disorder);
+            PC_LAUNCHED(ctx, "plain order");
+            a.ordered = true;
+            a.disorder = d_disorder;
+            ++launches;
+        }
         plain_launch(a, f->primes.data(), ctx->sm_count, st);
         PC_LAUNCHED(ctx, "plain match");
+        ++launches;
     }
     PC_CHECK(ctx, cudaEventRecord(ctx->ev[7], st));
     // the counters and the first records in one copy
@@ -2385,7 +2441,7 @@ extern "C" int pc_run_plain(pc_ctx *ctx, const pc_filters *f, const pc_buf *us, 
     if (stats) {
         stats->kernel_ms = elapsed_ms(ctx->ev[6], ctx->ev[7]);
         stats->outputs = n;
-        stats->launches = nu && nv ? 1 : 0;
+        stats->launches = launches;
     }
     const uint64_t copy = std::min(n, out_cap), got = stage ? std::min(copy, first) : 0;
     if (got) memcpy(out, stage + ng + 3, 16 * got);
@@ -2849,6 +2905,7 @@ static int plain_static_on(int device, const uint64_t *us, uint64_t nu, const ui
         a.counts = (uint64_t *)(base + o_counts);
         a.out = (uint64_t *)(base + o_out);
         a.out_cap = out_cap;
+        a.ordered = plain_ordered(a) && std::is_sorted(vs, vs + nv);
         plain_launch(a, primes, std::max(sm, 1), st);
         e = cudaGetLastError();
         if (e != cudaSuccess) return static_cuda(err, err_len, e, "plain match launch");
