@@ -54,6 +54,10 @@ int pc_device_info(const pc_ctx *ctx, int *sm_count, int *cc_major, int *cc_mino
 int pc_host_alloc(uint64_t bytes, void **out);
 int pc_host_free(void *p);
 int pc_sync(pc_ctx *ctx);
+/* Passes that write one list from many CTAs (focus windows, root lists) wait for their predecessors' counts; a wait that
+ * does not end within `polls` (2^22 when the context is made: seconds) ends the call with PC_ARITHMETIC.  A window batch
+ * (pc_multi_*) whose pass gave up once refuses all its later results. */
+int pc_wait_limit(pc_ctx *ctx, uint32_t polls);
 /* Device timestamps on the context's stream (slot 0..7) and the milliseconds between two. */
 int pc_mark(pc_ctx *ctx, int slot);
 int pc_elapsed(pc_ctx *ctx, int from_slot, int to_slot, double *ms);

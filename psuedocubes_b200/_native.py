@@ -24,7 +24,7 @@ PC_OK, PC_OVERFLOW, PC_INVALID, PC_ARITHMETIC, PC_TIMEOUT, PC_NOMEM, PC_CUDA = r
 #: Every symbol include/pcube.h declares.
 SYMBOLS = ('pc_version', 'pc_device_count', 'pc_last_error', 'pc_init', 'pc_free', 'pc_mem_info', 'pc_copy_info',
            'pc_host_alloc', 'pc_host_free',
-           'pc_device_info', 'pc_sync', 'pc_mark', 'pc_elapsed', 'pc_buf_upload', 'pc_buf_download', 'pc_buf_size', 'pc_buf_free',
+           'pc_device_info', 'pc_sync', 'pc_wait_limit', 'pc_mark', 'pc_elapsed', 'pc_buf_upload', 'pc_buf_download', 'pc_buf_size', 'pc_buf_free',
            'pc_buf_searchsorted', 'pc_focus_create', 'pc_focus_free', 'pc_focus_info', 'pc_focus_window',
            'pc_filters_create', 'pc_filters_free', 'pc_run_batch', 'pc_run_lease', 'pc_run_leases', 'pc_multi_create',
            'pc_multi_run', 'pc_multi_layout', 'pc_multi_results', 'pc_multi_free', 'pc_run_plain',
@@ -88,6 +88,7 @@ def lib() -> ctypes.CDLL:
     so.pc_device_info.argtypes = [_P, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int),
                                   ctypes.POINTER(ctypes.c_int), ctypes.c_char_p, ctypes.c_int]
     so.pc_sync.argtypes = [_P]
+    so.pc_wait_limit.argtypes = [_P, _U32]
     so.pc_mark.argtypes = [_P, ctypes.c_int]
     so.pc_elapsed.argtypes = [_P, ctypes.c_int, ctypes.c_int, ctypes.POINTER(ctypes.c_double)]
     so.pc_buf_upload.argtypes = [_P, _U64P, _U64, pp]

@@ -23,6 +23,7 @@ struct pc_ctx {
     uint64_t cap = 0, in_use = 0, peak = 0;
     uint64_t h2d = 0, d2h = 0;       // bytes the library has copied to and from the host
     int sm_count = 0, cc_major = 0, cc_minor = 0;
+    uint32_t polls = 1u << 22;       // of one wait between the tiles of a pass before it gives up
     StageBuffer stage;               // PC_STAGE_BYTES of page-locked memory for results
     char name[256] = {};
     std::string err;
@@ -300,14 +301,12 @@ __device__ __forceinline__ uint64_t group_prefix(uint64_t n, uint32_t lane, F be
 // ------------------------------------------------------------------------------------------
 // Exclusive prefix over the tiles of one launch (decoupled look-back).  A tile's state is one word:
 // value << 2 | 1 (its own sum) or 2 (its own and all before it), zeroed before the launch.
-constexpr uint32_t LOOK_BACK_SPINS = 1u << 22;   // polls of one wait before it gives up
-
 // Values of the tiles before `tile`, by warp 0: it publishes the tile's own sum, then adds the states of
 // the 32 tiles before it, and of the 32 before those, until one already holds its whole prefix.  Tiles take
-// ascending tickets, so every tile waited for is running or done; a wait that does not end in LOOK_BACK_SPINS
+// ascending tickets, so every tile waited for is running or done; a wait that does not end in `polls`
 // polls sets *stuck and goes on, and the host refuses the result.
-__device__ __forceinline__ uint64_t look_back(volatile unsigned long long *state, uint64_t *stuck, uint64_t tile,
-                                              uint64_t own, uint32_t lane) {
+__device__ __forceinline__ uint64_t look_back(volatile unsigned long long *state, uint64_t *stuck, uint32_t polls,
+                                              uint64_t tile, uint64_t own, uint32_t lane) {
     if (tile == 0) {
         if (lane == 0) state[0] = own << 2 | 2;
         return 0;
@@ -317,7 +316,7 @@ __device__ __forceinline__ uint64_t look_back(volatile unsigned long long *state
     for (int64_t at = (int64_t)tile - 1 - lane;; at -= 32) {
         unsigned long long s = at < 0 ? 2 : state[at];
         for (uint32_t spin = 0; __any_sync(0xffffffffu, (s & 3) == 0); ++spin) {
-            if (spin == LOOK_BACK_SPINS) {
+            if (spin == polls) {
                 if (lane == 0) *stuck = 1;
                 s |= 2;
             } else if ((s & 3) == 0) {

@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(ROOT_THREADS) k_roots(const RootParams p, unsi
 // list over 1e6 numbers took 33 us, now 29.5 (p = 1999: 59.5 -> 52; 2e7 numbers, where every SM has work: 41.5 -> 43.5).
 __global__ void __launch_bounds__(LIST_THREADS) k_root_list(const RootParams p,
                                                             unsigned long long *__restrict__ ticket, uint64_t ntiles,
-                                                            uint64_t *__restrict__ stuck, uint64_t *__restrict__ total,
+                                                            uint64_t *__restrict__ stuck, uint32_t polls, uint64_t *__restrict__ total,
                                                             uint32_t *__restrict__ out, uint64_t cap) {
     extern __shared__ uint4 smem[];
     __shared__ uint64_t tile_s, before_s;
@@ -308,7 +308,7 @@ __global__ void __launch_bounds__(LIST_THREADS) k_root_list(const RootParams p,
     __syncthreads();
     if (warp == 0) {
         const uint32_t all = __reduce_add_sync(0xffffffffu, lane < LIST_K / 32 ? sum_s[lane] : 0u);
-        const uint64_t before = look_back(ticket + 1, stuck, tile, all, lane);
+        const uint64_t before = look_back(ticket + 1, stuck, polls, tile, all, lane);
         if (lane == 0) {
             before_s = before;
             if (tile + 1 == ntiles) *total = before + all;
@@ -404,7 +404,7 @@ extern "C" int pc_cube_roots(pc_ctx *ctx, uint64_t first, uint64_t last, uint32_
             const size_t smem = rp.table_bytes() + std::max(rp.table_words * 4, LIST_K / 32 * LIST_STAGE * 2);
             PC_CHECK(ctx, cudaFuncSetAttribute(k_root_list, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             k_root_list<<<(unsigned)ntiles, LIST_THREADS, smem, ctx->stream>>>(
-                rp, (unsigned long long *)d_scan + 2, ntiles, d_scan + 1, d_scan, d_out, room);
+                rp, (unsigned long long *)d_scan + 2, ntiles, d_scan + 1, ctx->polls, d_scan, d_out, room);
             PC_LAUNCHED(ctx, "cube root list");
         }
         if (kernel_ms) PC_CHECK(ctx, cudaEventRecord(ctx->ev[1], ctx->stream));

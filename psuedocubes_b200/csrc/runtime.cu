@@ -164,6 +164,12 @@ extern "C" int pc_sync(pc_ctx *ctx) {
     return PC_OK;
 }
 
+extern "C" int pc_wait_limit(pc_ctx *ctx, uint32_t polls) {
+    if (!ctx) return PC_INVALID;
+    ctx->polls = polls;
+    return PC_OK;
+}
+
 extern "C" int pc_mark(pc_ctx *ctx, int slot) {
     if (slot < 0 || slot >= 8) return pc_fail(ctx, PC_INVALID, "timer slot out of range");
     PC_CHECK(ctx, cudaEventRecord(ctx->marks[slot], ctx->stream));

@@ -2132,17 +2132,18 @@ int engine_launch(Engine &E, bool events, bool capturing, int *launches) {
     return PC_OK;
 }
 
-// A finished run's report, already on the host (head: its scalars and deep counts): whether the deep slices held
-// every survivor, whether a window pass gave up, rows outside the subtile geometry, outputs that did not fit
+// A finished run's report, already on the host (head: its scalars and deep counts): whether a window pass gave up (its
+// lists then mean nothing), whether the deep slices held every survivor, rows outside the subtile geometry, outputs that did not fit
 // and underflows.
 int engine_check(Engine &E, const uint64_t *head, const uint64_t *counts, bool &outgrown) {
     const uint32_t *deep = (const uint32_t *)(head + E.o_deep);
     E.deep_max = 0;
     if (E.nu && E.nv)
         for (int b = 0; b < E.grid; ++b) E.deep_max = std::max(E.deep_max, deep[b]);
+    outgrown = false;
+    if (head[Engine::STUCK]) return pc_fail(E.ctx, PC_ARITHMETIC, "window pass did not finish");
     outgrown = E.deep_max > E.deep_cap;
     if (outgrown) return PC_OK;
-    if (head[Engine::STUCK]) return pc_fail(E.ctx, PC_ARITHMETIC, "window pass did not finish");
     if (head[Engine::BAD]) return pc_fail(E.ctx, PC_INVALID, "v row outside the subtile geometry");
     if (head[Engine::NOUT] > E.out_cap) return pc_fail(E.ctx, PC_OVERFLOW, "output overflow; attempt cannot commit");
     for (uint64_t t = 0; t < E.ntiles; ++t) {

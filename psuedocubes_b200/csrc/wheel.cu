@@ -165,6 +165,7 @@ struct WinOut {
     uint64_t cap;                      // entries of out
     uint64_t *stuck;                   // set when a look-back wait ran out
     uint64_t ntiles;
+    uint32_t polls;                    // most of one such wait
 };
 
 // Walks a warp's consecutive units.  The first is found by a binary search over the windows' first units
@@ -359,7 +360,7 @@ __global__ void __launch_bounds__(WT, 4) k_windows(const WinDesc *__restrict__ m
     __syncthreads();
     if (warp == 0) {
         const uint32_t all = __reduce_add_sync(0xffffffffu, lane < WIN_WARPS ? sum_s[lane] : 0u);
-        const uint64_t before = look_back(o.state, o.stuck, tile, all, lane);
+        const uint64_t before = look_back(o.state, o.stuck, o.polls, tile, all, lane);
         if (lane == 0) {
             before_s = before;
             if (tile + 1 == o.ntiles) o.starts[ndesc] = before + all;
@@ -677,6 +678,7 @@ int winbatch_emit(pc_ctx *ctx, const WinBatch &wb, uint64_t *out, uint64_t out_c
     o.out = out;
     o.cap = out_cap;
     o.ntiles = tiles;
+    o.polls = ctx->polls;
     return windows_launch<true>(ctx, wb, nullptr, o);
 }
 
