@@ -41,7 +41,7 @@ def verify(n: int, p: int) -> dict[str, Any]:
 # the interpreter lock inside its array operations).
 
 VECTOR_MIN = 2048          # fewer values: verify() one by one
-SMALL_VECTOR_MIN = 4       # fewer values: the scalar predicate one by one
+SMALL_VECTOR_MIN = 512     # fewer values times primes <= p: the scalar predicate one by one (even at 456 for p = 619, 500 for 199)
 MATERIALISE_MAX = 1 << 20  # more non-cubes than this: the rows are built when read
 
 
