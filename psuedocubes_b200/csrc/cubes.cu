@@ -162,9 +162,9 @@ __device__ __forceinline__ uint32_t class_bits(const RootParams &p, uint64_t k, 
 // fall in 32 different banks.  A prime above STRIKE hits a word in eight at most and would have a pattern to
 // itself: it is struck out instead, multiple by multiple in the warp's bitmap in shared memory, a lane per prime
 // (about one shared OR of a warp per prime where the pattern takes RUN + 1 loads and 1.5 RUN operations).
-// Bound: the patterns' marking (some 15 us whatever the range) and those loads and ORs, one per clock and SM.  4e8 numbers
-// with p = 619: 201 us with all 30 residues and patterns that wrapped per lane, 61 us with a pattern for every prime, 39 us
-// now (primes above 128 struck out: 41); all below 2^32 with p = 1999, whose patterns left room for 3 words: 2,052 -> 359.
+// Bound: marking the patterns and the first task (19 us for a range of one task per SM), then those loads and ORs, one per
+// clock and SM.  4e8 numbers with p = 619: 39 us (all 30 residues and patterns that wrap per lane 201, a pattern for every prime 61,
+// primes above 128 struck out 41); all below 2^32 with p = 1999, whose patterns would leave room for 3 words: 2,052 -> 359.
 constexpr uint32_t STRIKE = 256;   // the square root of ROOT_GROUP_MAX: no two larger primes share a pattern
 template <int RUN>
 __global__ void __launch_bounds__(ROOT_THREADS) k_roots(const RootParams p, unsigned long long *__restrict__ total) {
@@ -246,8 +246,8 @@ __global__ void __launch_bounds__(ROOT_THREADS) k_roots(const RootParams p, unsi
 // its classes, so number order is lane order, then k, then class.  The tile's place in
 // the list comes from a look-back over the tiles before it (out may be null: count only).  A warp's roots
 // are staged in the patterns' space, which nothing reads any more, and stored coalesced.  Bound: latency, of marking the
-// patterns and of a thread's way through all groups.  With a thread per word, 128 of them, sieving all eight classes a
-// list over 1e6 numbers took 33 us, now 29.5 (p = 1999: 59.5 -> 52; 2e7 numbers, where every SM has work: 41.5 -> 43.5).
+// patterns and of a thread's way through all groups.  Against a thread per word, 128 of them, sieving all eight classes: a
+// list over 1e6 numbers 33 -> 29.5 us (p = 1999: 59.5 -> 52; 2e7 numbers, where every SM has work: 41.5 -> 43.5).
 __global__ void __launch_bounds__(LIST_THREADS) k_root_list(const RootParams p,
                                                             unsigned long long *__restrict__ ticket, uint64_t ntiles,
                                                             uint64_t *__restrict__ stuck, uint32_t polls, uint64_t *__restrict__ total,

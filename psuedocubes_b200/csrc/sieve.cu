@@ -284,10 +284,10 @@ __device__ __forceinline__ uint32_t stage_count_le(const uint32_t *a, uint32_t t
 // spans segments each warp does the same for its own 32 rows in the list, and a row on its own where even these
 // span segments or the moduli are too large for 64-bit bounds.
 //
-// Bound: the latency of its dependent loads and instruction issue (0.5 per cycle); 48 registers, for 40 warps per SM,
-// took a lease's launch from 0.46 to 0.41 ms (40 registers spill: 0.41, and slower for fewer rows).  Sixteen rows per
-// thread whose bounds advanced through the list in global memory waited on L2: 0.85 ms for a lease's 1.6e7 rows and 50
-// us for a batch's 6e4, which gave work to 30 SMs (now 7 us).
+// Bound: the latency of its dependent loads and instruction issue (0.5 per cycle).  A lease's 1.6e7 rows: 0.41 ms at 48
+// registers, for 40 warps per SM (at more 0.46; 40 registers spill and are slower for fewer rows).  Against sixteen rows per
+// thread whose bounds advance through the list in global memory, waiting on L2: a lease 0.85 -> 0.41 ms, a batch's
+// 6e4 rows 50 -> 7 us.
 template <int ROWS>
 __global__ void __launch_bounds__(PREP_T, 5) k_vprep(const PrepArgs a) {
     constexpr uint32_t PREP_STAGE = ROWS > 4 ? 2048 : 1024;      // u entries staged per bound
@@ -459,8 +459,8 @@ __global__ void __launch_bounds__(PREP_T, 5) k_vprep(const PrepArgs a) {
 
 // Per subtile: u count and v count of its envelope (searchsorted bounds of
 // batch_experiment.py:37-43, as list-independent differences).  A warp per subtile, eight lanes per bound.  Bound:
-// the latency of the searches' dependent loads (a thread per subtile with four searches in turn: 13 us for a
-// batch, now 5 us; 37 us for a lease's 16,384 subtiles either way).
+// the latency of the searches' dependent loads (against a thread per subtile with four searches in turn: a batch
+// 13 -> 5 us, a lease's 16,384 subtiles 37 us either way).
 __global__ void __launch_bounds__(256) k_geometry(const uint64_t *__restrict__ us, const uint64_t *__restrict__ vs,
                                                   const SegDev *__restrict__ seg, const uint32_t *__restrict__ tile_seg,
                                                   uint64_t ntiles, uint64_t *__restrict__ geometry) {
@@ -488,7 +488,7 @@ __global__ void __launch_bounds__(256) k_geometry(const uint64_t *__restrict__ u
 // Per u block of UB entries: [va, vb) of v rows whose [left, right) meets the block, and the
 // sub-range [f0, f1) of rows covering the whole block (left <= start and right >= stop); left and
 // right are monotone in the row index within a segment, so all four are searches: a warp per block, eight lanes
-// each (a thread per block with four searches in turn: 24 us for a batch, 57 us for a lease; now 5 and 18 us).
+// each (against a thread per block with four searches in turn: a batch 24 -> 5 us, a lease 57 -> 18).
 __global__ void __launch_bounds__(256) k_blocks(const VRec *__restrict__ rec, const SegDev *__restrict__ seg, uint32_t nseg,
                                                 uint32_t UB, uint64_t nblocks, uint4 *__restrict__ bv,
                                                 uint32_t *__restrict__ blk_seg) {
@@ -624,7 +624,7 @@ __device__ __forceinline__ void block_residues(const uint64_t *__restrict__ us, 
 // pattern from offset 32 g + q - t on, one funnel shift, and a warp transpose turns 32 columns into 32 rows' words.
 // Before they are stored the lanes rotate their units, so that at each store eight neighbouring lanes, whose rows
 // lie a multiple of the banks apart, write four different units.  (Two units per warp and filter, stored from two
-// lane halves, met four bank conflicts a store and ten shuffles per word pair: 15.5 us of a block's 18; now 11 of 16.5.
+// lane halves, meet four bank conflicts a store and ten shuffles per word pair: 15.5 -> 11 us of a block's 16.5.
 // Eight units at a time have no conflicts, but their 32 words spill: 13.4.)
 template <int NB, int K>
 __device__ __forceinline__ void build_rows(const FamDev &F, uint4 *__restrict__ rows, const uint16_t *__restrict__ t_s,
@@ -1183,8 +1183,8 @@ __device__ __forceinline__ uint32_t mod_limbs(const uint32_t h[6], const FiltC &
 // Exact later filters on every deep record: x = uB - vA in two 64-bit limbs, filters first..nres-1
 // of the record's family with group counters, then the output record.  A lane tests the next DEEP_ALONE
 // filters on its own record; the few records that pass them (1 in 6,000 where each keeps a third) are then
-// tested one by one by the whole warp, a filter per lane, so none waits for eighty dependent table loads (a lane
-// per record to the end: 32 us for a batch, most of it one record's chain; now 8 us).
+// tested one by one by the whole warp, a filter per lane, so none waits for eighty dependent table loads (against a
+// lane per record to the end, where one record's chain is most of the time: a batch 32 -> 8 us).
 constexpr uint32_t DEEP_ALONE = 8;
 
 __global__ void __launch_bounds__(256) k_deep(const DeepArgs a) {
@@ -1274,10 +1274,9 @@ __global__ void __launch_bounds__(256) k_deep(const DeepArgs a) {
 // v*A mod q and its exact u interval (clipped to the CTA's entries) through shared memory, so a position
 // costs one subtraction and one bitmap lookup per filter (x mod q = (uB - vA) mod q).  The 1 in 81
 // positions that pass are queued per warp and finished 32 at a time in 128-bit arithmetic, filter by
-// filter.  The work is split over u chunks and v runs, so a tile of ten v rows fills the device: with a
-// warp per v row such a tile took 570 us, bound by the one warp that walked 17,400 u entries of a row; now
-// 11 us.  It takes 275 instructions of a warp for 128 positions, so from 64 v rows on (a tile of 7 10^6 positions)
-// k_plain_rows takes over.
+// filter.  The work is split over u chunks and v runs, so a tile of ten v rows fills the device (against a
+// warp per v row, which walks 17,400 u entries: 570 -> 11 us).  It takes 275 instructions of a warp for 128 positions, so
+// from 64 v rows on (a tile of 7 10^6 positions) k_plain_rows takes over.
 
 constexpr uint32_t PLAIN_T = 256, PLAIN_PER = 4, PLAIN_U = PLAIN_T * PLAIN_PER;   // threads, u entries per thread, per CTA
 constexpr uint32_t PLAIN_V = 64;                  // v rows staged at a time
@@ -2018,8 +2017,10 @@ int engine_prepare(Engine &E, const pc_tuning *tuning, Scratch &hold) {
     return PC_OK;
 }
 
-// What a block costs beyond its v rows, in rows: building sum(q) rows and the ends of its item took 26 us where
-// 215 v rows of seven filters take a microsecond (p = 619: sum(q) = 1567).
+// What a block counts beyond its v rows, in rows: 25 sum(q) / NB, 26 us at p = 619 (sum(q) = 1567), where 215 v rows of seven
+// filters take a microsecond.  That is more than building its rows takes (16.5 us), as a share that starts inside a block
+// builds it again and is charged nothing for it: with 16 sum(q) / NB a batch's k_match and k_deep take 101 us instead of 94, 24 batches
+// 1.10 ms instead of 1.04, 48 windows 0.458 instead of 0.388; 200 windows and 512 the same.
 uint32_t block_cost(const Engine &E) {
     uint32_t rows = 0;
     for (const FamDev &d : E.famdev) rows = std::max(rows, d.total_rows);

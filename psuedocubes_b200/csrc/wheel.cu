@@ -105,7 +105,6 @@ struct FocusDev {
     const uint32_t *rows;
     uint64_t M1, count1, words1, stride;
     uint32_t nT, pad;
-    uint32_t tq[PC_MAX_WHEEL_T];
     uint32_t t_m1mod[PC_MAX_WHEEL_T];
     uint32_t t_row0[PC_MAX_WHEEL_T];
     ModQ tmq[PC_MAX_WHEEL_T];
@@ -281,8 +280,8 @@ __device__ __forceinline__ uint32_t popc128(uint4 b) { return __popc(b.x) + __po
 // entry) writes them word by word after the look-back instead, one bit per lane.
 //
 // Bound: L2 (per lease 1.07 GB of row words, one 32-byte sector of W1 for each of 26M values, 0.2 GB of
-// stores) and the look-back's latency.  The two windows of a lease take 0.46 ms; a count pass, a scan and an
-// emit pass with one wheel word per lane took 1.15 ms, and 512 uneven windows 0.86 ms (now 0.35 ms).
+// stores) and the look-back's latency.  Against a count pass, a scan and an emit pass with one wheel word per lane: the
+// two windows of a lease 1.15 -> 0.46 ms, 512 uneven windows 0.86 -> 0.35 ms.
 template <bool EMIT, bool FEW>
 __global__ void __launch_bounds__(WT, 4) k_windows(const WinDesc *__restrict__ many, uint32_t ndesc,
                                                 const FocusDev *__restrict__ many_foci, uint64_t units, uint32_t rounds,
@@ -572,7 +571,6 @@ FocusDev focus_dev(const pc_focus *f) {
     d.stride = f->stride;
     d.nT = f->nT;
     for (uint32_t t = 0; t < f->nT; ++t) {
-        d.tq[t] = f->tq[t];
         d.t_m1mod[t] = f->t_m1mod[t];
         d.t_row0[t] = f->t_row0[t];
         d.tmq[t] = make_modq(f->tq[t]);
@@ -719,10 +717,9 @@ void set_rings(pc_focus *f, const Ring *rings, uint32_t n) {
 // enumerated on the host (period by period, so in order; a few thousand entries).  Then up to six rings
 // at a time: the sorted values of one whole period of the larger modulus are a window of the smaller wheel
 // with those rings as bitset rows, written by k_windows like any other.  That tests 32 candidates of the
-// smaller wheel per word and ring; a bit sieve over [0, M1), which this replaces, walked all M1
-// positions twice (0.33 and 0.48 ms a pass for the two foci of a (7, 6) split, whose wheels now take
-// 26 and 24 us).  The host keeps one wheel entry in 128 for planning, not the whole wheel (0.27 and 0.82 ms
-// of copies).
+// smaller wheel per word and ring, where a bit sieve walks all M1 positions of [0, M1) (the two foci of a (7, 6)
+// split: 0.33 and 0.48 ms a pass, two passes -> 26 and 24 us).  The host keeps one wheel entry in 128 for planning, not
+// the whole wheel (0.27 and 0.82 ms of copies).
 int focus_tables(pc_ctx *ctx, pc_focus *f, const std::vector<Ring> &rings, uint32_t nS) {
     Scratch hold(ctx);
     std::vector<std::vector<char>> ok(rings.size());
@@ -873,7 +870,7 @@ int winbatch_run(pc_ctx *ctx, Scratch &hold, const pc_focus *const *focus, const
     uint64_t room = (uint64_t)(expect * 1.01 + 8 * std::sqrt(expect)) + 1024;
     room = std::min(std::min(room, most), cap);
     // A few words: the kernel writes them to the page-locked stage itself.  With the descriptors as parameters
-    // that saves an allocation, an upload and a copy a call: a tile of 10^6 positions (two window calls) 160 -> 137 us.
+    // that saves an allocation, an upload and a copy a call.
     std::vector<uint64_t> pageable;
     const StageLoan stage = pc_stage(ctx, (n + 2) * 8);
     uint64_t *got = stage.get();

@@ -34,6 +34,7 @@ from typing import Any
 
 import numpy as np
 
+from .accounting import digest_decimals
 from .batched import BatchedEngine, Window
 from .cubes import genuine_cube_count
 from .focus import Config, Tile
@@ -45,10 +46,10 @@ A_RINGS = (2, 7, 13, 31, 43, 73, 79, 127, 139, 157, 181)   # the rings of A619, 
 B_RINGS = (9, 19, 37, 61, 67, 97, 103, 109, 151, 163)      # the rings of B619, ascending
 SERVED_PRIMES = (499, 523, 541, 547, 571, 577, 601, 607, 613, 619)
 X_MAX = 3 * 10**27
-#: device seconds per u entry, per v entry and per focused position.  A u entry costs its window
-#: generation plus its share of the matcher's fixed per-block work (pattern load, residue rows,
-#: barriers: about 30 us of one CTA per 1024-entry block, measured on served steps whose blocks
-#: met ~200 v rows each); a v entry its bounds and pieces; a position its share of the bitset tier.
+#: device seconds per u entry, per v entry and per focused position, by which the planner weighs splits.  A u entry
+#: counts its window generation and its share of the matcher's fixed work per 1024-entry block, at 30 us of one CTA; a v
+#: entry its bounds and pieces; a position its share of the bitset tier.  The split decides the reported
+#: populations, so these are part of the results: they stay although a block's rows now take 16.5 us.
 COST_U, COST_V, COST_POSITION = 200e-12, 100e-12, 0.08e-12
 U_WINDOW, V_WINDOW, P_WINDOW = 1 << 24, 1 << 22, 2 * 10**10
 STEP_U, STEP_V, STEP_P, STEP_WINDOWS = 1 << 27, 1 << 24, 2 * 10**11, 512
@@ -236,12 +237,6 @@ def verify_outputs(records: np.ndarray, lo: int, hi: int, p: int) -> tuple[list[
     return values, int(cubes.sum()), hits
 
 
-def _digest_values(values: list[int]) -> str:
-    """digest() of the decimal strings of ascending values, formatted in one pass."""
-    import hashlib
-    return hashlib.sha256(('[' + ','.join('"%d"' % n for n in values) + ']\n').encode()).hexdigest()
-
-
 def _finish(work: Work) -> dict[str, Any]:
     """Host verification and the result record of a completed request."""
     c, req = work.config, work.request
@@ -251,7 +246,7 @@ def _finish(work: Work) -> dict[str, Any]:
                 focus_split=[work.plan.a, work.plan.b], filter_groups=c.filter_groups(),
                 valid_focused_candidates=work.positions, group_survivors=list(work.groups),
                 local_survivors=len(values), genuine_cubes=ncubes, cpu_confirmed_hits=hits,
-                output_sha256=_digest_values(values), values=values, windows=work.windows)
+                output_sha256=digest_decimals([str(n) for n in values]), values=values, windows=work.windows)
 
 
 class ServedLoop:
