@@ -18,7 +18,7 @@ def sieve_primes(p: int) -> list[int]:
     return list(_primes(p))
 
 
-@lru_cache(maxsize=256)
+@lru_cache(maxsize=32)
 def _primes(p: int) -> tuple[int, ...]:
     if p < 2:
         return ()
@@ -39,7 +39,7 @@ def allowed(q: int) -> tuple[int, ...]:
     return tuple(range(1, q))
 
 
-@lru_cache(maxsize=None)
+@lru_cache(maxsize=1100)        # the 1,028 primes that the device takes as filters (below 8192): 4 MB
 def ring_bytes(q: int) -> bytes:
     """One byte per residue r of q: 1 when r is allowed."""
     ring = bytearray(q)

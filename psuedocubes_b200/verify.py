@@ -79,7 +79,7 @@ def icbrt_many(lo: np.ndarray, hi: np.ndarray) -> np.ndarray:
     return a
 
 
-@lru_cache(maxsize=None)
+@lru_cache(maxsize=1100)        # the 1,028 primes that the device takes as filters (below 8192): 4 MB
 def _fails(q: int) -> np.ndarray:
     """Per residue r of a prime q: r fails verify()'s test (r = 0, or r^((q-1)/3) != 1 when q = 1 mod 3)."""
     r = np.arange(q, dtype=np.int64)
