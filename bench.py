@@ -36,9 +36,9 @@ BATCHES_TOTAL = 108298517
 LEASE_BATCHES = 256
 OPS_PER_POSITION = 0.53071   # algorithmic 32-bit lane-ops per focused position (3W + 18S1 + 12T + 24Nv)
 # DRAM bytes per focused position of k_match from one ncu capture of a full lease (first seeded
-# lease; dram__bytes_read.sum + dram__bytes_write.sum of the k_match launch: 716,375,552 + 29,217,280
-# bytes over 274,244,194,629 positions; profiles/)
-DRAM_BYTES_PER_POSITION = (716_375_552 + 29_217_280) / 274244194629
+# lease; dram__bytes_read.sum + dram__bytes_write.sum of the k_match launch: 716.82 + 28.30 MB
+# over 274,244,194,629 positions; profiles/)
+DRAM_BYTES_PER_POSITION = (716.82e6 + 28.30e6) / 274244194629
 
 
 def seeded_first_batch() -> int:
@@ -528,8 +528,8 @@ CUBE_METRIC = 'cube roots checked/s (genuine-cube control, p=619, roots of (1e27
 
 def cube_ops_per_root(p: int) -> tuple[float, int]:
     """Lane operations per number of the device sieve and its prime groups, as pc_cube_roots forms them: 8 of 30
-    numbers are sieved, 32 to a word; a word takes a pattern load, a funnel shift and an OR per group of primes
-    (products <= 2^16) up to 256, and five operations per multiple of a larger prime."""
+    numbers are sieved, 32 to a word; a word takes a pattern load, a funnel shift and half a three-input OR per group of
+    primes (products <= 2^16) up to 256, and five operations per multiple of a larger prime."""
     primes = [q for q in range(7, p + 1) if all(q % d for d in range(2, int(q**0.5) + 1))]
     groups, product = 0, None
     for q in primes:
@@ -539,7 +539,7 @@ def cube_ops_per_root(p: int) -> tuple[float, int]:
             groups, product = groups + 1, q
         else:
             product *= q
-    return (3 * groups + 5 * sum(32 / q for q in primes if q > 256)) * 8 / 30 / 32, groups
+    return (2.5 * groups + 5 * sum(32 / q for q in primes if q > 256)) * 8 / 30 / 32, groups
 
 
 def reference_cube_count(first: int, last: int, p: int) -> tuple[int, float]:
