@@ -1951,12 +1951,16 @@ struct Engine {
     }
 };
 
+// Slices of `cap` records; of none when they cannot be had, so that a later run of the same engine stores nothing, finds
+// them outgrown and asks again.
 int engine_deep_alloc(Engine &E, uint32_t cap) {
     if (E.d_deep) pc_release(E.ctx, E.d_deep, E.deep_bytes);
     E.d_deep = nullptr;
-    E.deep_cap = cap;
+    E.deep_cap = 0;
     E.deep_bytes = (uint64_t)E.grid * cap * sizeof(uint4);
-    return pc_alloc(E.ctx, (void **)&E.d_deep, E.deep_bytes);
+    const int rc = pc_alloc(E.ctx, (void **)&E.d_deep, E.deep_bytes);
+    if (!rc) E.deep_cap = cap;
+    return rc;
 }
 
 int engine_prepare(Engine &E, const pc_tuning *tuning, Scratch &hold) {
@@ -2125,7 +2129,7 @@ int engine_launch(Engine &E, bool events, bool capturing, int *launches) {
         da.out = E.d_out();
         da.out_cap = E.out_cap;
         da.n_out = E.scalar(Engine::NOUT);
-        k_deep<<<dim3(std::min<uint32_t>((E.deep_cap + 255) / 256, 8), (unsigned)E.grid), 256, 0, st>>>(da);
+        k_deep<<<dim3(std::max(1u, std::min<uint32_t>((E.deep_cap + 255) / 256, 8)), (unsigned)E.grid), 256, 0, st>>>(da);
         PC_LAUNCHED(ctx, "deep");
         *launches += 4;
     }
@@ -2603,10 +2607,18 @@ int multi_eager(pc_ctx *ctx, pc_multi *m, pc_stats *stats) {
     PC_CHECK(ctx, cudaEventRecord(ctx->ev[5], ctx->stream));
     m->counts.resize(E.ntiles * E.stride);
     m->geometry.resize(2 * E.ntiles);
+    const uint32_t deep_cap = E.deep_cap;
     rc = engine_run(E, m->counts.data(), m->geometry.data(), &m->n_out, &launches, [&](uint64_t n) {
         m->out.resize(2 * n);
         return m->out.data();
     });
+    if (E.deep_cap != deep_cap && m->exec) {              // the recorded graph writes to the slices that were
+        cudaGraphExecDestroy(m->exec);
+        cudaGraphDestroy(m->graph);
+        m->exec = nullptr;
+        m->graph = nullptr;
+    }
+    if (!E.deep_cap) m->ran = false;                      // the next run sizes the slices anew before it records
     m->from = m->counts.data();
     m->geo_from = m->geometry.data();
     m->launches = launches;
