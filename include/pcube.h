@@ -200,9 +200,10 @@ int pc_multi_run(pc_ctx *ctx, pc_multi *m, uint32_t flags, pc_stats *stats);
  * info[0..7]: subtiles, counters per subtile (stride), padded u entries, v entries, deep slice
  * capacity, bitset filters, block words, threads. */
 int pc_multi_layout(const pc_multi *m, uint32_t *tile_base, uint64_t *sizes, uint64_t *info);
-/* Results of the last run: counts [subtiles x stride] (focused positions, the ng group survivors
- * of the window's family, outputs, underflows), geometry [subtiles x 2], out [min(n_out, out_cap)
- * x 2] with the global subtile in the high half of limb 1, as pc_run_batch. */
+/* Results of the last run (PC_INVALID when there is none or it failed): counts [subtiles x stride]
+ * (focused positions, the ng group survivors of the window's family, outputs, underflows), geometry
+ * [subtiles x 2], out [min(n_out, out_cap) x 2] with the global subtile in the high half of limb 1, as
+ * pc_run_batch. */
 int pc_multi_results(pc_ctx *ctx, const pc_multi *m, uint64_t *counts, uint64_t *geometry, uint64_t *out,
                      uint64_t out_cap, uint64_t *n_out);
 int pc_multi_free(pc_ctx *ctx, pc_multi *m);

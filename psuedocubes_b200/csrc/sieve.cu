@@ -2618,7 +2618,6 @@ int multi_eager(pc_ctx *ctx, pc_multi *m, pc_stats *stats) {
         m->exec = nullptr;
         m->graph = nullptr;
     }
-    if (!E.deep_cap) m->ran = false;                      // the next run sizes the slices anew before it records
     m->from = m->counts.data();
     m->geo_from = m->geometry.data();
     m->launches = launches;
@@ -2711,6 +2710,8 @@ extern "C" int pc_multi_run(pc_ctx *ctx, pc_multi *m, uint32_t flags, pc_stats *
         if (!m->exec) rc = multi_capture(ctx, m);
         if (!rc) rc = multi_replay(ctx, m, stats);
     }
+    // a failed run leaves no results, and the next one runs eagerly (and sizes its slices) before it replays a graph
+    if (rc) m->ran = false;
     if (stats) {
         stats->total_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
         stats->h2d_bytes = ctx->h2d - h2d0;

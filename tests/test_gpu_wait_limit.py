@@ -70,3 +70,23 @@ def test_a_window_batch_that_gave_up_stays_refused(runtime, graph):
     assert results(other) == results(good) == want
     other.close()
     good.close()
+
+
+@pytest.mark.parametrize('graph', [False, True])
+def test_no_results_of_a_failed_run(runtime, graph):
+    """A batch that has run and then gives up has no results: neither the old ones nor a mixture."""
+    engine = BatchedEngine(runtime)
+    batch = engine.plan([Window(619, LOW, LOW + 4 * 10**10)])
+    batch.run(graph=graph)
+    assert batch.positions() > 0
+    runtime.lib.pc_wait_limit(runtime.ctx, 0)
+    with pytest.raises(ArithmeticError, match='did not finish'):
+        batch.run()                                      # a recorded graph keeps the limit it was recorded with
+    runtime.lib.pc_wait_limit(runtime.ctx, DEFAULT)
+    with pytest.raises(ValueError, match='has not run'):
+        batch.raw()
+    with pytest.raises(ArithmeticError, match='did not finish'):
+        batch.run(graph=graph)
+    with pytest.raises(ValueError, match='has not run'):
+        batch.raw()
+    batch.close()
