@@ -21,8 +21,7 @@ from . import _native as N
 from .accounting import EMPTY_DIGEST, digest_decimals, scope_list
 from .focus import Config, Tile
 from .gpu import MASK, DeviceArray, Filters, GPUFocus, Matcher, Runtime, launch_plan
-from .predicate import is_perfect_cube, local3
-from .tables import sieve_primes
+from .predicate import is_perfect_cube, local3, primes_upto
 from .verify import MATERIALISE_MAX, SMALL_VECTOR_MIN, VECTOR_MIN, local_and_cubes, verify, verify_many
 
 
@@ -144,7 +143,7 @@ def verify_values(config: Config, values: list[int]) -> Sequence[dict[str, Any]]
         if not hits.all_valid:
             raise ArithmeticError('independent witness verification failed')
         return list(hits) if len(hits) <= MATERIALISE_MAX else hits
-    if len(values) * len(sieve_primes(config.p)) >= SMALL_VECTOR_MIN and config.hi < 1 << 96:
+    if len(values) * len(primes_upto(config.p)) >= SMALL_VECTOR_MIN and config.hi < 1 << 96:
         if any(not config.lo < n <= config.hi for n in (min(values), max(values))):
             raise ArithmeticError('GPU/CPU disagreement')
         ok, cubes = local_and_cubes(values, config.p)
