@@ -426,7 +426,7 @@ struct Ring {
     std::vector<uint32_t> res;
 };
 
-int focus_tables(pc_ctx *ctx, pc_focus *f, const std::vector<Ring> &rings, uint32_t nS);
+int focus_tables(pc_ctx *ctx, pc_focus *f, const std::vector<Ring> &rings, uint32_t nS, uint64_t base_steps);
 
 }  // namespace
 
@@ -460,6 +460,7 @@ extern "C" int pc_focus_create(pc_ctx *ctx, uint64_t M, uint32_t nrings, const u
     // Choose the T rings: the fewest largest rings whose removal makes the sieve over M1 and
     // the tables fit; among the feasible, the smallest table budget use wins ties.
     uint32_t chosen = UINT32_MAX;
+    uint64_t tables_bytes = 0;
     for (uint32_t nT = 0; nT <= std::min<uint32_t>(PC_MAX_WHEEL_T, nrings); ++nT) {
         uint64_t M1 = M, count1_lo = f->count_lo, count1_hi = f->count_hi, rowsum = 0;
         for (uint32_t k = nrings - nT; k < nrings; ++k) {
@@ -474,6 +475,7 @@ extern "C" int pc_focus_create(pc_ctx *ctx, uint64_t M, uint32_t nrings, const u
         uint64_t bytes = count1_lo * 8 + rowsum * words1 * 4;
         if (bytes <= table_budget) {
             chosen = nT;
+            tables_bytes = bytes;
             break;
         }
     }
@@ -483,12 +485,18 @@ extern "C" int pc_focus_create(pc_ctx *ctx, uint64_t M, uint32_t nrings, const u
     }
     f->nT = chosen;
     const uint32_t nS = nrings - chosen;
-    const int rc = focus_tables(ctx, f, rings, nS);
-    if (rc) {
+    int rc = focus_tables(ctx, f, rings, nS, BASE_STEPS);
+    // tables that fit the memory cap, but not with the scratch of their making: the whole wheel comes from the host
+    for (bool again = rc == PC_NOMEM; rc; again = false) {
         pc_release(ctx, f->W1, f->W1_bytes);
         pc_release(ctx, f->rows, f->rows_bytes);
-        delete f;
-        return rc;
+        f->W1 = nullptr;
+        f->rows = nullptr;
+        if (!again || ctx->in_use + tables_bytes > ctx->cap) {
+            delete f;
+            return rc;
+        }
+        rc = focus_tables(ctx, f, rings, nS, UINT64_MAX);
     }
     f->build_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_start).count();
     *out = f;
@@ -719,8 +727,8 @@ void set_rings(pc_focus *f, const Ring *rings, uint32_t n) {
 // with those rings as bitset rows, written by k_windows like any other.  That tests 32 candidates of the
 // smaller wheel per word and ring, where a bit sieve walks all M1 positions of [0, M1) (the two foci of a (7, 6)
 // split: 0.33 and 0.48 ms a pass, two passes -> 26 and 24 us).  The host keeps one wheel entry in 128 for planning, not
-// the whole wheel (0.27 and 0.82 ms of copies).
-int focus_tables(pc_ctx *ctx, pc_focus *f, const std::vector<Ring> &rings, uint32_t nS) {
+// the whole wheel (0.27 and 0.82 ms of copies).  `base_steps`: most candidates of a ring's step on the host.
+int focus_tables(pc_ctx *ctx, pc_focus *f, const std::vector<Ring> &rings, uint32_t nS, uint64_t base_steps) {
     Scratch hold(ctx);
     std::vector<std::vector<char>> ok(rings.size());
     for (size_t k = 0; k < rings.size(); ++k) {
@@ -730,7 +738,7 @@ int focus_tables(pc_ctx *ctx, pc_focus *f, const std::vector<Ring> &rings, uint3
     std::vector<uint64_t> base(1, 0), next;
     uint64_t M = 1, expect = 1;
     uint32_t k = 0;
-    for (; k < nS && base.size() * rings[k].q <= BASE_STEPS; ++k) {
+    for (; k < nS && base.size() * rings[k].q <= base_steps; ++k) {
         const uint32_t q = rings[k].q;
         next.clear();
         for (uint32_t period = 0; period < q; ++period)
@@ -810,14 +818,19 @@ int focus_tables(pc_ctx *ctx, pc_focus *f, const std::vector<Ring> &rings, uint3
     set_rings(f, rings.data() + nS, (uint32_t)rings.size() - nS);
     rc = pc_alloc(ctx, (void **)&f->rows, f->rows_bytes);
     if (!rc && f->nT) rc = wheel_rows(ctx, f, rings.data() + nS, f->nT, d_pat, off.data() + nS);
-    uint64_t *d_sample = nullptr;
-    const uint64_t samples = (f->count1 + SAMPLE - 1) / SAMPLE;
-    if (!rc) rc = hold.get(&d_sample, samples);
     if (rc) return rc;
-    k_sample<<<(unsigned)((samples + WT - 1) / WT), WT, 0, ctx->stream>>>(f->W1, samples, d_sample);
-    PC_LAUNCHED(ctx, "wheel samples");
+    const uint64_t samples = (f->count1 + SAMPLE - 1) / SAMPLE;
     f->sample.resize(samples);
-    PC_CHECK(ctx, pc_copy(ctx, f->sample.data(), d_sample, samples * 8, cudaMemcpyDeviceToHost));
+    if (levels.empty()) {
+        for (uint64_t i = 0; i < samples; ++i) f->sample[i] = base[i * SAMPLE];
+    } else {
+        uint64_t *d_sample = nullptr;
+        rc = hold.get(&d_sample, samples);
+        if (rc) return rc;
+        k_sample<<<(unsigned)((samples + WT - 1) / WT), WT, 0, ctx->stream>>>(f->W1, samples, d_sample);
+        PC_LAUNCHED(ctx, "wheel samples");
+        PC_CHECK(ctx, pc_copy(ctx, f->sample.data(), d_sample, samples * 8, cudaMemcpyDeviceToHost));
+    }
     for (const auto &l : levels)
         PC_CHECK(ctx, pc_copy(ctx, l->got, l->wb.d_scan + 1 + win_tiles(l->wb), sizeof(l->got), cudaMemcpyDeviceToHost));
     PC_CHECK(ctx, cudaStreamSynchronize(ctx->stream));

@@ -96,3 +96,34 @@ def test_root_list_that_just_fits(tight, p, n):
         with pytest.raises(MemoryError):
             list_roots(runtime, first, first + n - 1, p)
     del taken
+
+
+@pytest.mark.parametrize('A, B, budget', [(2 * 5 * 11 * 17 * 23 * 29, 9, 0), (2 * 5 * 11 * 17 * 23 * 29 * 41, 9 * 7 * 13, 0),
+                                          (599 * 593 * 2, 9 * 587, 0), (math.prod(A_RINGS[:7]), math.prod(B_RINGS[:6]), 0),
+                                          (math.prod(A_RINGS[:7]), math.prod(B_RINGS[:6]), 1 << 20)])
+def test_focus_tables_that_just_fit(A, B, budget):
+    """A context with room for a focus's tables and 16 KB, far less than the scratch of their making on the device."""
+    config = Config(619, 0, 10**9, A, B)
+    for focus in config.focuses():
+        roomy = Runtime(time.monotonic() + 300, 1 << 30)
+        gpu = GPUFocus(roomy, focus, budget)
+        span = min(3000 * focus.modulus, 50_000 * focus.modulus // focus.count)
+        low = focus.modulus // 3
+        want = gpu.window(low, low + span, cap=1 << 22).get()
+        tables, shape = gpu.table_bytes, (gpu.wheel_modulus, gpu.wheel_size, gpu.bitset_rings, gpu.count)
+        tight = Runtime(time.monotonic() + 300, tables // 256 * 256 + 4 * SPARE)
+        other = GPUFocus(tight, focus, budget)
+        assert (other.wheel_modulus, other.wheel_size, other.bitset_rings, other.count) == shape
+        low_room = left(tight)
+        assert 0 <= low_room <= 4 * SPARE
+        few = want[:50]
+        assert np.array_equal(other.window(low, int(few[-1]) + 1, cap=1 << 22).get(), few)
+        del other
+        tight.close()
+        tight = Runtime(time.monotonic() + 300, max(256, tables // 256 * 256 - 1024))
+        if tables > 4096:
+            with pytest.raises(MemoryError):
+                GPUFocus(tight, focus, budget)
+        tight.close()
+        del gpu
+        roomy.close()
